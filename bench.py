@@ -53,19 +53,12 @@ WORKLOAD = ("LDPC decoder batch: 512 codeblocks, BG1 Z=384 (K=8448, rate 1/3) an
 # Algorithmic integer operations per edge update: v2c saturating subtraction, infinity guard, abs,
 # three for the min1/min2 update, sign XOR, two for the message select and sign, promotion add.
 INT_OPS_PER_EDGE = 10
-LDPC_KERNEL_NAMES = ["ldpc_decode_kernel (one lifted lane per thread)",
-                     "ldpc_decode_x2_kernel (two lifted lanes per thread for even Z > 192)",
-                     "ldpc_decode_split_kernel (two lanes per thread pair, row edges split over the pair)",
-                     "ldpc_decode_z_kernel (two lifted lanes per thread, Z = 384 specialised, f16 soft-bit pairs)",
-                     "ldpc_decode_zs_kernel (Z = 384 specialised, row edges split over a thread pair)"]
-# ncu figures of one launch of the LDPC batch per kernel (pg_ldpc_kernel id): DRAM bytes read +
-# written, and pipe utilisation in % of active cycles. Kernel 1 at four CTAs per SM, kernel 3 at
-# two (the bench default).
-LDPC_NCU = {
-    1: {"traffic": 24246528, "pipes": {"alu": 55.5, "fma": 32.3, "lsu": 24.9, "issue_active": 59.6,
-                                       "sm_active_pct_of_elapsed": 60.4}},
-    3: {"traffic": 11546880, "pipes": {"alu": 50.3, "issue_active": 53.3, "sm_active_pct_of_elapsed": 81.0}},
-}
+LDPC_KERNEL_NAMES = (["ldpc_decode_kernel (one lifted lane per thread)"]
+                     + 4 * ["ldpc_decode_pair_kernel (two lifted lanes per lane pair, 2 or 4 threads per pair)"])
+# ncu figures of one launch of the LDPC batch with the lane-pair kernel: pipe utilisation in % of active
+# cycles.
+LDPC_NCU = {k: {"pipes": {"alu": 56.0, "fma": 46.0, "issue_active": 64.0, "sm_active_pct_of_elapsed": 89.0}}
+            for k in range(1, 5)}
 # Integer-instruction throughput probe (the LDPC roofline denominator), built by
 # ocudu-dapp-platform_b200/measure/Makefile.
 PROBE_SO = os.path.join(ROOT, "ocudu-dapp-platform_b200", "measure", "_lib", "libpg_probe.so")

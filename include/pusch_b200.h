@@ -136,19 +136,16 @@ int pg_set_kernel_timing(pg_context* ctx, int enabled);
  * or a negative value when none was recorded. */
 float pg_last_kernel_ms(pg_context* ctx);
 
-/* LDPC decoding kernels; every one gives the same bits and iteration counts. No counterpart in the
- * reference, whose decoder runs one codeblock per CPU task. */
+/* LDPC decoding kernels; both give the same bits and iteration counts. No counterpart in the
+ * reference, whose decoder runs one codeblock per CPU task. TWO_LANES, SPLIT, Z384 and Z384_SPLIT name
+ * the same kernel: two lifted lanes per lane pair as f16x2 halves, 384 threads per codeblock (two per
+ * lane pair above Z = 192, four below), up to two CTAs per SM. */
 enum pg_ldpc_kernel {
-  PG_LDPC_KERNEL_ONE_LANE  = 0, /* 384 threads per codeblock, one lifted lane per thread, two CTAs per SM */
-  PG_LDPC_KERNEL_TWO_LANES = 1, /* 192 threads per codeblock; even Z > 192: two lanes per thread as f16x2
-                                   halves; four CTAs per SM */
-  PG_LDPC_KERNEL_SPLIT     = 2, /* 384 threads per codeblock; even Z > 192: two lanes per thread pair, each
-                                   row's edges split between the two threads; two CTAs per SM */
-  PG_LDPC_KERNEL_Z384      = 3, /* 192 threads per codeblock; Z = 384 with the lifted edge tables in shared
-                                   memory and f16 soft-bit pairs stored once, other Z as TWO_LANES; up to
-                                   three CTAs per SM */
-  PG_LDPC_KERNEL_Z384_SPLIT = 4 /* 384 threads per codeblock; Z = 384 as Z384 with each row's edges split
-                                   over the two threads of a lane pair, other Z as SPLIT; two CTAs per SM */
+  PG_LDPC_KERNEL_ONE_LANE   = 0, /* 384 threads per codeblock, one lifted lane per thread, two CTAs per SM */
+  PG_LDPC_KERNEL_TWO_LANES  = 1,
+  PG_LDPC_KERNEL_SPLIT      = 2,
+  PG_LDPC_KERNEL_Z384       = 3,
+  PG_LDPC_KERNEL_Z384_SPLIT = 4
 };
 
 /* Selects the kernel of the context's batch decodes (pg_ldpc_decode_batch_{host,device,resident}
@@ -157,13 +154,13 @@ int pg_set_ldpc_kernel(pg_context* ctx, int kernel);
 /* Work order of the context's batch decodes: the codeblocks as given, or longest first (the
  * default): an estimate of each codeblock's decoding time from its input (the edges its rows cover
  * times Z, over the LLR magnitude per message bit) orders the persistent decoders' work list, so that
- * the long decodes start first. Results do not depend on the order. */
+ * the long decodes start first (when the codeblocks outnumber the CTAs). Results do not depend on the order. */
 enum pg_ldpc_order { PG_LDPC_ORDER_GIVEN = 0, PG_LDPC_ORDER_LONGEST_FIRST = 1 };
 int pg_set_ldpc_order(pg_context* ctx, int mode);
 /* The kernel of the context's batch decodes (pg_ldpc_kernel), or a negative error code. */
 int pg_get_ldpc_kernel(const pg_context* ctx);
-/* Resident CTAs per SM of the context's batch decodes (1-4, capped by the kernel's own limit; 0:
- * the kernel's limit, the default). Fewer CTAs than codeblocks make the persistent CTAs share the
+/* Resident CTAs per SM of the context's batch decodes (1-4, capped by the kernel's own limit; 0, the
+ * default: by the batch size). Fewer CTAs than codeblocks make the persistent CTAs share the
  * codeblocks dynamically; more make every codeblock start at once. */
 int pg_set_ldpc_ctas_per_sm(pg_context* ctx, int ctas_per_sm);
 
@@ -556,10 +553,10 @@ typedef struct pg_pusch_plan_tuning {
   int rm_ctas_per_cb;       /* rate dematching: CTAs per codeblock, 1..32 (default 8) */
   int demod_res_per_thread; /* demodulation: resource elements per thread, 1..8 (default 1) */
   int demod_block;          /* demodulation: threads per CTA, 64, 128 or 256 (default 256) */
-  int ldpc_ctas_per_sm;     /* persistent LDPC decoders: CTAs per SM, 1..4 (default 2; the one-lane-per-
-                               thread decoder holds at most 2) */
+  int ldpc_ctas_per_sm;     /* persistent LDPC decoders: CTAs per SM, 1..4 (default 2, which is also the most
+                               a kernel holds) */
   int ldpc_kernel;          /* LDPC decoder (pg_ldpc_kernel), PG_LDPC_KERNEL_ONE_LANE .. _Z384_SPLIT
-                               (default PG_LDPC_KERNEL_Z384) */
+                               (default PG_LDPC_KERNEL_Z384, the lane-pair decoder) */
   int ldpc_order;           /* work order of the persistent decoders: 0 = largest codeblocks first, fixed
                                when the plan is created; 1 = longest predicted decode first, from every
                                execution's LLRs (pg_set_ldpc_order's estimate; default 1) */

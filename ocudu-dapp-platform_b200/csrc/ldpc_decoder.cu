@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(kThreads, 2) ldpc_decode_kernel(const pg_ldpc_
                                                               int8_t* __restrict__ c2v_all,
                                                               const uint32_t* __restrict__ crc_pow,
                                                               const uint32_t* __restrict__ order, int n,
-                                                              int* __restrict__ counter, int skip_z)
+                                                              int* __restrict__ counter)
 {
   __shared__ smem_t sm;
   __shared__ int    s_work;
@@ -520,9 +520,6 @@ __global__ void __launch_bounds__(kThreads, 2) ldpc_decode_kernel(const pg_ldpc_
     }
     const int        cb = order != nullptr ? (int)order[w] : w;
     const pg_ldpc_cb d  = descs[cb];
-    if (d.lifting_size == skip_z) {
-      continue; // left to ldpc_decode_x2_kernel
-    }
     if (d.lifting_size == 384) {
       decode_codeblock<384, kThreads, pg::kMaxZ>(d, sm, llrs, bits, iterations, c2v_all, crc_pow, cb, blockIdx.x);
     } else {
@@ -532,65 +529,56 @@ __global__ void __launch_bounds__(kThreads, 2) ldpc_decode_kernel(const pg_ldpc_
 }
 
 // ---------------------------------------------------------------------------------------------
-// Two-lanes-per-thread decoder: one 192-thread CTA per codeblock, every lifting size.
+// Lane-pair decoder: even lifting sizes, H = Z / 2. A lane pair j (0 <= j < H) is check lanes j and
+// j + H, carried as the two halves of one f16x2 register by T adjacent threads, which split the
+// edges of every row.
 //
-// Pair mode (even Z > 192, H = Z / 2): thread j (0 <= j < H) carries check lanes j and j + H as
-// the two halves of one f16x2 register. For an edge of shift s the two variable lanes it reads,
-// (j + s) mod Z and (j + H + s) mod Z, differ by H, so soft bits live twice in shared memory and
-// the shifted pair is one 16-bit word: D[col][w] = (soft[col][w], soft[col][(w + H) mod Z]).
-// The reference's int8 rules become exact f16x2 identities:
-//   v2c      = x == +-127 ? x : clamp(x - c, -120, 120)       (reference)
-//   v        = min(max(clamp(x - c, -120, 120), 104x - 12984), 104x + 12984)  (fused
-//              multiply-adds; for |x| <= 120 the bounds lie outside [-120, 120], for x = +-127
-//              they are +-224; in the first iteration c = 0 and x is not clamped, and the bounds
-//              keep every |x| <= 126 as it is)
-//              so v = v2c, except that a saturated soft bit gives +-224 instead of +-127. Both
-//              exceed every magnitude the minimum search starts from (120) and keep the sign, so
-//              the row's minima, sign and messages are the same; and +-224 plus any message
-//              (|c2v| <= 96) stays above 120 in magnitude, so the soft update below gives +-127
-//              back without the reference's separate test of |v2c| == 127.
-//   min1/min2/sign: min.xorsign.abs keeps min(|.|) and accumulates the sign product in min1's sign
-//   c2v      = sign(product of the others) * (|v2c| == min1 ? s2 : s1),
-//              magnitude = s2 + (s1 - s2) * (|v| != min1), the comparison as f16 1.0 / 0.0, sign by
-//              XOR of sign bits
-//   soft     = |v2c| == 127 ? v2c : promote(c2v + v2c) = promote(c2v + v),
-//              promote(t) = clamp(8t - 7 clamp(t, +-120), +-127)
-//   scale    s = (m * 52428) >> 16 from a table indexed by the f16 bit pattern of m over 16.
-// Every value used is an integer of magnitude at most 2,560 (even above 2,048), so f16 arithmetic
-// (11-bit significand) on it is exact; the bounds are exact where they decide (x = +-127).
-// Storage is int8 in offset binary (byte = value + 128): f16 bits 0x6400 | byte are 1024 + byte, so
-// one byte permute and one f16x2 subtraction of 1152 give the values, and an addition of 1152 and a
-// byte permute give the bytes back, exactly. Check-to-variable messages are byte pairs per (edge,
-// thread) in the global slab.
+// Soft bits: E[col][k] = (soft[col][k], soft[col][k + H]) as one f16x2 word, 0 <= k < H, in shared
+// memory. For an edge of shift s, lane j reads variable lane (j + s) mod Z and lane j + H reads
+// (j + H + s) mod Z: both are halves of the same word k = (j + s') mod H with s' = s mod H, swapped
+// when (j + s' >= H) differs from (s >= H). The edge table in shared memory holds what pair_edge needs. Rows are padded to a multiple of T edges with an edge to a constant column of
+// saturated positive soft bits, which changes no minimum, sign or message of the row.
 //
-// Scalar mode (Z <= 192): the one-lane arithmetic of ldpc_decode_kernel with 192 threads.
-constexpr int kX2Threads  = 192; // = kMaxZ / 2
-constexpr int kScaleTab   = 1408;
-constexpr int kX2MaxPerSm = 4;   // resident CTAs per SM (registers)
-
-template <int NT>
-struct __align__(16) smem_pair_nt_t {
-  uint16_t D[pg::kMaxNodes * pg::kMaxZ]; // soft-bit pairs, column stride Z
-  uint32_t edge[pg::kBg1Edges];          // col*Z << 16 | s
-  uint32_t hard[(22 * pg::kMaxZ) / 32];
-  uint32_t red[NT / 32];
-  int      s_last;
-  int      s_done;
-};
-using smem_pair_t      = smem_pair_nt_t<kX2Threads>;
-using smem_x2_scalar_t = smem_scalar_t<kX2Threads, kX2Threads>;
-constexpr size_t kX2Smem = sizeof(smem_pair_t) > sizeof(smem_x2_scalar_t) ? sizeof(smem_pair_t)
-                                                                           : sizeof(smem_x2_scalar_t);
-
-// Split decoder: 384 threads per codeblock. Pair mode (even Z > 192) runs two threads per lane
-// pair, each taking every second edge of a row; other lifting sizes run the one-lane arithmetic
-// with one thread per lane.
-constexpr int kSplitThreads  = 384;
-constexpr int kSplitMaxPerSm = 2;
-using smem_split_pair_t      = smem_pair_nt_t<kSplitThreads>;
-using smem_split_scalar_t    = smem_scalar_t<kSplitThreads, pg::kMaxZ>;
-constexpr size_t kSplitSmem  = sizeof(smem_split_pair_t) > sizeof(smem_split_scalar_t) ? sizeof(smem_split_pair_t)
-                                                                                        : sizeof(smem_split_scalar_t);
+// Arithmetic: the reference's int8 rules as exact f16x2 identities (every value that decides is an
+// integer of magnitude at most 2,048):
+//   soft x       finite when |x| <= 120; any larger magnitude is the reference's +-127. The promotion
+//                of a sum above 120 is not done when the sum is stored but when it is read: the
+//                stored sum (at most 120 + 96) is compared with 120 there.
+//   v2c          v = min(max(clamp(x - c, +-120), 400x - 48128), 400x + 48128), fused multiply-adds: for
+//                |x| <= 120 the bounds lie outside [-120, 120]; from |x| = 121 they are at least 272 in
+//                magnitude with x's sign (or infinite). So a saturated v never is the row's minimum
+//                (the search starts at 120), keeps its sign, and v + c is again above 120 (|c| <= 96):
+//                a saturated soft bit stays saturated. Messages are finite, so no infinity meets its
+//                negative.
+//   min1/min2/sign: min.xorsign.abs keeps min(|.|) and accumulates the sign product in min1's sign.
+//   scale        floor(m * 52428 / 2^16) for integer 0 <= m <= 120 is max(fma(m, f16(0.8), 1023.5) -
+//                1024, 0): the fused multiply-add rounds once, to an integer (the spacing of f16 in
+//                [1024, 2048)), and f16(0.8) = 0.7998046875 errs by at most 0.024 at m = 120, inside
+//                the 0.1 margin of every rounding decision (checked for every m).
+//   c2v          (|v| == min1 ? s2 : s1) with the sign product of the others by XOR of sign bits.
+//   soft         c + v.
+// Whole input nodes are clamped to +-64. In a ragged tail (fewer LLRs than the node) the values 121 to
+// 126 are finite in the first iteration, which this reading rule cannot tell from a sum: a codeblock
+// that holds one runs its first iteration through pair_row_ragged, which promotes when it stores.
+//
+// Check-to-variable messages are offset-binary byte pairs (value + 128: f16 bits 0x6400 | byte are
+// 1024 + byte), two edges to a 32-bit word, one word column per thread; each thread reads only what
+// it wrote. They stay in shared memory when the rows that the codeblock runs fit there (behind the
+// columns that those rows use), else in the CTA's global slab.
+constexpr uint32_t kH120     = 0x57805780u; // 120
+constexpr uint32_t kHm120    = 0xd780d780u; // -120
+constexpr uint32_t kH126p5   = 0x57e857e8u; // 126.5
+constexpr uint32_t kH400     = 0x5e405e40u; // 400
+constexpr uint32_t kH48128   = 0x79e079e0u; // 48128
+constexpr uint32_t kHm48128  = 0xf9e0f9e0u; // -48128
+constexpr uint32_t kH1152    = 0x64806480u; // 1152 = 1024 + 128
+constexpr uint32_t kAbs      = 0x7fff7fffu;
+constexpr uint32_t kSign     = 0x80008000u;
+constexpr uint32_t kSat      = 0x60006000u; // the top two exponent bits
+constexpr uint32_t kHDummy   = 0x70007000u; // 8192, the constant column
+constexpr uint32_t kH0p8     = 0x3a663a66u; // f16(0.8) = 0.7998046875
+constexpr uint32_t kH1023p5  = 0x63ff63ffu; // 1023.5
+constexpr uint32_t kHm1024   = 0xe400e400u; // -1024
 
 __device__ __forceinline__ uint32_t h2_sub(uint32_t a, uint32_t b)
 {
@@ -608,12 +596,6 @@ __device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c)
 {
   uint32_t r;
   asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
-  return r;
-}
-__device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b)
-{
-  uint32_t r;
-  asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
   return r;
 }
 __device__ __forceinline__ uint32_t h2_min(uint32_t a, uint32_t b)
@@ -640,246 +622,274 @@ __device__ __forceinline__ uint32_t h2_max_xs(uint32_t a, uint32_t b)
   asm("max.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
   return r;
 }
-
-// f16x2 constants (both halves equal).
-constexpr uint32_t kH120    = 0x57805780u; // 120
-constexpr uint32_t kHm120   = 0xd780d780u; // -120
-constexpr uint32_t kH127    = 0x57f057f0u; // 127
-constexpr uint32_t kHm127   = 0xd7f0d7f0u; // -127
-constexpr uint32_t kH104    = 0x56805680u; // 104
-constexpr uint32_t kHm12984 = 0xf257f257u; // -12984
-constexpr uint32_t kH12984  = 0x72577257u; // 12984
-constexpr uint32_t kH8      = 0x48004800u; // 8
-constexpr uint32_t kHm7     = 0xc700c700u; // -7
-constexpr uint32_t kH1152   = 0x64806480u; // 1152 = 1024 + 128
-constexpr uint32_t kAbs     = 0x7fff7fffu;
-constexpr uint32_t kSign    = 0x80008000u;
+// All ones in the halves where |a| > b, or |a| == b.
+__device__ __forceinline__ uint32_t h2_abs_gt_mask(uint32_t a, uint32_t b)
+{
+  const __half2 x = __habs2(*reinterpret_cast<const __half2*>(&a));
+  return __hgt2_mask(x, *reinterpret_cast<const __half2*>(&b));
+}
+__device__ __forceinline__ uint32_t h2_abs_eq_mask(uint32_t a, uint32_t b)
+{
+  const __half2 x = __habs2(*reinterpret_cast<const __half2*>(&a));
+  return __heq2_mask(x, *reinterpret_cast<const __half2*>(&b));
+}
+// 1.0 in the halves where |a| != b, else 0.0.
+__device__ __forceinline__ uint32_t h2_abs_ne(uint32_t a, uint32_t b)
+{
+  const __half2 r = __hne2(__habs2(*reinterpret_cast<const __half2*>(&a)), *reinterpret_cast<const __half2*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
 
 // Offset-binary byte pair -> f16x2 integers (low byte first).
 __device__ __forceinline__ uint32_t bytes_to_h2(uint32_t b)
 {
   return h2_sub(__byte_perm(b, 0x6464u, 0x5140u), kH1152);
 }
-__device__ __forceinline__ uint32_t h2_to_bytes_biased(uint32_t c)
+
+__device__ __forceinline__ uint32_t pair_scale(uint32_t m)
 {
-  return h2_add(c, kH1152); // bytes 0 and 2 are the offset-binary values
+  return h2_max(h2_add(h2_fma(m, kH0p8, kH1023p5), kHm1024), 0u);
 }
 
-__device__ __forceinline__ uint32_t x2_scale(const uint16_t* __restrict__ tab, uint32_t m)
+// Shared-memory accesses by 32-bit shared address (the soft-bit addresses of the edge table are
+// absolute, so that no base is added per edge).
+__device__ __forceinline__ uint32_t lds_u32(uint32_t adr)
 {
-  return (uint32_t)__ldg(tab + ((m & 0xffffu) >> 4)) | ((uint32_t)__ldg(tab + (m >> 20)) << 16);
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(adr));
+  return v;
+}
+__device__ __forceinline__ uint4 lds_v4(uint32_t adr)
+{
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(adr));
+  return v;
+}
+__device__ __forceinline__ void sts_u32(uint32_t adr, uint32_t v)
+{
+  asm volatile("st.shared.u32 [%0], %1;" ::"r"(adr), "r"(v));
 }
 
-__device__ __forceinline__ uint32_t h2_ne(uint32_t a, uint32_t b)
+// Tables of the base graphs, indexed by [graph], and of their rows padded to a multiple of T = 2 << lg
+// edges ([lg][graph]): first padded edge and first message word (in units of the active
+// threads) of each row. In global memory: threads read different entries.
+struct pair_tables {
+  uint16_t edge_v[2][pg::kBg1Edges][8];
+  uint8_t  edge_col[2][pg::kBg1Edges];
+  uint8_t  edge_row[2][pg::kBg1Edges];
+  uint8_t  row_deg[2][pg::kBg1Rows];
+  uint8_t  row_sync[2][pg::kBg1Rows]; // the row is the last of its step
+  uint16_t row_e0[2][pg::kBg1Rows + 1];
+  uint16_t pad_e0[2][2][pg::kBg1Rows + 1];
+  uint16_t msg0[2][2][pg::kBg1Rows + 1];
+};
+__device__ pair_tables g_pair_tables;
+
+constexpr int      kPairMaxEdges = 460;  // padded edges of a graph, T <= 4 (316 + 3 * 46 at most)
+constexpr uint32_t kPairTabBytes = kPairMaxEdges * 16;
+constexpr uint32_t kPairMinSmem  = kPairTabBytes + (pg::kMaxNodes + 1) * (pg::kMaxZ / 2) * 4; // every column
+constexpr int      kOddMaxZ      = 16;   // odd lifting sizes are at most 15
+
+struct pair_shared {
+  uint4    row[pg::kBg1Rows + 1]; // first padded edge, first message word, edges per thread, step end
+  int      last;
+  int      ragged;
+  uint32_t crc[2];
+  int      zero[2];
+  int      work;
+};
+
+// Byte offset in E and byte-permute selector of edge table entry c for lane pair j. The decoder is
+// bound by the ALU pipe (comparisons, selects, logic, byte permutes: 64 lanes a cycle on an SM), so
+// both are formed on the FP32 pipe: w = 1 when the edge wraps (the saturated sum of j and 1 - (H - s')
+// is 0 or 1), and the integers travel as the bits of denormal numbers, on which an FP32 multiply-add by
+// w is exact: adr = (4 j + base) - w 4 H, sel = sel0 + w dsel.
+__device__ __forceinline__ void pair_edge(const uint4 c, const float jf, const float j4d, const float nh4d,
+                                          uint32_t& adr, uint32_t& sel)
 {
-  uint32_t r;
-  asm("set.ne.f16x2.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-  return r;
+  const float w = __saturatef(__fadd_rn(jf, __uint_as_float(c.y)));
+  adr           = __float_as_uint(__fmaf_rn(w, nh4d, __fadd_rn(j4d, __uint_as_float(c.x))));
+  sel           = __float_as_uint(__fmaf_rn(w, __uint_as_float(c.w), __uint_as_float(c.z)));
 }
 
-// v2c of one edge (saturated soft bits as +-224) from its soft-bit pair x and its stored
-// check-to-variable pair.
-template <bool FIRST>
-__device__ __forceinline__ uint32_t pair_v2c(const uint32_t x, const uint16_t* __restrict__ c2v)
+// The partial (min1, min2, sign) of the T threads of a lane pair meet through shuffles.
+template <int T>
+__device__ __forceinline__ void pair_reduce(uint32_t& min1, uint32_t& min2)
 {
-  uint32_t d = x;
+#pragma unroll
+  for (int o = 1; o < T; o <<= 1) {
+    const uint32_t o1 = __shfl_xor_sync(0xffffffffu, min1, o);
+    const uint32_t o2 = __shfl_xor_sync(0xffffffffu, min2, o);
+    min2              = h2_min_xs(h2_min_xs(min2, o2), h2_max_xs(min1, o1));
+    min1              = h2_min_xs(min1, o1);
+  }
+}
+
+// One row for this thread's NE edges (table entries zt[0 .. NE - 1], message words msg[0], msg[nta],
+// ...). FIRST: the first iteration, whose messages are still zero.
+template <int NE, bool FIRST, int T>
+__device__ __forceinline__ void pair_row(const uint32_t zt, const float jf, const float j4d, const float nh4d,
+                                         uint32_t* msg, const bool active)
+{
+  constexpr int NW = (NE + 1) / 2;
+  uint32_t      m[NW], v[NE], adr[NE], sel[NE];
   if (!FIRST) {
-    d = h2_min(h2_max(h2_sub(x, bytes_to_h2(*c2v)), kHm120), kH120);
-  }
-  return h2_min(h2_max(d, h2_fma(x, kH104, kHm12984)), h2_fma(x, kH104, kH12984));
-}
-
-// One layer for thread j. Rows of degree up to 10 keep each edge's v2c, soft-bit position and
-// partner position from the first pass; the degree-19 rows keep the v2c of their first ten edges
-// and recompute the rest (the soft bits and messages they read are not yet overwritten), so that
-// they stay within the register budget of four CTAs per SM.
-template <int DEG, bool FIRST>
-__device__ __forceinline__ void row_update_pair(const unsigned j, const unsigned Z, const unsigned H,
-                                                uint16_t* __restrict__ D, const uint32_t* __restrict__ edge,
-                                                uint16_t* __restrict__ c2v_row, const uint16_t* __restrict__ tab)
-{
-  constexpr bool KEEP = DEG <= 10;
-  constexpr int  NV   = KEEP ? DEG : 10;
-  uint32_t       v[NV];
-  unsigned       pos[KEEP ? DEG : 1], par[KEEP ? DEG : 1];
-  uint32_t       min1 = kH120, min2 = kH120;
-#pragma unroll
-  for (int e = 0; e < DEG; ++e) {
-    const uint32_t ed = edge[e];
-    const unsigned p0 = j + (ed & 0xffffu);
-    const unsigned w  = min(p0, p0 - Z); // (j + s) mod Z
-    const unsigned p  = w + (ed >> 16);
-    if constexpr (KEEP) {
-      pos[e] = p;
-      par[e] = w < H ? p + H : p - H;
-    }
-    const uint32_t vv = pair_v2c<FIRST>(bytes_to_h2(D[p]), c2v_row + e * kX2Threads);
-    if (e < NV) {
-      v[e < NV ? e : 0] = vv;
-    }
-    const uint32_t t = h2_max_xs(min1, vv);
-    min2             = h2_min_xs(min2, t);
-    min1             = h2_min_xs(min1, vv);
-  }
-  const uint32_t m1  = min1 & kAbs;
-  const uint32_t s1  = x2_scale(tab, m1);
-  const uint32_t s2  = x2_scale(tab, min2 & kAbs);
-  const uint32_t nds = h2_sub(s1, s2);
-  const uint32_t sgn = min1 & kSign;  // sign product of every v2c of the row
-#pragma unroll
-  for (int e = 0; e < DEG; ++e) {
-    unsigned p, q;
-    if constexpr (KEEP) {
-      p = pos[e];
-      q = par[e];
+    if constexpr (NW == 2) {
+      const uint2 q = *reinterpret_cast<const uint2*>(msg);
+      m[0] = q.x, m[NW - 1] = q.y;
     } else {
-      const uint32_t ed = edge[e];
-      const unsigned p0 = j + (ed & 0xffffu);
-      const unsigned w  = min(p0, p0 - Z);
-      p                 = w + (ed >> 16);
-      q                 = w < H ? p + H : p - H;
-    }
-    const uint32_t vv  = e < NV ? v[e < NV ? e : 0] : pair_v2c<FIRST>(bytes_to_h2(D[p]), c2v_row + e * kX2Threads);
-    const uint32_t mag = h2_fma(nds, h2_ne(vv & kAbs, m1), s2);
-    const uint32_t c   = mag ^ ((sgn ^ vv) & kSign);
-    c2v_row[e * kX2Threads] = (uint16_t)__byte_perm(h2_to_bytes_biased(c), 0, 0x0020);
-    const uint32_t t   = h2_add(c, vv);
-    const uint32_t cl  = h2_min(h2_max(t, kHm120), kH120);
-    uint32_t       u   = h2_fma(cl, kHm7, h2_mul(t, kH8));
-    u                  = h2_min(h2_max(u, kHm127), kH127);
-    const uint32_t ub  = h2_to_bytes_biased(u);
-    D[p] = (uint16_t)__byte_perm(ub, 0, 0x0020);
-    D[q] = (uint16_t)__byte_perm(ub, 0, 0x0002);
-  }
-}
-
-// One layer for lane pair j split over two threads: thread t (0 or 1) takes edges t, t + 2, ... of
-// the row (a thread with an odd-degree row's missing last edge contributes +120, which changes no
-// minimum and no sign), the two partial (min1, min2, sign) meet through one shuffle, and each
-// thread updates its own edges. With at most ten edges per thread every row keeps its v2c, soft-bit
-// positions and partner positions in registers. Threads past the last lane pair (j >= H) run the
-// row without loads or stores, so that every shuffle has its whole warp.
-template <int DEG, bool FIRST>
-__device__ __forceinline__ void row_update_split(const unsigned j, const unsigned t, const unsigned Z, const unsigned H,
-                                                 uint16_t* __restrict__ D, const uint32_t* __restrict__ edge,
-                                                 uint16_t* __restrict__ c2v_row, const uint16_t* __restrict__ tab)
-{
-  constexpr int NE     = (DEG + 1) / 2;
-  const bool    active = j < H;
-  uint32_t      v[NE];
-  unsigned      pos[NE], par[NE];
-  uint32_t      min1 = kH120, min2 = kH120;
 #pragma unroll
-  for (int k = 0; k < NE; ++k) {
-    const unsigned e     = 2 * k + t;
-    const bool     valid = active && ((DEG % 2) == 0 || k + 1 < NE || e < DEG);
-    const uint32_t ed    = edge[valid ? e : 0];
-    const unsigned p0    = j + (ed & 0xffffu);
-    const unsigned w     = min(p0, p0 - Z); // (j + s) mod Z
-    const unsigned p     = w + (ed >> 16);
-    pos[k]               = p;
-    par[k]               = w < H ? p + H : p - H;
-    uint32_t vv          = kH120;
-    if (valid) {
-      vv = pair_v2c<FIRST>(bytes_to_h2(D[p]), c2v_row + e * kX2Threads);
+      for (int w = 0; w < NW; ++w) {
+        m[w] = msg[w];
+      }
     }
-    v[k]             = vv;
-    const uint32_t x = h2_max_xs(min1, vv);
-    min2             = h2_min_xs(min2, x);
-    min1             = h2_min_xs(min1, vv);
   }
-  const uint32_t o1 = __shfl_xor_sync(0xffffffffu, min1, 1);
-  const uint32_t o2 = __shfl_xor_sync(0xffffffffu, min2, 1);
-  min2              = h2_min_xs(h2_min_xs(min2, o2), h2_max_xs(min1, o1));
-  min1              = h2_min_xs(min1, o1);
+  uint32_t min1 = kH120, min2 = kH120;
+#pragma unroll
+  for (int e = 0; e < NE; ++e) {
+    pair_edge(lds_v4(zt + 16 * e), jf, j4d, nh4d, adr[e], sel[e]);
+    const uint32_t x = __byte_perm(lds_u32(adr[e]), 0, sel[e]);
+    uint32_t       d = x;
+    if (!FIRST) {
+      const uint32_t c = h2_sub(__byte_perm(m[e / 2], 0x64646464u, (e & 1) ? 0x4342u : 0x4140u), kH1152);
+      d                = h2_min(h2_max(h2_sub(x, c), kHm120), kH120);
+    }
+    v[e]             = h2_min(h2_max(d, h2_fma(x, kH400, kHm48128)), h2_fma(x, kH400, kH48128));
+    const uint32_t t = h2_max_xs(min1, v[e]);
+    min2             = h2_min_xs(min2, t);
+    min1             = h2_min_xs(min1, v[e]);
+  }
+  pair_reduce<T>(min1, min2);
   const uint32_t m1  = min1 & kAbs;
-  const uint32_t s1  = x2_scale(tab, m1);
-  const uint32_t s2  = x2_scale(tab, min2 & kAbs);
-  const uint32_t nds = h2_sub(s1, s2);
   const uint32_t sgn = min1 & kSign; // sign product of every v2c of the row
+  const uint32_t s1  = pair_scale(m1) ^ sgn;
+  const uint32_t s2  = pair_scale(min2 & kAbs) ^ sgn;
+  const uint32_t ds  = h2_sub(s1, s2);
 #pragma unroll
-  for (int k = 0; k < NE; ++k) {
-    const unsigned e     = 2 * k + t;
-    const bool     valid = active && ((DEG % 2) == 0 || k + 1 < NE || e < DEG);
-    if (valid) {
-      const uint32_t vv  = v[k];
-      const uint32_t mag = h2_fma(nds, h2_ne(vv & kAbs, m1), s2);
-      const uint32_t c   = mag ^ ((sgn ^ vv) & kSign);
-      c2v_row[e * kX2Threads] = (uint16_t)__byte_perm(h2_to_bytes_biased(c), 0, 0x0020);
-      const uint32_t tt  = h2_add(c, vv);
-      const uint32_t cl  = h2_min(h2_max(tt, kHm120), kH120);
-      uint32_t       u   = h2_fma(cl, kHm7, h2_mul(tt, kH8));
-      u                  = h2_min(h2_max(u, kHm127), kH127);
-      const uint32_t ub  = h2_to_bytes_biased(u);
-      D[pos[k]]          = (uint16_t)__byte_perm(ub, 0, 0x0020);
-      D[par[k]]          = (uint16_t)__byte_perm(ub, 0, 0x0002);
+  for (int e = 0; e < NE; ++e) {
+    const uint32_t c = h2_fma(ds, h2_abs_ne(v[e], m1), s2) ^ (v[e] & kSign);
+    if (active) {
+      sts_u32(adr[e], __byte_perm(h2_add(c, v[e]), 0, sel[e]));
+    }
+    v[e] = h2_add(c, kH1152); // bytes 0 and 2 are the offset-binary messages
+  }
+#pragma unroll
+  for (int w = 0; w < NW; ++w) {
+    m[w] = __byte_perm(v[2 * w], v[2 * w + 1 < NE ? 2 * w + 1 : 2 * w], 0x6420u);
+  }
+  if constexpr (NW == 2) {
+    *reinterpret_cast<uint2*>(msg) = make_uint2(m[0], m[NW - 1]);
+  } else {
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      msg[w] = m[w];
     }
   }
 }
 
-template <bool FIRST>
-__device__ __forceinline__ void row_dispatch_split(int deg, unsigned j, unsigned t, unsigned Z, unsigned H,
-                                                   uint16_t* D, const uint32_t* edge, uint16_t* c2v_row,
-                                                   const uint16_t* tab)
+// The first iteration's row with the promotion where the soft bit is stored, for codeblocks whose
+// ragged tail holds magnitudes of 121 to 126: soft bits up to 126 are finite. Any ne; each edge's v2c is
+// formed again in the second pass.
+template <int T>
+__device__ __noinline__ void pair_row_ragged(const int ne, const uint32_t zt, const float jf, const float j4d,
+                                             const float nh4d, uint32_t* msg, const bool active)
 {
-  switch (deg) {
-    case 3: row_update_split<3, FIRST>(j, t, Z, H, D, edge, c2v_row, tab); break;
-    case 4: row_update_split<4, FIRST>(j, t, Z, H, D, edge, c2v_row, tab); break;
-    case 5: row_update_split<5, FIRST>(j, t, Z, H, D, edge, c2v_row, tab); break;
-    case 6: row_update_split<6, FIRST>(j, t, Z, H, D, edge, c2v_row, tab); break;
-    case 7: row_update_split<7, FIRST>(j, t, Z, H, D, edge, c2v_row, tab); break;
-    case 8: row_update_split<8, FIRST>(j, t, Z, H, D, edge, c2v_row, tab); break;
-    case 9: row_update_split<9, FIRST>(j, t, Z, H, D, edge, c2v_row, tab); break;
-    case 10: row_update_split<10, FIRST>(j, t, Z, H, D, edge, c2v_row, tab); break;
-    default: row_update_split<19, FIRST>(j, t, Z, H, D, edge, c2v_row, tab); break;
+  uint32_t min1 = kH120, min2 = kH120, adr, sel;
+#pragma unroll 1
+  for (int e = 0; e < ne; ++e) {
+    pair_edge(lds_v4(zt + 16 * e), jf, j4d, nh4d, adr, sel);
+    const uint32_t x = __byte_perm(lds_u32(adr), 0, sel);
+    const uint32_t v = x | (h2_abs_gt_mask(x, kH126p5) & kSat);
+    const uint32_t t = h2_max_xs(min1, v);
+    min2             = h2_min_xs(min2, t);
+    min1             = h2_min_xs(min1, v);
+  }
+  pair_reduce<T>(min1, min2);
+  const uint32_t m1  = min1 & kAbs;
+  const uint32_t sgn = min1 & kSign;
+  const uint32_t s1  = pair_scale(m1) ^ sgn;
+  const uint32_t s2  = pair_scale(min2 & kAbs) ^ sgn;
+  uint32_t       pack = 0;
+#pragma unroll 1
+  for (int e = 0; e < ne; ++e) {
+    pair_edge(lds_v4(zt + 16 * e), jf, j4d, nh4d, adr, sel);
+    const uint32_t x  = __byte_perm(lds_u32(adr), 0, sel);
+    const uint32_t v  = x | (h2_abs_gt_mask(x, kH126p5) & kSat);
+    const uint32_t eq = h2_abs_eq_mask(v, m1);
+    const uint32_t c  = ((eq & s2) | (~eq & s1)) ^ (v & kSign);
+    const uint32_t b  = h2_add(c, kH1152);
+    pack              = (e & 1) ? __byte_perm(pack, b, 0x6420u) : b;
+    if ((e & 1) != 0 || e + 1 == ne) {
+      msg[e / 2] = (e & 1) ? pack : __byte_perm(pack, pack, 0x6420u);
+    }
+    const uint32_t u = h2_add(c, v);
+    if (active) {
+      sts_u32(adr, __byte_perm(u | (h2_abs_gt_mask(u, kH120) & kSat), 0, sel));
+    }
   }
 }
 
-template <bool FIRST>
-__device__ __forceinline__ void row_dispatch_pair(int deg, unsigned j, unsigned Z, unsigned H, uint16_t* D,
-                                                  const uint32_t* edge, uint16_t* c2v_row, const uint16_t* tab)
+template <bool FIRST, int T>
+__device__ __forceinline__ void pair_row_dispatch(const int ne, const uint32_t tpart16, const uint32_t zt,
+                                                  const float jf, const float j4d, const float nh4d, uint32_t* msg,
+                                                  const bool active)
 {
-  switch (deg) {
-    case 3: row_update_pair<3, FIRST>(j, Z, H, D, edge, c2v_row, tab); break;
-    case 4: row_update_pair<4, FIRST>(j, Z, H, D, edge, c2v_row, tab); break;
-    case 5: row_update_pair<5, FIRST>(j, Z, H, D, edge, c2v_row, tab); break;
-    case 6: row_update_pair<6, FIRST>(j, Z, H, D, edge, c2v_row, tab); break;
-    case 7: row_update_pair<7, FIRST>(j, Z, H, D, edge, c2v_row, tab); break;
-    case 8: row_update_pair<8, FIRST>(j, Z, H, D, edge, c2v_row, tab); break;
-    case 9: row_update_pair<9, FIRST>(j, Z, H, D, edge, c2v_row, tab); break;
-    case 10: row_update_pair<10, FIRST>(j, Z, H, D, edge, c2v_row, tab); break;
-    default: row_update_pair<19, FIRST>(j, Z, H, D, edge, c2v_row, tab); break;
+  // Base-graph row degrees: BG1 {3..10, 19}, BG2 {3..10}.
+#define PG_PAIR_ROW(n) \
+  pair_row<n, FIRST, T>(zt + tpart16 * (n), jf, j4d, nh4d, msg + threadIdx.x * (((n) + 1) / 2), active)
+  if constexpr (T == 2) {
+    switch (ne) {
+      case 2: PG_PAIR_ROW(2); break;
+      case 3: PG_PAIR_ROW(3); break;
+      case 4: PG_PAIR_ROW(4); break;
+      case 5: PG_PAIR_ROW(5); break;
+      default: PG_PAIR_ROW(10); break;
+    }
+  } else {
+    switch (ne) {
+      case 1: PG_PAIR_ROW(1); break;
+      case 2: PG_PAIR_ROW(2); break;
+      case 3: PG_PAIR_ROW(3); break;
+      default: PG_PAIR_ROW(5); break;
+    }
   }
+#undef PG_PAIR_ROW
+}
+
+// f16 soft bit -> hard bit: soft <= 0 (either zero counts as 0).
+__device__ __forceinline__ bool pair_hard(uint32_t h)
+{
+  return (h & 0x8000u) != 0 || (h & 0x7fffu) == 0;
 }
 
 // Eight input LLRs from index k (any k; outside [0, n) they are zero) as soft bits in offset
 // binary, four per word: whole nodes (index < nof_full) clamped to +-64, a ragged tail as is
 // (ldpc_decoder_impl.cpp:147-188). last: one past the last non-zero LLR seen (the trailing-zero trim,
-// ldpc_decoder_impl.cpp:66-71).
+// ldpc_decoder_impl.cpp:66-71); ragged: a tail value of magnitude 121 to 126 was seen.
 __device__ __forceinline__ void fetch8(const int8_t* __restrict__ in, int k, int n, int nof_full, bool aligned,
-                                       int& last, uint32_t& w0, uint32_t& w1)
+                                       int& last, int& ragged, uint32_t& w0, uint32_t& w1)
 {
-  int v[8];
-  if (aligned && k >= 0 && k + 8 <= n) {
+  if (aligned && k >= 0 && k + 8 <= nof_full) {
     const uint2 q = __ldg(reinterpret_cast<const uint2*>(in + k));
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      v[i]     = (int)(int8_t)(q.x >> (8 * i));
-      v[i + 4] = (int)(int8_t)(q.y >> (8 * i));
+    if ((q.x | q.y) != 0) {
+      last = max(last, k + (q.y != 0 ? 8 - (__clz(q.y) >> 3) : 4 - (__clz(q.x) >> 3)));
     }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      v[i] = (k + i >= 0 && k + i < n) ? (int)__ldg(in + k + i) : 0;
-    }
+    w0 = __vmaxs4(__vmins4(q.x, 0x40404040u), 0xc0c0c0c0u) ^ 0x80808080u;
+    w1 = __vmaxs4(__vmins4(q.y, 0x40404040u), 0xc0c0c0c0u) ^ 0x80808080u;
+    return;
   }
   w0 = 0;
   w1 = 0;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int kk = k + i;
-    last         = v[i] != 0 ? kk + 1 : last;
-    const int x  = kk < nof_full ? max(-64, min(64, v[i])) : v[i];
+    int       x  = (kk >= 0 && kk < n) ? (int)__ldg(in + kk) : 0;
+    last         = x != 0 ? max(last, kk + 1) : last;
+    if (kk < nof_full) {
+      x = max(-64, min(64, x));
+    } else {
+      ragged |= (abs(x) > 120 && abs(x) < 127) ? 1 : 0;
+    }
     const uint32_t b = (uint32_t)(x + 128);
     if (i < 4) {
       w0 |= b << (8 * i);
@@ -889,89 +899,140 @@ __device__ __forceinline__ void fetch8(const int8_t* __restrict__ in, int k, int
   }
 }
 
-// Decodes codeblock cb (even Z > 192) with check-to-variable slab `slab`: NT threads, T threads per
-// lane pair (NT = 192 * T).
-template <int NT, int T>
-__device__ void decode_codeblock_pair(const pg_ldpc_cb& d, smem_pair_nt_t<NT>& sm, const int8_t* __restrict__ llrs,
-                                      uint8_t* __restrict__ bits, int32_t* __restrict__ iterations,
-                                      int8_t* __restrict__ c2v_all, const uint32_t* __restrict__ crc_pow,
-                                      const uint16_t* __restrict__ scale_tab, const int cb, const int slab)
+// Decodes codeblock cb (even Z <= 2 NT / T) with T threads per lane pair; smem: smem_bytes of dynamic
+// shared memory (at least kPairMinSmem); slab: the CTA's global message slab.
+template <int T, int NT>
+__device__ __forceinline__ void decode_codeblock_pair(const pg_ldpc_cb& d, pair_shared& sh, unsigned char* smem,
+                                                      const uint32_t smem_bytes, const int8_t* __restrict__ llrs,
+                                                      uint8_t* __restrict__ bits, int32_t* __restrict__ iterations,
+                                                      uint32_t* slab, const uint32_t* __restrict__ crc_pow,
+                                                      const int cb)
 {
-  static_assert(NT == kX2Threads * T && (T == 1 || T == 2), "one or two threads per lane pair");
-  const int tid = threadIdx.x;
-  const int bg  = d.base_graph;
-  const int Z   = (int)d.lifting_size;
-  const int H   = Z >> 1;
-  const int set = (Z <= pg::kMaxZ) ? dev_set_index(Z) : -1;
-  if ((bg != 1 && bg != 2) || set < 0 || (Z & 15) != 0) {
+  constexpr int LG  = T == 2 ? 0 : 1; // index of the T-dependent tables
+  const int     tid = threadIdx.x;
+  const int     bg  = d.base_graph;
+  const int     Z   = (int)d.lifting_size;
+  const int     H   = Z >> 1;
+  const int     set = dev_set_index(Z);
+  if ((bg != 1 && bg != 2) || set < 0) {
     if (tid == 0) {
       iterations[cb] = -1;
     }
     return;
   }
-  const int     g        = bg - 1;
-  const int     Kb       = bg == 1 ? 22 : 10;
-  const int     nrows    = bg == 1 ? pg::kBg1Rows : pg::kBg2Rows;
-  const int     nedges   = bg == 1 ? pg::kBg1Edges : pg::kBg2Edges;
-  const int     nfull    = bg == 1 ? 68 : 52;
-  const int     msg_len  = Kb * Z;
-  const int     n        = (int)d.nof_llrs;
-  const int8_t* in       = llrs + d.llr_offset;
-  uint16_t*     c2v      = reinterpret_cast<uint16_t*>(c2v_all + (size_t)slab * pg::kC2vStride);
-  const int     nbytes   = (msg_len + 7) / 8;
-  uint8_t*      out      = bits + d.out_offset;
-  const int     crc_poly = d.crc_poly;
-  const int     nwords   = (msg_len + 31) / 32;
-  uint16_t*     D        = sm.D;
+  const int          g        = bg - 1;
+  const int          Kb       = bg == 1 ? 22 : 10;
+  const int          nrows    = bg == 1 ? pg::kBg1Rows : pg::kBg2Rows;
+  const int          nedges   = bg == 1 ? pg::kBg1Edges : pg::kBg2Edges;
+  const int          nfull    = bg == 1 ? 68 : 52;
+  const int          msg_len  = Kb * Z;
+  const int          n        = (int)d.nof_llrs;
+  const int8_t*      in       = llrs + d.llr_offset;
+  const int          nbytes   = (msg_len + 7) / 8;
+  uint8_t*           out      = bits + d.out_offset;
+  const int          crc_poly = d.crc_poly;
+  const uint32_t     h4       = 4u * (uint32_t)H;
+  const pair_tables& tb       = g_pair_tables;
+  uint4*             tab      = reinterpret_cast<uint4*>(smem);
+  unsigned char*     E        = smem + kPairTabBytes; // the constant column, then the graph's columns
+  const uint32_t     tab_s    = (uint32_t)__cvta_generic_to_shared(tab);
+  const uint32_t     E_s      = (uint32_t)__cvta_generic_to_shared(E);
+  const int          nta      = (T * H + 31) & ~31;   // threads of the rows (whole warps)
+  const bool         active   = tid < T * H;
+  const uint32_t     jp       = (uint32_t)(active ? tid / T : H - 1);
 
+  // Edge table of this lifting size, row list, constant column.
   for (int e = tid; e < nedges; e += NT) {
-    const int col = c_edge_col[g][e];
-    const int s   = c_edge_v[g][e][set] % Z;
-    sm.edge[e]    = ((uint32_t)(col * Z) << 16) | (uint32_t)s;
+    const int      r    = tb.edge_row[g][e];
+    const uint32_t s    = (uint32_t)tb.edge_v[g][e][set] % (uint32_t)Z;
+    const bool     up   = s >= (uint32_t)H;
+    const uint32_t sp   = up ? s - (uint32_t)H : s;
+    // {shared address of (col, s'), 1 - (H - s') as a float, selector 0x3210 or (swapped) 0x1032, its change when
+    // the edge wraps (sign and magnitude)}
+    tab[tb.pad_e0[LG][g][r] + e - tb.row_e0[g][r]] =
+        make_uint4(E_s + h4 * (1u + tb.edge_col[g][e]) + 4u * sp, __float_as_uint(1.f - (float)(H - (int)sp)),
+                   up ? 0x1032u : 0x3210u, up ? 0x21deu : 0x800021deu);
+  }
+  for (int r = tid; r < nrows; r += NT) {
+    const int deg = tb.row_deg[g][r];
+    const int p0 = tb.pad_e0[LG][g][r], p1 = tb.pad_e0[LG][g][r + 1];
+    for (int k = deg; k < p1 - p0; ++k) {
+      tab[p0 + k] = make_uint4(E_s, __float_as_uint(-1024.f), 0x3210u, 0u); // the constant column
+    }
+    sh.row[r] = make_uint4(tab_s + 16u * (uint32_t)p0, (uint32_t)(nta * tb.msg0[LG][g][r]), (uint32_t)((p1 - p0) / T),
+                           (uint32_t)tb.row_sync[g][r]);
+  }
+  for (int k = tid; k < H; k += NT) {
+    reinterpret_cast<uint32_t*>(E)[k] = kHDummy;
   }
   if (tid == 0) {
-    sm.s_last = 0;
-    sm.s_done = 0;
+    sh.last   = 0;
+    sh.ragged = 0;
+    sh.crc[0] = sh.crc[1] = 0;
+    sh.zero[0] = sh.zero[1] = 0;
   }
   __syncthreads();
 
-  // Soft bits, eight lanes of each half of a column per thread step (2Z punctured zeros, then the
-  // input), both copies: D[col][w0 + i] = (soft[w0 + i], soft[w0 + H + i]) and the swapped pair at
-  // w0 + H + i.
+  // Soft bits as f16 pairs (2Z punctured zeros, then the input): eight pairs per thread step when
+  // the node halves are multiples of eight lanes, else one.
   {
-    const int  per_col  = H / 8;
-    const int  nchunks  = nfull * per_col;
-    const int  nof_full = (n / Z) * Z;
-    const bool aligned  = (reinterpret_cast<uintptr_t>(in) & 7u) == 0;
-    int        last     = 0;
+    const int nof_full = (n / Z) * Z;
+    int       last = 0, ragged = 0;
+    uint32_t* E0 = reinterpret_cast<uint32_t*>(E) + H;
+    if ((H & 7) == 0) {
+      const int      per_col = H >> 3;
+      const int      nchunks = nfull * per_col;
+      const uint32_t inv     = 0xffffffffu / (uint32_t)per_col + 1u;
+      const bool     aligned = (reinterpret_cast<uintptr_t>(in) & 7u) == 0;
+#pragma unroll 2
+      for (int q = tid; q < nchunks; q += NT) {
+        const int col = per_col == 1 ? q : (int)__umulhi((uint32_t)q, inv);
+        const int w0  = (q - col * per_col) * 8;
+        const int k   = (col - 2) * Z + w0;
+        uint32_t  l0, l1, u0, u1;
+        fetch8(in, k, n, nof_full, aligned, last, ragged, l0, l1);
+        fetch8(in, k + H, n, nof_full, aligned, last, ragged, u0, u1);
+        const uint32_t p0 = __byte_perm(l0, u0, 0x5140), p1 = __byte_perm(l0, u0, 0x7362);
+        const uint32_t p2 = __byte_perm(l1, u1, 0x5140), p3 = __byte_perm(l1, u1, 0x7362);
+        uint32_t*      o = E0 + col * H + w0;
+        *reinterpret_cast<uint4*>(o) =
+            make_uint4(bytes_to_h2(p0), bytes_to_h2(p0 >> 16), bytes_to_h2(p1), bytes_to_h2(p1 >> 16));
+        *reinterpret_cast<uint4*>(o + 4) =
+            make_uint4(bytes_to_h2(p2), bytes_to_h2(p2 >> 16), bytes_to_h2(p3), bytes_to_h2(p3 >> 16));
+      }
+    } else {
+      const int      nwords = nfull * H;
+      const uint32_t inv    = 0xffffffffu / (uint32_t)H + 1u;
 #pragma unroll 4
-    for (int q = tid; q < nchunks; q += NT) {
-      const int col = q / per_col;
-      const int w0  = (q - col * per_col) * 8;
-      const int k   = (col - 2) * Z + w0;
-      uint32_t  l0, l1, h0, h1;
-      fetch8(in, k, n, nof_full, aligned, last, l0, l1);
-      fetch8(in, k + H, n, nof_full, aligned, last, h0, h1);
-      uint4 lo, hi;
-      lo.x = __byte_perm(l0, h0, 0x5140);
-      lo.y = __byte_perm(l0, h0, 0x7362);
-      lo.z = __byte_perm(l1, h1, 0x5140);
-      lo.w = __byte_perm(l1, h1, 0x7362);
-      hi.x = __byte_perm(h0, l0, 0x5140);
-      hi.y = __byte_perm(h0, l0, 0x7362);
-      hi.z = __byte_perm(h1, l1, 0x5140);
-      hi.w = __byte_perm(h1, l1, 0x7362);
-      *reinterpret_cast<uint4*>(D + col * Z + w0)     = lo;
-      *reinterpret_cast<uint4*>(D + col * Z + w0 + H) = hi;
+      for (int q = tid; q < nwords; q += NT) {
+        const int col = H == 1 ? q : (int)__umulhi((uint32_t)q, inv);
+        const int k   = (col - 2) * Z + (q - col * H);
+        int       x[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int kk = k + i * H;
+          x[i]         = (kk >= 0 && kk < n) ? (int)__ldg(in + kk) : 0;
+          last         = x[i] != 0 ? max(last, kk + 1) : last;
+          if (kk < nof_full) {
+            x[i] = max(-64, min(64, x[i]));
+          } else {
+            ragged |= (abs(x[i]) > 120 && abs(x[i]) < 127) ? 1 : 0;
+          }
+        }
+        E0[q] = bytes_to_h2((uint32_t)(x[0] + 128) | ((uint32_t)(x[1] + 128) << 8));
+      }
     }
-    last = warp_max(last);
+    last = __reduce_max_sync(0xffffffffu, last);
     if ((tid & 31) == 0 && last > 0) {
-      atomicMax(&sm.s_last, last);
+      atomicMax(&sh.last, last);
+    }
+    if (ragged) {
+      sh.ragged = 1;
     }
   }
   __syncthreads();
 
-  const int input_size = sm.s_last;
+  const int input_size = sh.last;
   if (input_size < msg_len) {
     for (int b = tid; b < nbytes; b += NT) {
       out[b] = 0xff;
@@ -979,757 +1040,200 @@ __device__ void decode_codeblock_pair(const pg_ldpc_cb& d, smem_pair_nt_t<NT>& s
     if (tid == 0) {
       iterations[cb] = 0;
     }
-    __syncthreads();
     return;
   }
   int cb_len = max(input_size + 2 * Z, (Kb + 4) * Z);
   cb_len     = ((cb_len + Z - 1) / Z) * Z;
-  const int nof_layers = min(cb_len / Z - Kb, nrows);
+  const int      nof_layers = min(cb_len / Z - Kb, nrows);
+  const bool     ragged     = sh.ragged != 0;
+  const int      order      = crc_poly == PG_CRC16 ? 16 : 24;
+  const uint32_t* pow_tab   = crc_pow + (size_t)(crc_poly <= PG_CRC24B ? crc_poly : 0) * pg::kCrcPowLen;
+  const int      crc_len    = msg_len - (int)d.nof_filler_bits;
 
-  int order = 24;
-  if (crc_poly == PG_CRC16) {
-    order = 16;
-  }
-  const uint32_t* pow_tab = crc_pow + (size_t)(crc_poly <= PG_CRC24B ? crc_poly : 0) * pg::kCrcPowLen;
-  const int       crc_len = msg_len - (int)d.nof_filler_bits;
-
-  int            result = 0;
-  const int      max_it = d.max_iterations;
-  const int      lane   = tid & 31;
-  const unsigned j      = (unsigned)tid;
-  const int nsteps = steps_for_layers(g, nof_layers);
-  for (int it = 0; it < max_it; ++it) {
-    for (int st = 0; st < nsteps; ++st) {
-      // Messages are read from the second iteration on: prefetch the next step's.
-      if (it > 0 || st + 1 == nsteps) {
-        prefetch_step(g, st + 1 < nsteps ? st + 1 : 0, nof_layers, tid, reinterpret_cast<const char*>(c2v),
-                      kX2Threads * 2);
-      }
-      const int r0 = c_step_row0[g][st];
-      const int r1 = min(r0 + (int)c_step_nrows[g][st], nof_layers);
-      if (T == 1 && tid < H) {
-        for (int r = r0; r < r1; ++r) {
-          const int deg     = c_row_deg[g][r];
-          const int e0      = c_row_e0[g][r];
-          uint16_t* c2v_row = c2v + (size_t)e0 * kX2Threads + tid;
-          if (it == 0) {
-            row_dispatch_pair<true>(deg, j, (unsigned)Z, (unsigned)H, D, sm.edge + e0, c2v_row, scale_tab);
-          } else {
-            row_dispatch_pair<false>(deg, j, (unsigned)Z, (unsigned)H, D, sm.edge + e0, c2v_row, scale_tab);
-          }
-        }
-      } else if (T == 2 && tid < ((2 * H + 31) & ~31)) {
-        const unsigned jp = (unsigned)tid >> 1, tp = (unsigned)tid & 1u;
-        for (int r = r0; r < r1; ++r) {
-          const int deg     = c_row_deg[g][r];
-          const int e0      = c_row_e0[g][r];
-          uint16_t* c2v_row = c2v + (size_t)e0 * kX2Threads + jp;
-          if (it == 0) {
-            row_dispatch_split<true>(deg, jp, tp, (unsigned)Z, (unsigned)H, D, sm.edge + e0, c2v_row, scale_tab);
-          } else {
-            row_dispatch_split<false>(deg, jp, tp, (unsigned)Z, (unsigned)H, D, sm.edge + e0, c2v_row, scale_tab);
-          }
-        }
-      }
-      __syncthreads();
-    }
-
-    // Hard decisions (soft <= 0: offset byte <= 128; the low byte of D[i] is soft bit i), zero
-    // check and CRC: one 32-bit word per warp step, lane k holding bit k of the word (MSB first
-    // after the reversal); each set bit within the CRC length adds x^e mod g.
-    int      zero = 0;
-    uint32_t crc  = 0;
-    for (int wi = tid >> 5; wi < nwords; wi += NT / 32) {
-      const int      idx = 32 * wi + lane;
-      const uint32_t b   = idx < msg_len ? (D[idx] & 0xffu) : 0xffu;
-      const bool     bit = b <= 128u;
-      zero |= b == 128u;
-      const uint32_t w = __brev(__ballot_sync(0xffffffffu, bit));
-      if (lane == 0) {
-        sm.hard[wi] = w;
-      }
-      if (crc_poly != PG_CRC_NONE && bit && idx < crc_len) {
-        crc ^= __ldg(pow_tab + (crc_len - 1 - idx + order));
-      }
-    }
-    zero = __syncthreads_or(zero);
-    crc  = warp_xor(crc);
-    if (lane == 0) {
-      sm.red[tid >> 5] = crc;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      uint32_t t = 0;
-      for (int w = 0; w < NT / 32; ++w) {
-        t ^= sm.red[w];
-      }
-      sm.s_done = (crc_poly != PG_CRC_NONE && !zero && t == 0) ? 1 : 0;
-    }
-    __syncthreads();
-    if (sm.s_done) {
-      result = it + 1;
-      break;
-    }
-  }
-
-  if (crc_poly == PG_CRC_NONE) {
-    // Syndrome check over the processed rows (ldpc_decoder_impl.cpp:329-387), both lanes.
-    int bad = 0;
-    if (tid < H) {
-      int e0 = 0;
-      for (int r = 0; r < nof_layers; ++r) {
-        const int deg    = c_row_deg[g][r];
-        uint32_t  parity = 0;
-        for (int e = 0; e < deg; ++e) {
-          const uint32_t ed = sm.edge[e0 + e];
-          const unsigned p0 = j + (ed & 0xffffu);
-          const uint32_t x  = D[min(p0, p0 - (unsigned)Z) + (ed >> 16)];
-          const uint32_t lo = x & 0xffu, hi = x >> 8;
-          bad |= (lo == 128u) | (hi == 128u);
-          parity ^= (uint32_t)(lo <= 128u) | ((uint32_t)(hi <= 128u) << 1);
-        }
-        bad |= parity != 0;
-        e0 += deg;
-      }
-    }
-    bad      = __syncthreads_or(bad);
-    int zero = 0;
-    for (int i = tid; i < msg_len; i += NT) {
-      zero |= (D[i] & 0xffu) == 128u;
-    }
-    zero   = __syncthreads_or(zero);
-    result = (!bad && !zero) ? max_it : 0;
-  }
-
-  for (int b = tid; b < nbytes; b += NT) {
-    out[b] = (uint8_t)(sm.hard[b >> 2] >> (24 - 8 * (b & 3)));
-  }
-  if (tid == 0) {
-    iterations[cb] = result;
-  }
-  __syncthreads();
-}
-
-// ---------------------------------------------------------------------------------------------
-// Lifting size 384 (every large transport block): the two-lanes-per-thread arithmetic above with
-// everything that depends on Z fixed at compile time and the soft bits stored once, as f16.
-//
-// Thread j (0 <= j < 192) carries check lanes j and j + 192. Soft bits: E[col][k] = (soft[col][k],
-// soft[col][k + 192]) as one f16x2 word, 0 <= k < 192 (52 KB for BG1, so four CTAs share an SM).
-// For an edge of shift s, lane j reads variable lane (j + s) mod 384 and lane j + 192 reads
-// (j + 192 + s) mod 384: both are halves of the same word k = (j + s') mod 192 with s' = s mod 192,
-// swapped when (j + s' >= 192) differs from (s >= 192). Per edge the constant tables give 4 s', the
-// column's byte offset and the byte-permute selector of the wrapped case (c_z_*, set for Z = 384
-// at table upload); the selector of the unwrapped case differs from it by 0x2222.
-// The 0.8 scaling, floor(m * 52428 / 2^16) for integer 0 <= m <= 120, is
-// max(fma(m, f16(0.8), 1023.5) - 1024, 0) in f16: the fused multiply-add rounds once, to an integer
-// (the spacing of f16 in [1024, 2048)), and f16(0.8) = 0.7998046875 errs by at most 0.024 at
-// m = 120, inside the 0.1 margin of every rounding decision (checked for every m).
-// Check-to-variable messages are offset-binary byte pairs per (edge, thread) in the L2 slab, as in
-// the two-lanes-per-thread decoder.
-// Saturation: the soft update keeps 8t - 7 clamp(t, +-120) without the final clamp to +-127, so a
-// soft bit the reference saturates to +-127 is here any magnitude of at least 128 (or f16
-// infinity). Such a value acts as +-127 everywhere it is used: its bounds 104x -+ 12984 are at least
-// 328 in magnitude, so its v2c stays at least 328 (no minimum, no message-magnitude tie, the sign
-// kept) and its next soft update is again at least 128 in magnitude; the hard decision reads only
-// the sign. The message magnitudes are at most 96 and finite, so no infinity meets its negative.
-constexpr int kZ384      = 384;
-constexpr int kZH        = 192;
-constexpr int kZThreads  = 192;
-constexpr int kZMaxPerSm = 4;   // register budget of the launch bounds (80 registers a thread)
-constexpr int kZResidentPerSm = 3; // resident CTAs per SM: shared memory (soft bits + edge tables)
-constexpr int kZ19Keep   = 8;  // v2c kept in registers by rows above kZKeepDeg edges
-constexpr int kZKeepDeg  = 10; // rows of up to this many edges keep v2c, address and selector
-
-__constant__ uint32_t c_z_sp4[2][pg::kBg1Edges]; // 4 (s mod 192)
-__constant__ uint32_t c_z_col[2][pg::kBg1Edges]; // byte offset of the edge's column in E
-__constant__ uint32_t c_z_sel[2][pg::kBg1Edges]; // selector when j + s' >= 192
-
-template <int NT>
-struct __align__(16) smem_z_nt_t {
-  uint32_t E[pg::kMaxNodes * kZH];
-  uint32_t hard[(22 * kZ384) / 32];
-  uint32_t red[NT / 32];
-  int      s_last;
-  int      s_done;
-};
-using smem_z_t = smem_z_nt_t<kZThreads>;
-
-constexpr uint32_t kH0p8     = 0x3a663a66u; // f16(0.8) = 0.7998046875
-constexpr uint32_t kH1023p5  = 0x63ff63ffu; // 1023.5
-constexpr uint32_t kHm1024   = 0xe400e400u; // -1024
-
-__device__ __forceinline__ uint32_t z_scale(uint32_t m)
-{
-  return h2_max(h2_add(h2_fma(m, kH0p8, kH1023p5), kHm1024), 0u);
-}
-
-__device__ __forceinline__ uint32_t lds_u32(const unsigned char* base, uint32_t off)
-{
-  return *reinterpret_cast<const uint32_t*>(base + off);
-}
-__device__ __forceinline__ void sts_u32(unsigned char* base, uint32_t off, uint32_t v)
-{
-  *reinterpret_cast<uint32_t*>(base + off) = v;
-}
-
-// Byte offset in E and byte-permute selector of edge e (global edge index) for thread j (j4 = 4 j),
-// from the CTA's copy of the edge table: {4 (s mod 192), column byte offset, selector when
-// j + s' >= 192, selector otherwise}.
-__device__ __forceinline__ void z_edge(const uint4* __restrict__ zt, const int e, const uint32_t j4, uint32_t& adr,
-                                       uint32_t& sel)
-{
-  const uint4    c  = zt[e];
-  const uint32_t t4 = j4 + c.x;
-  const uint32_t k4 = __viaddmin_u32(t4, 0u - 4u * kZH, t4); // (j + s') mod 192, times 4
-  sel               = k4 == t4 ? c.w : c.z;
-  adr               = k4 + c.y;
-}
-
-// The edge tables of both base graphs in shared memory (one copy per CTA, filled once per launch).
-__device__ __forceinline__ void z_load_edge_tables(uint4* zt)
-{
-  for (int i = threadIdx.x; i < 2 * pg::kBg1Edges; i += blockDim.x) {
-    const int      g = i / pg::kBg1Edges, e = i - g * pg::kBg1Edges;
-    const uint32_t sw = c_z_sel[g][e];
-    zt[i]             = make_uint4(c_z_sp4[g][e], c_z_col[g][e], sw, sw ^ 0x2222u);
-  }
-  __syncthreads();
-}
-
-// One layer (base-graph row of degree DEG, first edge e0) for thread j. Rows of up to kZKeepDeg
-// edges keep each edge's v2c, address and selector from the first pass; the degree-19 rows keep
-// the v2c of their first kZ19Keep edges and recompute the rest (the soft bits and messages they
-// read are not yet overwritten), so that four CTAs fit an SM without spills.
-template <int DEG, bool FIRST>
-__device__ __forceinline__ void row_update_z(const uint4* __restrict__ zt, const int e0, const uint32_t j4, unsigned char* E,
-                                             uint16_t* __restrict__ c2v_row)
-{
-  constexpr bool KEEP = DEG <= kZKeepDeg;
-  constexpr int  NV   = KEEP ? DEG : kZ19Keep;
-  uint32_t       v[NV];
-  uint32_t       adr[KEEP ? DEG : 1], sel[KEEP ? DEG : 1];
-  uint32_t       min1 = kH120, min2 = kH120;
-#pragma unroll
-  for (int e = 0; e < DEG; ++e) {
-    uint32_t a, s;
-    z_edge(zt, e0 + e, j4, a, s);
-    if constexpr (KEEP) {
-      adr[e] = a;
-      sel[e] = s;
-    }
-    const uint32_t vv = pair_v2c<FIRST>(__byte_perm(lds_u32(E, a), 0, s), c2v_row + e * kZH);
-    if (e < NV) {
-      v[e < NV ? e : 0] = vv;
-    }
-    const uint32_t t  = h2_max_xs(min1, vv);
-    min2              = h2_min_xs(min2, t);
-    min1              = h2_min_xs(min1, vv);
-  }
-  const uint32_t m1  = min1 & kAbs;
-  const uint32_t s1  = z_scale(m1);
-  const uint32_t s2  = z_scale(min2 & kAbs);
-  const uint32_t nds = h2_sub(s1, s2);
-  const uint32_t sgn = min1 & kSign; // sign product of every v2c of the row
-#pragma unroll
-  for (int e = 0; e < DEG; ++e) {
-    uint32_t a, s;
-    if constexpr (KEEP) {
-      a = adr[e];
-      s = sel[e];
-    } else {
-      z_edge(zt, e0 + e, j4, a, s);
-    }
-    const uint32_t vv  = e < NV ? v[e < NV ? e : 0]
-                                : pair_v2c<FIRST>(__byte_perm(lds_u32(E, a), 0, s), c2v_row + e * kZH);
-    const uint32_t mag = h2_fma(nds, h2_ne(vv & kAbs, m1), s2);
-    const uint32_t c   = mag ^ ((sgn ^ vv) & kSign);
-    c2v_row[e * kZH] = (uint16_t)__byte_perm(h2_to_bytes_biased(c), 0, 0x0020);
-    const uint32_t tt  = h2_add(c, vv);
-    const uint32_t cl  = h2_min(h2_max(tt, kHm120), kH120);
-    const uint32_t u   = h2_fma(cl, kHm7, h2_mul(tt, kH8));
-    sts_u32(E, a, __byte_perm(u, 0, s));
-  }
-}
-
-// The same layer split over the two threads of lane pair j (t = 0, 1): thread t takes edges t,
-// t + 2, ... (a missing last edge of an odd-degree row contributes +120, which changes no minimum
-// and no sign), the two partial (min1, min2, sign) meet through one shuffle, and each thread updates
-// its own edges.
-template <int DEG, bool FIRST>
-__device__ __forceinline__ void row_update_z_split(const uint4* __restrict__ zt, const int e0, const uint32_t j4, const int t,
-                                                   unsigned char* E, uint16_t* __restrict__ c2v_row)
-{
-  constexpr int  NE   = (DEG + 1) / 2;
-  constexpr bool KEEP = NE <= 3; // wider rows recompute address and selector (register budget)
-  uint32_t       v[NE], adr[KEEP ? NE : 1], sel[KEEP ? NE : 1];
-  uint32_t       min1 = kH120, min2 = kH120;
-#pragma unroll
-  for (int k = 0; k < NE; ++k) {
-    const int  e     = 2 * k + t;
-    const bool valid = (DEG % 2) == 0 || k + 1 < NE || e < DEG;
-    uint32_t   vv    = kH120;
-    if (valid) {
-      uint32_t a, s;
-      z_edge(zt, e0 + e, j4, a, s);
-      if constexpr (KEEP) {
-        adr[k] = a;
-        sel[k] = s;
-      }
-      vv = pair_v2c<FIRST>(__byte_perm(lds_u32(E, a), 0, s), c2v_row + e * kZH);
-    }
-    v[k]             = vv;
-    const uint32_t x = h2_max_xs(min1, vv);
-    min2             = h2_min_xs(min2, x);
-    min1             = h2_min_xs(min1, vv);
-  }
-  const uint32_t o1 = __shfl_xor_sync(0xffffffffu, min1, 1);
-  const uint32_t o2 = __shfl_xor_sync(0xffffffffu, min2, 1);
-  min2              = h2_min_xs(h2_min_xs(min2, o2), h2_max_xs(min1, o1));
-  min1              = h2_min_xs(min1, o1);
-  const uint32_t m1  = min1 & kAbs;
-  const uint32_t s1  = z_scale(m1);
-  const uint32_t s2  = z_scale(min2 & kAbs);
-  const uint32_t nds = h2_sub(s1, s2);
-  const uint32_t sgn = min1 & kSign; // sign product of every v2c of the row
-#pragma unroll
-  for (int k = 0; k < NE; ++k) {
-    const int  e     = 2 * k + t;
-    const bool valid = (DEG % 2) == 0 || k + 1 < NE || e < DEG;
-    if (valid) {
-      uint32_t a, s;
-      if constexpr (KEEP) {
-        a = adr[k];
-        s = sel[k];
-      } else {
-        z_edge(zt, e0 + e, j4, a, s);
-      }
-      const uint32_t vv  = v[k];
-      const uint32_t mag = h2_fma(nds, h2_ne(vv & kAbs, m1), s2);
-      const uint32_t c   = mag ^ ((sgn ^ vv) & kSign);
-      c2v_row[e * kZH]   = (uint16_t)__byte_perm(h2_to_bytes_biased(c), 0, 0x0020);
-      const uint32_t tt  = h2_add(c, vv);
-      const uint32_t cl  = h2_min(h2_max(tt, kHm120), kH120);
-      const uint32_t u   = h2_fma(cl, kHm7, h2_mul(tt, kH8));
-      sts_u32(E, a, __byte_perm(u, 0, s));
-    }
-  }
-}
-
-template <bool FIRST>
-__device__ __forceinline__ void row_dispatch_z_split(int deg, const uint4* zt, int e0, uint32_t j4, int t, unsigned char* E,
-                                                     uint16_t* c2v_row)
-{
-  switch (deg) {
-    case 3: row_update_z_split<3, FIRST>(zt, e0, j4, t, E, c2v_row); break;
-    case 4: row_update_z_split<4, FIRST>(zt, e0, j4, t, E, c2v_row); break;
-    case 5: row_update_z_split<5, FIRST>(zt, e0, j4, t, E, c2v_row); break;
-    case 6: row_update_z_split<6, FIRST>(zt, e0, j4, t, E, c2v_row); break;
-    case 7: row_update_z_split<7, FIRST>(zt, e0, j4, t, E, c2v_row); break;
-    case 8: row_update_z_split<8, FIRST>(zt, e0, j4, t, E, c2v_row); break;
-    case 9: row_update_z_split<9, FIRST>(zt, e0, j4, t, E, c2v_row); break;
-    case 10: row_update_z_split<10, FIRST>(zt, e0, j4, t, E, c2v_row); break;
-    default: row_update_z_split<19, FIRST>(zt, e0, j4, t, E, c2v_row); break;
-  }
-}
-
-template <bool FIRST>
-__device__ __forceinline__ void row_dispatch_z(int deg, const uint4* zt, int e0, uint32_t j4, unsigned char* E, uint16_t* c2v_row)
-{
-  switch (deg) {
-    case 3: row_update_z<3, FIRST>(zt, e0, j4, E, c2v_row); break;
-    case 4: row_update_z<4, FIRST>(zt, e0, j4, E, c2v_row); break;
-    case 5: row_update_z<5, FIRST>(zt, e0, j4, E, c2v_row); break;
-    case 6: row_update_z<6, FIRST>(zt, e0, j4, E, c2v_row); break;
-    case 7: row_update_z<7, FIRST>(zt, e0, j4, E, c2v_row); break;
-    case 8: row_update_z<8, FIRST>(zt, e0, j4, E, c2v_row); break;
-    case 9: row_update_z<9, FIRST>(zt, e0, j4, E, c2v_row); break;
-    case 10: row_update_z<10, FIRST>(zt, e0, j4, E, c2v_row); break;
-    default: row_update_z<19, FIRST>(zt, e0, j4, E, c2v_row); break;
-  }
-}
-
-// f16 soft bit -> hard bit: soft <= 0 (either zero counts as 0).
-__device__ __forceinline__ bool z_hard(uint32_t h)
-{
-  return (h & 0x8000u) != 0 || (h & 0x7fffu) == 0;
-}
-
-// Decodes codeblock cb (Z = 384) with check-to-variable slab `slab`: NT threads, T = NT / 192 per
-// lane pair (T = 2: each row's edges split between the pair's two threads).
-template <int NT>
-__device__ void decode_codeblock_z384(const pg_ldpc_cb& d, smem_z_nt_t<NT>& sm, const uint4* __restrict__ ztab,
-                                      const int8_t* __restrict__ llrs,
-                                      uint8_t* __restrict__ bits, int32_t* __restrict__ iterations,
-                                      int8_t* __restrict__ c2v_all, const uint32_t* __restrict__ crc_pow, const int cb,
-                                      const int slab)
-{
-  constexpr int T = NT / kZH;
-  static_assert(NT == kZH || NT == 2 * kZH, "one or two threads per lane pair");
-  const int tid = threadIdx.x;
-  const int bg  = d.base_graph;
-  if (bg != 1 && bg != 2) {
-    if (tid == 0) {
-      iterations[cb] = -1;
-    }
-    return;
-  }
-  const int      g        = bg - 1;
-  const uint4*   zt       = ztab + g * pg::kBg1Edges;
-  const int      Kb       = bg == 1 ? 22 : 10;
-  const int      nrows    = bg == 1 ? pg::kBg1Rows : pg::kBg2Rows;
-  const int      nfull    = bg == 1 ? 68 : 52;
-  const int      msg_len  = Kb * kZ384;
-  const int      n        = (int)d.nof_llrs;
-  const int8_t*  in       = llrs + d.llr_offset;
-  uint16_t*      c2v      = reinterpret_cast<uint16_t*>(c2v_all + (size_t)slab * pg::kC2vStride);
-  const int      nbytes   = msg_len / 8;
-  uint8_t*       out      = bits + d.out_offset;
-  const int      crc_poly = d.crc_poly;
-  const int      nwords   = msg_len / 32;
-  unsigned char* E        = reinterpret_cast<unsigned char*>(sm.E);
-  const int      jp       = T == 1 ? tid : tid >> 1; // lane pair
-  const int      tp       = T == 1 ? 0 : tid & 1;
-  const uint32_t j4       = 4u * (uint32_t)jp;
-
-  if (tid == 0) {
-    sm.s_last = 0;
-    sm.s_done = 0;
-  }
-  __syncthreads();
-
-  // Soft bits as f16 pairs, eight pairs per thread step (2Z punctured zeros, then the input).
-  {
-    constexpr int per_col  = kZH / 8;
-    const int     nchunks  = nfull * per_col;
-    const int     nof_full = (n / kZ384) * kZ384;
-    const bool    aligned  = (reinterpret_cast<uintptr_t>(in) & 7u) == 0;
-    int           last     = 0;
-#pragma unroll 2
-    for (int q = tid; q < nchunks; q += NT) {
-      const int col = q / per_col;
-      const int w0  = (q - col * per_col) * 8;
-      const int k   = (col - 2) * kZ384 + w0;
-      uint32_t  l0, l1, h0, h1;
-      fetch8(in, k, n, nof_full, aligned, last, l0, l1);
-      fetch8(in, k + kZH, n, nof_full, aligned, last, h0, h1);
-      const uint32_t p0 = __byte_perm(l0, h0, 0x5140), p1 = __byte_perm(l0, h0, 0x7362);
-      const uint32_t p2 = __byte_perm(l1, h1, 0x5140), p3 = __byte_perm(l1, h1, 0x7362);
-      uint4          a, b;
-      a.x = bytes_to_h2(p0);
-      a.y = bytes_to_h2(p0 >> 16);
-      a.z = bytes_to_h2(p1);
-      a.w = bytes_to_h2(p1 >> 16);
-      b.x = bytes_to_h2(p2);
-      b.y = bytes_to_h2(p2 >> 16);
-      b.z = bytes_to_h2(p3);
-      b.w = bytes_to_h2(p3 >> 16);
-      *reinterpret_cast<uint4*>(sm.E + col * kZH + w0)     = a;
-      *reinterpret_cast<uint4*>(sm.E + col * kZH + w0 + 4) = b;
-    }
-    last = warp_max(last);
-    if ((tid & 31) == 0 && last > 0) {
-      atomicMax(&sm.s_last, last);
-    }
-  }
-  __syncthreads();
-
-  const int input_size = sm.s_last;
-  if (input_size < msg_len) {
-    for (int b = tid; b < nbytes; b += NT) {
-      out[b] = 0xff;
-    }
-    if (tid == 0) {
-      iterations[cb] = 0;
-    }
-    __syncthreads();
-    return;
-  }
-  int cb_len = max(input_size + 2 * kZ384, (Kb + 4) * kZ384);
-  cb_len     = ((cb_len + kZ384 - 1) / kZ384) * kZ384;
-  const int nof_layers = min(cb_len / kZ384 - Kb, nrows);
-
-  int order = 24;
-  if (crc_poly == PG_CRC16) {
-    order = 16;
-  }
-  const uint32_t* pow_tab = crc_pow + (size_t)(crc_poly <= PG_CRC24B ? crc_poly : 0) * pg::kCrcPowLen;
-  const int       crc_len = msg_len - (int)d.nof_filler_bits;
+  // Messages: behind the columns of the rows that run (the columns past them hold only zeros).
+  const uint32_t o_msg   = kPairTabBytes + ((h4 * (uint32_t)(1 + Kb + nof_layers) + 15u) & ~15u);
+  const uint32_t msg_len_bytes = 4u * (uint32_t)nta * tb.msg0[LG][g][nof_layers];
+  uint32_t* msg = (o_msg + msg_len_bytes <= smem_bytes ? reinterpret_cast<uint32_t*>(smem + o_msg) : slab);
 
   int       result = 0;
   const int max_it = d.max_iterations;
   const int lane   = tid & 31;
-  const int nsteps = steps_for_layers(g, nof_layers);
+  const int tpart  = tid % T;
+  const int cgrp   = tid / H; // column group of the hard-decision phase
+  const int ngrp   = NT / H;
+  const uint32_t tpart16 = 16u * (uint32_t)tpart;
+  const float jf   = (float)jp; // lane pair, its byte offset and -4 H as denormals (pair_edge)
+  const float j4d  = __uint_as_float(4u * jp);
+  const float nh4d = __uint_as_float(0x80000000u | h4);
   for (int it = 0; it < max_it; ++it) {
-    for (int st = 0; st < nsteps; ++st) {
-      if (it > 0 || st + 1 == nsteps) {
-        prefetch_step(g, st + 1 < nsteps ? st + 1 : 0, nof_layers, tid, reinterpret_cast<const char*>(c2v),
-                      kZH * 2);
-      }
-      const int r0 = c_step_row0[g][st];
-      const int r1 = min(r0 + (int)c_step_nrows[g][st], nof_layers);
-      for (int r = r0; r < r1; ++r) {
-        const int deg     = c_row_deg[g][r];
-        const int e0      = c_row_e0[g][r];
-        uint16_t* c2v_row = c2v + (size_t)e0 * kZH + jp;
-        if (T == 1) {
-          if (it == 0) {
-            row_dispatch_z<true>(deg, zt, e0, j4, E, c2v_row);
-          } else {
-            row_dispatch_z<false>(deg, zt, e0, j4, E, c2v_row);
-          }
+    if (tid < nta) {
+      for (int r = 0; r < nof_layers; ++r) {
+        const uint4  rd = sh.row[r];
+        const int    ne = (int)rd.z;
+        uint32_t*    mr = msg + rd.y;
+        if (it > 0) {
+          pair_row_dispatch<false, T>(ne, tpart16, rd.x, jf, j4d, nh4d, mr, active);
+        } else if (!ragged) {
+          pair_row_dispatch<true, T>(ne, tpart16, rd.x, jf, j4d, nh4d, mr, active);
         } else {
-          if (it == 0) {
-            row_dispatch_z_split<true>(deg, zt, e0, j4, tp, E, c2v_row);
-          } else {
-            row_dispatch_z_split<false>(deg, zt, e0, j4, tp, E, c2v_row);
+          pair_row_ragged<T>(ne, rd.x + tpart16 * ne, jf, j4d, nh4d, mr + tid * ((ne + 1) / 2), active);
+        }
+        if (rd.w != 0 && r + 1 < nof_layers) {
+          asm volatile("bar.sync 1, %0;" ::"r"(nta) : "memory");
+        }
+      }
+    }
+    __syncthreads();
+
+    // Hard decisions (soft <= 0), zero check and CRC: lane pair k of every ngrp-th message column; each
+    // set bit within the CRC length adds x^e mod g.
+    bool     zero = false;
+    uint32_t crc  = 0;
+    if (cgrp < ngrp) {
+      const int       k  = tid - cgrp * H;
+      const uint32_t* Ec = reinterpret_cast<const uint32_t*>(E) + H + k;
+#pragma unroll 4
+      for (int c = cgrp; c < Kb; c += ngrp) {
+        const uint32_t x  = Ec[c * H];
+        const int      i0 = c * Z + k, i1 = i0 + H;
+        zero |= (x & 0x7fffu) == 0 || (x & 0x7fff0000u) == 0;
+        if (crc_poly != PG_CRC_NONE) {
+          if (pair_hard(x & 0xffffu) && i0 < crc_len) {
+            crc ^= __ldg(pow_tab + (crc_len - 1 - i0 + order));
+          }
+          if (pair_hard(x >> 16) && i1 < crc_len) {
+            crc ^= __ldg(pow_tab + (crc_len - 1 - i1 + order));
           }
         }
       }
-      __syncthreads();
     }
-
-    // Hard decisions (soft <= 0), zero check and CRC: one 32-bit word per warp step, lane k
-    // holding bit 32 wi + k (MSB first after the reversal); message bit i of column c = i / 384,
-    // lane w = i mod 384 is half (w >= 192) of E[c][w mod 192].
-    int      zero = 0;
-    uint32_t crc  = 0;
-    for (int wi = tid >> 5; wi < nwords; wi += NT / 32) {
-      const int      idx = 32 * wi + lane;
-      const int      col = idx / kZ384;
-      const int      w   = idx - col * kZ384;
-      const uint32_t x   = sm.E[col * kZH + (w < kZH ? w : w - kZH)];
-      const uint32_t h   = w < kZH ? (x & 0xffffu) : (x >> 16);
-      const bool     bit = z_hard(h);
-      zero |= (h & 0x7fffu) == 0;
-      const uint32_t wd = __brev(__ballot_sync(0xffffffffu, bit));
-      if (lane == 0) {
-        sm.hard[wi] = wd;
-      }
-      if (crc_poly != PG_CRC_NONE && bit && idx < crc_len) {
-        crc ^= __ldg(pow_tab + (crc_len - 1 - idx + order));
-      }
-    }
-    zero = __syncthreads_or(zero);
-    crc  = warp_xor(crc);
+    crc  = __reduce_xor_sync(0xffffffffu, crc);
+    zero = __any_sync(0xffffffffu, zero);
     if (lane == 0) {
-      sm.red[tid >> 5] = crc;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      uint32_t t = 0;
-      for (int w = 0; w < NT / 32; ++w) {
-        t ^= sm.red[w];
+      if (crc != 0) {
+        atomicXor(&sh.crc[it & 1], crc);
       }
-      sm.s_done = (crc_poly != PG_CRC_NONE && !zero && t == 0) ? 1 : 0;
+      if (zero) {
+        sh.zero[it & 1] = 1;
+      }
     }
     __syncthreads();
-    if (sm.s_done) {
+    const bool done = crc_poly != PG_CRC_NONE && sh.zero[it & 1] == 0 && sh.crc[it & 1] == 0;
+    if (tid == 0) {
+      sh.crc[(it + 1) & 1]  = 0; // last read before this iteration's rows
+      sh.zero[(it + 1) & 1] = 0;
+    }
+    if (done) {
       result = it + 1;
       break;
     }
   }
 
   if (crc_poly == PG_CRC_NONE) {
-    // Syndrome check over the processed rows (ldpc_decoder_impl.cpp:329-387), both lanes.
-    int bad = 0;
-    int e0  = 0;
-    for (int r = 0; r < nof_layers && tid < kZH; ++r) {
-      const int deg    = c_row_deg[g][r];
-      uint32_t  parity = 0;
-      for (int e = 0; e < deg; ++e) {
-        uint32_t a, s;
-        z_edge(zt, e0 + e, 4u * (uint32_t)tid, a, s);
-        const uint32_t x  = __byte_perm(lds_u32(E, a), 0, s);
-        const uint32_t lo = x & 0xffffu, hi = x >> 16;
-        bad |= ((lo & 0x7fffu) == 0) | ((hi & 0x7fffu) == 0);
-        parity ^= (uint32_t)z_hard(lo) | ((uint32_t)z_hard(hi) << 1);
+    // Syndrome check over the processed rows (ldpc_decoder_impl.cpp:329-387), both lanes (the padding
+    // edges read a positive soft bit). A zero soft bit of a row or of the message fails too.
+    int bad = max_it > 0 ? sh.zero[(max_it - 1) & 1] : 1;
+    if (active && tpart == 0) {
+      for (int r = 0; r < nof_layers; ++r) {
+        const uint4 rd     = sh.row[r];
+        uint32_t    parity = 0;
+        for (int e = 0; e < (int)rd.z * T; ++e) {
+          uint32_t a, s;
+          pair_edge(lds_v4(rd.x + 16 * e), jf, j4d, nh4d, a, s);
+          const uint32_t x = __byte_perm(lds_u32(a), 0, s);
+          bad |= ((x & 0x7fffu) == 0) | ((x & 0x7fff0000u) == 0);
+          parity ^= (uint32_t)pair_hard(x & 0xffffu) | ((uint32_t)pair_hard(x >> 16) << 1);
+        }
+        bad |= parity != 0;
       }
-      bad |= parity != 0;
-      e0 += deg;
     }
-    bad      = __syncthreads_or(bad);
-    int zero = 0;
-    for (int i = tid; i < msg_len; i += NT) {
-      const int      col = i / kZ384;
-      const int      w   = i - col * kZ384;
-      const uint32_t x   = sm.E[col * kZH + (w < kZH ? w : w - kZH)];
-      zero |= (((w < kZH ? x : x >> 16) & 0x7fffu) == 0);
-    }
-    zero   = __syncthreads_or(zero);
-    result = (!bad && !zero) ? max_it : 0;
+    bad    = __syncthreads_or(bad);
+    result = !bad ? max_it : 0;
   }
 
-  for (int b = tid; b < nbytes; b += NT) {
-    out[b] = (uint8_t)(sm.hard[b >> 2] >> (24 - 8 * (b & 3)));
+  // Decoded bits: one 32-bit word per warp step, lane k holding bit 32 wi + k (MSB first after the
+  // reversal); message bit i of column c = i / Z, lane w = i mod Z is half (w >= H) of E[c][w mod H].
+  {
+    const uint32_t inv = 0xffffffffu / (uint32_t)Z + 1u;
+    for (int wi = tid >> 5; wi < (msg_len + 31) / 32; wi += NT / 32) {
+      const int idx = 32 * wi + lane;
+      bool      bit = false;
+      if (idx < msg_len) {
+        const int      col = (int)__umulhi((uint32_t)idx, inv);
+        const int      w   = idx - col * Z;
+        const uint32_t x   = reinterpret_cast<const uint32_t*>(E)[H + col * H + (w < H ? w : w - H)];
+        bit                = pair_hard(w < H ? (x & 0xffffu) : (x >> 16));
+      }
+      const uint32_t wd = __brev(__ballot_sync(0xffffffffu, bit));
+      if (lane < 4 && 4 * wi + lane < nbytes) {
+        out[4 * wi + lane] = (uint8_t)(wd >> (24 - 8 * lane));
+      }
+    }
   }
   if (tid == 0) {
     iterations[cb] = result;
   }
-  __syncthreads();
 }
 
-constexpr size_t kZSmem = sizeof(smem_z_t) > kX2Smem ? sizeof(smem_z_t) : kX2Smem;
+constexpr int kPairThreads = 384;
+constexpr int kPairPerSm   = 2;
+constexpr int kPairMaxSmem = 227 * 1024 - (((int)sizeof(pair_shared) + 15) & ~15); // dynamic, one CTA per SM
 
-// Persistent decoder of a work list, every lifting size: Z = 384 through decode_codeblock_z384,
-// other even Z > 192 in pair mode, Z <= 192 with the one-lane arithmetic (192 threads, four CTAs
-// per SM).
-__global__ void __launch_bounds__(kZThreads, kZMaxPerSm) ldpc_decode_z_kernel(const pg_ldpc_cb* __restrict__ descs,
-                                                                      const int8_t* __restrict__ llrs,
-                                                                      uint8_t* __restrict__ bits,
-                                                                      int32_t* __restrict__ iterations,
-                                                                      int8_t* __restrict__ c2v_all,
-                                                                      const uint32_t* __restrict__ crc_pow,
-                                                                      const uint16_t* __restrict__ scale_tab,
-                                                                      const uint32_t* __restrict__ order, int n,
-                                                                      int* __restrict__ counter)
+// Dynamic shared memory of a launch with per_sm CTAs on each SM (228 KB, 1 KB of it reserved per CTA).
+int pair_smem(int per_sm)
 {
-  extern __shared__ __align__(16) unsigned char smem_z_raw[];
-  __shared__ int   s_work;
-  __shared__ uint4 s_ztab[2 * pg::kBg1Edges];
-  z_load_edge_tables(s_ztab);
-  for (;;) {
-    if (threadIdx.x == 0) {
-      s_work = atomicAdd(counter, 1);
-    }
-    __syncthreads();
-    const int w = s_work;
-    __syncthreads();
-    if (w >= n) {
-      break;
-    }
+  const int share = 228 * 1024 / per_sm - 1024 - (((int)sizeof(pair_shared) + 15) & ~15);
+  return std::min(share, kPairMaxSmem) & ~127;
+}
+static_assert(kPairMinSmem + 2048 <= 228 * 1024 / kPairPerSm, "every column fits next to the other CTAs");
+
+// Persistent decoder of a work list, every lifting size: each CTA takes codeblock order[w] (or w), w
+// its own index first, then from *counter (zero before the launch when n exceeds the grid). Two
+// threads per lane pair above Z = 192, four below; odd lifting sizes (Z <= 15) with the one-lane
+// arithmetic.
+//
+// Bound: at 512 codeblocks the ALU pipe and latency (24 warps per SM), with few codeblocks latency
+// alone (12 warps). B200, against the kernel this one replaced (two lanes per thread, one thread per
+// lane pair, Z = 384 only, messages in L2): 512 codeblocks BG1/BG2 Z = 384, 0.528 -> 0.364 ms; 6
+// codeblocks BG1 Z = 384, 257 -> 155 us; 200 codeblocks of many sizes, 302 -> 190 us. One thread per
+// lane pair (192 threads, three CTAs per SM) took 0.415 ms, 200 us and 268 us.
+__global__ void __launch_bounds__(kPairThreads, kPairPerSm)
+    ldpc_decode_pair_kernel(const pg_ldpc_cb* __restrict__ descs, const int8_t* __restrict__ llrs,
+                            uint8_t* __restrict__ bits, int32_t* __restrict__ iterations, int8_t* __restrict__ c2v_all,
+                            const uint32_t* __restrict__ crc_pow, const uint32_t* __restrict__ order, int n,
+                            int* __restrict__ counter, uint32_t smem_bytes)
+{
+  extern __shared__ __align__(16) unsigned char smem_pair[];
+  __shared__ pair_shared sh;
+  constexpr int NT   = kPairThreads;
+  uint32_t*     slab = reinterpret_cast<uint32_t*>(c2v_all + (size_t)blockIdx.x * pg::kPairSlab);
+  for (int w = blockIdx.x; w < n;) {
     const int        cb = order != nullptr ? (int)order[w] : w;
     const pg_ldpc_cb d  = descs[cb];
-    if (d.lifting_size == kZ384) {
-      decode_codeblock_z384<kZThreads>(d, *reinterpret_cast<smem_z_t*>(smem_z_raw), s_ztab, llrs, bits, iterations,
-                                       c2v_all, crc_pow, cb, blockIdx.x);
-    } else if (d.lifting_size > kX2Threads) {
-      decode_codeblock_pair<kX2Threads, 1>(d, *reinterpret_cast<smem_pair_t*>(smem_z_raw), llrs, bits, iterations,
-                                           c2v_all, crc_pow, scale_tab, cb, blockIdx.x);
+    const int        Z  = d.lifting_size;
+    if ((Z & 1) != 0 || Z < 2 || Z > pg::kMaxZ) {
+      if (Z < kOddMaxZ) {
+        decode_codeblock<0, NT, kOddMaxZ>(d, *reinterpret_cast<smem_scalar_t<NT, kOddMaxZ>*>(smem_pair), llrs, bits,
+                                          iterations, reinterpret_cast<int8_t*>(slab), crc_pow, cb, 0);
+      } else if (threadIdx.x == 0) {
+        iterations[cb] = -1;
+      }
+    } else if (Z <= NT / 2) {
+      decode_codeblock_pair<4, NT>(d, sh, smem_pair, smem_bytes, llrs, bits, iterations, slab, crc_pow, cb);
     } else {
-      decode_codeblock<0, kX2Threads, kX2Threads>(d, *reinterpret_cast<smem_x2_scalar_t*>(smem_z_raw), llrs, bits,
-                                                  iterations, c2v_all, crc_pow, cb, blockIdx.x);
-      __syncthreads();
+      decode_codeblock_pair<2, NT>(d, sh, smem_pair, smem_bytes, llrs, bits, iterations, slab, crc_pow, cb);
     }
-  }
-}
-
-// The Z = 384 decoder with two threads per lane pair (384 threads, two CTAs per SM): each row's
-// edges are split between the pair, which halves the latency of a layer, for batches whose time is
-// set by their slowest codeblocks. Other lifting sizes as ldpc_decode_split_kernel.
-constexpr int    kZsThreads  = 2 * kZH;
-constexpr int    kZsMaxPerSm = 2;
-constexpr size_t kZsSmem     = std::max(sizeof(smem_z_nt_t<kZsThreads>), kSplitSmem);
-
-__global__ void __launch_bounds__(kZsThreads, kZsMaxPerSm) ldpc_decode_zs_kernel(
-    const pg_ldpc_cb* __restrict__ descs, const int8_t* __restrict__ llrs, uint8_t* __restrict__ bits,
-    int32_t* __restrict__ iterations, int8_t* __restrict__ c2v_all, const uint32_t* __restrict__ crc_pow,
-    const uint16_t* __restrict__ scale_tab, const uint32_t* __restrict__ order, int n, int* __restrict__ counter)
-{
-  extern __shared__ __align__(16) unsigned char smem_zs_raw[];
-  __shared__ int   s_work;
-  __shared__ uint4 s_ztab[2 * pg::kBg1Edges];
-  z_load_edge_tables(s_ztab);
-  for (;;) {
-    if (threadIdx.x == 0) {
-      s_work = atomicAdd(counter, 1);
-    }
-    __syncthreads();
-    const int w = s_work;
-    __syncthreads();
-    if (w >= n) {
+    if (n <= (int)gridDim.x) {
       break;
     }
-    const int        cb = order != nullptr ? (int)order[w] : w;
-    const pg_ldpc_cb d  = descs[cb];
-    if (d.lifting_size == kZ384) {
-      decode_codeblock_z384<kZsThreads>(d, *reinterpret_cast<smem_z_nt_t<kZsThreads>*>(smem_zs_raw), s_ztab, llrs,
-                                        bits, iterations, c2v_all, crc_pow, cb, blockIdx.x);
-    } else if (d.lifting_size > kX2Threads && (d.lifting_size & 1) == 0) {
-      decode_codeblock_pair<kSplitThreads, 2>(d, *reinterpret_cast<smem_split_pair_t*>(smem_zs_raw), llrs, bits,
-                                              iterations, c2v_all, crc_pow, scale_tab, cb, blockIdx.x);
-    } else {
-      decode_codeblock<0, kSplitThreads, pg::kMaxZ>(d, *reinterpret_cast<smem_split_scalar_t*>(smem_zs_raw), llrs,
-                                                    bits, iterations, c2v_all, crc_pow, cb, blockIdx.x);
-      __syncthreads();
-    }
-  }
-}
-
-// Persistent decoder of a work list, every lifting size: each CTA takes the next work index from
-// *counter, decodes codeblock order[w] (or w) in pair mode (even Z > 192) or scalar mode (Z <= 192)
-// with slab blockIdx.x, and stops when the n codeblocks are taken.
-__global__ void __launch_bounds__(kX2Threads, kX2MaxPerSm) ldpc_decode_x2_kernel(const pg_ldpc_cb* __restrict__ descs,
-                                                                        const int8_t* __restrict__ llrs,
-                                                                        uint8_t* __restrict__ bits,
-                                                                        int32_t* __restrict__ iterations,
-                                                                        int8_t* __restrict__ c2v_all,
-                                                                        const uint32_t* __restrict__ crc_pow,
-                                                                        const uint16_t* __restrict__ scale_tab,
-                                                                        const uint32_t* __restrict__ order, int n,
-                                                                        int* __restrict__ counter)
-{
-  extern __shared__ __align__(16) unsigned char smem_x2_raw[];
-  __shared__ int s_work;
-  for (;;) {
+    __syncthreads();
     if (threadIdx.x == 0) {
-      s_work = atomicAdd(counter, 1);
+      sh.work = (int)gridDim.x + atomicAdd(counter, 1);
     }
     __syncthreads();
-    const int w = s_work;
-    __syncthreads();
-    if (w >= n) {
-      break;
-    }
-    const int        cb = order != nullptr ? (int)order[w] : w;
-    const pg_ldpc_cb d  = descs[cb];
-    if (d.lifting_size > kX2Threads) {
-      decode_codeblock_pair<kX2Threads, 1>(d, *reinterpret_cast<smem_pair_t*>(smem_x2_raw), llrs, bits, iterations,
-                                           c2v_all, crc_pow, scale_tab, cb, blockIdx.x);
-    } else {
-      decode_codeblock<0, kX2Threads, kX2Threads>(d, *reinterpret_cast<smem_x2_scalar_t*>(smem_x2_raw), llrs, bits,
-                                                  iterations, c2v_all, crc_pow, cb, blockIdx.x);
-      __syncthreads();
-    }
+    w = sh.work;
   }
 }
-
-// Persistent split decoder of a work list, every lifting size: 384 threads per codeblock, pair mode
-// with two threads per lane pair for even Z > 192, the one-lane arithmetic otherwise.
-__global__ void __launch_bounds__(kSplitThreads, kSplitMaxPerSm) ldpc_decode_split_kernel(
-    const pg_ldpc_cb* __restrict__ descs, const int8_t* __restrict__ llrs, uint8_t* __restrict__ bits,
-    int32_t* __restrict__ iterations, int8_t* __restrict__ c2v_all, const uint32_t* __restrict__ crc_pow,
-    const uint16_t* __restrict__ scale_tab, const uint32_t* __restrict__ order, int n, int* __restrict__ counter)
-{
-  extern __shared__ __align__(16) unsigned char smem_split_raw[];
-  __shared__ int s_work;
-  for (;;) {
-    if (threadIdx.x == 0) {
-      s_work = atomicAdd(counter, 1);
-    }
-    __syncthreads();
-    const int w = s_work;
-    __syncthreads();
-    if (w >= n) {
-      break;
-    }
-    const int        cb = order != nullptr ? (int)order[w] : w;
-    const pg_ldpc_cb d  = descs[cb];
-    if (d.lifting_size > kX2Threads && (d.lifting_size & 1) == 0) {
-      decode_codeblock_pair<kSplitThreads, 2>(d, *reinterpret_cast<smem_split_pair_t*>(smem_split_raw), llrs, bits,
-                                              iterations, c2v_all, crc_pow, scale_tab, cb, blockIdx.x);
-    } else if (d.lifting_size == 384) {
-      decode_codeblock<384, kSplitThreads, pg::kMaxZ>(d, *reinterpret_cast<smem_split_scalar_t*>(smem_split_raw), llrs,
-                                                      bits, iterations, c2v_all, crc_pow, cb, blockIdx.x);
-      __syncthreads();
-    } else {
-      decode_codeblock<0, kSplitThreads, pg::kMaxZ>(d, *reinterpret_cast<smem_split_scalar_t*>(smem_split_raw), llrs,
-                                                    bits, iterations, c2v_all, crc_pow, cb, blockIdx.x);
-      __syncthreads();
-    }
-  }
-}
-
 
 // Longest-first work order of a batch for the persistent decoders. A codeblock's expected decoding
 // time is its work per iteration (the edges of the check rows its input reaches, as the decoder
@@ -1904,67 +1408,7 @@ int ldpc_upload_tables(pg_context* ctx)
   for (int r = 0; r < PG_BG2_ROWS; ++r) {
     deg[1][r] = PG_BG2_ROW_DEG[r];
   }
-  // Scale table of the two-lanes-per-thread decoder: f16 bits of (m * 52428) >> 16 at (f16 bits of
-  // m) >> 4, m = 0 .. 127.
-  uint16_t scale[kScaleTab] = {};
-  for (int m = 0; m <= 127; ++m) {
-    const uint16_t key = __half_as_ushort(__float2half_rn((float)m)) >> 4;
-    scale[key]         = __half_as_ushort(__float2half_rn((float)((m * 52428) >> 16)));
-  }
-  // Edge tables of the Z = 384 decoder (lifting set index 1): 4 (s mod 192), the column's byte
-  // offset in the f16-pair soft bits and the byte-permute selector of the wrapped case (halves
-  // swapped unless s >= 192).
-  uint32_t z_sp4[2][kBg1Edges] = {}, z_col[2][kBg1Edges] = {}, z_sel[2][kBg1Edges] = {};
-  for (int gi = 0; gi < 2; ++gi) {
-    const int ne = gi == 0 ? PG_BG1_EDGES : PG_BG2_EDGES;
-    for (int e = 0; e < ne; ++e) {
-      const uint32_t s = (uint32_t)v[gi][e][1] % (uint32_t)kZ384;
-      z_sp4[gi][e]     = 4u * (s % (uint32_t)kZH);
-      z_col[gi][e]     = 4u * (uint32_t)kZH * col[gi][e];
-      z_sel[gi][e]     = s >= (uint32_t)kZH ? 0x3210u : 0x1032u;
-    }
-  }
   int rc = check_cuda(ctx, cudaMemcpyToSymbol(c_edge_col, col, sizeof(col)), "cudaMemcpyToSymbol(edge_col)");
-  if (rc == PG_OK) {
-    rc = check_cuda(ctx, cudaMemcpyToSymbol(c_z_sp4, z_sp4, sizeof(z_sp4)), "cudaMemcpyToSymbol(z_sp4)");
-  }
-  if (rc == PG_OK) {
-    rc = check_cuda(ctx, cudaMemcpyToSymbol(c_z_col, z_col, sizeof(z_col)), "cudaMemcpyToSymbol(z_col)");
-  }
-  if (rc == PG_OK) {
-    rc = check_cuda(ctx, cudaMemcpyToSymbol(c_z_sel, z_sel, sizeof(z_sel)), "cudaMemcpyToSymbol(z_sel)");
-  }
-  if (rc == PG_OK) {
-    rc = check_cuda(ctx,
-                    cudaFuncSetAttribute(ldpc_decode_z_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kZSmem),
-                    "cudaFuncSetAttribute(ldpc_decode_z_kernel)");
-  }
-  if (rc == PG_OK) {
-    rc = check_cuda(ctx,
-                    cudaFuncSetAttribute(ldpc_decode_zs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kZsSmem),
-                    "cudaFuncSetAttribute(ldpc_decode_zs_kernel)");
-  }
-  if (rc == PG_OK) {
-    rc = check_cuda(ctx, cudaMalloc(&ctx->dev.ldpc_scale, sizeof(scale)), "cudaMalloc(scale table)");
-  }
-  if (rc == PG_OK) {
-    rc = check_cuda(ctx, cudaMemcpy(ctx->dev.ldpc_scale, scale, sizeof(scale), cudaMemcpyHostToDevice),
-                    "cudaMemcpy(scale table)");
-  }
-  if (rc == PG_OK) {
-    rc = check_cuda(ctx,
-                    cudaFuncSetAttribute(ldpc_decode_x2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kX2Smem),
-                    "cudaFuncSetAttribute(ldpc_decode_x2_kernel)");
-  }
-  if (rc == PG_OK) {
-    rc = check_cuda(ctx,
-                    cudaFuncSetAttribute(ldpc_decode_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kSplitSmem),
-                    "cudaFuncSetAttribute(ldpc_decode_split_kernel)");
-  }
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaMemcpyToSymbol(c_edge_v, v, sizeof(v)), "cudaMemcpyToSymbol(edge_v)");
   }
@@ -2012,6 +1456,37 @@ int ldpc_upload_tables(pg_context* ctx)
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaMemcpyToSymbol(c_row_e0, row_e0, sizeof(row_e0)), "cudaMemcpyToSymbol(row_e0)");
   }
+  static pair_tables pt; // the same values in every call
+  for (int gi = 0; gi < 2; ++gi) {
+    const int rows = gi == 0 ? PG_BG1_ROWS : PG_BG2_ROWS;
+    for (int r = 0; r < rows; ++r) {
+      pt.row_deg[gi][r]    = deg[gi][r];
+      pt.row_e0[gi][r + 1] = row_e0[gi][r + 1];
+      for (int e = row_e0[gi][r]; e < row_e0[gi][r + 1]; ++e) {
+        pt.edge_row[gi][e] = (uint8_t)r;
+        pt.edge_col[gi][e] = col[gi][e];
+        std::copy(v[gi][e], v[gi][e] + 8, pt.edge_v[gi][e]);
+      }
+      for (int lg = 0; lg < 2; ++lg) {
+        const int t                = 2 << lg;
+        const int ne               = (deg[gi][r] + t - 1) / t;
+        pt.pad_e0[lg][gi][r + 1]   = (uint16_t)(pt.pad_e0[lg][gi][r] + ne * t);
+        pt.msg0[lg][gi][r + 1]     = (uint16_t)(pt.msg0[lg][gi][r] + (ne + 1) / 2);
+      }
+    }
+    for (int st = 0; st < nsteps[gi]; ++st) {
+      pt.row_sync[gi][step_row0[gi][st] + step_nrows[gi][st] - 1] = 1;
+    }
+  }
+  if (rc == PG_OK) {
+    rc = check_cuda(ctx, cudaMemcpyToSymbol(g_pair_tables, &pt, sizeof(pt)), "cudaMemcpyToSymbol(pair tables)");
+  }
+  if (rc == PG_OK) {
+    rc = check_cuda(ctx,
+                    cudaFuncSetAttribute(ldpc_decode_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         kPairMaxSmem),
+                    "cudaFuncSetAttribute(ldpc_decode_pair_kernel)");
+  }
   if (rc == PG_OK) {
     // Device address of the static scratch on this context's device (current here), looked up
     // once so that the static-scratch entry makes no runtime call besides its launch.
@@ -2027,17 +1502,35 @@ int ldpc_launch(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_
   return ldpc_launch_scratch(ctx, descs_dev, n, llrs, bits, iterations, ctx->dev.c2v, stream);
 }
 
+// CTAs of the decoder the context's batch decodes launch for n codeblocks: one per SM up to one and a half
+// codeblocks per SM (their messages then stay in shared memory: 200 codeblocks of many sizes 234 us
+// against 245 with two per SM), two per SM above (512 codeblocks 378 us against 462 with one).
+static int batch_ctas(const pg_context* ctx, int n)
+{
+  const int per_sm = ctx->ldpc_ctas_per_sm > 0 ? ctx->ldpc_ctas_per_sm : (2 * n <= 3 * ctx->sm_count ? 1 : kPairPerSm);
+  return std::min(n, ldpc_max_ctas(ctx, per_sm, ctx->ldpc_kernel));
+}
+
+int ldpc_max_ctas(const pg_context* ctx, int per_sm, int kernel)
+{
+  return kernel == PG_LDPC_KERNEL_ONE_LANE ? std::min(per_sm * ctx->sm_count, ctx->ldpc_ctas)
+                                           : std::min(per_sm, kPairPerSm) * ctx->sm_count;
+}
+
 int ldpc_launch_scratch(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* bits,
                         int32_t* iterations, int8_t* c2v, cudaStream_t stream)
 {
+  const int       ctas  = batch_ctas(ctx, n);
   const uint32_t* order = nullptr;
-  if (ctx->ldpc_order_mode == PG_LDPC_ORDER_LONGEST_FIRST && n > 1 && n <= ctx->max_codeblocks) {
+  // With a CTA for every codeblock all start at once, and their order decides nothing.
+  if (ctx->ldpc_order_mode == PG_LDPC_ORDER_LONGEST_FIRST && n > ctas && n <= ctx->max_codeblocks) {
     if (int rc = ldpc_order_launch(ctx, descs_dev, n, llrs, ctx->dev.ldpc_keys, ctx->dev.ldpc_order, stream)) {
       return rc;
     }
     order = ctx->dev.ldpc_order;
   }
-  return ldpc_launch_persistent(ctx, descs_dev, n, llrs, bits, iterations, c2v, order, ctx->dev.ldpc_counter, stream);
+  return ldpc_launch_persistent(ctx, descs_dev, n, llrs, bits, iterations, c2v, order, ctx->dev.ldpc_counter, stream,
+                                ctas, ctx->ldpc_kernel);
 }
 
 int ldpc_order_launch(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* keys,
@@ -2079,58 +1572,30 @@ int ldpc_resident_ctas(pg_context* ctx)
 
 int ldpc_launch_persistent(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* bits,
                            int32_t* iterations, int8_t* c2v, const uint32_t* order, int* counter,
-                           cudaStream_t stream)
-{
-  const int per_sm = ctx->ldpc_ctas_per_sm > 0 ? ctx->ldpc_ctas_per_sm : kX2MaxPerSm;
-  return ldpc_launch_persistent(ctx, descs_dev, n, llrs, bits, iterations, c2v, order, counter, stream,
-                                per_sm * ctx->sm_count, PG_LDPC_KIND_ALL | ldpc_route(ctx->ldpc_kernel));
-}
-
-int ldpc_launch_persistent(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* bits,
-                           int32_t* iterations, int8_t* c2v, const uint32_t* order, int* counter,
-                           cudaStream_t stream, int max_ctas, int kinds)
+                           cudaStream_t stream, int max_ctas, int kernel)
 {
   if (n == 0) {
     return PG_OK;
   }
-  if (int rc = check_cuda(ctx, cudaMemsetAsync(counter, 0, 2 * sizeof(int), stream), "cudaMemsetAsync(ldpc counter)")) {
-    return rc;
+  const int grid = std::max(1, std::min(n, max_ctas));
+  if (n > grid || kernel == PG_LDPC_KERNEL_ONE_LANE) {
+    if (int rc = check_cuda(ctx, cudaMemsetAsync(counter, 0, sizeof(int), stream), "cudaMemsetAsync(ldpc counter)")) {
+      return rc;
+    }
   }
   const unsigned int rec_flags = timing_record_flags(ctx, stream);
   if (ctx->timed) {
     cudaEventRecordWithFlags(ctx->ev_start, stream, rec_flags);
   }
-  // PG_LDPC_ROUTE_Z: the Z = 384 kernel (three per SM, pair mode and one-lane arithmetic for the
-  // other lifting sizes);
-  // PG_LDPC_ROUTE_SPLIT: the split kernel decodes every codeblock (two CTAs per SM);
-  // PG_LDPC_ROUTE_X2: the two-lanes-per-thread kernel (four per SM); neither: ldpc_decode_kernel
-  // (two per SM). The caller provides a slab per CTA (min(n, max_ctas) slabs, max_ctas <= four
-  // per SM).
   int rc = PG_OK;
-  if (kinds & PG_LDPC_ROUTE_ZS) {
-    const int grid_zs = std::max(1, std::min(n, std::min(max_ctas, kZsMaxPerSm * ctx->sm_count)));
-    ldpc_decode_zs_kernel<<<grid_zs, kZsThreads, kZsSmem, stream>>>(
-        descs_dev, llrs, bits, iterations, c2v, ctx->dev.crc_pow, ctx->dev.ldpc_scale, order, n, counter + 1);
-    rc = check_cuda(ctx, cudaGetLastError(), "ldpc_decode_zs_kernel launch");
-  } else if (kinds & PG_LDPC_ROUTE_Z) {
-    const int grid_z = std::max(1, std::min(n, std::min(max_ctas, kZResidentPerSm * ctx->sm_count)));
-    ldpc_decode_z_kernel<<<grid_z, kZThreads, kZSmem, stream>>>(
-        descs_dev, llrs, bits, iterations, c2v, ctx->dev.crc_pow, ctx->dev.ldpc_scale, order, n, counter + 1);
-    rc = check_cuda(ctx, cudaGetLastError(), "ldpc_decode_z_kernel launch");
-  } else if (kinds & PG_LDPC_ROUTE_SPLIT) {
-    const int grid_s = std::max(1, std::min(n, std::min(max_ctas, kSplitMaxPerSm * ctx->sm_count)));
-    ldpc_decode_split_kernel<<<grid_s, kSplitThreads, kSplitSmem, stream>>>(
-        descs_dev, llrs, bits, iterations, c2v, ctx->dev.crc_pow, ctx->dev.ldpc_scale, order, n, counter + 1);
-    rc = check_cuda(ctx, cudaGetLastError(), "ldpc_decode_split_kernel launch");
-  } else if (kinds & PG_LDPC_ROUTE_X2) {
-    const int grid_x2 = std::max(1, std::min(n, std::min(max_ctas, kX2MaxPerSm * ctx->sm_count)));
-    ldpc_decode_x2_kernel<<<grid_x2, kX2Threads, kX2Smem, stream>>>(
-        descs_dev, llrs, bits, iterations, c2v, ctx->dev.crc_pow, ctx->dev.ldpc_scale, order, n, counter + 1);
-    rc = check_cuda(ctx, cudaGetLastError(), "ldpc_decode_x2_kernel launch");
+  if (kernel != PG_LDPC_KERNEL_ONE_LANE) {
+    const int smem = pair_smem((grid + ctx->sm_count - 1) / ctx->sm_count);
+    ldpc_decode_pair_kernel<<<grid, kPairThreads, smem, stream>>>(descs_dev, llrs, bits, iterations, c2v,
+                                                                  ctx->dev.crc_pow, order, n, counter, (uint32_t)smem);
+    rc = check_cuda(ctx, cudaGetLastError(), "ldpc_decode_pair_kernel launch");
   } else {
-    const int grid = std::max(1, std::min(n, std::min(max_ctas, ctx->ldpc_ctas)));
     ldpc_decode_kernel<<<grid, kThreads, 0, stream>>>(descs_dev, llrs, bits, iterations, c2v, ctx->dev.crc_pow, order,
-                                                      n, counter, 0);
+                                                      n, counter);
     rc = check_cuda(ctx, cudaGetLastError(), "ldpc_decode_kernel launch");
   }
   if (ctx->timed) {
@@ -2193,7 +1658,7 @@ extern "C" int pg_ldpc_decode_batch_static_scratch(pg_context* ctx, const pg_ldp
     cudaEventRecordWithFlags(ctx->ev_start, s, rec_flags);
   }
   ldpc_decode_kernel<<<nof_cbs, kThreads, 0, s>>>(cbs_dev, llrs, bits, iterations, ctx->static_c2v, ctx->dev.crc_pow,
-                                                  nullptr, nof_cbs, nullptr, 0);
+                                                  nullptr, nof_cbs, nullptr);
   int rc = pg::check_cuda(ctx, cudaGetLastError(), "ldpc_decode_kernel launch (static scratch)");
   if (ctx->timed) {
     cudaEventRecordWithFlags(ctx->ev_stop, s, rec_flags);

@@ -277,10 +277,8 @@ int pg_create(const pg_config* cfg, pg_context** out)
     rc = check_cuda(ctx, cudaEventCreateWithFlags(&ctx->ev_desc, cudaEventDisableTiming), "cudaEventCreate");
   }
   if (rc == PG_OK) {
-    // One slab per resident decoder CTA: at most four per SM (two of twice the size for the Z = 384
-    // decoder), and at most one per codeblock.
-    rc = check_cuda(ctx,
-                    cudaMalloc(&ctx->dev.c2v, (size_t)std::max(cfg->max_codeblocks, 4 * ctx->sm_count) * kC2vStride),
+    // One slab per resident decoder CTA.
+    rc = check_cuda(ctx, cudaMalloc(&ctx->dev.c2v, (size_t)kLdpcSlabsPerSm * ctx->sm_count * kPairSlab),
                     "cudaMalloc(check-to-variable scratch)");
   }
   if (rc == PG_OK) {
@@ -393,7 +391,6 @@ void pg_destroy(pg_context* ctx)
   cudaFree(ctx->dev.ldpc_counter);
   cudaFree(ctx->dev.ldpc_keys);
   cudaFree(ctx->dev.ldpc_order);
-  cudaFree(ctx->dev.ldpc_scale);
   if (ctx->host_descs) {
     cudaFreeHost(ctx->host_descs);
   }

@@ -20,7 +20,11 @@ constexpr int kBg2Edges      = 197;
 constexpr int kMaxNodes      = 68;  // BG1 variable nodes before shortening
 constexpr int kMaxRowDegree  = 19;
 constexpr int kCrcPowLen     = 22 * kMaxZ + 64;  // x^e mod g for every exponent a codeblock CRC needs
-constexpr int kC2vStride     = kBg1Edges * kMaxZ; // check-to-variable bytes per codeblock
+constexpr int kC2vStride     = kBg1Edges * kMaxZ; // check-to-variable bytes per codeblock, one per edge and lane
+// Message slab of one lane-pair decoder CTA: BG1 at Z = 384 with its rows padded to two threads per
+// lane pair has 101 words per thread and 384 threads (155,136 bytes), the largest of its layouts.
+constexpr int kPairSlab      = 155648;
+constexpr int kLdpcSlabsPerSm = 2;      // decoder CTAs per SM, at most (both kernels)
 constexpr uint32_t kGoldWords = (14u * 3276u * 2u * 8u + 64u * 32u) / 32u + 2u; // Gold-sequence words per basis
 
 inline int kb_of(int bg) { return bg == 1 ? 22 : 10; }
@@ -66,7 +70,6 @@ struct device_buffers {
   int*         ldpc_counter = nullptr; // work counters of the persistent decoders (two ints)
   uint8_t*     ldpc_keys    = nullptr; // max_codeblocks work-order keys of the batch decodes
   uint32_t*    ldpc_order   = nullptr; // max_codeblocks work-order entries
-  uint16_t*    ldpc_scale   = nullptr; // scale table of the two-lanes-per-thread decoder
   size_t       llr_cap     = 0;
   size_t       bits_cap    = 0;
 };
@@ -261,43 +264,21 @@ int demap_launch(pg_context* ctx, int qm, int n, const float2* sym, const float*
 // Enqueues the batched decoder; descs_dev holds n descriptors in device memory.
 int ldpc_launch(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* bits,
                 int32_t* iterations, cudaStream_t stream);
-// Same with a caller-provided check-to-variable scratch of min(n, ldpc_ctas) * kC2vStride bytes.
+// Same with a caller-provided check-to-variable scratch of kLdpcSlabsPerSm * sm_count * kPairSlab bytes.
 int ldpc_launch_scratch(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* bits,
                         int32_t* iterations, int8_t* c2v, cudaStream_t stream);
 // Hardest-first work order (ldpc_score_kernel + ldpc_sort_kernel): keys n bytes, order n entries.
 int ldpc_order_launch(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* keys,
                       uint32_t* order, cudaStream_t stream);
-// Persistent launch: min(n, ldpc_ctas) CTAs take codeblocks order[0..n) (identity when order is
-// null) from *counter (device int, zeroed here on the stream); c2v holds one slab per CTA.
+// CTAs a launch of the kernel (pg_ldpc_kernel) may have with per_sm of them on each SM, within the
+// kernel's own limit.
+int ldpc_max_ctas(const pg_context* ctx, int per_sm, int kernel);
+// Persistent launch: min(n, max_ctas) CTAs (max_ctas from ldpc_max_ctas) take codeblocks order[0..n)
+// (identity when order is null) from *counter (device int, zeroed here on the stream); c2v holds one
+// slab (kPairSlab bytes) per CTA.
 int ldpc_launch_persistent(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* bits,
                            int32_t* iterations, int8_t* c2v, const uint32_t* order, int* counter,
-                           cudaStream_t stream);
-// Kinds of codeblocks a work list may hold: Z = 384 (two-lanes-per-thread decoder) and others.
-// PG_LDPC_ROUTE_X2 routes the Z = 384 codeblocks to the two-lanes-per-thread decoder; without it
-// ldpc_decode_kernel decodes every codeblock.
-enum {
-  PG_LDPC_KIND_OTHER  = 1,
-  PG_LDPC_KIND_Z384   = 2,
-  PG_LDPC_KIND_ALL    = 3,
-  PG_LDPC_ROUTE_X2    = 4,
-  PG_LDPC_ROUTE_SPLIT = 8,
-  PG_LDPC_ROUTE_Z     = 16,
-  PG_LDPC_ROUTE_ZS    = 32
-};
-// Route flags of a pg_ldpc_kernel value.
-inline int ldpc_route(int kernel)
-{
-  return kernel == PG_LDPC_KERNEL_TWO_LANES ? PG_LDPC_ROUTE_X2
-         : kernel == PG_LDPC_KERNEL_SPLIT   ? PG_LDPC_ROUTE_SPLIT
-         : kernel == PG_LDPC_KERNEL_Z384    ? PG_LDPC_ROUTE_Z
-         : kernel == PG_LDPC_KERNEL_Z384_SPLIT ? PG_LDPC_ROUTE_ZS
-                                            : 0;
-}
-// Same with at most max_ctas CTAs per decoder kernel, launching only the decoders of `kinds`.
-// counter: two device ints; c2v: one slab (kC2vStride bytes) per CTA.
-int ldpc_launch_persistent(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* bits,
-                           int32_t* iterations, int8_t* c2v, const uint32_t* order, int* counter,
-                           cudaStream_t stream, int max_ctas, int kinds);
+                           cudaStream_t stream, int max_ctas, int kernel);
 // CTAs of ldpc_decode_kernel resident on the whole device.
 int ldpc_resident_ctas(pg_context* ctx);
 

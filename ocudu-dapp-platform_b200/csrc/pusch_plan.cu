@@ -40,7 +40,6 @@ struct pg_pusch_plan {
   size_t                   grid_words = 0, tb_bytes = 0, nof_llrs = 0, dev_bytes = 0, est_total = 0;
   uint32_t                 total_tiles = 0; // demodulation tiles
   int                      max_rb   = 1;
-  int                      ldpc_kinds = 0; // PG_LDPC_KIND_* present in the plan
   std::vector<pg_pusch_ue> ues;
   std::vector<pg_rm_cb>    rm;                 // rate-dematch descriptors (host copy, for HARQ updates)
   std::vector<int>         tb_first, tb_ncb;   // codeblocks of each UE
@@ -262,6 +261,18 @@ std::vector<uint32_t> unplaced_list(const std::vector<uint8_t>& placed)
   return list;
 }
 
+// Decoder CTAs of the plan's launch, and whether an execution orders the codeblocks on the device: only
+// when they outnumber the CTAs (otherwise all start at once).
+int ldpc_ctas(const pg_pusch_plan* p)
+{
+  return std::min(p->nof_cbs, ldpc_max_ctas(p->ctx, p->tuning.ldpc_ctas_per_sm, p->tuning.ldpc_kernel));
+}
+
+bool ldpc_ordered(const pg_pusch_plan* p)
+{
+  return p->tuning.ldpc_order != 0 && p->nof_cbs > ldpc_ctas(p);
+}
+
 int enqueue(pg_pusch_plan* p, const uint32_t* grids, uint8_t* tb_out, pg_sch_result* results,
             pg_port_result* port_results, cudaStream_t s)
 {
@@ -331,15 +342,14 @@ int enqueue(pg_pusch_plan* p, const uint32_t* grids, uint8_t* tb_out, pg_sch_res
                              p->tuning.rm_ctas_per_cb, p->d_unplaced);
   }
   const uint32_t* order = p->d_order_static;
-  if (rc == PG_OK && p->nof_cbs > 1 && p->tuning.ldpc_order != 0) {
+  if (rc == PG_OK && ldpc_ordered(p)) {
     // Longest first: the decoders take the codeblocks by the predicted decoding time of their input.
     rc    = ldpc_order_launch(ctx, p->d_ldpc, p->nof_cbs, p->d_rm_out, p->d_keys, p->d_order, s);
     order = p->d_order;
   }
   if (rc == PG_OK) {
     rc = ldpc_launch_persistent(ctx, p->d_ldpc, p->nof_cbs, p->d_rm_out, p->d_cb_bits, p->d_iters, p->d_c2v,
-                                order, p->d_counter, s, p->tuning.ldpc_ctas_per_sm * ctx->sm_count,
-                                p->ldpc_kinds | ldpc_route(p->tuning.ldpc_kernel));
+                                order, p->d_counter, s, ldpc_ctas(p), p->tuning.ldpc_kernel);
   }
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaMemsetAsync(tb_out, 0, p->tb_bytes, s), "cudaMemsetAsync(tb)");
@@ -609,12 +619,8 @@ int pg_pusch_plan_create_uci(pg_context* ctx, const pg_pusch_ue* ues, const pg_p
     cost[c]             = (uint64_t)l.lifting_size * std::min<uint64_t>(w.rm[c].rm_length + l.nof_filler_bits, l.nof_llrs);
   }
   std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return cost[a] > cost[b]; });
-  p->ldpc_kinds = 0;
-  for (const pg_ldpc_cb& l : w.ldpc) {
-    p->ldpc_kinds |= l.lifting_size == 384 ? PG_LDPC_KIND_Z384 : PG_LDPC_KIND_OTHER;
-  }
-  // One check-to-variable slab per decoder CTA: up to four per SM, at most one per codeblock.
-  const int ldpc_slabs = std::max(1, std::min(p->nof_cbs, 4 * ctx->sm_count));
+  // One check-to-variable slab per decoder CTA, at most one per codeblock.
+  const int ldpc_slabs = std::max(1, std::min(p->nof_cbs, kLdpcSlabsPerSm * ctx->sm_count));
 
   // Device image: descriptors first (uploaded once), then the workspace.
   const size_t o_ues    = 0;
@@ -658,7 +664,7 @@ int pg_pusch_plan_create_uci(pg_context* ctx, const pg_pusch_ue* ues, const pg_p
   const size_t o_keys   = o_it + al((size_t)p->nof_cbs * 4);
   const size_t o_cnt    = o_keys + al((size_t)p->nof_cbs);
   const size_t o_c2v    = o_cnt + al(sizeof(int));
-  const size_t o_grid   = o_c2v + al((size_t)ldpc_slabs * kC2vStride);
+  const size_t o_grid   = o_c2v + al((size_t)ldpc_slabs * kPairSlab);
   const size_t o_tbout  = o_grid + al(grid_words * 4);
   const size_t o_res    = o_tbout + al(p->tb_bytes);
   const size_t o_epart  = o_res + al((size_t)nof_ues * sizeof(pg_sch_result));
@@ -810,7 +816,7 @@ int pg_pusch_plan_info(const pg_pusch_plan* plan, pg_pusch_plan_info_t* info)
   // [device work order: score, sort], LDPC, TB assembly, results.
   info->nof_kernels = 2u + (plan->le_net != nullptr ? 3u : 0u) + 1u + (plan->uci_w.nitems > 0 ? 1u : 0u) +
                       (plan->uci_nshort > 0 ? 1u : 0u) + (plan->polar_n > 0 ? 1u : 0u) +
-                      (plan->unplaced.empty() ? 0u : 1u) + (plan->nof_cbs > 1 && plan->tuning.ldpc_order != 0 ? 2u : 0u) +
+                      (plan->unplaced.empty() ? 0u : 1u) + (ldpc_ordered(plan) ? 2u : 0u) +
                       3u;
   info->h2d_grid_bytes = (uint32_t)std::min<size_t>(plan->h2d_grid_bytes, 0xffffffffu);
   return PG_OK;
@@ -1117,7 +1123,7 @@ int pg_pusch_plan_autotune(pg_pusch_plan* plan, const uint32_t* grids, int reps,
   static const int rm_c[]    = {2, 4, 8, 16, 32};
   static const int res_c[]   = {1, 2, 4};
   static const int blk_c[]   = {64, 128, 256};
-  static const int ldpc_c[]  = {1, 2, 3, 4};
+  static const int ldpc_c[]  = {1, 2};
   pg_pusch_plan_tuning cur   = plan->tuning;
   float                cur_ms = 0.f;
   // UEs set to combine would accumulate every timed execution into their soft buffers: keep a
@@ -1175,12 +1181,6 @@ int pg_pusch_plan_autotune(pg_pusch_plan* plan, const uint32_t* grids, int reps,
     for (int v : ldpc_c) {
       pg_pusch_plan_tuning c = cur;
       c.ldpc_ctas_per_sm     = v;
-      if (rc == PG_OK) rc = try_set(c);
-    }
-    for (int v : {PG_LDPC_KERNEL_ONE_LANE, PG_LDPC_KERNEL_TWO_LANES, PG_LDPC_KERNEL_SPLIT, PG_LDPC_KERNEL_Z384,
-                  PG_LDPC_KERNEL_Z384_SPLIT}) {
-      pg_pusch_plan_tuning c = cur;
-      c.ldpc_kernel          = v;
       if (rc == PG_OK) rc = try_set(c);
     }
     for (int v : {0, 1}) {
