@@ -572,10 +572,12 @@ constexpr uint32_t kH400     = 0x5e405e40u; // 400
 constexpr uint32_t kH48128   = 0x79e079e0u; // 48128
 constexpr uint32_t kHm48128  = 0xf9e0f9e0u; // -48128
 constexpr uint32_t kH1152    = 0x64806480u; // 1152 = 1024 + 128
+constexpr uint32_t kHm1152   = 0xe480e480u; // -1152
 constexpr uint32_t kAbs      = 0x7fff7fffu;
 constexpr uint32_t kSign     = 0x80008000u;
 constexpr uint32_t kSat      = 0x60006000u; // the top two exponent bits
-constexpr uint32_t kHDummy   = 0x70007000u; // 8192, the constant column
+constexpr uint32_t kH8192    = 0x70007000u; // 8192 (the constant column)
+constexpr uint32_t kH0       = 0x00000000u; // 0
 constexpr uint32_t kH0p8     = 0x3a663a66u; // f16(0.8) = 0.7998046875
 constexpr uint32_t kH1023p5  = 0x63ff63ffu; // 1023.5
 constexpr uint32_t kHm1024   = 0xe400e400u; // -1024
@@ -643,12 +645,12 @@ __device__ __forceinline__ uint32_t h2_abs_ne(uint32_t a, uint32_t b)
 // Offset-binary byte pair -> f16x2 integers (low byte first).
 __device__ __forceinline__ uint32_t bytes_to_h2(uint32_t b)
 {
-  return h2_sub(__byte_perm(b, 0x6464u, 0x5140u), kH1152);
+  return h2_add(__byte_perm(b, 0x6464u, 0x5140u), kHm1152);
 }
 
 __device__ __forceinline__ uint32_t pair_scale(uint32_t m)
 {
-  return h2_max(h2_add(h2_fma(m, kH0p8, kH1023p5), kHm1024), 0u);
+  return h2_max(h2_add(h2_fma(m, kH0p8, kH1023p5), kHm1024), kH0);
 }
 
 // Shared-memory accesses by 32-bit shared address (the soft-bit addresses of the edge table are
@@ -751,7 +753,7 @@ __device__ __forceinline__ void pair_row(const uint32_t zt, const float jf, cons
     const uint32_t x = __byte_perm(lds_u32(adr[e]), 0, sel[e]);
     uint32_t       d = x;
     if (!FIRST) {
-      const uint32_t c = h2_sub(__byte_perm(m[e / 2], 0x64646464u, (e & 1) ? 0x4342u : 0x4140u), kH1152);
+      const uint32_t c = h2_add(__byte_perm(m[e / 2], 0x64646464u, (e & 1) ? 0x4342u : 0x4140u), kHm1152);
       d                = h2_min(h2_max(h2_sub(x, c), kHm120), kH120);
     }
     v[e]             = h2_min(h2_max(d, h2_fma(x, kH400, kHm48128)), h2_fma(x, kH400, kH48128));
@@ -963,7 +965,7 @@ __device__ __forceinline__ void decode_codeblock_pair(const pg_ldpc_cb& d, pair_
                            (uint32_t)tb.row_sync[g][r]);
   }
   for (int k = tid; k < H; k += NT) {
-    reinterpret_cast<uint32_t*>(E)[k] = kHDummy;
+    reinterpret_cast<uint32_t*>(E)[k] = kH8192;
   }
   if (tid == 0) {
     sh.last   = 0;
