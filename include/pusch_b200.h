@@ -647,7 +647,7 @@ typedef struct pg_le_adam {
 size_t pg_le_nof_params(void);
 /* Rows of the network's layout for a list of UEs (12 nof_rb per port and layer, plus gaps). */
 size_t pg_le_rows(const pg_pusch_ue* ues, int nof_ues);
-/* Creates a network with buffers for max_rows rows (about 2.1 KB of device memory per row). The
+/* Creates a network with buffers for max_rows rows (about 3.4 KB of device memory per row). The
  * parameters start at zero: set them with pg_le_set_params. */
 int  pg_le_create(pg_context* ctx, int max_rows, pg_le_net** out);
 void pg_le_destroy(pg_le_net* net);

@@ -91,15 +91,14 @@ struct pg_le_net {
   float*      grads    = nullptr;
   float*      adam_m   = nullptr;
   float*      adam_v   = nullptr;
-  uint16_t*   wf       = nullptr; // packed forward weights
-  uint16_t*   wt       = nullptr; // packed transposed weights (input gradients)
-  uint16_t*   wp       = nullptr; // packed weights of the fused inference kernel (taps along N)
+  uint16_t*   wp       = nullptr; // packed weights of the fused kernel (taps along N)
+  uint16_t*   wpt      = nullptr; // the same of the transposed convolutions (input gradients)
   uint16_t*   x        = nullptr; // [2][R][8]
   uint16_t*   act[8]   = {};      // act[1..7]: [8][R][8] (act[0] = x)
   uint16_t*   mid[kBlocks] = {};  // [8][R][8]
   uint16_t*   y        = nullptr; // [2][R][8]
   uint16_t*   dy       = nullptr; // [2][R][8]
-  uint16_t*   g0 = nullptr, *g1 = nullptr, *h = nullptr; // [8][R][8] gradients
+  uint16_t*   g[kLayers - 1] = {}; // g[l]: [8][R][8] gradient of layer l's output (before it: dy)
   uint8_t*    row_valid = nullptr;
   pg::le_seq* seqs      = nullptr;
   float*      gseq      = nullptr;
@@ -310,12 +309,11 @@ __device__ __forceinline__ uint16_t bf16_bits(float f)
   return *reinterpret_cast<const uint16_t*>(&b);
 }
 
-// Adam step (when update != 0) on every parameter, then the packed BF16 copies of the weights for
-// the forward and the input-gradient convolutions and for the fused inference kernel; the gradients
-// are cleared for the next step.
+// Adam step (when update != 0) on every parameter, then the packed BF16 copies of the weights for the
+// fused kernel's forward and input-gradient passes (the latter W'[ci][co][t] = W[co][ci][4 - t]); the
+// gradients are cleared for the next step.
 __global__ void le_adam_kernel(float* __restrict__ p, float* __restrict__ grad, float* __restrict__ m,
-                               float* __restrict__ v, uint16_t* __restrict__ wf, uint16_t* __restrict__ wt,
-                               uint16_t* __restrict__ wp, int total,
+                               float* __restrict__ v, uint16_t* __restrict__ wp, uint16_t* __restrict__ wpt, int total,
                                int update, float lr, float b1, float b2, float eps, float wd, float bc1, float bc2)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -348,9 +346,8 @@ __global__ void le_adam_kernel(float* __restrict__ p, float* __restrict__ grad, 
     const int ci = r / L.cout;
     const int co = r - ci * L.cout;
     const uint16_t b = bf16_bits(w);
-    wf[L.p_off + ((t * (L.cin / 8) + ci / 8) * L.cout + co) * 8 + (ci & 7)]              = b;
-    wt[L.p_off + (((kTaps - 1 - t) * (L.cout / 8) + co / 8) * L.cin + ci) * 8 + (co & 7)] = b;
-    wp[L.p_off + (((ci / 8) * kTaps + (kTaps - 1 - t)) * L.cout + co) * 8 + (ci & 7)]     = b;
+    wp[L.p_off + (((ci / 8) * kTaps + (kTaps - 1 - t)) * L.cout + co) * 8 + (ci & 7)] = b;
+    wpt[L.p_off + (((co / 8) * kTaps + t) * L.cin + ci) * 8 + (co & 7)]              = b;
   }
 }
 
@@ -359,7 +356,7 @@ size_t al(size_t x)
   return (x + 255) & ~(size_t)255;
 }
 // ---------------------------------------------------------------------------------------------
-// Fused inference: the whole network per window of 512 rows in one kernel, activations in shared
+// The whole network per window of 512 rows in one kernel, activations in shared
 // memory, accumulators in tensor memory, each layer's weights brought in by 1-D bulk copies while
 // the previous layer computes. Every layer loses two exact rows at each window edge (its taps reach
 // two rows beyond), so after 14 layers the central 456 rows are exact and are the ones stored:
@@ -416,9 +413,36 @@ constexpr uint32_t kFCopy     = kFWB;  // bytes per bulk copy: one per layer (16
 constexpr uint32_t kFCols     = 512;   // TMEM columns: 128 accumulators per M tile, then 64 per tile
                                        // of packed bf16 block input (the residual two layers on)
 constexpr uint32_t kFColRes   = 256;
+constexpr uint32_t kFZeroB    = 2 * 128 * 16;          // training: a zero A tile (two chunks of 128 pairs)
+constexpr uint32_t kFOffZero  = ((uint32_t)kFSmem + 127u) & ~127u;
+constexpr size_t   kFSmemTrain = kFOffZero + kFZeroB;
+static_assert(kFSmemTrain <= 227 * 1024, "shared memory of the fused kernel's training modes");
 static_assert(kFOffW % 16 == 0 && kFOffBias % 16 == 0 && kFOffBar % 8 == 0, "smem layout");
 static_assert(kFSmem <= 227 * 1024, "shared memory of the fused kernel");
 static_assert(kFChunkB % 16 == 0 && kFSmem < (1u << 18), "descriptor start addresses: 14 bits of 16-byte units");
+
+// Modes. Training stores every layer's output (the exact central rows) to memory as well, for the
+// backward pass. The backward pass is the same network of 13 layers on the output gradient: layer l is
+// the transposed convolution of network layer 13 - l, its output the gradient of network layer
+// 12 - l's output - no bias, the residual of a block as in the forward pass (the gradient that passed by
+// the block), and the ReLU replaced by the mask of the forward activation (its values are positive where
+// the ReLU passed), read from memory while the layer's MMAs run. Both passes are one launch instead of
+// one per layer, whose tile loads, MMAs and epilogues ran one after the other: at 96,000 rows the forward
+// pass takes 92 us (446 us in 14 launches before), the input gradients 122 us (545 us in 13). Bound: the
+// epilogues and the activation traffic (tensor pipe 31 % and 24 % of active cycles).
+enum fused_mode { kFInfer, kFTrain, kFBackward };
+
+struct fused_io {
+  uint4*       out[kLayers - 1];  // kFTrain: outputs of layers 0 .. 12; kFBackward: gradients
+  const uint4* mask[kLayers - 1]; // kFBackward: forward activation that masks layer l's output
+};
+
+// The bf16 values of word w kept where those of word m are positive (ReLU outputs: +0 or positive).
+__device__ __forceinline__ uint32_t mask_positive(uint32_t w, uint32_t m)
+{
+  const __nv_bfloat162 z = __floats2bfloat162_rn(0.f, 0.f);
+  return w & __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&m), z);
+}
 
 __device__ __forceinline__ uint32_t layer_weight_bytes(int l)
 {
@@ -438,10 +462,13 @@ __device__ __forceinline__ void fused_load_weights(const uint16_t* __restrict__ 
 
 // The MMAs of one input shift s (x[2 r' + s], all input chunks) of M tile c. The descriptors are
 // formed once; each MMA adds its constant offset (16-byte units) to the start-address field, which
-// stays below 2^14 (shared memory < 256 KB), so no carry reaches the LBO field. Shift -1 comes first
-// in each tile and initialises both halves of the accumulator (N = 2 cout, no accumulation on the
-// first chunk); every other MMA accumulates.
-template <int CIN, int COUT, int S>
+// stays below 2^14 (shared memory < 256 KB), so no carry reaches the LBO field. Inference: shift -1 comes
+// first in each tile and initialises both halves of the accumulator (N = 2 cout, no accumulation on the
+// first chunk); every other MMA accumulates. Training (ZEROED): an MMA of a zero A tile initialises both
+// halves and the shifts follow in ascending order, so that every output row sums its taps 0 to 4 in
+// order, as one convolution per layer (conv1d_fwd_kernel) does, and the activations and gradients equal
+// those of such a chain bit for bit.
+template <int CIN, int COUT, int S, bool ZEROED>
 __device__ __forceinline__ void fused_issue_shift(uint64_t a0, uint64_t b0, uint32_t d)
 {
   constexpr uint32_t idesc_pair = make_idesc(128, 2 * COUT, false, false);
@@ -461,28 +488,34 @@ __device__ __forceinline__ void fused_issue_shift(uint64_t a0, uint64_t b0, uint
     } else if (S == -2) {
       mma_bf16(d, ad, bd, idesc_one, 1u);
     } else {
-      mma_bf16(d, ad, bd, idesc_pair, (S == -1 && kc == 0) ? 0u : 1u);
+      mma_bf16(d, ad, bd, idesc_pair, (!ZEROED && S == -1 && kc == 0) ? 0u : 1u);
     }
   }
 }
 
 // The MMAs of M tile c of one layer: part 0 the shifts that read no pair beyond the tile's end
 // (-1, -2, 0, 1), part 1 the two that read the next tile's first pair (2, 3), part 2 all six.
-template <int CIN, int COUT>
-__device__ __forceinline__ void fused_issue_tile(int c, int part, uint32_t src, uint32_t wb, uint32_t tmem)
+template <int CIN, int COUT, bool ZEROED>
+__device__ __forceinline__ void fused_issue_tile(int c, int part, uint32_t src, uint32_t wb, uint32_t tmem, uint32_t zero)
 {
   const uint64_t a0 = make_desc(src + (uint32_t)(c * 128) * 16u, kFChunkB, 128);
   const uint64_t b0 = make_desc(wb, (uint32_t)kTaps * COUT * 16, 128);
   const uint32_t d  = tmem + (uint32_t)(c * 128);
   if (part != 1) {
-    fused_issue_shift<CIN, COUT, -1>(a0, b0, d);
-    fused_issue_shift<CIN, COUT, -2>(a0, b0, d);
-    fused_issue_shift<CIN, COUT, 0>(a0, b0, d);
-    fused_issue_shift<CIN, COUT, 1>(a0, b0, d);
+    if (ZEROED) {
+      mma_bf16(d, make_desc(zero, kFZeroB / 2, 128), b0, make_idesc(128, 2 * COUT, false, false), 0u);
+      fused_issue_shift<CIN, COUT, -2, ZEROED>(a0, b0, d);
+      fused_issue_shift<CIN, COUT, -1, ZEROED>(a0, b0, d);
+    } else {
+      fused_issue_shift<CIN, COUT, -1, ZEROED>(a0, b0, d);
+      fused_issue_shift<CIN, COUT, -2, ZEROED>(a0, b0, d);
+    }
+    fused_issue_shift<CIN, COUT, 0, ZEROED>(a0, b0, d);
+    fused_issue_shift<CIN, COUT, 1, ZEROED>(a0, b0, d);
   }
   if (part != 0) {
-    fused_issue_shift<CIN, COUT, 2>(a0, b0, d);
-    fused_issue_shift<CIN, COUT, 3>(a0, b0, d);
+    fused_issue_shift<CIN, COUT, 2, ZEROED>(a0, b0, d);
+    fused_issue_shift<CIN, COUT, 3, ZEROED>(a0, b0, d);
   }
 }
 
@@ -506,13 +539,16 @@ __device__ __forceinline__ uint32_t fused_line(int plane, int chunk, int pair) /
   return ((uint32_t)(plane * 8 + chunk)) * kFChunkB + (uint32_t)pair * 16u;
 }
 
+template <int MODE>
 __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const uint4* __restrict__ x,
                                                                         const uint8_t* __restrict__ row_valid,
                                                                         const uint16_t* __restrict__ wp,
                                                                         const float* __restrict__ params, int R,
                                                                         int n_full, int n_win, uint4* __restrict__ y,
-                                                                        int* __restrict__ err)
+                                                                        int* __restrict__ err,
+                                                                        const __grid_constant__ fused_io io)
 {
+  constexpr int NL = MODE == kFBackward ? kLayers - 1 : kLayers;
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char*     buf_a    = smem;
   unsigned char*     buf_b    = smem + kFActB;
@@ -533,11 +569,15 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
     const int b = i >> 5, pl = (i >> 4) & 1, ch = (i >> 1) & 7, e = i & 1;
     *reinterpret_cast<uint4*>(smem + b * kFActB + fused_line(pl, ch, e ? kFPRows - 1 : 0)) = make_uint4(0, 0, 0, 0);
   }
-  for (int i = tid; i < kLayers * kCh; i += kFThreads) {
+  for (int i = tid; MODE != kFBackward && i < kLayers * kCh; i += kFThreads) {
     const int        l = i / kCh, co = i - l * kCh;
     const layer_desc L = c_layers[l];
     bias_s[i]          = co < L.cout ? params[L.w_off + kTaps * L.cin * L.cout + co] : 0.f;
   }
+  for (int i = tid; MODE != kFInfer && i < (int)kFZeroB / 16; i += kFThreads) {
+    *reinterpret_cast<uint4*>(smem + kFOffZero + 16 * i) = make_uint4(0, 0, 0, 0);
+  }
+  const uint32_t zero_s   = smem_u32(smem + kFOffZero);
   const bool     producer = warp == kFEpiWarps;
   const uint32_t bar_mma  = smem_u32(&bars[0]);           // + 8c
   const uint32_t bar_epi  = smem_u32(&bars[kFTiles]);     // + 8c
@@ -557,7 +597,7 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
     mbar_init(bar_w + 8u, 1);
     *abort_sm = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    fused_load_weights(wp, 0, wbuf0, bar_w);
+    fused_load_weights(wp, MODE == kFBackward ? kLayers - 1 : 0, wbuf0, bar_w);
   }
   tc_fence_before();
   __syncthreads();
@@ -598,7 +638,7 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
     }
     if (producer) {
       if (lane == 0) {
-        for (int l = 0; l < kLayers; ++l) {
+        for (int l = 0; l < NL; ++l) {
           const uint32_t s   = step + (uint32_t)l;
           const uint32_t src = (l & 1) ? act_a : act_b;
           if (!fused_wait(bar_w + 8u * (s & 1), (s >> 1) & 1u, abort_sm, err)) {
@@ -607,11 +647,11 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
           const uint32_t wb    = wbuf0 + (s & 1) * kFWB;
           auto           issue = [&](int c, int part) {
             if (l == 0) {
-              fused_issue_tile<kInCh, kCh>(c, part, src, wb, tmem);
-            } else if (l == kLayers - 1) {
-              fused_issue_tile<kCh, kOutCh>(c, part, src, wb, tmem);
+              fused_issue_tile<kInCh, kCh, MODE != kFInfer>(c, part, src, wb, tmem, zero_s);
+            } else if (MODE != kFBackward && l == kLayers - 1) {
+              fused_issue_tile<kCh, kOutCh, MODE != kFInfer>(c, part, src, wb, tmem, zero_s);
             } else {
-              fused_issue_tile<kCh, kCh>(c, part, src, wb, tmem);
+              fused_issue_tile<kCh, kCh, MODE != kFInfer>(c, part, src, wb, tmem, zero_s);
             }
           };
           // Layer 0 follows the window barrier. Later layers: tile 0's first part reads tile 0 of
@@ -634,8 +674,9 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
             mma_issued = s + 1;
             break;
           }
-          if (l + 1 < kLayers || win + (int)gridDim.x < n_win) {
-            fused_load_weights(wp, (l + 1) % kLayers, wbuf0 + ((s + 1) & 1) * kFWB, bar_w + 8u * ((s + 1) & 1));
+          if (l + 1 < NL || win + (int)gridDim.x < n_win) {
+            const int nx = (l + 1) % NL;
+            fused_load_weights(wp, MODE == kFBackward ? kLayers - 1 - nx : nx, wbuf0 + ((s + 1) & 1) * kFWB, bar_w + 8u * ((s + 1) & 1));
             ++w_issued;
           }
           if (l > 0) {
@@ -660,9 +701,19 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
       }
       __syncwarp();
     } else {
-      for (int l = 0; l < kLayers; ++l) {
+      for (int l = 0; l < NL; ++l) {
         const uint32_t s = step + (uint32_t)l;
         for (int c = 0; c < kFTiles; ++c) {
+          // Backward: the forward activations of this step's outputs, loaded while its MMAs run.
+          uint4 mk[4];
+          if (MODE == kFBackward && (two || c == 0)) {
+            const int    g  = base + 2 * (c * 128 + q * 32 + lane) + (cs >> 1);
+            const uint4* mp = io.mask[l] + (size_t)((cs & 1) * 4) * R + g;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              mk[k] = (g >= 0 && g < R) ? __ldg(mp + (size_t)k * R) : make_uint4(0, 0, 0, 0);
+            }
+          }
           // One lane polls the barrier and tells the others: probes from all 32 lanes take
           // shared-memory cycles from the tensor cores' operand reads (measured 13 % slower).
           bool ok = false;
@@ -674,7 +725,7 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
             tc_fence_after();
             const int      pr  = c * 128 + q * 32 + lane;                 // window row pair
             const uint32_t tad = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 128);
-            if (l < kLayers - 1) {
+            if (MODE == kFBackward || l < kLayers - 1) {
               // 32 output channels (chunks 4 hh .. 4 hh + 3) of one row: one TMEM load of the
               // accumulators, then straight-line arithmetic. Layers 0, 2, .. 12 write the block
               // input, kept as packed bf16 in TMEM as well, where the second layer of the next block
@@ -684,6 +735,9 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
               const bool     second = l >= 2 && (l & 1) == 0;
               const bool     keep   = (l & 1) == 0;
               unsigned char* dst    = (l & 1) ? buf_b : buf_a;
+              const int      wr     = 2 * pr + plane; // window row
+              const bool     store  = MODE != kFInfer && wr >= kFMargin && wr < kFMargin + nout && base + wr < R;
+              uint4*         op     = MODE != kFInfer ? io.out[l] + (size_t)(hh * 4) * R + (base + wr) : nullptr;
               uint4*         p      = reinterpret_cast<uint4*>(dst + fused_line(plane, hh * 4, pr + 1));
               constexpr int  kStep  = kFChunkB / 16; // uint4 per chunk
               const float*   bl     = bias_s + l * kCh + hh * 32;
@@ -708,7 +762,7 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
                 float        o[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                  o[j] = v[8 * k + j] + bb[j];
+                  o[j] = v[8 * k + j] + (MODE == kFBackward ? 0.f : bb[j]);
                 }
                 if (second) {
 #pragma unroll
@@ -719,13 +773,23 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
                   }
                 }
                 uint4 pk = make_uint4(0, 0, 0, 0);
-                if (valid) {
+                if (MODE == kFBackward) {
+                  if (valid) {
+                    pk = make_uint4(mask_positive(pack_bf16x2(o[0], o[1]), mk[k].x),
+                                    mask_positive(pack_bf16x2(o[2], o[3]), mk[k].y),
+                                    mask_positive(pack_bf16x2(o[4], o[5]), mk[k].z),
+                                    mask_positive(pack_bf16x2(o[6], o[7]), mk[k].w));
+                  }
+                } else if (valid) {
                   pk = make_uint4(pack_bf16x2(fmaxf(o[0], 0.f), fmaxf(o[1], 0.f)),
                                   pack_bf16x2(fmaxf(o[2], 0.f), fmaxf(o[3], 0.f)),
                                   pack_bf16x2(fmaxf(o[4], 0.f), fmaxf(o[5], 0.f)),
                                   pack_bf16x2(fmaxf(o[6], 0.f), fmaxf(o[7], 0.f)));
                 }
                 p[k * kStep] = pk;
+                if (MODE != kFInfer && store) {
+                  op[(size_t)k * R] = pk;
+                }
                 kept[4 * k] = pk.x, kept[4 * k + 1] = pk.y, kept[4 * k + 2] = pk.z, kept[4 * k + 3] = pk.w;
               }
               if (keep) {
@@ -764,7 +828,7 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
         }
       }
     }
-    step += kLayers;
+    step += NL;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -791,9 +855,6 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
   }
 }
 
-int fused_forward(pg_le_net* net, int R, cudaStream_t s);
-
-
 int check_err_status(pg_le_net* net)
 {
   int e = 0;
@@ -802,29 +863,6 @@ int check_err_status(pg_le_net* net)
     return rc;
   }
   return e != 0 ? pg::set_error(net->ctx, PG_ERR_TIMEOUT, "a tensor-core completion wait expired") : PG_OK;
-}
-
-int forward(pg_le_net* net, int R, cudaStream_t s)
-{
-  pg_context*        ctx = net->ctx;
-  const layer_table& T   = layers();
-  auto w  = [&](int i) { return (const void*)(net->wf + T.l[i].p_off); };
-  auto b  = [&](int i) { return (const float*)(net->params + T.l[i].w_off + kTaps * T.l[i].cin * T.l[i].cout); };
-  int  rc = pg::conv_forward_launch(ctx, kInCh, kCh, net->x, w(0), b(0), nullptr, nullptr, net->act[1],
-                                    net->row_valid, R, 1, net->err, s);
-  for (int k = 0; k < kBlocks && rc == PG_OK; ++k) {
-    rc = pg::conv_forward_launch(ctx, kCh, kCh, net->act[k + 1], w(1 + 2 * k), b(1 + 2 * k), nullptr, nullptr,
-                                 net->mid[k], net->row_valid, R, 1, net->err, s);
-    if (rc == PG_OK) {
-      rc = pg::conv_forward_launch(ctx, kCh, kCh, net->mid[k], w(2 + 2 * k), b(2 + 2 * k), net->act[k + 1], nullptr,
-                                   net->act[k + 2], net->row_valid, R, 1, net->err, s);
-    }
-  }
-  if (rc == PG_OK) {
-    rc = pg::conv_forward_launch(ctx, kCh, kOutCh, net->act[kBlocks + 1], w(kLayers - 1), b(kLayers - 1), nullptr,
-                                 nullptr, net->y, net->row_valid, R, 0, net->err, s);
-  }
-  return rc;
 }
 
 // Windows of the fused kernel over R rows: n_full two-tile windows, then one-tile windows up to
@@ -848,7 +886,8 @@ void fused_windows(int R, int sms, int* n_full, int* n_win)
   }
 }
 
-int fused_forward(pg_le_net* net, int R, cudaStream_t s)
+template <int MODE>
+int fused_launch(pg_le_net* net, const uint16_t* x, const uint16_t* wp, int R, const fused_io& io, cudaStream_t s)
 {
   if (R <= 0) {
     return PG_OK;
@@ -856,50 +895,55 @@ int fused_forward(pg_le_net* net, int R, cudaStream_t s)
   int n_full = 0, n_win = 0;
   fused_windows(R, net->ctx->sm_count, &n_full, &n_win);
   const int grid = std::max(1, std::min(n_win, net->ctx->sm_count));
-  le_fused_forward_kernel<<<grid, kFThreads, kFSmem, s>>>(reinterpret_cast<const uint4*>(net->x), net->row_valid,
-                                                          net->wp, net->params, R, n_full, n_win,
-                                                          reinterpret_cast<uint4*>(net->y), net->err);
+  le_fused_forward_kernel<MODE><<<grid, kFThreads, MODE == kFInfer ? kFSmem : kFSmemTrain, s>>>(reinterpret_cast<const uint4*>(x), net->row_valid, wp,
+                                                                net->params, R, n_full, n_win,
+                                                                reinterpret_cast<uint4*>(net->y), net->err, io);
   return pg::check_cuda(net->ctx, cudaGetLastError(), "le_fused_forward_kernel launch");
 }
 
+int fused_forward(pg_le_net* net, int R, cudaStream_t s)
+{
+  return fused_launch<kFInfer>(net, net->x, net->wp, R, fused_io{}, s);
+}
+
+// Output of network layer l (0 .. 12).
+uint16_t* layer_out(pg_le_net* net, int l)
+{
+  return (l & 1) ? net->mid[(l - 1) / 2] : net->act[l / 2 + 1];
+}
+
+// The network on net->x with every layer's output kept for backward().
+int forward(pg_le_net* net, int R, cudaStream_t s)
+{
+  fused_io io{};
+  for (int l = 0; l < kLayers - 1; ++l) {
+    io.out[l] = reinterpret_cast<uint4*>(layer_out(net, l));
+  }
+  return fused_launch<kFTrain>(net, net->x, net->wp, R, io, s);
+}
+
 // Gradients of every parameter (added to net->grads) from net->dy and the activations of the last
-// forward pass.
+// forward pass: the input gradients of every layer in one launch, then the weight and bias gradients of
+// every layer in another.
 int backward(pg_le_net* net, int R, cudaStream_t s)
 {
-  pg_context*        ctx = net->ctx;
-  const layer_table& T   = layers();
-  auto wt = [&](int i) { return (const void*)(net->wt + T.l[i].p_off); };
-  auto gw = [&](int i) { return net->grads + T.l[i].w_off; };
-  auto gb = [&](int i) { return net->grads + T.l[i].w_off + kTaps * T.l[i].cin * T.l[i].cout; };
-  const int last = kLayers - 1;
-  uint16_t* top  = net->act[kBlocks + 1];
-  int rc = pg::conv_wgrad_launch(ctx, kCh, kOutCh, top, net->dy, R, gw(last), gb(last), net->err, s);
-  if (rc == PG_OK) {
-    rc = pg::conv_forward_launch(ctx, kOutCh, kCh, net->dy, wt(last), nullptr, nullptr, top, net->g0, net->row_valid,
-                                 R, 0, net->err, s);
+  const layer_table& T = layers();
+  fused_io           io{};
+  for (int l = 0; l < kLayers - 1; ++l) {
+    io.out[l]  = reinterpret_cast<uint4*>(net->g[kLayers - 2 - l]);
+    io.mask[l] = reinterpret_cast<const uint4*>(layer_out(net, kLayers - 2 - l));
   }
-  uint16_t* G = net->g0;
-  uint16_t* Gn = net->g1;
-  for (int k = kBlocks - 1; k >= 0 && rc == PG_OK; --k) {
-    const int l2 = 2 + 2 * k, l1 = 1 + 2 * k;
-    rc = pg::conv_wgrad_launch(ctx, kCh, kCh, net->mid[k], G, R, gw(l2), gb(l2), net->err, s);
-    if (rc == PG_OK) {
-      rc = pg::conv_forward_launch(ctx, kCh, kCh, G, wt(l2), nullptr, nullptr, net->mid[k], net->h, net->row_valid, R,
-                                   0, net->err, s);
-    }
-    if (rc == PG_OK) {
-      rc = pg::conv_wgrad_launch(ctx, kCh, kCh, net->act[k + 1], net->h, R, gw(l1), gb(l1), net->err, s);
-    }
-    if (rc == PG_OK) {
-      rc = pg::conv_forward_launch(ctx, kCh, kCh, net->h, wt(l1), nullptr, G, net->act[k + 1], Gn, net->row_valid, R,
-                                   0, net->err, s);
-    }
-    std::swap(G, Gn);
+  int rc = fused_launch<kFBackward>(net, net->dy, net->wpt, R, io, s);
+  if (rc != PG_OK) {
+    return rc;
   }
-  if (rc == PG_OK) {
-    rc = pg::conv_wgrad_launch(ctx, kInCh, kCh, net->x, G, R, gw(0), gb(0), net->err, s);
+  pg::wgrad_layer wl[kLayers];
+  for (int l = 0; l < kLayers; ++l) {
+    const layer_desc& d = T.l[l];
+    wl[l] = {l == 0 ? net->x : layer_out(net, l - 1), l == kLayers - 1 ? net->dy : net->g[l],
+             net->grads + d.w_off, net->grads + d.w_off + kTaps * d.cin * d.cout, d.cin, d.cout};
   }
-  return rc;
+  return pg::conv_wgrad_launch(net->ctx, wl, kLayers, R, net->err, s);
 }
 
 int pack_launch(pg_le_net* net, int update, const pg_le_adam* opt, cudaStream_t s)
@@ -916,8 +960,8 @@ int pack_launch(pg_le_net* net, int update, const pg_le_adam* opt, cudaStream_t 
     bc1 = 1.f - std::pow(b1, (float)net->step);
     bc2 = 1.f - std::pow(b2, (float)net->step);
   }
-  le_adam_kernel<<<(total + 255) / 256, 256, 0, s>>>(net->params, net->grads, net->adam_m, net->adam_v, net->wf,
-                                                     net->wt, net->wp, total, update, lr, b1, b2, eps, wd, bc1, bc2);
+  le_adam_kernel<<<(total + 255) / 256, 256, 0, s>>>(net->params, net->grads, net->adam_m, net->adam_v, net->wp,
+                                                     net->wpt, total, update, lr, b1, b2, eps, wd, bc1, bc2);
   return pg::check_cuda(net->ctx, cudaGetLastError(), "le_adam_kernel launch");
 }
 
@@ -1045,8 +1089,7 @@ int pg_le_create(pg_context* ctx, int max_rows, pg_le_net** out)
     return o;
   };
   const size_t o_p = take(P * 4), o_g = take(P * 4), o_m = take(P * 4), o_v = take(P * 4);
-  const size_t o_wf = take((size_t)T.npacked * 2), o_wt = take((size_t)T.npacked * 2),
-               o_wp = take((size_t)T.npacked * 2);
+  const size_t o_wp = take((size_t)T.npacked * 2), o_wpt = take((size_t)T.npacked * 2);
   const size_t o_x = take(R * 32), o_y = take(R * 32), o_dy = take(R * 32);
   size_t o_act[8] = {}, o_mid[kBlocks] = {};
   for (int i = 1; i <= kBlocks + 1; ++i) {
@@ -1055,20 +1098,36 @@ int pg_le_create(pg_context* ctx, int max_rows, pg_le_net** out)
   for (int i = 0; i < kBlocks; ++i) {
     o_mid[i] = take(R * 128);
   }
-  const size_t o_g0 = take(R * 128), o_g1 = take(R * 128), o_h = take(R * 128);
   const size_t o_rv = take(R), o_seq = take((size_t)n->max_seqs * sizeof(le_seq)),
                o_gs = take((size_t)n->max_seqs * 4), o_err = take(4), o_loss = take(8);
+  const size_t cleared = off; // the gradients are written before they are read
+  size_t o_grad[kLayers - 1] = {};
+  for (int i = 0; i < kLayers - 1; ++i) {
+    o_grad[i] = take(R * 128);
+  }
   int rc = check_cuda(ctx, cudaSetDevice(ctx->device), "cudaSetDevice");
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaMalloc(&n->dev, off), "cudaMalloc(learned estimator)");
   }
   if (rc == PG_OK) {
-    rc = check_cuda(ctx, cudaMemset(n->dev, 0, off), "cudaMemset(learned estimator)");
+    rc = check_cuda(ctx, cudaMemset(n->dev, 0, cleared), "cudaMemset(learned estimator)");
   }
   if (rc == PG_OK) {
     rc = check_cuda(ctx,
-                    cudaFuncSetAttribute(le_fused_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                    cudaFuncSetAttribute(le_fused_forward_kernel<kFInfer>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kFSmem),
+                    "cudaFuncSetAttribute(le_fused_forward_kernel)");
+  }
+  if (rc == PG_OK) {
+    rc = check_cuda(ctx,
+                    cudaFuncSetAttribute(le_fused_forward_kernel<kFTrain>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)kFSmemTrain),
+                    "cudaFuncSetAttribute(le_fused_forward_kernel)");
+  }
+  if (rc == PG_OK) {
+    rc = check_cuda(ctx,
+                    cudaFuncSetAttribute(le_fused_forward_kernel<kFBackward>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFSmemTrain),
                     "cudaFuncSetAttribute(le_fused_forward_kernel)");
   }
   if (rc == PG_OK) {
@@ -1086,9 +1145,8 @@ int pg_le_create(pg_context* ctx, int max_rows, pg_le_net** out)
   n->grads     = reinterpret_cast<float*>(b + o_g);
   n->adam_m    = reinterpret_cast<float*>(b + o_m);
   n->adam_v    = reinterpret_cast<float*>(b + o_v);
-  n->wf        = reinterpret_cast<uint16_t*>(b + o_wf);
-  n->wt        = reinterpret_cast<uint16_t*>(b + o_wt);
   n->wp        = reinterpret_cast<uint16_t*>(b + o_wp);
+  n->wpt       = reinterpret_cast<uint16_t*>(b + o_wpt);
   n->x         = reinterpret_cast<uint16_t*>(b + o_x);
   n->y         = reinterpret_cast<uint16_t*>(b + o_y);
   n->dy        = reinterpret_cast<uint16_t*>(b + o_dy);
@@ -1099,9 +1157,9 @@ int pg_le_create(pg_context* ctx, int max_rows, pg_le_net** out)
   for (int i = 0; i < kBlocks; ++i) {
     n->mid[i] = reinterpret_cast<uint16_t*>(b + o_mid[i]);
   }
-  n->g0        = reinterpret_cast<uint16_t*>(b + o_g0);
-  n->g1        = reinterpret_cast<uint16_t*>(b + o_g1);
-  n->h         = reinterpret_cast<uint16_t*>(b + o_h);
+  for (int i = 0; i < kLayers - 1; ++i) {
+    n->g[i] = reinterpret_cast<uint16_t*>(b + o_grad[i]);
+  }
   n->row_valid = b + o_rv;
   n->seqs      = reinterpret_cast<le_seq*>(b + o_seq);
   n->gseq      = reinterpret_cast<float*>(b + o_gs);

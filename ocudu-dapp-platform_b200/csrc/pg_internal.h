@@ -284,13 +284,21 @@ int ldpc_resident_ctas(pg_context* ctx);
 
 // Tensor-core 1-D convolutions (tc_conv1d.cu): kernel attributes, the forward launch over an
 // activation buffer of R rows ([C/8][R][8] bf16; bias, res and mask may be null) and the weight
-// gradient (adds to dw[5][cin][cout] and, when db is not null, to db[cout]).
+// gradients of up to kMaxWgradLayers layers (each adds to dw[5][cin][cout] and, when db is not null, to
+// db[cout]).
 int conv_setup(pg_context* ctx);
 int conv_forward_launch(pg_context* ctx, int cin, int cout, const void* x, const void* w, const float* bias,
                         const void* res, const void* mask, void* y, const uint8_t* row_valid, int R, int relu,
                         int* err, cudaStream_t s);
-int conv_wgrad_launch(pg_context* ctx, int cin, int cout, const void* x, const void* dy, int R, float* dw, float* db,
-                      int* err, cudaStream_t s);
+struct wgrad_layer {
+  const void* x;
+  const void* dy;
+  float*      dw;
+  float*      db;
+  int         cin, cout;
+};
+constexpr int kMaxWgradLayers = 14;
+int conv_wgrad_launch(pg_context* ctx, const wgrad_layer* layers, int n, int R, int* err, cudaStream_t s);
 
 // Learned channel estimator (learned_est.cu): one allocation sequence of the network's row layout
 // (a (UE, receive port, layer) allocation of 12 nof_rb rows).

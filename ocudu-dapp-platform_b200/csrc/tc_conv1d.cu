@@ -23,6 +23,8 @@
 
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 namespace {
 
 using namespace pg::tc;
@@ -199,197 +201,321 @@ __global__ void __launch_bounds__(kConvThreads) conv1d_fwd_kernel(const uint4* _
 }
 
 // ---------------------------------------------------------------------------------------------
-// Weight gradient. D[m][co] = sum_r A[m][r] * dY[r][co] over the K tiles (128 rows) of this CTA's
-// row range, with m = (tap, ci): the input tile is staged as kCopies row-shifted copies
-// (copy k holds X[r0 - 2 + k + j]), so that the 16 eight-channel groups of one M tile of 128 sit at
-// a uniform stride; M tile j adds j * kCopies rows to the start address. CIN = 64: 2 copies, 3 M
-// tiles (taps 0-1, 2-3, 4 and a discarded 5th); CIN = 16: 8 copies, 1 M tile (taps 0-4 and three
-// discarded). Both operands are MN-major without swizzle (SBO = stride of the 8-element MN groups,
-// LBO = stride of the 8-row K groups). Two smem stages: the loads of tile i + 1 overlap the MMAs of
-// tile i. Epilogue: FP32 partial sums added to dw[t][ci][co] with vector atomics.
-constexpr int kWgTile     = 128;
-constexpr int kWgCopyRows = kWgTile + 8;
+// Weight and bias gradients of a list of layers, one launch. Per layer D[m][co] = sum_r A[m][r] * dY[r][co]
+// over K tiles of 128 rows, with m = (tap, ci): the input tile is staged as `copies` row-shifted copies
+// (copy k holds X[r0 - 2 + k + j]), so that the 16 eight-channel groups of one M tile of 128 sit at a
+// uniform stride; M tile j adds j * copies rows to the start address. CIN = 64: 2 copies, 3 M tiles (taps
+// 0-1, 2-3, 4 and a discarded 5th); CIN = 16: 8 copies, 1 M tile (taps 0-4 and three discarded). Both
+// operands are MN-major without swizzle (SBO = stride of the 8-element MN groups, LBO = stride of the
+// 8-row K groups).
+//
+// The tiles of all layers form one list that is split evenly over one CTA per SM (about 70 tiles each at
+// 96,000 rows and 14 layers, so that few CTAs add to one layer's gradients), and a ring of four stages is
+// filled by bulk copies (one per 8-channel column and copy) ahead of the MMAs. Warp 0 issues the MMAs,
+// warp 1 the copies (and zeroes the rows outside [0, R)), warps 2 and 3 sum dY for the bias gradient from
+// the same stage, and warps 4 to 7 add each group of four tiles' FP32 accumulators (two sets in tensor
+// memory, one filled while the other is read) to FP32 sums in registers, so that no sum of more than 512
+// rows is formed in the tensor cores. When a CTA's run of tiles of one layer ends, its sums are added to
+// dw[t][ci][co] with vector atomics. At 96,000 rows the 14 layers take 105 us (722 us with one launch per
+// layer, two synchronous stages and a second launch for the bias); bound by the rate at which one thread
+// issues the MMAs and by the loads.
+constexpr int      kWgTile     = 128;
+constexpr int      kWgCopyRows = kWgTile + 8;
+constexpr int      kWgStages   = 4;
+constexpr uint32_t kWgABytes   = 16u * kWgCopyRows * 16u;
+constexpr uint32_t kWgBBytes   = 8u * kWgTile * 16u;
+constexpr uint32_t kWgStageB   = kWgABytes + kWgBBytes;
+constexpr int      kWgThreads  = 256;
+constexpr int      kWgGroup    = 4;   // tiles per accumulator set
+constexpr uint32_t kWgCols     = 512; // two sets of up to 3 M tiles x 64 columns, 256 columns apart
+constexpr size_t   kWgSmem     = kWgStages * (size_t)kWgStageB + 8 * (2 * kWgStages + 4) + 24;
+static_assert(kWgStageB % 128 == 0 && kWgSmem <= 227 * 1024, "shared memory of the weight-gradient kernel");
 
-template <int CIN, int COUT>
-struct wg_cfg {
-  static constexpr int      kInChunks   = CIN / 8;
-  static constexpr int      kCopies     = 16 / kInChunks;
-  static constexpr int      kMTiles     = (kTapCount + kCopies - 1) / kCopies;
-  static constexpr uint32_t kABytes     = 16u * kWgCopyRows * 16u;
-  static constexpr uint32_t kBBytes     = (uint32_t)(COUT / 8) * kWgTile * 16u;
-  static constexpr uint32_t kStageBytes = kABytes + kBBytes;
-  static constexpr uint32_t kCols       = tmem_cols<kMTiles * COUT>();
-  static constexpr size_t   kSmem       = 2 * (size_t)kStageBytes + 32;
+struct wg_args {
+  pg::wgrad_layer l[pg::kMaxWgradLayers];
+  int             n;
 };
 
+// The MMAs of one stage: the descriptors are formed once and each MMA adds a constant to their
+// start-address fields (16-byte units, below 2^14, so no carry reaches the next field). Formed per MMA by
+// the one issuing thread they set the time of a tile (154 us for the 14 layers at 96,000 rows).
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(kConvThreads) conv1d_wgrad_kernel(const uint4* __restrict__ x,
-                                                                    const uint4* __restrict__ dy, int R,
-                                                                    int tiles_per_cta, float* __restrict__ dw,
-                                                                    int* __restrict__ err)
+__device__ __forceinline__ void wgrad_issue_tile(uint32_t ab, uint32_t d, uint32_t acc)
 {
-  using C = wg_cfg<CIN, COUT>;
-  extern __shared__ __align__(128) unsigned char smem[];
-  uint64_t*  mbar    = reinterpret_cast<uint64_t*>(smem + 2 * C::kStageBytes);
-  uint32_t*  tmem_sm = reinterpret_cast<uint32_t*>(mbar + 2);
-  uint32_t*  ok_sm   = tmem_sm + 1;
-  const int  tid     = threadIdx.x;
-  const int  warp    = tid >> 5;
-  const int  ntiles  = (R + kWgTile - 1) / kWgTile;
-  const int  t0      = blockIdx.x * tiles_per_cta;
-  const int  nt      = min(ntiles, t0 + tiles_per_cta) - t0;
-  if (nt <= 0) {
-    return;
+  constexpr int      kCopies = 16 / (CIN / 8);
+  constexpr int      kMTiles = (kTapCount + kCopies - 1) / kCopies;
+  constexpr uint32_t idesc   = make_idesc(kTileRows, COUT, true, true);
+  const uint64_t     a0      = make_desc(ab, 128, kWgCopyRows * 16);
+  const uint64_t     b0      = make_desc(ab + kWgABytes, 128, kWgTile * 16);
+#pragma unroll
+  for (int ks = 0; ks < kWgTile / 16; ++ks) {
+#pragma unroll
+    for (int j = 0; j < kMTiles; ++j) {
+      mma_bf16(d + (uint32_t)(j * COUT), a0 + (uint64_t)(j * kCopies + ks * 16), b0 + (uint64_t)(ks * 16), idesc,
+               ks > 0 ? 1u : acc);
+    }
   }
+}
+
+__global__ void __launch_bounds__(kWgThreads, 1) conv1d_wgrad_kernel(const __grid_constant__ wg_args args, int R,
+                                                                       int* __restrict__ err)
+{
+  extern __shared__ __align__(128) unsigned char smem[];
+  uint64_t*          bars     = reinterpret_cast<uint64_t*>(smem + kWgStages * kWgStageB);
+  uint32_t*          tmem_sm  = reinterpret_cast<uint32_t*>(bars + 2 * kWgStages + 4);
+  volatile uint32_t* abort_sm = tmem_sm + 1;
+  const uint32_t     bar_full = smem_u32(&bars[0]);             // + 8 stage: copies landed
+  const uint32_t     bar_free = smem_u32(&bars[kWgStages]);     // + 8 stage: MMAs and bias sums done
+  const uint32_t     bar_acc  = smem_u32(&bars[2 * kWgStages]);     // + 8 set: accumulators of a group complete
+  const uint32_t     bar_read = smem_u32(&bars[2 * kWgStages + 2]); // + 8 set: they have been read
+  const uint32_t     base     = smem_u32(smem);
+  const int          tid      = threadIdx.x;
+  const int          warp     = tid >> 5;
+  const int          lane     = tid & 31;
   if (warp == 0) {
-    tmem_alloc(smem_u32(tmem_sm), C::kCols);
+    tmem_alloc(smem_u32(tmem_sm), kWgCols);
   }
   if (tid == 0) {
-    mbar_init(smem_u32(&mbar[0]), 1);
-    mbar_init(smem_u32(&mbar[1]), 1);
+    for (int i = 0; i < kWgStages; ++i) {
+      mbar_init(bar_full + 8u * i, 1);
+      mbar_init(bar_free + 8u * i, 3); // the MMA commit and the two bias warps
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar_acc + 8u * i, 1);
+      mbar_init(bar_read + 8u * i, 4); // the four accumulating warps
+    }
+    *abort_sm = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem  = *tmem_sm;
-  const uint32_t idesc = make_idesc(kTileRows, COUT, true, true);
-  const uint4    zero  = make_uint4(0, 0, 0, 0);
-  bool           ok    = true;
-
-  for (int i = 0; i < nt; ++i) {
-    const int      st = i & 1;
-    unsigned char* A  = smem + st * C::kStageBytes;
-    unsigned char* B  = A + C::kABytes;
-    if (i >= 2) {
-      // The stage is free once the MMAs of tile i - 2 (commit number (i - 2) / 2 on its barrier)
-      // have completed.
-      if (tid == 0) {
-        const bool done = mbar_wait_bounded(smem_u32(&mbar[st]), (uint32_t)((i - 2) >> 1) & 1u);
-        *ok_sm          = done ? 1u : 0u;
-        if (!done) {
-          atomicExch(err, 1);
-        }
-      }
-      __syncthreads();
-      ok = *ok_sm != 0;
-      if (!ok) {
-        break;
-      }
+  const uint32_t tmem   = *tmem_sm;
+  const int      ntiles = (R + kWgTile - 1) / kWgTile;
+  const long     total  = (long)args.n * ntiles;
+  const long     t_end  = total * (blockIdx.x + 1) / gridDim.x;
+  auto wait = [&](uint32_t bar, uint32_t parity) {
+    if (*abort_sm != 0) {
+      return false;
     }
-    const int r0 = (t0 + i) * kWgTile;
-    uint4*    As = reinterpret_cast<uint4*>(A);
-    for (int q = tid; q < 16 * kWgCopyRows; q += kConvThreads) {
-      const int g  = q / kWgCopyRows;
-      const int j  = q - g * kWgCopyRows;
-      const int k  = g / C::kInChunks;
-      const int c  = g - k * C::kInChunks;
-      const int gr = r0 - 2 + k + j;
-      As[q]        = (gr >= 0 && gr < R) ? x[(size_t)c * R + gr] : zero;
+    if (mbar_wait_bounded(bar, parity)) {
+      return true;
     }
-    uint4* Bs = reinterpret_cast<uint4*>(B);
-    for (int q = tid; q < (COUT / 8) * kWgTile; q += kConvThreads) {
-      const int c  = q / kWgTile;
-      const int j  = q - c * kWgTile;
-      const int gr = r0 + j;
-      Bs[q]        = gr < R ? dy[(size_t)c * R + gr] : zero;
-    }
-    fence_async_shared();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    if (tid == 0) {
-      const uint32_t ab = smem_u32(A);
-      const uint32_t bb = smem_u32(B);
-#pragma unroll
-      for (int ks = 0; ks < kWgTile / 16; ++ks) {
-        const uint64_t bd = make_desc(bb + (uint32_t)ks * 256u, 128, kWgTile * 16);
-#pragma unroll
-        for (int j = 0; j < C::kMTiles; ++j) {
-          const uint64_t ad =
-              make_desc(ab + (uint32_t)(j * C::kCopies) * 16u + (uint32_t)ks * 256u, 128, kWgCopyRows * 16);
-          mma_bf16(tmem + (uint32_t)(j * COUT), ad, bd, idesc, (i > 0 || ks > 0) ? 1u : 0u);
-        }
-      }
-      mma_commit(smem_u32(&mbar[st]));
-    }
-  }
-  if (ok) {
-    const int last = nt - 1;
-    if (tid == 0) {
-      const bool done = mbar_wait_bounded(smem_u32(&mbar[last & 1]), (uint32_t)(last >> 1) & 1u);
-      *ok_sm          = done ? 1u : 0u;
-      if (!done) {
-        atomicExch(err, 1);
-      }
-    }
-    __syncthreads();
-    tc_fence_after();
-    ok = *ok_sm != 0;
-  }
-  if (ok) {
-    // Thread = TMEM lane m of every M tile: group g = m / 8 (copy k, chunk c), lane e = m % 8.
-    const int      m   = warp * 32 + (tid & 31);
-    const int      g   = m >> 3;
-    const int      k   = g / C::kInChunks;
-    const int      ci  = 8 * (g - k * C::kInChunks) + (m & 7);
-    const uint32_t tad = tmem + ((uint32_t)(warp * 32) << 16);
-#pragma unroll
-    for (int j = 0; j < C::kMTiles; ++j) {
-      const int tap = j * C::kCopies + k;
-#pragma unroll
-      for (int cc = 0; cc < COUT / 16; ++cc) {
-        float v[16];
-        tmem_ld16(tad + (uint32_t)(j * COUT + cc * 16), v);
-        if (tap < kTapCount) {
-          float4* dst = reinterpret_cast<float4*>(dw + ((size_t)tap * CIN + ci) * COUT + cc * 16);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            atomicAdd(dst + q, make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
+    *abort_sm = 1;
+    atomicExch(err, 1);
+    return false;
+  };
+  uint32_t k0 = 0; // tiles of the earlier runs: tile k of this CTA goes to stage k mod kWgStages
+  uint32_t g0 = 0; // groups of the earlier runs: group g uses accumulator set g mod 2
+  for (long t = total * blockIdx.x / gridDim.x; t < t_end;) {
+    const int              li     = (int)(t / ntiles);
+    const int              tile0  = (int)(t - (long)li * ntiles);
+    const int              nt     = (int)min((long)(ntiles - tile0), t_end - t);
+    const pg::wgrad_layer& L      = args.l[li];
+    const int              inch   = L.cin / 8;
+    const int              copies = 16 / inch;
+    const int              mt     = (kTapCount + copies - 1) / copies;
+    const int              bch    = L.cout / 8;
+    const int              ngrp   = (nt + kWgGroup - 1) / kWgGroup;
+    if (warp == 0) {
+      if (lane == 0) {
+        for (int i = 0; i < nt; ++i) {
+          const uint32_t k = k0 + (uint32_t)i, st = k % kWgStages;
+          const uint32_t grp = g0 + (uint32_t)(i / kWgGroup), set = grp & 1u;
+          if (i % kWgGroup == 0 && grp >= 2 && !wait(bar_read + 8u * set, (grp / 2 - 1u) & 1u)) {
+            break;
+          }
+          if (!wait(bar_full + 8u * st, (k / kWgStages) & 1u)) {
+            break;
+          }
+          tc_fence_after();
+          const uint32_t ab = base + st * kWgStageB, acc = i % kWgGroup > 0 ? 1u : 0u, d = tmem + 256u * set;
+          if (L.cin == 16) {
+            wgrad_issue_tile<16, 64>(ab, d, acc);
+          } else if (L.cout == 16) {
+            wgrad_issue_tile<64, 16>(ab, d, acc);
+          } else {
+            wgrad_issue_tile<64, 64>(ab, d, acc);
+          }
+          mma_commit(bar_free + 8u * st);
+          if (i % kWgGroup == kWgGroup - 1 || i + 1 == nt) {
+            mma_commit(bar_acc + 8u * set);
           }
         }
+      }
+      __syncwarp();
+    } else if (warp == 1) {
+      // Lane g: column g of A (copy g / inch, chunk g % inch), lane 16 + c: column c of B.
+      const int    ak  = lane / inch;
+      const int    col = lane < 16 ? lane - ak * inch : lane - 16;
+      const bool   on  = lane < 16 || col < bch;
+      const uint4* src = static_cast<const uint4*>(lane < 16 ? L.x : L.dy) + (size_t)(on ? col : 0) * R;
+      const int    len = lane < 16 ? kWgCopyRows : kWgTile;
+      for (int i = 0; i < nt; ++i) {
+        const uint32_t k = k0 + (uint32_t)i, st = k % kWgStages;
+        bool           ok = true;
+        if (lane == 0 && k >= kWgStages) {
+          ok = wait(bar_free + 8u * st, (k / kWgStages - 1u) & 1u);
+        }
+        if (__shfl_sync(0xffffffffu, ok ? 1 : 0, 0) == 0) {
+          break;
+        }
+        const int      r0  = (tile0 + i) * kWgTile + (lane < 16 ? ak - 2 : 0); // first row of the column
+        const int      lo  = on ? max(0, -r0) : 0;
+        const int      hi  = on ? max(lo, min(len, R - r0)) : 0;
+        const uint32_t dst = base + st * kWgStageB + (lane < 16 ? (uint32_t)lane * (kWgCopyRows * 16u)
+                                                               : kWgABytes + (uint32_t)col * (kWgTile * 16u));
+        if (on && hi - lo < len) {
+          for (int r = 0; r < len; ++r) {
+            if (r < lo || r >= hi) {
+              *reinterpret_cast<uint4*>(smem + (dst - base) + 16 * r) = make_uint4(0, 0, 0, 0);
+            }
+          }
+          fence_async_shared();
+        }
+        const uint32_t bytes = __reduce_add_sync(0xffffffffu, 16u * (uint32_t)(hi - lo));
+        __syncwarp();
+        if (lane == 0) {
+          mbar_expect_tx(bar_full + 8u * st, bytes);
+        }
+        __syncwarp();
+        if (hi > lo) {
+          bulk_g2s(dst + 16u * (uint32_t)lo, src + r0 + lo, 16u * (uint32_t)(hi - lo), bar_full + 8u * st);
+        }
+      }
+    } else if (warp < 4) {
+      // Thread: rows bt % 8, + 8, ... of dY column bt / 8.
+      float      bsum[8] = {};
+      const int  bt = tid - 64, c = bt >> 3;
+      const bool on = c < bch && L.db != nullptr;
+      for (int i = 0; i < nt; ++i) {
+        const uint32_t k = k0 + (uint32_t)i, st = k % kWgStages;
+        bool           ok = true;
+        if (lane == 0) {
+          ok = wait(bar_full + 8u * st, (k / kWgStages) & 1u);
+        }
+        if (__shfl_sync(0xffffffffu, ok ? 1 : 0, 0) == 0) {
+          break;
+        }
+        __syncwarp(); // the copies that lane 0 waited for are visible to the warp
+        if (on) {
+          const uint4* p = reinterpret_cast<const uint4*>(smem + st * kWgStageB + kWgABytes) + c * kWgTile + (bt & 7);
+          float        tsum[8] = {}; // of the tile
+#pragma unroll
+          for (int r = 0; r < kWgTile / 8; ++r) {
+            const uint4           v = p[8 * r];
+            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              tsum[2 * j] += __low2float(h[j]);
+              tsum[2 * j + 1] += __high2float(h[j]);
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            bsum[j] += tsum[j];
+          }
+        }
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(bar_free + 8u * st);
+        }
+      }
+      const bool whole = __shfl_sync(0xffffffffu, *abort_sm == 0 ? 1 : 0, 0) != 0;
+      if (on && whole) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float v = bsum[j];
+          v += __shfl_xor_sync(0xffu << (lane & 24), v, 1);
+          v += __shfl_xor_sync(0xffu << (lane & 24), v, 2);
+          v += __shfl_xor_sync(0xffu << (lane & 24), v, 4);
+          if ((bt & 7) == 0) {
+            atomicAdd(L.db + 8 * c + j, v);
+          }
+        }
+      }
+    } else {
+      // Thread = TMEM lane m of every M tile: group mg = m / 8 (copy ck, chunk), lane m % 8.
+      const int      m  = tid - 128;
+      const int      mg = m >> 3;
+      const int      ck = mg / inch;
+      const int      ci = 8 * (mg - ck * inch) + (m & 7);
+      const int      nc = mt * L.cout / 16; // 16-column pieces
+      float          acc[12][16];
+#pragma unroll
+      for (int p = 0; p < 12; ++p) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+          acc[p][q] = 0.f;
+        }
+      }
+      for (int i = 0; i < ngrp; ++i) {
+        const uint32_t grp = g0 + (uint32_t)i, set = grp & 1u;
+        bool           ok  = true;
+        if (lane == 0) {
+          ok = wait(bar_acc + 8u * set, (grp / 2) & 1u);
+        }
+        if (__shfl_sync(0xffffffffu, ok ? 1 : 0, 0) == 0) {
+          break;
+        }
+        tc_fence_after();
+        const uint32_t tad = tmem + 256u * set + ((uint32_t)((warp & 3) * 32) << 16);
+#pragma unroll
+        for (int p = 0; p < 12; ++p) {
+          if (p < nc) {
+            float v[16];
+            tmem_ld16(tad + 16u * (uint32_t)p, v);
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+              acc[p][q] += v[q];
+            }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(bar_read + 8u * set);
+        }
+      }
+      if (*abort_sm == 0) {
+        const int per = L.cout / 16; // pieces per M tile
+#pragma unroll
+        for (int p = 0; p < 12; ++p) {
+          const int j = p / per, tap = j * copies + ck;
+          if (p < nc && tap < kTapCount) {
+            float4* dst = reinterpret_cast<float4*>(L.dw + ((size_t)tap * L.cin + ci) * L.cout + (p - j * per) * 16);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              atomicAdd(dst + q, make_float4(acc[p][4 * q], acc[p][4 * q + 1], acc[p][4 * q + 2], acc[p][4 * q + 3]));
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();
+    if (*abort_sm != 0) {
+      break;
+    }
+    g0 += (uint32_t)ngrp;
+    k0 += (uint32_t)nt;
+    t += nt;
+  }
+  // After a failure: wait (bounded) for the copies and MMAs that may be in flight (a barrier's phase in
+  // flight is one of the two parities; the other returns at once).
+  if (*abort_sm != 0) {
+    if (tid == 0) {
+      mma_commit(bar_acc);
+    }
+    if (tid < kWgStages + 2) {
+      for (uint32_t ph = 0; ph < 2; ++ph) {
+        (void)mbar_wait_bounded(tid < kWgStages ? bar_full + 8u * tid : bar_acc + 8u * (tid - kWgStages), ph);
       }
     }
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
-    tmem_dealloc(tmem, C::kCols);
-  }
-}
-
-// Bias gradient db[co] += sum over rows of dY[r][co]: blockIdx.y = 8-channel chunk, grid-stride rows.
-__global__ void conv1d_bias_grad_kernel(const uint4* __restrict__ dy, int R, float* __restrict__ db)
-{
-  __shared__ float part[8];
-  const int c = blockIdx.y;
-  if (threadIdx.x < 8) {
-    part[threadIdx.x] = 0.f;
-  }
-  __syncthreads();
-  float acc[8] = {};
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < R; r += gridDim.x * blockDim.x) {
-    const uint4           v = dy[(size_t)c * R + r];
-    const __nv_bfloat16*  b = reinterpret_cast<const __nv_bfloat16*>(&v);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      acc[j] += __bfloat162float(b[j]);
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    float s = acc[j];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      s += __shfl_xor_sync(0xffffffffu, s, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-      atomicAdd(&part[j], s);
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < 8) {
-    atomicAdd(&db[8 * c + threadIdx.x], part[threadIdx.x]);
+    tmem_dealloc(tmem, kWgCols);
   }
 }
 
@@ -409,15 +535,6 @@ int fwd_setup()
 }
 
 template <int CIN, int COUT>
-int wg_setup()
-{
-  return cudaFuncSetAttribute(conv1d_wgrad_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)wg_cfg<CIN, COUT>::kSmem) == cudaSuccess
-             ? PG_OK
-             : PG_ERR_CUDA;
-}
-
-template <int CIN, int COUT>
 int fwd_launch(pg_context* ctx, const void* x, const void* w, const float* bias, const void* res, const void* mask,
                void* y, const uint8_t* row_valid, int R, int relu, int* err, cudaStream_t s)
 {
@@ -427,24 +544,6 @@ int fwd_launch(pg_context* ctx, const void* x, const void* w, const float* bias,
       static_cast<const uint4*>(x), static_cast<const uint4*>(w), bias, static_cast<const uint4*>(res),
       static_cast<const uint4*>(mask), static_cast<uint4*>(y), row_valid, R, relu, err);
   return pg::check_cuda(ctx, cudaGetLastError(), "conv1d_fwd_kernel launch");
-}
-
-template <int CIN, int COUT>
-int wg_launch(pg_context* ctx, const void* x, const void* dy, int R, float* dw, float* db, int* err, cudaStream_t s)
-{
-  const int ntiles = (R + kWgTile - 1) / kWgTile;
-  // At least four K tiles per CTA (fewer partial sums to add), at most two CTAs per SM.
-  const int per    = std::max(4, (ntiles + 2 * ctx->sm_count - 1) / (2 * ctx->sm_count));
-  const int grid   = (ntiles + per - 1) / per;
-  conv1d_wgrad_kernel<CIN, COUT><<<grid, kConvThreads, wg_cfg<CIN, COUT>::kSmem, s>>>(
-      static_cast<const uint4*>(x), static_cast<const uint4*>(dy), R, per, dw, err);
-  int rc = pg::check_cuda(ctx, cudaGetLastError(), "conv1d_wgrad_kernel launch");
-  if (rc == PG_OK && db != nullptr) {
-    const int bgrid = std::max(1, std::min((R + 255) / 256, ctx->sm_count));
-    conv1d_bias_grad_kernel<<<dim3(bgrid, COUT / 8), 256, 0, s>>>(static_cast<const uint4*>(dy), R, db);
-    rc = pg::check_cuda(ctx, cudaGetLastError(), "conv1d_bias_grad_kernel launch");
-  }
-  return rc;
 }
 
 } // namespace
@@ -460,14 +559,9 @@ int conv_setup(pg_context* ctx)
   if (rc == PG_OK) {
     rc = fwd_setup<64, 16>();
   }
-  if (rc == PG_OK) {
-    rc = wg_setup<16, 64>();
-  }
-  if (rc == PG_OK) {
-    rc = wg_setup<64, 64>();
-  }
-  if (rc == PG_OK) {
-    rc = wg_setup<64, 16>();
+  if (rc == PG_OK && cudaFuncSetAttribute(conv1d_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)kWgSmem) != cudaSuccess) {
+    rc = PG_ERR_CUDA;
   }
   if (rc != PG_OK) {
     (void)cudaGetLastError();
@@ -495,22 +589,25 @@ int conv_forward_launch(pg_context* ctx, int cin, int cout, const void* x, const
   return set_error(ctx, PG_ERR_INVALID, "conv1d: channel counts must be (16,64), (64,64) or (64,16)");
 }
 
-int conv_wgrad_launch(pg_context* ctx, int cin, int cout, const void* x, const void* dy, int R, float* dw, float* db,
-                      int* err, cudaStream_t s)
+int conv_wgrad_launch(pg_context* ctx, const wgrad_layer* layers, int n, int R, int* err, cudaStream_t s)
 {
-  if (R <= 0) {
+  if (R <= 0 || n <= 0) {
     return PG_OK;
   }
-  if (cin == 16 && cout == 64) {
-    return wg_launch<16, 64>(ctx, x, dy, R, dw, db, err, s);
+  wg_args args{};
+  for (int i = 0; i < n; ++i) {
+    const int ci = layers[i].cin, co = layers[i].cout;
+    if (n > kMaxWgradLayers || !((ci == 16 && co == 64) || (ci == 64 && co == 64) || (ci == 64 && co == 16))) {
+      return set_error(ctx, PG_ERR_INVALID, "conv1d: channel counts must be (16,64), (64,64) or (64,16)");
+    }
+    args.l[i] = layers[i];
   }
-  if (cin == 64 && cout == 64) {
-    return wg_launch<64, 64>(ctx, x, dy, R, dw, db, err, s);
-  }
-  if (cin == 64 && cout == 16) {
-    return wg_launch<64, 16>(ctx, x, dy, R, dw, db, err, s);
-  }
-  return set_error(ctx, PG_ERR_INVALID, "conv1d: channel counts must be (16,64), (64,64) or (64,16)");
+  args.n = n;
+  // At least four K tiles per CTA (fewer partial sums to add), at most one CTA per SM.
+  const long tiles = (long)n * ((R + kWgTile - 1) / kWgTile);
+  const int  grid  = (int)std::max(1l, std::min((long)ctx->sm_count, tiles / 4));
+  conv1d_wgrad_kernel<<<grid, kWgThreads, kWgSmem, s>>>(args, R, err);
+  return check_cuda(ctx, cudaGetLastError(), "conv1d_wgrad_kernel launch");
 }
 
 } // namespace pg
@@ -554,5 +651,6 @@ extern "C" int pg_conv1d_backward_weights_device(pg_context* ctx, int cin, int c
   if (x == nullptr || dy == nullptr || dw == nullptr || err == nullptr || rows < 0) {
     return pg::set_error(ctx, PG_ERR_INVALID, "conv1d weight gradient: null buffer or negative row count");
   }
-  return pg::conv_wgrad_launch(ctx, cin, cout, x, dy, rows, dw, db, err, static_cast<cudaStream_t>(stream));
+  const pg::wgrad_layer layer = {x, dy, dw, db, cin, cout};
+  return pg::conv_wgrad_launch(ctx, &layer, 1, rows, err, static_cast<cudaStream_t>(stream));
 }
