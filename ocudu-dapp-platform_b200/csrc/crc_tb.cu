@@ -291,6 +291,42 @@ int tb_assemble_launch(pg_context* ctx, const pg_tb_desc* tbs_dev, int n, const 
   return check_cuda(ctx, cudaGetLastError(), "tb_assemble_kernel launch");
 }
 
+std::vector<ldpc_tb_cb> tb_join_in_decoder(const std::vector<pg_tb_desc>& tbs, const std::vector<pg_ldpc_cb>& cbs)
+{
+  std::vector<ldpc_tb_cb> out(cbs.size());
+  for (size_t t = 0; t < tbs.size(); ++t) {
+    const pg_tb_desc& d = tbs[t];
+    uint32_t          g;
+    int               order;
+    crc_poly_params((int)d.crc_poly, &g, &order);
+    auto mulmod = [&](uint32_t a, uint32_t b) {
+      uint32_t p = 0;
+      for (int i = order - 1; i >= 0; --i) {
+        p <<= 1;
+        p ^= (p >> order) & 1u ? g : 0u;
+        p ^= (b >> i) & 1u ? a : 0u;
+      }
+      return p;
+    };
+    uint32_t xp = 1; // x^P by squaring
+    for (int i = 31; i >= 0 && d.nof_cbs > 1; --i) {
+      xp = mulmod(xp, xp);
+      if ((d.cb_payload_bits >> i) & 1u) {
+        xp = mulmod(xp, 2u);
+      }
+    }
+    uint32_t f = 1; // x^((C - 1 - c) P)
+    for (uint32_t c = d.nof_cbs; c-- > 0;) {
+      if (d.nof_cbs > 1 && (d.cb_payload_bits % 8 != 0 || cbs[d.cb_first + c].lifting_size % 2 != 0)) {
+        return {};
+      }
+      out[d.cb_first + c] = {(uint32_t)t, f};
+      f                   = mulmod(f, xp);
+    }
+  }
+  return out;
+}
+
 void tb_chunk_list(const pg_tb_desc* tbs, int n, std::vector<uint32_t>& out)
 {
   out.clear();

@@ -694,6 +694,7 @@ constexpr int      kOddMaxZ      = 16;   // odd lifting sizes are at most 15
 
 struct pair_shared {
   uint4    row[pg::kBg1Rows + 1]; // first padded edge, first message word, edges per thread, step end
+  uint32_t tb_crc;
   int      last;
   int      ragged;
   uint32_t crc[2];
@@ -901,6 +902,71 @@ __device__ __forceinline__ void fetch8(const int8_t* __restrict__ in, int k, int
   }
 }
 
+// a(x) b(x) mod g(x) for a of degree below `order` (Horner over the bits of b).
+__device__ __forceinline__ uint32_t gf2_mulmod_horner(uint32_t a, uint32_t b, uint32_t g, int order)
+{
+  uint32_t p = 0;
+  for (int i = order - 1; i >= 0; --i) {
+    p <<= 1;
+    p ^= (p >> order) & 1u ? g : 0u;
+    p ^= (b >> i) & 1u ? a : 0u;
+  }
+  return p;
+}
+
+// Transport-block join in the decoder (sink.tbs not null): codeblock cb's part of the TB is stored by its
+// decoder, and the last codeblock of a TB to arrive forms the TB's result, so that nothing follows the
+// decoder in a slot (a TB assembly and a result kernel after it, with two fills, took 16 to 20 us of a
+// slot). First payload byte of the codeblock in the TB, and the bytes it stores.
+__device__ __forceinline__ uint8_t* tb_part(const pg::ldpc_tb_sink& sink, const pg_tb_desc& t, const int cb, int& nb)
+{
+  const uint32_t off = (uint32_t)(cb - (int)t.cb_first) * t.cb_payload_bits / 8u; // whole bytes (checked by the host)
+  const uint32_t all = t.tbs_bits / 8u;
+  nb                 = (int)min((t.cb_payload_bits + 7u) / 8u, all > off ? all - off : 0u);
+  return sink.tb_out + t.tb_out_offset + off;
+}
+
+// Called by the first warp when its thread 0 has stored iterations[cb] and added the codeblock's CRC.
+__device__ __forceinline__ void tb_arrive(const pg::ldpc_tb_sink& sink, const pg_tb_desc& t, const uint32_t tb,
+                                          const int32_t* iterations)
+{
+  const int lane = threadIdx.x & 31;
+  int       last = 0;
+  if (lane == 0) {
+    __threadfence();
+    last = atomicAdd(&sink.arrivals[tb], 1) == (int)t.nof_cbs - 1;
+  }
+  if (__shfl_sync(0xffffffffu, last, 0) == 0) {
+    return;
+  }
+  __threadfence();
+  // pusch_decoder_result: C == 1, the codeblock CRC is the TB CRC; C > 1, every codeblock CRC and the TB
+  // CRC. A failed codeblock counts max_iterations (pusch_decoder_impl.cpp:612-710).
+  const uint32_t maxit = sink.ues[tb].max_iterations;
+  uint32_t       ok = 0, sum = 0, mx = 0;
+  for (uint32_t c = lane; c < t.nof_cbs; c += 32) {
+    const int32_t  it  = __ldcg(iterations + t.cb_first + c);
+    const uint32_t run = it > 0 ? (uint32_t)it : maxit;
+    ok += it > 0 ? 1u : 0u;
+    sum += run;
+    mx = max(mx, run);
+  }
+  ok  = __reduce_add_sync(0xffffffffu, ok);
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  mx  = __reduce_max_sync(0xffffffffu, mx);
+  if (lane == 0) {
+    const uint32_t crc   = atomicExch(&sink.crc[tb], 0u); // zero again for the next execution
+    sink.arrivals[tb]    = 0;
+    pg_sch_result r;
+    r.tb_crc_ok          = (ok == t.nof_cbs && (t.nof_cbs == 1 || crc == 0)) ? 1u : 0u;
+    r.nof_cbs            = t.nof_cbs;
+    r.nof_cbs_crc_ok     = ok;
+    r.mean_iterations    = (float)sum / (float)t.nof_cbs;
+    r.max_iterations_run = mx;
+    sink.results[tb]     = r;
+  }
+}
+
 // Decodes codeblock cb (even Z <= 2 NT / T) with T threads per lane pair; smem: smem_bytes of dynamic
 // shared memory (at least kPairMinSmem); slab: the CTA's global message slab.
 template <int T, int NT>
@@ -908,7 +974,7 @@ __device__ __forceinline__ void decode_codeblock_pair(const pg_ldpc_cb& d, pair_
                                                       const uint32_t smem_bytes, const int8_t* __restrict__ llrs,
                                                       uint8_t* __restrict__ bits, int32_t* __restrict__ iterations,
                                                       uint32_t* slab, const uint32_t* __restrict__ crc_pow,
-                                                      const int cb)
+                                                      const int cb, const pg::ldpc_tb_sink& sink)
 {
   constexpr int LG  = T == 2 ? 0 : 1; // index of the T-dependent tables
   const int     tid = threadIdx.x;
@@ -930,8 +996,15 @@ __device__ __forceinline__ void decode_codeblock_pair(const pg_ldpc_cb& d, pair_
   const int          msg_len  = Kb * Z;
   const int          n        = (int)d.nof_llrs;
   const int8_t*      in       = llrs + d.llr_offset;
-  const int          nbytes   = (msg_len + 7) / 8;
+  int                nbytes   = (msg_len + 7) / 8;
   uint8_t*           out      = bits + d.out_offset;
+  uint32_t           tbi      = 0; // TB of the codeblock
+  pg_tb_desc         td       = {};
+  if (sink.tbs != nullptr) {
+    tbi = sink.cbs[cb].tb;
+    td  = sink.tbs[tbi];
+    out = tb_part(sink, td, cb, nbytes);
+  }
   const int          crc_poly = d.crc_poly;
   const uint32_t     h4       = 4u * (uint32_t)H;
   const pair_tables& tb       = g_pair_tables;
@@ -970,6 +1043,7 @@ __device__ __forceinline__ void decode_codeblock_pair(const pg_ldpc_cb& d, pair_
   if (tid == 0) {
     sh.last   = 0;
     sh.ragged = 0;
+    sh.tb_crc = 0;
     sh.crc[0] = sh.crc[1] = 0;
     sh.zero[0] = sh.zero[1] = 0;
   }
@@ -1041,6 +1115,9 @@ __device__ __forceinline__ void decode_codeblock_pair(const pg_ldpc_cb& d, pair_
     }
     if (tid == 0) {
       iterations[cb] = 0;
+    }
+    if (sink.tbs != nullptr && tid < 32) {
+      tb_arrive(sink, td, tbi, iterations);
     }
     return;
   }
@@ -1157,7 +1234,7 @@ __device__ __forceinline__ void decode_codeblock_pair(const pg_ldpc_cb& d, pair_
   // reversal); message bit i of column c = i / Z, lane w = i mod Z is half (w >= H) of E[c][w mod H].
   {
     const uint32_t inv = 0xffffffffu / (uint32_t)Z + 1u;
-    for (int wi = tid >> 5; wi < (msg_len + 31) / 32; wi += NT / 32) {
+    for (int wi = tid >> 5; wi < (nbytes + 3) / 4; wi += NT / 32) {
       const int idx = 32 * wi + lane;
       bool      bit = false;
       if (idx < msg_len) {
@@ -1172,8 +1249,44 @@ __device__ __forceinline__ void decode_codeblock_pair(const pg_ldpc_cb& d, pair_
       }
     }
   }
+  if (sink.tbs != nullptr && td.nof_cbs > 1 && result > 0) {
+    // The payload's remainder, shifted to its place in the TB.
+    const uint32_t* ptab = crc_pow + (size_t)td.crc_poly * pg::kCrcPowLen;
+    const int       P    = (int)td.cb_payload_bits;
+    uint32_t        crc  = 0;
+    if (cgrp < ngrp) {
+      const int       k  = tid - cgrp * H;
+      const uint32_t* Ec = reinterpret_cast<const uint32_t*>(E) + H + k;
+#pragma unroll 4
+      for (int c = cgrp; c < Kb; c += ngrp) {
+        const uint32_t x  = Ec[c * H];
+        const int      i0 = c * Z + k, i1 = i0 + H;
+        if (pair_hard(x & 0xffffu) && i0 < P) {
+          crc ^= __ldg(ptab + (P - 1 - i0));
+        }
+        if (pair_hard(x >> 16) && i1 < P) {
+          crc ^= __ldg(ptab + (P - 1 - i1));
+        }
+      }
+    }
+    crc = __reduce_xor_sync(0xffffffffu, crc);
+    if (lane == 0 && crc != 0) {
+      atomicXor(&sh.tb_crc, crc);
+    }
+    __syncthreads();
+    if (tid == 0) {
+      uint32_t gp;
+      int      go;
+      pg::crc_poly_params((int)td.crc_poly, &gp, &go);
+      atomicXor(&sink.crc[tbi], gf2_mulmod_horner(sh.tb_crc, sink.cbs[cb].factor, gp, go));
+    }
+  }
   if (tid == 0) {
     iterations[cb] = result;
+  }
+  if (sink.tbs != nullptr && tid < 32) {
+    __syncwarp();
+    tb_arrive(sink, td, tbi, iterations);
   }
 }
 
@@ -1203,7 +1316,7 @@ __global__ void __launch_bounds__(kPairThreads, kPairPerSm)
     ldpc_decode_pair_kernel(const pg_ldpc_cb* __restrict__ descs, const int8_t* __restrict__ llrs,
                             uint8_t* __restrict__ bits, int32_t* __restrict__ iterations, int8_t* __restrict__ c2v_all,
                             const uint32_t* __restrict__ crc_pow, const uint32_t* __restrict__ order, int n,
-                            int* __restrict__ counter, uint32_t smem_bytes)
+                            int* __restrict__ counter, uint32_t smem_bytes, const __grid_constant__ pg::ldpc_tb_sink sink)
 {
   extern __shared__ __align__(16) unsigned char smem_pair[];
   __shared__ pair_shared sh;
@@ -1217,13 +1330,27 @@ __global__ void __launch_bounds__(kPairThreads, kPairPerSm)
       if (Z < kOddMaxZ) {
         decode_codeblock<0, NT, kOddMaxZ>(d, *reinterpret_cast<smem_scalar_t<NT, kOddMaxZ>*>(smem_pair), llrs, bits,
                                           iterations, reinterpret_cast<int8_t*>(slab), crc_pow, cb, 0);
+        if (sink.tbs != nullptr) {
+          // A TB of one codeblock (checked by the host): its bytes are the first of the decoded bits.
+          const uint32_t   tb = sink.cbs[cb].tb;
+          const pg_tb_desc td = sink.tbs[tb];
+          int              nb;
+          uint8_t*         out = tb_part(sink, td, cb, nb);
+          __syncthreads();
+          for (int b = threadIdx.x; b < nb; b += NT) {
+            out[b] = bits[d.out_offset + b];
+          }
+          if (threadIdx.x < 32) {
+            tb_arrive(sink, td, tb, iterations);
+          }
+        }
       } else if (threadIdx.x == 0) {
         iterations[cb] = -1;
       }
     } else if (Z <= NT / 2) {
-      decode_codeblock_pair<4, NT>(d, sh, smem_pair, smem_bytes, llrs, bits, iterations, slab, crc_pow, cb);
+      decode_codeblock_pair<4, NT>(d, sh, smem_pair, smem_bytes, llrs, bits, iterations, slab, crc_pow, cb, sink);
     } else {
-      decode_codeblock_pair<2, NT>(d, sh, smem_pair, smem_bytes, llrs, bits, iterations, slab, crc_pow, cb);
+      decode_codeblock_pair<2, NT>(d, sh, smem_pair, smem_bytes, llrs, bits, iterations, slab, crc_pow, cb, sink);
     }
     if (n <= (int)gridDim.x) {
       break;
@@ -1574,13 +1701,13 @@ int ldpc_resident_ctas(pg_context* ctx)
 
 int ldpc_launch_persistent(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* bits,
                            int32_t* iterations, int8_t* c2v, const uint32_t* order, int* counter,
-                           cudaStream_t stream, int max_ctas, int kernel)
+                           cudaStream_t stream, int max_ctas, int kernel, const ldpc_tb_sink* sink, bool counter_zero)
 {
   if (n == 0) {
     return PG_OK;
   }
   const int grid = std::max(1, std::min(n, max_ctas));
-  if (n > grid || kernel == PG_LDPC_KERNEL_ONE_LANE) {
+  if (!counter_zero && (n > grid || kernel == PG_LDPC_KERNEL_ONE_LANE)) {
     if (int rc = check_cuda(ctx, cudaMemsetAsync(counter, 0, sizeof(int), stream), "cudaMemsetAsync(ldpc counter)")) {
       return rc;
     }
@@ -1593,7 +1720,8 @@ int ldpc_launch_persistent(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, 
   if (kernel != PG_LDPC_KERNEL_ONE_LANE) {
     const int smem = pair_smem((grid + ctx->sm_count - 1) / ctx->sm_count);
     ldpc_decode_pair_kernel<<<grid, kPairThreads, smem, stream>>>(descs_dev, llrs, bits, iterations, c2v,
-                                                                  ctx->dev.crc_pow, order, n, counter, (uint32_t)smem);
+                                                                  ctx->dev.crc_pow, order, n, counter, (uint32_t)smem,
+                                                                  sink != nullptr ? *sink : ldpc_tb_sink{});
     rc = check_cuda(ctx, cudaGetLastError(), "ldpc_decode_pair_kernel launch");
   } else {
     ldpc_decode_kernel<<<grid, kThreads, 0, stream>>>(descs_dev, llrs, bits, iterations, c2v, ctx->dev.crc_pow, order,

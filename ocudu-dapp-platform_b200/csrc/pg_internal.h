@@ -166,8 +166,9 @@ int rate_dematch_launch(pg_context* ctx, const pg_rm_cb* descs_dev, int n, const
 // Writes what rate dematching leaves at the positions no LLR reaches (+127 at the fillers, 0
 // elsewhere) over the whole circular buffer of every codeblock with placed[c] = 1, to be done
 // before the demodulator stores those codeblocks' LLRs in place.
+// The same launch zeroes tb_out (tb_bytes) and *counter.
 int rm_prefill_launch(pg_context* ctx, const pg_rm_cb* descs_dev, int n, const uint8_t* placed, int8_t* out,
-                      cudaStream_t stream);
+                      uint8_t* tb_out, size_t tb_bytes, int* counter, cudaStream_t stream);
 void crc_tables_host(uint32_t* tab);
 int crc_launch(pg_context* ctx, const pg_crc_item* items_dev, int n, const uint8_t* data, uint32_t* out,
                cudaStream_t stream);
@@ -270,15 +271,36 @@ int ldpc_launch_scratch(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, con
 // Hardest-first work order (ldpc_score_kernel + ldpc_sort_kernel): keys n bytes, order n entries.
 int ldpc_order_launch(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* keys,
                       uint32_t* order, cudaStream_t stream);
+// Transport-block join of the lane-pair decoder: with tbs set, codeblock cb's payload goes to its place in
+// tb_out instead of the decoder's bit output, and the last codeblock of each TB writes results[tb]. Every
+// TB has one codeblock, or codeblocks of an even lifting size with payloads of whole bytes
+// (tb_join_in_decoder). cbs[cb]: TB and x^((C - 1 - c) P) mod the TB's CRC polynomial for codeblock c of C
+// with P payload bits. crc and arrivals (one entry per TB) are zero before a launch and after it.
+struct ldpc_tb_cb {
+  uint32_t tb;
+  uint32_t factor;
+};
+struct ldpc_tb_sink {
+  const pg_tb_desc*  tbs      = nullptr;
+  const pg_pusch_ue* ues      = nullptr;
+  const ldpc_tb_cb*  cbs      = nullptr;
+  uint8_t*           tb_out   = nullptr;
+  uint32_t*          crc      = nullptr;
+  int*               arrivals = nullptr;
+  pg_sch_result*     results  = nullptr;
+};
+// The entries of ldpc_tb_sink::cbs for the TBs of a work list; empty when a TB needs the separate join.
+std::vector<ldpc_tb_cb> tb_join_in_decoder(const std::vector<pg_tb_desc>& tbs, const std::vector<pg_ldpc_cb>& cbs);
 // CTAs a launch of the kernel (pg_ldpc_kernel) may have with per_sm of them on each SM, within the
 // kernel's own limit.
 int ldpc_max_ctas(const pg_context* ctx, int per_sm, int kernel);
 // Persistent launch: min(n, max_ctas) CTAs (max_ctas from ldpc_max_ctas) take codeblocks order[0..n)
-// (identity when order is null) from *counter (device int, zeroed here on the stream); c2v holds one
-// slab (kPairSlab bytes) per CTA.
+// (identity when order is null) from *counter (device int, zeroed here on the stream unless counter_zero);
+// c2v holds one slab (kPairSlab bytes) per CTA.
 int ldpc_launch_persistent(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* bits,
                            int32_t* iterations, int8_t* c2v, const uint32_t* order, int* counter,
-                           cudaStream_t stream, int max_ctas, int kernel);
+                           cudaStream_t stream, int max_ctas, int kernel, const ldpc_tb_sink* sink = nullptr,
+                           bool counter_zero = false);
 // CTAs of ldpc_decode_kernel resident on the whole device.
 int ldpc_resident_ctas(pg_context* ctx);
 

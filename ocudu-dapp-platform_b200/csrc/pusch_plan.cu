@@ -100,6 +100,8 @@ struct pg_pusch_plan {
   int8_t*         d_c2v    = nullptr;
   uint32_t*       d_order  = nullptr; // per-execution work order (device ordering)
   uint32_t*       d_order_static = nullptr; // largest codeblocks first, fixed at creation
+  ldpc_tb_cb*     d_tb_cbs       = nullptr; // TB join in the decoder (null: separate kernels)
+  uint32_t*       d_join         = nullptr; // its per-TB CRC and arrival words, zero between executions
   uint32_t*       d_tb_chunks    = nullptr; // TB-assembly work items (TB | chunk << 16)
   int             tb_nchunks     = 0;
   uint8_t*        d_keys   = nullptr; // work-order keys of the codeblocks // LDPC work order: largest codeblocks first
@@ -273,6 +275,12 @@ bool ldpc_ordered(const pg_pusch_plan* p)
   return p->tuning.ldpc_order != 0 && p->nof_cbs > ldpc_ctas(p);
 }
 
+// Whether the decoder joins the TBs and writes the results (the lane-pair kernel, TBs it can join).
+bool joined(const pg_pusch_plan* p)
+{
+  return p->d_tb_cbs != nullptr && p->tuning.ldpc_kernel != PG_LDPC_KERNEL_ONE_LANE;
+}
+
 int enqueue(pg_pusch_plan* p, const uint32_t* grids, uint8_t* tb_out, pg_sch_result* results,
             pg_port_result* port_results, cudaStream_t s)
 {
@@ -284,7 +292,7 @@ int enqueue(pg_pusch_plan* p, const uint32_t* grids, uint8_t* tb_out, pg_sch_res
     rc = check_cuda(ctx, cudaStreamWaitEvent(p->aux, p->ev_fork, 0), "cudaStreamWaitEvent(fork)");
   }
   if (rc == PG_OK) {
-    rc = rm_prefill_launch(ctx, p->d_rm, p->nof_cbs, p->d_placed, p->d_rm_out, p->aux);
+    rc = rm_prefill_launch(ctx, p->d_rm, p->nof_cbs, p->d_placed, p->d_rm_out, tb_out, p->tb_bytes, p->d_counter, p->aux);
   }
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaEventRecord(p->ev_join, p->aux), "cudaEventRecord(join)");
@@ -347,21 +355,22 @@ int enqueue(pg_pusch_plan* p, const uint32_t* grids, uint8_t* tb_out, pg_sch_res
     rc    = ldpc_order_launch(ctx, p->d_ldpc, p->nof_cbs, p->d_rm_out, p->d_keys, p->d_order, s);
     order = p->d_order;
   }
+  ldpc_tb_sink sink;
+  if (joined(p)) {
+    sink = {p->d_tb, p->d_ues, p->d_tb_cbs, tb_out, p->d_join, reinterpret_cast<int*>(p->d_join + p->nof_ues), results};
+  }
   if (rc == PG_OK) {
     rc = ldpc_launch_persistent(ctx, p->d_ldpc, p->nof_cbs, p->d_rm_out, p->d_cb_bits, p->d_iters, p->d_c2v,
-                                order, p->d_counter, s, ldpc_ctas(p), p->tuning.ldpc_kernel);
+                                order, p->d_counter, s, ldpc_ctas(p), p->tuning.ldpc_kernel, &sink, true);
   }
-  if (rc == PG_OK) {
-    rc = check_cuda(ctx, cudaMemsetAsync(tb_out, 0, p->tb_bytes, s), "cudaMemsetAsync(tb)");
-  }
-  if (rc == PG_OK) {
+  if (rc == PG_OK && !joined(p)) {
     rc = tb_assemble_launch(ctx, p->d_tb, p->nof_ues, p->d_cb_bits, p->d_cb_off, tb_out, p->d_tb_crc, s, p->d_tb_chunks,
                             p->tb_nchunks);
-  }
-  if (rc == PG_OK) {
-    sch_results_kernel<<<(p->nof_ues + 127) / 128, 128, 0, s>>>(p->d_tb, p->d_ues, p->nof_ues, p->d_iters, p->d_tb_crc,
-                                                                 results);
-    rc = check_cuda(ctx, cudaGetLastError(), "sch_results_kernel launch");
+    if (rc == PG_OK) {
+      sch_results_kernel<<<(p->nof_ues + 127) / 128, 128, 0, s>>>(p->d_tb, p->d_ues, p->nof_ues, p->d_iters,
+                                                                   p->d_tb_crc, results);
+      rc = check_cuda(ctx, cudaGetLastError(), "sch_results_kernel launch");
+    }
   }
   if (rc == PG_OK && p->uci_w.nitems > 0 && p->polar_n > 0) {
     rc = check_cuda(ctx, cudaStreamWaitEvent(s, p->ev_ujoin, 0), "cudaStreamWaitEvent(UCI join)");
@@ -634,7 +643,9 @@ int pg_pusch_plan_create_uci(pg_context* ctx, const pg_pusch_ue* ues, const pg_p
   tb_chunk_list(w.tbd.data(), (int)w.tbd.size(), tb_chunks);
   p->tb_nchunks         = (int)tb_chunks.size();
   const size_t o_tbch   = o_ostat + al(order.size() * 4);
-  const size_t o_seqoff = o_tbch + al(tb_chunks.size() * 4);
+  const std::vector<ldpc_tb_cb> join = tb_join_in_decoder(w.tbd, w.ldpc);
+  const size_t o_join   = o_tbch + al(tb_chunks.size() * 4);
+  const size_t o_seqoff = o_join + al(join.size() * sizeof(ldpc_tb_cb));
   const size_t o_reoff  = o_seqoff + al((size_t)nof_ues * 4);
   std::vector<uint32_t> est_work;
   uint32_t              pilot_words = 0;
@@ -674,7 +685,8 @@ int pg_pusch_plan_create_uci(pg_context* ctx, const pg_pusch_ue* ues, const pg_p
   const size_t o_uvalid = o_ubits + al((size_t)nof_ues * sizeof(pg_pusch_uci_result));
   const size_t o_polb   = o_uvalid + al((size_t)std::max(1, p->uci_nmsg));
   const size_t o_pbits  = o_polb + al(polar_bits_total);
-  p->dev_bytes          = o_pbits + al((size_t)pilot_words * 4);
+  const size_t o_jwords = o_pbits + al((size_t)pilot_words * 4);
+  p->dev_bytes          = o_jwords + al((size_t)nof_ues * 8);
 
   const size_t h_res  = 0;
   const size_t h_pr   = h_res + al((size_t)nof_ues * sizeof(pg_sch_result));
@@ -743,6 +755,11 @@ int pg_pusch_plan_create_uci(pg_context* ctx, const pg_pusch_ue* ues, const pg_p
   std::memcpy(h + o_order, order.data(), order.size() * 4);
   std::memcpy(h + o_ostat, order.data(), order.size() * 4);
   std::memcpy(h + o_tbch, tb_chunks.data(), tb_chunks.size() * 4);
+  if (!join.empty()) {
+    p->d_tb_cbs = reinterpret_cast<ldpc_tb_cb*>(b + o_join);
+    std::memcpy(h + o_join, join.data(), join.size() * sizeof(ldpc_tb_cb));
+  }
+  p->d_join = reinterpret_cast<uint32_t*>(b + o_jwords);
   std::memcpy(h + o_seqoff, seq_off.data(), (size_t)nof_ues * 4);
   std::memcpy(h + o_reoff, tile_map.data(), tile_map.size() * 4);
   std::memcpy(h + o_ework, est_work.data(), est_work.size() * 4);
@@ -769,6 +786,9 @@ int pg_pusch_plan_create_uci(pg_context* ctx, const pg_pusch_ue* ues, const pg_p
   }
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaMemsetAsync(b + o_earr, 0, (size_t)nof_ues * 16, s), "cudaMemsetAsync(arrivals)");
+  }
+  if (rc == PG_OK) {
+    rc = check_cuda(ctx, cudaMemsetAsync(p->d_join, 0, (size_t)nof_ues * 8, s), "cudaMemsetAsync(TB join)");
   }
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaMemsetAsync(b + o_ubits, 0, (size_t)nof_ues * sizeof(pg_pusch_uci_result), s),
@@ -813,11 +833,11 @@ int pg_pusch_plan_info(const pg_pusch_plan* plan, pg_pusch_plan_info_t* info)
   info->device_bytes   = plan->dev_bytes;
   // The kernels enqueue() launches: prefill, estimation, [learned: features, network, corrections],
   // demodulation, [UCI: demultiplexing, detection], [rate dematching of the codeblocks not placed],
-  // [device work order: score, sort], LDPC, TB assembly, results.
+  // [device work order: score, sort], LDPC [separate join: TB assembly, results].
   info->nof_kernels = 2u + (plan->le_net != nullptr ? 3u : 0u) + 1u + (plan->uci_w.nitems > 0 ? 1u : 0u) +
                       (plan->uci_nshort > 0 ? 1u : 0u) + (plan->polar_n > 0 ? 1u : 0u) +
                       (plan->unplaced.empty() ? 0u : 1u) + (ldpc_ordered(plan) ? 2u : 0u) +
-                      3u;
+                      (joined(plan) ? 1u : 3u);
   info->h2d_grid_bytes = (uint32_t)std::min<size_t>(plan->h2d_grid_bytes, 0xffffffffu);
   return PG_OK;
 }

@@ -173,8 +173,29 @@ __global__ void __launch_bounds__(kRmThreads) rate_dematch_kernel(const pg_rm_cb
 // boundary are stored one by one.
 __global__ void __launch_bounds__(kRmThreads) rm_prefill_kernel(const pg_rm_cb* __restrict__ cbs,
                                                                 const uint8_t* __restrict__ placed,
-                                                                int8_t* __restrict__ out_all)
+                                                                int8_t* __restrict__ out_all, uint8_t* __restrict__ tb_out,
+                                                                size_t tb_bytes, int* __restrict__ counter)
 {
+  // The TB buffer (bytes between the TBs stay zero) and the decoders' work counter.
+  {
+    const size_t nthr = (size_t)gridDim.x * gridDim.y * kRmThreads;
+    const size_t t0   = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kRmThreads + threadIdx.x;
+    const size_t head = min(tb_bytes, (size_t)((16u - (unsigned)(reinterpret_cast<uintptr_t>(tb_out) & 15u)) & 15u));
+    const size_t nvec = (tb_bytes - head) / 16;
+    uint4*       v    = reinterpret_cast<uint4*>(tb_out + head);
+    for (size_t q = t0; q < nvec; q += nthr) {
+      v[q] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    if (t0 < head) {
+      tb_out[t0] = 0;
+    }
+    if (head + 16 * nvec + t0 < tb_bytes) {
+      tb_out[head + 16 * nvec + t0] = 0;
+    }
+    if (t0 == 0) {
+      *counter = 0;
+    }
+  }
   if (placed[blockIdx.x] == 0) {
     return;
   }
@@ -276,13 +297,13 @@ int rate_dematch_launch(pg_context* ctx, const pg_rm_cb* descs_dev, int n, const
 }
 
 int rm_prefill_launch(pg_context* ctx, const pg_rm_cb* descs_dev, int n, const uint8_t* placed, int8_t* out,
-                      cudaStream_t stream)
+                      uint8_t* tb_out, size_t tb_bytes, int* counter, cudaStream_t stream)
 {
   if (n == 0) {
     return PG_OK;
   }
   // N <= 25,344 bytes = 1,584 chunks: two CTAs of 256 threads per codeblock, about three stores each.
-  rm_prefill_kernel<<<dim3(n, 2), kRmThreads, 0, stream>>>(descs_dev, placed, out);
+  rm_prefill_kernel<<<dim3(n, 2), kRmThreads, 0, stream>>>(descs_dev, placed, out, tb_out, tb_bytes, counter);
   return check_cuda(ctx, cudaGetLastError(), "rm_prefill_kernel launch");
 }
 
