@@ -146,34 +146,49 @@ __device__ __forceinline__ float2 cmulconjf(float2 a, float2 b) // a * conj(b)
   return make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
 }
 
-__device__ void virtual_pilots(float2* out, const float2* base, int nv, bool is_start)
+// Virtual pilots of one end of one sequence, by a group of eight lanes (lane i of the group is pilot i;
+// nv <= 8): linear fit of |h| and of the unwrapped arg(h) over nv pilots (port_channel_estimator_helpers.cpp
+// compute_v_pilots / add_v_pilots), evaluated at the nv positions before or after them. The magnitudes,
+// arguments and output phases are formed one per lane; every lane takes the sums over the pilots in
+// pilot order. Latency-bound: by one thread the chain of hypotf, atan2f and sincosf made the estimation of a
+// one-UE slot 9.5 us and of a 16-cell slot 17.4 us; by groups 6.8 and 14.7 us. `on` (alike in a group):
+// the group has pilots to write; the whole warp calls.
+constexpr int kVGroup = 8;
+
+__device__ __forceinline__ void virtual_pilots(float2* out, const float2* base, int nv, bool is_start, bool on)
 {
-  // Linear fit of |h| and of the unwrapped arg(h) over nv pilots (port_channel_estimator_helpers.cpp
-  // compute_v_pilots / add_v_pilots), evaluated at the nv positions before or after them.
+  const int i = (int)(threadIdx.x & (kVGroup - 1));
+  float     a = 0.f, g = 0.f;
+  if (on && i < nv) {
+    a = hypotf(base[i].x, base[i].y);
+    g = atan2f(base[i].y, base[i].x);
+  }
   float arg_prev = 0.f, acc = 0.f;
   float mean_abs = 0.f, mean_arg = 0.f, sxa = 0.f, sxg = 0.f;
-  float args[kMaxV], abss[kMaxV];
-  for (int i = 0; i < nv; ++i) {
-    const float a = hypotf(base[i].x, base[i].y);
-    float       g = atan2f(base[i].y, base[i].x);
-    if (i > 0) {
-      // unwrap: keep consecutive differences within (-pi, pi].
-      float d = g - arg_prev;
-      if (d > 3.14159265358979f) {
-        acc -= 6.28318530717959f;
-      } else if (d < -3.14159265358979f) {
-        acc += 6.28318530717959f;
+#pragma unroll
+  for (int k = 0; k < kVGroup; ++k) {
+    const float ak = __shfl_sync(0xffffffffu, a, k, kVGroup);
+    const float gk = __shfl_sync(0xffffffffu, g, k, kVGroup);
+    if (k < nv) {
+      if (k > 0) {
+        // unwrap: keep consecutive differences within (-pi, pi].
+        const float d = gk - arg_prev;
+        if (d > 3.14159265358979f) {
+          acc -= 6.28318530717959f;
+        } else if (d < -3.14159265358979f) {
+          acc += 6.28318530717959f;
+        }
       }
+      arg_prev        = gk;
+      const float arg = gk + acc;
+      mean_abs += ak;
+      mean_arg += arg;
+      sxa += ak * (float)k;
+      sxg += arg * (float)k;
     }
-    arg_prev = g;
-    abss[i]  = a;
-    args[i]  = g + acc;
   }
-  for (int i = 0; i < nv; ++i) {
-    mean_abs += abss[i];
-    mean_arg += args[i];
-    sxa += abss[i] * (float)i;
-    sxg += args[i] * (float)i;
+  if (!on || i >= nv) {
+    return;
   }
   mean_abs /= (float)nv;
   mean_arg /= (float)nv;
@@ -185,13 +200,11 @@ __device__ void virtual_pilots(float2* out, const float2* base, int nv, bool is_
   const float sg     = (sxg - mean_x * mean_arg * (float)nv) / den;
   const float ig     = mean_arg - sg * mean_x;
   const int   voff   = is_start ? -nv : nv;
-  for (int i = 0; i < nv; ++i) {
-    const float iv  = (float)(i + voff);
-    const float rho = sa * iv + ia;
-    float       s, c;
-    sincosf(sg * iv + ig + (rho > 0.f ? 0.f : 3.14159265358979f), &s, &c);
-    out[i] = make_float2(fabsf(rho) * c, fabsf(rho) * s);
-  }
+  const float iv     = (float)(i + voff);
+  const float rho    = sa * iv + ia;
+  float       s, c;
+  sincosf(sg * iv + ig + (rho > 0.f ? 0.f : 3.14159265358979f), &s, &c);
+  out[i] = make_float2(fabsf(rho) * c, fabsf(rho) * s);
 }
 
 __global__ void __launch_bounds__(kEstThreads) pusch_estimate_kernel(const pg_pusch_ue* __restrict__ ues,
@@ -321,14 +334,11 @@ __global__ void __launch_bounds__(kEstThreads) pusch_estimate_kernel(const pg_pu
   const int ntaps = tsel == 2 ? 15 : (tsel == 1 ? 11 : 5);
   const int mid   = ntaps / 2;
   const int nv    = nrb == 1 ? npil : mid;
-  if (tid < nd * nl * 2) {
-    const int d = tid / (nl * 2), l = (tid / 2) % nl, side = tid & 1;
+  if (tid < 64) { // eight groups: up to two DM-RS symbols, two layers, both ends
+    const int q = tid / kVGroup, d = min(q / (nl * 2), nd - 1), l = (q / 2) % nl, side = q & 1;
     float2*   e = ext(d, l);
-    if (side == 0) {
-      virtual_pilots(e + kMaxV - nv, e + kMaxV, nv, true);
-    } else {
-      virtual_pilots(e + kMaxV + npil, e + kMaxV + npil - nv, nv, false);
-    }
+    virtual_pilots(side == 0 ? e + kMaxV - nv : e + kMaxV + npil, side == 0 ? e + kMaxV : e + kMaxV + npil - nv, nv,
+                   side == 0, q < nd * nl * 2);
   }
   __syncthreads();
   // The smoothed pilots go straight to the even subcarriers of the output; the odd ones are filled
@@ -558,14 +568,11 @@ __global__ void __launch_bounds__(kChunkThreads) pusch_estimate_chunk_kernel(con
   const int mid   = ntaps / 2;
   const int nv    = nrb == 1 ? npil : mid;
   const int ks    = min(k1 + 1, npil); // smoothed pilots k0 .. ks - 1
-  if (tid < nd * nl * 2) {
-    const int d = tid / (nl * 2), l = (tid / 2) % nl, side = tid & 1;
+  if (tid < 64) { // eight groups: up to two DM-RS symbols, two layers, both ends
+    const int q = tid / kVGroup, d = min(q / (nl * 2), nd - 1), l = (q / 2) % nl, side = q & 1;
     float2*   e = s_ls[d][l];
-    if (side == 0 && k0 == 0) {
-      virtual_pilots(e - nv - t0, e - t0, nv, true);
-    } else if (side == 1 && ks - 1 + mid >= npil) {
-      virtual_pilots(e + npil - t0, e + npil - nv - t0, nv, false);
-    }
+    virtual_pilots(side == 0 ? e - nv - t0 : e + npil - t0, side == 0 ? e - t0 : e + npil - nv - t0, nv, side == 0,
+                   q < nd * nl * 2 && (side == 0 ? k0 == 0 : ks - 1 + mid >= npil));
   }
   __syncthreads();
 
