@@ -51,22 +51,23 @@ struct pg_pusch_plan {
   void*           dev      = nullptr;
   pg_pusch_ue*    d_ues    = nullptr;
   // UCI on PUSCH: the demultiplexer's device blob and work shape, the detector's message items,
-  // the UCI soft bits, detected bits (pg_pusch_uci_result layout per UE) and validity per message.
+  // the UCI soft bits; in pinned host memory, which the decoders store to, the detected bits
+  // (pg_pusch_uci_result layout per UE) and validity per message.
   void*           d_uci_blob  = nullptr;
   uci_demux_work  uci_w;
   void*           d_uci_items = nullptr;
   int             uci_nmsg    = 0;
   int8_t*         d_uci_llr   = nullptr;
-  uint8_t*        d_uci_bits  = nullptr;
-  uint8_t*        d_uci_valid = nullptr;
+  uint8_t*        uci_bits    = nullptr;
+  uint8_t*        uci_valid   = nullptr;
   std::vector<int> uci_msg_ue, uci_msg_kind; // per message: UE and 0 HARQ-ACK / 1 CSI Part 1
   // Polar-coded messages (after the short-block ones in the message order): their descriptors,
-  // their decoded bits, and per message the bit offset (in the short-block results or the polar
+  // their decoded bits (pinned host memory), and per message the bit offset (in the short-block results or the polar
   // bits) and the size.
   int              uci_nshort   = 0;
   int              polar_n      = 0;
   void*            d_polar_cbs  = nullptr;
-  uint8_t*         d_polar_bits = nullptr;
+  uint8_t*         polar_bits   = nullptr;
   std::vector<uint32_t> uci_msg_off, uci_msg_nbits;
   rm_direct*      d_direct   = nullptr; // per UE: fused rate-dematch placement of the demodulator
   uint8_t*        d_placed   = nullptr; // per codeblock: 1 when the demodulator places its LLRs
@@ -77,8 +78,9 @@ struct pg_pusch_plan {
   cudaStream_t    aux        = nullptr;
   cudaEvent_t     ev_fork    = nullptr;
   cudaEvent_t     ev_join    = nullptr;
-  cudaEvent_t     ev_ufork   = nullptr; // polar UCI decoding on the aux stream, beside the UL-SCH stages
+  cudaEvent_t     ev_ufork   = nullptr; // UCI decoding on the aux stream, beside the UL-SCH stages
   cudaEvent_t     ev_ujoin   = nullptr;
+  cudaEvent_t     ev_uread   = nullptr; // orders the host's reads of the UCI results
   uint32_t*       d_est_work = nullptr; // channel-estimation work list and per-(UE, port) first items
   void*           d_est_part = nullptr; // its partial sums
   int*            d_est_arr  = nullptr; // per-(UE, port) arrival counters, zero between executions
@@ -289,6 +291,10 @@ int enqueue(pg_pusch_plan* p, const uint32_t* grids, uint8_t* tb_out, pg_sch_res
   // execution on this stream, whose decoder read the buffers, precedes the fork).
   int rc = check_cuda(ctx, cudaEventRecord(p->ev_fork, s), "cudaEventRecord(fork)");
   if (rc == PG_OK) {
+    rc = estimate_launch(ctx, p->d_ues, p->nof_ues, p->d_est_work, p->est_nwork, p->d_est_part, p->d_est_arr, grids,
+                         p->d_est, p->le_net != nullptr ? p->d_ls : nullptr, port_results, s, p->d_pilot_bits);
+  }
+  if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaStreamWaitEvent(p->aux, p->ev_fork, 0), "cudaStreamWaitEvent(fork)");
   }
   if (rc == PG_OK) {
@@ -296,10 +302,6 @@ int enqueue(pg_pusch_plan* p, const uint32_t* grids, uint8_t* tb_out, pg_sch_res
   }
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaEventRecord(p->ev_join, p->aux), "cudaEventRecord(join)");
-  }
-  if (rc == PG_OK) {
-    rc = estimate_launch(ctx, p->d_ues, p->nof_ues, p->d_est_work, p->est_nwork, p->d_est_part, p->d_est_arr, grids,
-                         p->d_est, p->le_net != nullptr ? p->d_ls : nullptr, port_results, s, p->d_pilot_bits);
   }
   if (rc == PG_OK && p->le_net != nullptr) {
     const unsigned int flags = timing_record_flags(ctx, s);
@@ -326,23 +328,23 @@ int enqueue(pg_pusch_plan* p, const uint32_t* grids, uint8_t* tb_out, pg_sch_res
     // UCI UEs: their codewords into the UL-SCH stream (in the codeword buffer, after the codewords)
     // and the HARQ-ACK / CSI Part 1 streams, then the short-block detection of the messages.
     rc = uci_demux_launch(ctx, p->d_uci_blob, p->uci_w, p->d_llr, p->d_llr, p->d_uci_llr, p->d_uci_llr, s);
+    // The UCI decoders read only the demultiplexed UCI streams: a branch of their own that overlaps rate
+    // dematching and LDPC decoding, joined at the end.
     if (rc == PG_OK) {
-      rc = uci_detect_launch(ctx, p->d_uci_items, p->uci_nshort, p->d_uci_llr, p->d_uci_bits, p->d_uci_valid, s);
+      rc = check_cuda(ctx, cudaEventRecord(p->ev_ufork, s), "cudaEventRecord(UCI fork)");
+    }
+    if (rc == PG_OK) {
+      rc = check_cuda(ctx, cudaStreamWaitEvent(p->aux, p->ev_ufork, 0), "cudaStreamWaitEvent(UCI fork)");
     }
     if (rc == PG_OK && p->polar_n > 0) {
-      // The polar decoders read only the demultiplexed UCI streams: a branch of their own that
-      // overlaps rate dematching and LDPC decoding, joined at the end.
-      rc = check_cuda(ctx, cudaEventRecord(p->ev_ufork, s), "cudaEventRecord(UCI fork)");
-      if (rc == PG_OK) {
-        rc = check_cuda(ctx, cudaStreamWaitEvent(p->aux, p->ev_ufork, 0), "cudaStreamWaitEvent(UCI fork)");
-      }
-      if (rc == PG_OK) {
-        rc = uci_polar_launch_dev(ctx, p->d_polar_cbs, p->polar_n, p->d_uci_llr, p->d_polar_bits,
-                                  p->d_uci_valid + p->uci_nshort, p->aux);
-      }
-      if (rc == PG_OK) {
-        rc = check_cuda(ctx, cudaEventRecord(p->ev_ujoin, p->aux), "cudaEventRecord(UCI join)");
-      }
+      rc = uci_polar_launch_dev(ctx, p->d_polar_cbs, p->polar_n, p->d_uci_llr, p->polar_bits,
+                                p->uci_valid + p->uci_nshort, p->aux);
+    }
+    if (rc == PG_OK) {
+      rc = uci_detect_launch(ctx, p->d_uci_items, p->uci_nshort, p->d_uci_llr, p->uci_bits, p->uci_valid, p->aux);
+    }
+    if (rc == PG_OK) {
+      rc = check_cuda(ctx, cudaEventRecord(p->ev_ujoin, p->aux), "cudaEventRecord(UCI join)");
     }
   }
   if (rc == PG_OK && !p->unplaced.empty()) {
@@ -372,7 +374,7 @@ int enqueue(pg_pusch_plan* p, const uint32_t* grids, uint8_t* tb_out, pg_sch_res
       rc = check_cuda(ctx, cudaGetLastError(), "sch_results_kernel launch");
     }
   }
-  if (rc == PG_OK && p->uci_w.nitems > 0 && p->polar_n > 0) {
+  if (rc == PG_OK && p->uci_w.nitems > 0) {
     rc = check_cuda(ctx, cudaStreamWaitEvent(s, p->ev_ujoin, 0), "cudaStreamWaitEvent(UCI join)");
   }
   return rc;
@@ -395,7 +397,7 @@ void release(pg_pusch_plan* p)
     cudaStreamDestroy(p->aux);
   }
   for (cudaEvent_t e : {p->ev_h2d, p->ev_stage_free[0], p->ev_stage_free[1], p->ev_done[0], p->ev_done[1],
-                        p->ev_done[2], p->ev_fork, p->ev_join, p->ev_ufork, p->ev_ujoin}) {
+                        p->ev_done[2], p->ev_fork, p->ev_join, p->ev_ufork, p->ev_ujoin, p->ev_uread}) {
     if (e) {
       cudaEventDestroy(e);
     }
@@ -407,6 +409,9 @@ void release(pg_pusch_plan* p)
   }
   if (p->host) {
     cudaFreeHost(p->host);
+  }
+  if (p->uci_bits) {
+    cudaFreeHost(p->uci_bits);
   }
   delete p;
 }
@@ -681,16 +686,16 @@ int pg_pusch_plan_create_uci(pg_context* ctx, const pg_pusch_ue* ues, const pg_p
   const size_t o_epart  = o_res + al((size_t)nof_ues * sizeof(pg_sch_result));
   const size_t o_earr   = o_epart + al((size_t)std::max(1, p->est_nwork) * 16);
   const size_t o_ullr   = o_earr + al((size_t)nof_ues * 16);
-  const size_t o_ubits  = o_ullr + al(uci_llr_total);
-  const size_t o_uvalid = o_ubits + al((size_t)nof_ues * sizeof(pg_pusch_uci_result));
-  const size_t o_polb   = o_uvalid + al((size_t)std::max(1, p->uci_nmsg));
-  const size_t o_pbits  = o_polb + al(polar_bits_total);
+  const size_t o_pbits  = o_ullr + al(uci_llr_total);
   const size_t o_jwords = o_pbits + al((size_t)pilot_words * 4);
   p->dev_bytes          = o_jwords + al((size_t)nof_ues * 8);
 
   const size_t h_res  = 0;
   const size_t h_pr   = h_res + al((size_t)nof_ues * sizeof(pg_sch_result));
   const size_t h_tb   = h_pr + al((size_t)nof_ues * 4 * sizeof(pg_port_result));
+  const size_t hu_valid = al((size_t)nof_ues * sizeof(pg_pusch_uci_result));
+  const size_t hu_polar = hu_valid + al((size_t)std::max(1, p->uci_nmsg));
+  const size_t hu_size  = hu_polar + al(polar_bits_total);
   const size_t h_size = std::max(h_tb + al(p->tb_bytes), desc_end);
 
   int rc = check_cuda(ctx, cudaSetDevice(ctx->device), "cudaSetDevice");
@@ -699,6 +704,14 @@ int pg_pusch_plan_create_uci(pg_context* ctx, const pg_pusch_ue* ues, const pg_p
   }
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaMallocHost(&p->host, h_size), "cudaMallocHost(plan)");
+  }
+  if (rc == PG_OK && !ucfg.empty()) {
+    rc = check_cuda(ctx, cudaMallocHost(&p->uci_bits, hu_size), "cudaMallocHost(UCI results)");
+    if (rc == PG_OK) {
+      std::memset(p->uci_bits, 0, hu_size);
+      p->uci_valid  = p->uci_bits + hu_valid;
+      p->polar_bits = p->uci_bits + hu_polar;
+    }
   }
   if (rc != PG_OK) {
     release(p);
@@ -739,10 +752,7 @@ int pg_pusch_plan_create_uci(pg_context* ctx, const pg_pusch_ue* ues, const pg_p
   p->d_uci_blob  = b + o_ublob;
   p->d_uci_items = b + o_uitems;
   p->d_uci_llr   = reinterpret_cast<int8_t*>(b + o_ullr);
-  p->d_uci_bits  = b + o_ubits;
-  p->d_uci_valid = b + o_uvalid;
   p->d_polar_cbs  = b + o_pcbs;
-  p->d_polar_bits = b + o_polb;
 
   // Descriptor image in pinned memory, one upload.
   uint8_t* h = static_cast<uint8_t*>(p->host);
@@ -776,7 +786,7 @@ int pg_pusch_plan_create_uci(pg_context* ctx, const pg_pusch_ue* ues, const pg_p
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaStreamCreateWithFlags(&p->aux, cudaStreamNonBlocking), "cudaStreamCreate(aux)");
   }
-  for (cudaEvent_t* e : {&p->ev_fork, &p->ev_join, &p->ev_ufork, &p->ev_ujoin}) {
+  for (cudaEvent_t* e : {&p->ev_fork, &p->ev_join, &p->ev_ufork, &p->ev_ujoin, &p->ev_uread}) {
     if (rc == PG_OK) {
       rc = check_cuda(ctx, cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate(fork/join)");
     }
@@ -789,10 +799,6 @@ int pg_pusch_plan_create_uci(pg_context* ctx, const pg_pusch_ue* ues, const pg_p
   }
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaMemsetAsync(p->d_join, 0, (size_t)nof_ues * 8, s), "cudaMemsetAsync(TB join)");
-  }
-  if (rc == PG_OK) {
-    rc = check_cuda(ctx, cudaMemsetAsync(b + o_ubits, 0, (size_t)nof_ues * sizeof(pg_pusch_uci_result), s),
-                    "cudaMemsetAsync(UCI results)");
   }
   if (rc == PG_OK) {
     rc = scrambling_launch(ctx, p->d_ues, nof_ues, max_words, p->d_seq_off, p->d_seq, s);
@@ -924,24 +930,26 @@ int pg_pusch_plan_set_learned(pg_pusch_plan* plan, pg_le_net* net, const uint8_t
   return PG_OK;
 }
 
+// Waits for the executions whose UCI results the caller reads. The decoders store them to pinned host
+// memory, so a read needs no copy; recording an event on the default stream keeps the order a copy on that
+// stream would have. (Two copies to pageable memory took 37 us a message.)
+static int wait_uci(pg_pusch_plan* plan)
+{
+  int rc = check_cuda(plan->ctx, cudaEventRecord(plan->ev_uread, nullptr), "cudaEventRecord(UCI read)");
+  return rc != PG_OK ? rc : check_cuda(plan->ctx, cudaEventSynchronize(plan->ev_uread), "cudaEventSynchronize(UCI read)");
+}
+
 int pg_pusch_plan_uci_results(pg_pusch_plan* plan, pg_pusch_uci_result* out)
 {
   if (plan == nullptr || out == nullptr) {
     return PG_ERR_INVALID;
   }
-  pg_context* ctx = plan->ctx;
   std::vector<pg_pusch_uci_result> r(plan->nof_ues);
-  std::vector<uint8_t>             valid(std::max(1, plan->uci_nmsg));
-  int rc = check_cuda(ctx,
-                      cudaMemcpy(r.data(), plan->d_uci_bits, r.size() * sizeof(pg_pusch_uci_result),
-                                 cudaMemcpyDeviceToHost),
-                      "D2H UCI bits");
-  if (rc == PG_OK && plan->uci_nmsg > 0) {
-    rc = check_cuda(ctx, cudaMemcpy(valid.data(), plan->d_uci_valid, (size_t)plan->uci_nmsg, cudaMemcpyDeviceToHost),
-                    "D2H UCI validity");
-  }
-  if (rc != PG_OK) {
-    return rc;
+  if (plan->uci_nmsg > 0) {
+    if (int rc = wait_uci(plan)) {
+      return rc;
+    }
+    std::memcpy(r.data(), plan->uci_bits, r.size() * sizeof(pg_pusch_uci_result));
   }
   for (int u = 0; u < plan->nof_ues; ++u) {
     r[u].harq_ack_valid  = 0;
@@ -949,7 +957,7 @@ int pg_pusch_plan_uci_results(pg_pusch_plan* plan, pg_pusch_uci_result* out)
   }
   for (int m = 0; m < plan->uci_nmsg; ++m) {
     pg_pusch_uci_result& x = r[plan->uci_msg_ue[m]];
-    (plan->uci_msg_kind[m] == 0 ? x.harq_ack_valid : x.csi_part1_valid) = valid[m];
+    (plan->uci_msg_kind[m] == 0 ? x.harq_ack_valid : x.csi_part1_valid) = plan->uci_valid[m];
   }
   std::memcpy(out, r.data(), r.size() * sizeof(pg_pusch_uci_result));
   return PG_OK;
@@ -975,12 +983,12 @@ int pg_pusch_plan_uci_message(pg_pusch_plan* plan, int ue, int field, uint8_t* b
   if (len < nbits) {
     return set_error(ctx, PG_ERR_INVALID, "bit buffer shorter than the message");
   }
-  const uint8_t* src = (m < plan->uci_nshort ? plan->d_uci_bits : plan->d_polar_bits) + plan->uci_msg_off[m];
-  int            rc  = check_cuda(ctx, cudaMemcpy(bits, src, nbits, cudaMemcpyDeviceToHost), "D2H UCI message");
-  if (rc == PG_OK) {
-    rc = check_cuda(ctx, cudaMemcpy(valid, plan->d_uci_valid + m, 1, cudaMemcpyDeviceToHost), "D2H UCI validity");
+  if (int rc = wait_uci(plan)) {
+    return rc;
   }
-  return rc;
+  std::memcpy(bits, (m < plan->uci_nshort ? plan->uci_bits : plan->polar_bits) + plan->uci_msg_off[m], nbits);
+  *valid = plan->uci_valid[m];
+  return PG_OK;
 }
 
 int pg_pusch_plan_set_harq(pg_pusch_plan* plan, const uint8_t* new_data, const uint8_t* rv)

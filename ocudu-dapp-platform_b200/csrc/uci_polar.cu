@@ -5,12 +5,12 @@
 // (polar_decoder_impl.cpp) and deallocator (polar_deallocator_impl.cpp), on the GPU.
 //
 // The host builds each codeblock's code (N, the information and parity-check sub-channels) once
-// per call; one CTA of two warps decodes one message, one warp per codeblock (a message longer than
-// 359 bits with at least 1088 soft bits, or of 1013 bits and more, has two codeblocks). A warp runs
-// the whole chain on its codeblock in shared memory: channel de-interleaving, bit selection and
-// sub-block de-interleaving into the decoder's input, the decoder's depth-first walk over rate-0,
-// rate-1 and rate-R nodes with the f / g / re-encoding steps spread over the 32 lanes, the
-// deallocation and the codeblock CRC. Every LLR operation is the reference's int8 arithmetic
+// per call; one CTA decodes one message (a message longer than 359 bits with at least 1088 soft bits,
+// or of 1013 bits and more, has two codeblocks). The CTA runs channel de-interleaving, bit selection
+// and sub-block de-interleaving into the decoder's input in shared memory; then one warp per codeblock
+// walks the rate-0, rate-1 and rate-R nodes depth first, with the f / g steps spread over the 32 lanes
+// and codewords and decoded bits held as bit words, one word a lane, and runs the deallocation and the
+// codeblock CRC. Every LLR operation is the reference's int8 arithmetic
 // (log_likelihood_ratio: saturated sum at +-120 with +-127 as infinity, soft_xor, hard bit v <= 0,
 // promotion sum on repetition).
 #include "pg_internal.h"
@@ -212,108 +212,154 @@ __device__ __forceinline__ int llr_soft_xor(int x, int y)
   return x * y < 0 ? -m : m;
 }
 
-constexpr int kRate0 = 0, kRateR = 2, kRate1 = 3; // polar_decoder_impl node_rate
+constexpr int kPolarThreads = 128;
 
-struct polar_warp_smem {
-  int8_t   e[kPolarEMax];          // de-interleaved soft bits, then the deallocated message bits
-  int8_t   llr[2 * kPolarNMax];    // stage s at offset 2^s - 1, 2^s values (s = 0 .. n)
-  uint8_t  est[kPolarNMax];        // codeword estimates (partial sums)
-  uint8_t  u[kPolarNMax];          // decoded sub-channel bits
-  uint8_t  type[2 * kPolarNMax];   // node types, stage s at offset 2N - (2N >> s)
-  uint32_t info[kPolarNMax / 32];
-  uint16_t pc[4];
+struct polar_cb_smem {
+  int8_t   e[kPolarEMax];          // de-interleaved soft bits
+  uint32_t in[kPolarEMax / 4 + 1]; // the received soft bits, then the deallocated message bits
+  int8_t   llr[2 * kPolarNMax];    // stage s (5 .. n) at offset 2^s, 2^s values
   int      valid;
 };
 
-// Node types of every stage (polar_decoder_impl.cpp:74-107): a leaf is rate 1 when it is in K_set,
-// rate 0 otherwise; a node of stage s is rate 0 (rate 1) when both children are, rate R otherwise.
-__device__ __forceinline__ void node_types(polar_warp_smem& sm, int n, int lane)
+// Bits of a word of sub-channels re-encoded by the polar transform: bit i ^= bit i + st for st = 1, 2, ...
+__device__ __forceinline__ uint32_t polar_transform_word(uint32_t x)
 {
-  const int N = 1 << n;
-  for (int j = lane; j < N; j += 32) {
-    sm.type[j] = ((sm.info[j >> 5] >> (j & 31)) & 1u) ? kRate1 : kRate0;
-  }
-  __syncwarp();
-  for (int st = 1; st <= n; ++st) {
-    const uint8_t* c = sm.type + (2 * N - ((2 * N) >> (st - 1)));
-    uint8_t*       t = sm.type + (2 * N - ((2 * N) >> st));
-    for (int j = lane; j < (N >> st); j += 32) {
-      const int a = c[2 * j], b = c[2 * j + 1];
-      t[j]        = (uint8_t)(a == b && a != kRateR ? a : kRateR);
-    }
-    __syncwarp();
-  }
+  x ^= (x >> 1) & 0x55555555u;
+  x ^= (x >> 2) & 0x33333333u;
+  x ^= (x >> 4) & 0x0f0f0f0fu;
+  x ^= (x >> 8) & 0x00ff00ffu;
+  x ^= x >> 16;
+  return x;
 }
 
-// One codeblock by one warp.
-__device__ void polar_decode_codeblock(const polar_cb& d, polar_warp_smem& sm, const int8_t* __restrict__ llrs,
-                                       uint8_t* __restrict__ bits)
+__device__ __forceinline__ int llr_f(int x, int y)
 {
-  const int lane = threadIdx.x & 31;
-  const int n    = d.n;
-  const int N    = 1 << n;
-  const int E    = (int)d.E;
-  const int K    = d.K;
-  const int8_t* f = llrs + d.llr_offset;
+  return (int)(int8_t)llr_soft_xor(x, y);
+}
 
-  for (int w = lane; w < kPolarNMax / 32; w += 32) {
-    sm.info[w] = d.info[w];
-  }
-  __syncwarp();
-  node_types(sm, n, lane);
-  if (lane < 4) {
-    sm.pc[lane] = d.pc[lane];
-  }
-  for (int i = lane; i < N; i += 32) {
-    sm.est[i] = 0;
-    sm.u[i]   = 0;
-  }
+__device__ __forceinline__ int llr_g(int x, int y, uint32_t bit)
+{
+  return (int)(int8_t)llr_sat_sum(y, bit == 0 ? x : -x);
+}
 
-  // Channel de-interleaver (polar_rate_dematcher_impl.cpp:53-79): the triangle of T rows, T the
-  // smallest with T (T + 1) / 2 >= E, filled row by row: row r holds positions
-  // r + c T - c (c - 1) / 2 for c = 0, 1, ... while below E, taking the input in (r, c) order.
-  int T = 1;
+// One node of stage S <= 5 (polar_decoder_impl.cpp:163-252) in registers: lane i < 2^S holds the LLR of the
+// node's element i, info its sub-channels' K_set bits; returns the node's codeword (bit i: element i) and
+// in u its decoded sub-channel bits. The two children share one copy of the code.
+template <int S>
+__device__ __forceinline__ uint32_t polar_node(int l, uint32_t info, uint32_t& u)
+{
+  constexpr uint32_t m = S == 5 ? 0xffffffffu : (1u << (1 << (S < 5 ? S : 0))) - 1u;
+  if (info == 0u) { // rate 0: zeros (:163-178)
+    u = 0u;
+    return 0u;
+  }
+  if (info == m) { // rate 1: hard decisions, re-encoded into the message bits (:180-205)
+    const uint32_t e = __ballot_sync(0xffffffffu, l <= 0) & m;
+    u                = polar_transform_word(e);
+    return e;
+  }
+  if constexpr (S > 0) {
+    constexpr int      h  = 1 << (S - 1);
+    constexpr uint32_t mh = (1u << h) - 1u;
+    const int          y  = __shfl_down_sync(0xffffffffu, l, h);
+    int                lc = llr_f(l, y); // left child (:214-218)
+    uint32_t           e0 = 0u, u0 = 0u;
+#pragma unroll 1
+    for (int half = 0;; ++half) {
+      uint32_t       uc;
+      const uint32_t e = polar_node<S - 1>(lc, half == 0 ? info & mh : info >> h, uc);
+      if (half == 1) {
+        u = u0 | (uc << h);
+        return (e0 ^ e) | (e << h); // (:240-252)
+      }
+      e0 = e;
+      u0 = uc;
+      lc = llr_g(l, y, (e0 >> (threadIdx.x & 31)) & 1u); // right child (:228-233)
+    }
+  }
+  return 0u;
+}
+
+// Rate dematching of one codeblock by the CTA: the soft bits into shared memory, the channel
+// de-interleaver, and bit selection with sub-block de-interleaving into the stage-n LLRs.
+__device__ __forceinline__ void polar_rate_dematch(const polar_cb& d, polar_cb_smem& sm, const int8_t* __restrict__ llrs)
+{
+  const int     tid = threadIdx.x;
+  const int     n   = d.n;
+  const int     N   = 1 << n;
+  const int     E   = (int)d.E;
+  const int     K   = d.K;
+  const int8_t* f   = llrs + d.llr_offset;
+
+  // By aligned words; an unaligned stream is shifted into place.
+  {
+    const uint32_t  sh = (uint32_t)(reinterpret_cast<uintptr_t>(f) & 3u);
+    const uint32_t* w  = reinterpret_cast<const uint32_t*>(f - sh);
+    const int       nw = (E + 3) / 4, last = (int)(sh + (uint32_t)E - 1u) / 4; // last word that holds a soft bit
+#pragma unroll 8
+    for (int i = tid; i < nw; i += kPolarThreads) {
+      const uint32_t lo = __ldg(w + i), hi = sh != 0 && i < last ? __ldg(w + i + 1) : 0u;
+      sm.in[i]          = __funnelshift_r(lo, hi, 8 * sh);
+    }
+  }
+  __syncthreads();
+  const int8_t* const fin = reinterpret_cast<const int8_t*>(sm.in);
+
+  // Channel de-interleaver (polar_rate_dematcher_impl.cpp:53-79): a triangle of T columns, T the smallest
+  // with T (T + 1) / 2 >= E, column c of T - c entries. Position S(c) + r, S(c) = c T - c (c - 1) / 2, is
+  // the entry (r, c); positions at or beyond E are missing: the last q columns whole and the last `rem`
+  // entries of the column before them. The input fills the rows in turn, one thread a row (T <= 128).
+  int T = (int)ceilf((sqrtf(8.0f * (float)E + 1.0f) - 1.0f) * 0.5f);
+  while (T > 1 && (T - 1) * T / 2 >= E) {
+    --T;
+  }
   while (T * (T + 1) / 2 < E) {
     ++T;
   }
-  int base = 0; // input index of the first entry of rows r0 ..
-  for (int r0 = 0; r0 < T; r0 += 32) {
-    const int r   = r0 + lane;
-    int       cnt = 0;
-    if (r < T) {
-      int i_in = r;
-      for (int c = 0; c < T - r && i_in < E; ++c) {
-        ++cnt;
-        i_in += T - c;
-      }
-    }
-    int incl = cnt; // inclusive prefix of the counts over the lanes
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) {
-        incl += t;
-      }
-    }
-    const int first = base + incl - cnt;
-    if (r < T) {
-      int i_in = r;
-      for (int c = 0; c < cnt; ++c) {
-        sm.e[i_in] = f[first + c];
-        i_in += T - c;
-      }
-    }
-    base += __shfl_sync(0xffffffffu, incl, 31);
+  const int miss = T * (T + 1) / 2 - E; // < T
+  int       q    = (int)((sqrtf(8.0f * (float)miss + 1.0f) - 1.0f) * 0.5f);
+  while (q * (q + 1) / 2 > miss) {
+    --q;
   }
-  __syncwarp();
+  while ((q + 1) * (q + 2) / 2 <= miss) {
+    ++q;
+  }
+  const int rem = miss - q * (q + 1) / 2;
+  for (int r = tid; r < T; r += kPolarThreads) {
+    const int a     = min(r, q);
+    const int cnt   = T - r - max(0, q - r) - (r <= q && r > q - rem ? 1 : 0);
+    const int first = r * T - r * (r - 1) / 2 - (a * q - a * (a - 1) / 2) - max(0, min(r, q + 1) - (q + 1 - rem));
+    int       i_in  = r;
+    int       c     = 0;
+    for (; c + 4 <= cnt; c += 4) {
+      int8_t x[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        x[k] = fin[first + c + k];
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        sm.e[i_in] = x[k];
+        i_in += T - c - k;
+      }
+    }
+    for (; c < cnt; ++c) {
+      sm.e[i_in] = fin[first + c];
+      i_in += T - c;
+    }
+  }
+  __syncthreads();
 
   // Bit selection (:21-50) and sub-block de-interleaving (:12-19) into the stage-n LLRs.
-  int8_t* const ln = sm.llr + (N - 1);
+  int8_t* const ln    = sm.llr + N;
   const bool    rep   = E >= N;
   const bool    punct = !rep && 16 * K <= 7 * E;
-  for (int j = lane; j < N; j += 32) {
+  const int     b     = N >> 5;
+  for (int j = tid; j < N; j += kPolarThreads) {
     int y;
     if (rep) {
       y = sm.e[j];
+#pragma unroll 4
       for (int k = j + N; k < E; k += N) {
         y = llr_promotion_sum(y, sm.e[k]);
       }
@@ -322,141 +368,187 @@ __device__ void polar_decode_codeblock(const polar_cb& d, polar_warp_smem& sm, c
     } else {
       y = j < E ? sm.e[j] : kLlrInf;
     }
-    const int b = N >> 5;
-    ln[c_polar_subblock[(32 * j) / N] * b + j % b] = (int8_t)y;
+    ln[c_polar_subblock[j >> (n - 5)] * b + (j & (b - 1))] = (int8_t)y;
   }
-  __syncwarp();
+  __syncthreads();
+}
 
-  // Simplified successive cancellation (polar_decoder_impl.cpp:163-316), depth first. phases holds
-  // two bits per stage: 0 = node entered, 1 = left child done, 2 = right child done.
-  int      s = n, j = 0;
+// Simplified successive cancellation (polar_decoder_impl.cpp:163-316) of one codeblock by one warp, depth
+// first, then deallocation and CRC. Lane w holds sub-channels 32 w .. 32 w + 31: their K_set bits, codeword
+// estimates and decoded bits. Stages above 5 keep their LLRs in shared memory; a node of stage 5 is decoded
+// in registers.
+__device__ __forceinline__ void polar_decode_codeblock(const polar_cb& d, polar_cb_smem& sm, uint8_t* __restrict__ bits)
+{
+  const int      lane  = threadIdx.x & 31;
+  const int      n     = d.n;
+  const int      N     = 1 << n;
+  const int      K     = d.K;
+  const uint32_t info  = lane < (N >> 5) ? d.info[lane] : 0u;
+  const uint32_t zeros = __ballot_sync(0xffffffffu, info == 0u); // words of rate 0 and of rate 1
+  const uint32_t ones  = __ballot_sync(0xffffffffu, info == 0xffffffffu);
+  uint32_t       cw = 0u, u = 0u;
+
+  // The node: stage s, words w0 .. w0 + 2^(s-5) - 1. phases holds two bits per stage: 0 = node entered,
+  // 1 = left child done, 2 = right child done.
+  int      s = n, w0 = 0;
   uint32_t phases = 0;
   for (;;) {
-    const int ph     = (int)((phases >> (2 * s)) & 3u);
-    bool      ascend = false;
-    const int h      = (1 << s) >> 1;
-    int8_t*   ls     = sm.llr + ((1 << s) - 1);
-    if (ph == 0) {
-      const int t = sm.type[2 * N - ((2 * N) >> s) + j];
-      if (t == kRate1) {
-        // Hard decisions of the node's LLRs, re-encoded into its message bits (:180-205).
-        const int p0 = j << s, sz = 1 << s;
-        for (int i = lane; i < sz; i += 32) {
-          const uint8_t b = ls[i] <= 0 ? 1 : 0;
-          sm.est[p0 + i]  = b;
-          sm.u[p0 + i]    = b;
-        }
-        __syncwarp();
-        for (int st = 1; st < sz; st <<= 1) {
-          for (int i = lane; i < sz; i += 32) {
-            if ((i & st) == 0) {
-              sm.u[p0 + i] ^= sm.u[p0 + i + st];
-            }
+    if (s == 5) {
+      uint32_t       uc;
+      const uint32_t e = polar_node<5>(sm.llr[32 + lane], __shfl_sync(0xffffffffu, info, w0), uc);
+      if (lane == w0) {
+        cw = e;
+        u  = uc;
+      }
+    } else {
+      const int      ph  = (int)((phases >> (2 * s)) & 3u);
+      const int      h   = 1 << (s - 1);
+      const int      cnt = 1 << (s - 5);
+      const uint32_t m   = (cnt == 32 ? 0xffffffffu : (1u << cnt) - 1u) << w0;
+      const int8_t*  ls  = sm.llr + (1 << s);
+      int8_t*        lc  = sm.llr + h;
+      const bool     in  = ((m >> lane) & 1u) != 0u;
+      if (ph == 0 && (zeros & m) == m) {
+        // rate 0: the words stay zero
+      } else if (ph == 0 && (ones & m) == m) {
+        for (int k = 0; k < cnt; ++k) {
+          const uint32_t e = __ballot_sync(0xffffffffu, ls[32 * k + lane] <= 0);
+          if (lane == w0 + k) {
+            cw = e;
+            u  = polar_transform_word(e);
           }
-          __syncwarp();
         }
-        ascend = true;
-      } else if (t == kRate0) {
-        ascend = true; // bits stay zero (:163-178)
-      } else {
-        // f: left child's LLRs soft_xor(first half, second half) (:214-218).
-        int8_t* lc = sm.llr + (h - 1);
-        for (int i = lane; i < h; i += 32) {
-          lc[i] = (int8_t)llr_soft_xor(ls[i], ls[i + h]);
+        for (int st = 1; st < cnt; st <<= 1) {
+          const uint32_t t = __shfl_down_sync(0xffffffffu, u, st);
+          if (in && ((lane - w0) & st) == 0) {
+            u ^= t;
+          }
+        }
+      } else if (ph < 2) {
+        __syncwarp();
+        if (ph == 0) {
+#pragma unroll 4
+          for (int i = lane; i < h; i += 32) {
+            lc[i] = (int8_t)llr_f(ls[i], ls[i + h]);
+          }
+        } else {
+#pragma unroll 4
+          for (int k = 0; k < (h >> 5); ++k) {
+            const int      i  = 32 * k + lane;
+            const uint32_t eb = __shfl_sync(0xffffffffu, cw, w0 + k);
+            lc[i]             = (int8_t)llr_g(ls[i], ls[i + h], (eb >> lane) & 1u);
+          }
         }
         __syncwarp();
-        phases = (phases & ~(3u << (2 * s))) | (1u << (2 * s));
+        phases = (phases & ~(3u << (2 * s))) | ((uint32_t)(ph + 1) << (2 * s));
+        w0 += ph == 0 ? 0 : cnt >> 1;
         --s;
-        j <<= 1;
         phases &= ~(3u << (2 * s));
         continue;
-      }
-    } else if (ph == 1) {
-      // g: right child's LLRs second half +- first half by the left child's codeword (:228-233).
-      int8_t*        lc = sm.llr + (h - 1);
-      const uint8_t* eb = sm.est + (j << s);
-      for (int i = lane; i < h; i += 32) {
-        const int x = ls[i], y = ls[i + h];
-        lc[i]       = (int8_t)llr_sat_sum(y, eb[i] == 0 ? x : -x);
-      }
-      __syncwarp();
-      phases = (phases & ~(3u << (2 * s))) | (2u << (2 * s));
-      --s;
-      j = 2 * j + 1;
-      phases &= ~(3u << (2 * s));
-      continue;
-    } else {
-      // Both children done: left codeword ^= right codeword (:240-252).
-      uint8_t* eb = sm.est + (j << s);
-      for (int i = lane; i < h; i += 32) {
-        eb[i] ^= eb[i + h];
-      }
-      __syncwarp();
-      ascend = true;
-    }
-    if (ascend) {
-      if (s == n) {
-        break;
-      }
-      ++s;
-      j >>= 1;
-    }
-  }
-
-  // Deallocation (polar_deallocator_impl.cpp:10-24) and the codeblock CRC over the K bits
-  // (uci_decoder_impl.cpp:74-92), one lane.
-  if (lane == 0) {
-    int     iPC = 0, iK = 0;
-    int8_t* msg = sm.e;
-    for (int w = 0; w < (N >> 5); ++w) {
-      uint32_t x = sm.info[w];
-      while (x != 0u) {
-        const int i = (w << 5) + __ffs(x) - 1;
-        x &= x - 1u;
-        if (i == sm.pc[iPC]) {
-          ++iPC;
-        } else if (iK < K) {
-          msg[iK++] = (int8_t)sm.u[i];
+      } else {
+        // Both children done: left codeword ^= right codeword (:240-252).
+        const uint32_t t = __shfl_down_sync(0xffffffffu, cw, cnt >> 1);
+        if (in && lane < w0 + (cnt >> 1)) {
+          cw ^= t;
         }
       }
     }
+    if (s == n) {
+      break;
+    }
+    ++s;
+    w0 &= ~((1 << (s - 5)) - 1);
+  }
+
+  // Deallocation (polar_deallocator_impl.cpp:10-24): a lane's first message index is the number of K_set
+  // entries of the lower sub-channels less the parity ones among them.
+  int8_t* const msg = reinterpret_cast<int8_t*>(sm.in);
+  {
+    uint32_t x = info;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t pc = d.pc[k];
+      if ((pc >> 5) == (uint32_t)lane) {
+        x &= ~(1u << (pc & 31u));
+      }
+    }
+    const int cnt  = __popc(x);
+    int       incl = cnt;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) {
+        incl += t;
+      }
+    }
+    int iK = incl - cnt;
+    while (x != 0u) {
+      const int i = __ffs(x) - 1;
+      x &= x - 1u;
+      if (iK < K) {
+        msg[iK] = (int8_t)((u >> i) & 1u);
+      }
+      ++iK;
+    }
+  }
+  __syncwarp();
+  // The codeblock CRC over the K bits (uci_decoder_impl.cpp:74-92): words of 32 bits by the warp, the
+  // register by every lane alike.
+  {
     const int      L    = d.crc_size;
     const uint32_t poly = L == 11 ? 0x621u : 0x21u; // CRC11 0xE21, CRC6 0x61 without the x^L term
     const uint32_t mask = (1u << L) - 1u;
     uint32_t       reg  = 0;
-    for (int i = 0; i < K; ++i) {
-      const uint32_t top = ((reg >> (L - 1)) ^ (uint32_t)msg[i]) & 1u;
-      reg                = (reg << 1) & mask;
-      if (top) {
-        reg ^= poly;
+    for (int i0 = 0; i0 < K; i0 += 32) {
+      const uint32_t w = __ballot_sync(0xffffffffu, i0 + lane < K && msg[i0 + lane] != 0);
+      const int      m = min(32, K - i0);
+      for (int i = 0; i < m; ++i) {
+        const uint32_t top = ((reg >> (L - 1)) ^ (w >> i)) & 1u;
+        reg                = ((reg << 1) & mask) ^ (top ? poly : 0u);
       }
     }
-    sm.valid = reg == 0u ? 1 : 0;
+    if (lane == 0) {
+      sm.valid = reg == 0u ? 1 : 0;
+    }
   }
-  __syncwarp();
   for (int i = lane; i < d.nbits; i += 32) {
-    bits[d.out_offset + i] = (uint8_t)sm.e[d.nof_filler + i];
+    bits[d.out_offset + i] = (uint8_t)msg[d.nof_filler + i];
   }
 }
 
-constexpr int kPolarThreads = 64; // one warp per codeblock
-
+// One CTA per message: all its warps prepare the decoder's input, then one warp decodes each codeblock.
+// Bound: latency, the chain of node steps. Six messages of 20 to 60 bits over up to 8192 soft bits took
+// 90 us with the walk down to single sub-channels in shared memory, bytes for codewords and one warp that
+// read its soft bits from global memory one by one; with stage 5 in registers and four warps that prepare the
+// input 42 us.
 __global__ void __launch_bounds__(kPolarThreads) uci_polar_kernel(const polar_cb* __restrict__ cbs, int n,
                                                                  const int8_t* __restrict__ llrs,
                                                                  uint8_t* __restrict__ bits,
                                                                  uint8_t* __restrict__ valid)
 {
-  __shared__ polar_warp_smem sm[2];
+  __shared__ polar_cb_smem sm[2];
+  __shared__ polar_cb      cb[2];
   const int msg  = blockIdx.x;
   const int warp = threadIdx.x >> 5;
   if (msg >= n) {
     return;
   }
-  const polar_cb& d = cbs[2 * msg + warp];
-  if (d.E > 0) {
-    polar_decode_codeblock(d, sm[warp], llrs, bits);
-  } else if ((threadIdx.x & 31) == 0) {
-    sm[warp].valid = 1;
+  constexpr int kWords = (int)(2 * sizeof(polar_cb) / 4);
+  static_assert(kWords <= kPolarThreads && alignof(polar_cb) == 4, "one word of the two descriptors per thread");
+  if ((int)threadIdx.x < kWords) {
+    reinterpret_cast<uint32_t*>(cb)[threadIdx.x] = reinterpret_cast<const uint32_t*>(cbs + 2 * (size_t)msg)[threadIdx.x];
+  }
+  __syncthreads();
+  for (int c = 0; c < 2; ++c) {
+    if (cb[c].E > 0) {
+      polar_rate_dematch(cb[c], sm[c], llrs);
+    }
+  }
+  if (warp < 2) {
+    if (cb[warp].E > 0) {
+      polar_decode_codeblock(cb[warp], sm[warp], bits);
+    } else if ((threadIdx.x & 31) == 0) {
+      sm[warp].valid = 1;
+    }
   }
   __syncthreads();
   // uci_decoder_impl.cpp:40-57: valid when every codeblock passes its CRC.
