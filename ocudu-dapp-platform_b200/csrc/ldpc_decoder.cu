@@ -536,7 +536,8 @@ __global__ void __launch_bounds__(kThreads, 2) ldpc_decode_kernel(const pg_ldpc_
 // Soft bits: E[col][k] = (soft[col][k], soft[col][k + H]) as one f16x2 word, 0 <= k < H, in shared
 // memory. For an edge of shift s, lane j reads variable lane (j + s) mod Z and lane j + H reads
 // (j + H + s) mod Z: both are halves of the same word k = (j + s') mod H with s' = s mod H, swapped
-// when (j + s' >= H) differs from (s >= H). The edge table in shared memory holds what pair_edge needs. Rows are padded to a multiple of T edges with an edge to a constant column of
+// when (j + s' >= H) differs from (s >= H). The edge table in shared memory holds what pair_edge needs. Rows are
+// padded to a multiple of T edges with an edge to a constant column of
 // saturated positive soft bits, which changes no minimum, sign or message of the row.
 //
 // Arithmetic: the reference's int8 rules as exact f16x2 identities (every value that decides is an
@@ -672,31 +673,30 @@ __device__ __forceinline__ void sts_u32(uint32_t adr, uint32_t v)
   asm volatile("st.shared.u32 [%0], %1;" ::"r"(adr), "r"(v));
 }
 
+constexpr int kPairMaxEdges = 460; // padded edges of a graph, T <= 4 (316 + 3 * 46 at most)
+
 // Tables of the base graphs, indexed by [graph], and of their rows padded to a multiple of T = 2 << lg
 // edges ([lg][graph]): first padded edge and first message word (in units of the active
 // threads) of each row. In global memory: threads read different entries.
 struct pair_tables {
-  uint16_t edge_v[2][pg::kBg1Edges][8];
-  uint8_t  edge_col[2][pg::kBg1Edges];
-  uint8_t  edge_row[2][pg::kBg1Edges];
-  uint8_t  row_deg[2][pg::kBg1Rows];
-  uint8_t  row_sync[2][pg::kBg1Rows]; // the row is the last of its step
-  uint16_t row_e0[2][pg::kBg1Rows + 1];
+  uint16_t pad_v[2][2][kPairMaxEdges][8]; // shift of each padded edge, per lifting set
+  uint8_t  pad_col[2][2][kPairMaxEdges];  // its column plus 1, 0 for an edge to the constant column
+  uint8_t  row_sync[2][pg::kBg1Rows];     // the row is the last of its step
   uint16_t pad_e0[2][2][pg::kBg1Rows + 1];
   uint16_t msg0[2][2][pg::kBg1Rows + 1];
 };
 __device__ pair_tables g_pair_tables;
 
-constexpr int      kPairMaxEdges = 460;  // padded edges of a graph, T <= 4 (316 + 3 * 46 at most)
 constexpr uint32_t kPairTabBytes = kPairMaxEdges * 16;
 constexpr uint32_t kPairMinSmem  = kPairTabBytes + (pg::kMaxNodes + 1) * (pg::kMaxZ / 2) * 4; // every column
 constexpr int      kOddMaxZ      = 16;   // odd lifting sizes are at most 15
 
+constexpr int kPairThreads = 384;
+
 struct pair_shared {
-  uint4    row[pg::kBg1Rows + 1]; // first padded edge, first message word, edges per thread, step end
+  uint4    row[pg::kBg1Rows + 1]; // first padded edge, first message byte, edges per thread, threads to meet after it or 0
   uint32_t tb_crc;
-  int      last;
-  int      ragged;
+  int      seen[kPairThreads / 32]; // per warp: twice the last non-zero LLR's end, plus 1 for a ragged value
   uint32_t crc[2];
   int      zero[2];
   int      work;
@@ -728,29 +728,93 @@ __device__ __forceinline__ void pair_reduce(uint32_t& min1, uint32_t& min2)
   }
 }
 
-// One row for this thread's NE edges (table entries zt[0 .. NE - 1], message words msg[0], msg[nta],
-// ...). FIRST: the first iteration, whose messages are still zero.
-template <int NE, bool FIRST, int T>
-__device__ __forceinline__ void pair_row(const uint32_t zt, const float jf, const float j4d, const float nh4d,
-                                         uint32_t* msg, const bool active)
-{
-  constexpr int NW = (NE + 1) / 2;
-  uint32_t      m[NW], v[NE], adr[NE], sel[NE];
-  if (!FIRST) {
+// A thread's message words of one row: in shared memory (a 32-bit address) or in the global slab.
+struct msg_shared {
+  uint32_t a;
+  __device__ __forceinline__ msg_shared at(uint32_t byte) const { return {a + byte}; }
+  template <int NW>
+  __device__ __forceinline__ void load(uint32_t* m) const
+  {
     if constexpr (NW == 2) {
-      const uint2 q = *reinterpret_cast<const uint2*>(msg);
+      asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(m[0]), "=r"(m[NW - 1]) : "r"(a));
+    } else {
+#pragma unroll
+      for (int w = 0; w < NW; ++w) {
+        m[w] = lds_u32(a + 4 * w);
+      }
+    }
+  }
+  template <int NW>
+  __device__ __forceinline__ void store(const uint32_t* m) const
+  {
+    if constexpr (NW == 2) {
+      asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(m[0]), "r"(m[NW - 1]) : "memory");
+    } else {
+#pragma unroll
+      for (int w = 0; w < NW; ++w) {
+        sts_u32(a + 4 * w, m[w]);
+      }
+    }
+  }
+};
+struct msg_global {
+  unsigned char* a;
+  __device__ __forceinline__ msg_global at(uint32_t byte) const { return {a + byte}; }
+  template <int NW>
+  __device__ __forceinline__ void load(uint32_t* m) const
+  {
+    if constexpr (NW == 2) {
+      const uint2 q = *reinterpret_cast<const uint2*>(a);
       m[0] = q.x, m[NW - 1] = q.y;
     } else {
 #pragma unroll
       for (int w = 0; w < NW; ++w) {
-        m[w] = msg[w];
+        m[w] = reinterpret_cast<const uint32_t*>(a)[w];
       }
     }
   }
-  uint32_t min1 = kH120, min2 = kH120;
+  template <int NW>
+  __device__ __forceinline__ void store(const uint32_t* m) const
+  {
+    if constexpr (NW == 2) {
+      *reinterpret_cast<uint2*>(a) = make_uint2(m[0], m[NW - 1]);
+    } else {
+#pragma unroll
+      for (int w = 0; w < NW; ++w) {
+        reinterpret_cast<uint32_t*>(a)[w] = m[w];
+      }
+    }
+  }
+};
+
+// The end of a step: the rows before it have stored their soft bits. A row meets the step before it only when
+// it reads soft bits; its edge table and messages, which no other thread writes, are read before that. nthreads: the threads of the rows, or 0.
+__device__ __forceinline__ void step_sync(const uint32_t nthreads)
+{
+  if (nthreads != 0) {
+    asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
+  }
+}
+
+// One row for this thread's NE edges (table entries zt[0 .. NE - 1], message words msg[0], msg[nta],
+// ...). FIRST: the first iteration, whose messages are still zero.
+template <int NE, bool FIRST, int T, class M>
+__device__ __forceinline__ void pair_row(const uint32_t zt, const float jf, const float j4d, const float nh4d,
+                                         const M msg, const bool active, const uint32_t sync)
+{
+  constexpr int NW = (NE + 1) / 2;
+  uint32_t      m[NW], v[NE], adr[NE], sel[NE];
+  if (!FIRST) {
+    msg.template load<NW>(m);
+  }
 #pragma unroll
   for (int e = 0; e < NE; ++e) {
     pair_edge(lds_v4(zt + 16 * e), jf, j4d, nh4d, adr[e], sel[e]);
+  }
+  step_sync(sync);
+  uint32_t min1 = kH120, min2 = kH120;
+#pragma unroll
+  for (int e = 0; e < NE; ++e) {
     const uint32_t x = __byte_perm(lds_u32(adr[e]), 0, sel[e]);
     uint32_t       d = x;
     if (!FIRST) {
@@ -780,14 +844,7 @@ __device__ __forceinline__ void pair_row(const uint32_t zt, const float jf, cons
   for (int w = 0; w < NW; ++w) {
     m[w] = __byte_perm(v[2 * w], v[2 * w + 1 < NE ? 2 * w + 1 : 2 * w], 0x6420u);
   }
-  if constexpr (NW == 2) {
-    *reinterpret_cast<uint2*>(msg) = make_uint2(m[0], m[NW - 1]);
-  } else {
-#pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      msg[w] = m[w];
-    }
-  }
+  msg.template store<NW>(m);
 }
 
 // The first iteration's row with the promotion where the soft bit is stored, for codeblocks whose
@@ -795,8 +852,9 @@ __device__ __forceinline__ void pair_row(const uint32_t zt, const float jf, cons
 // formed again in the second pass.
 template <int T>
 __device__ __noinline__ void pair_row_ragged(const int ne, const uint32_t zt, const float jf, const float j4d,
-                                             const float nh4d, uint32_t* msg, const bool active)
+                                             const float nh4d, uint32_t* msg, const bool active, const uint32_t sync)
 {
+  step_sync(sync);
   uint32_t min1 = kH120, min2 = kH120, adr, sel;
 #pragma unroll 1
   for (int e = 0; e < ne; ++e) {
@@ -832,31 +890,54 @@ __device__ __noinline__ void pair_row_ragged(const int ne, const uint32_t zt, co
   }
 }
 
-template <bool FIRST, int T>
-__device__ __forceinline__ void pair_row_dispatch(const int ne, const uint32_t tpart16, const uint32_t zt,
-                                                  const float jf, const float j4d, const float nh4d, uint32_t* msg,
-                                                  const bool active)
+// The rows of one iteration.
+template <bool FIRST, int T, class M>
+__device__ __forceinline__ void pair_rows(const pair_shared& sh, const int nof_layers, const uint32_t tpart16,
+                                          const float jf, const float j4d, const float nh4d, const M msg,
+                                          const bool active)
 {
-  // Base-graph row degrees: BG1 {3..10, 19}, BG2 {3..10}.
+  const uint32_t tid4 = 4u * threadIdx.x;
+  uint32_t       sync = 0; // the step before this row
+  uint4          rd   = sh.row[0];
+#pragma unroll 1
+  for (int r = 0; r < nof_layers; ++r) {
+    const uint4 next = sh.row[r + 1];
+    const int   ne   = (int)rd.z;
+    const M     mr   = msg.at(rd.y);
+    // Base-graph row degrees: BG1 {3..10, 19}, BG2 {3..10}.
 #define PG_PAIR_ROW(n) \
-  pair_row<n, FIRST, T>(zt + tpart16 * (n), jf, j4d, nh4d, msg + threadIdx.x * (((n) + 1) / 2), active)
-  if constexpr (T == 2) {
-    switch (ne) {
-      case 2: PG_PAIR_ROW(2); break;
-      case 3: PG_PAIR_ROW(3); break;
-      case 4: PG_PAIR_ROW(4); break;
-      case 5: PG_PAIR_ROW(5); break;
-      default: PG_PAIR_ROW(10); break;
+  pair_row<n, FIRST, T>(rd.x + tpart16 * (n), jf, j4d, nh4d, mr.at(tid4 * (((n) + 1) / 2)), active, sync)
+    if constexpr (T == 2) {
+      if (ne < 4) {
+        if (ne < 3) {
+          PG_PAIR_ROW(2);
+        } else {
+          PG_PAIR_ROW(3);
+        }
+      } else if (ne < 5) {
+        PG_PAIR_ROW(4);
+      } else if (ne < 6) {
+        PG_PAIR_ROW(5);
+      } else {
+        PG_PAIR_ROW(10);
+      }
+    } else {
+      if (ne < 3) {
+        if (ne < 2) {
+          PG_PAIR_ROW(1);
+        } else {
+          PG_PAIR_ROW(2);
+        }
+      } else if (ne < 4) {
+        PG_PAIR_ROW(3);
+      } else {
+        PG_PAIR_ROW(5);
+      }
     }
-  } else {
-    switch (ne) {
-      case 1: PG_PAIR_ROW(1); break;
-      case 2: PG_PAIR_ROW(2); break;
-      case 3: PG_PAIR_ROW(3); break;
-      default: PG_PAIR_ROW(5); break;
-    }
-  }
 #undef PG_PAIR_ROW
+    sync = rd.w;
+    rd   = next;
+  }
 }
 
 // f16 soft bit -> hard bit: soft <= 0 (either zero counts as 0).
@@ -865,15 +946,22 @@ __device__ __forceinline__ bool pair_hard(uint32_t h)
   return (h & 0x8000u) != 0 || (h & 0x7fffu) == 0;
 }
 
+constexpr int kFetchBatch = 5; // pieces of eight lane pairs per thread step: 68 columns of Z = 384 in one
+
 // Eight input LLRs from index k (any k; outside [0, n) they are zero) as soft bits in offset
 // binary, four per word: whole nodes (index < nof_full) clamped to +-64, a ragged tail as is
 // (ldpc_decoder_impl.cpp:147-188). last: one past the last non-zero LLR seen (the trailing-zero trim,
 // ldpc_decoder_impl.cpp:66-71); ragged: a tail value of magnitude 121 to 126 was seen.
-__device__ __forceinline__ void fetch8(const int8_t* __restrict__ in, int k, int n, int nof_full, bool aligned,
+// q: the eight LLRs where fetch_whole holds.
+__device__ __forceinline__ bool fetch_whole(int k, int nof_full, bool aligned)
+{
+  return aligned && k >= 0 && k + 8 <= nof_full;
+}
+
+__device__ __forceinline__ void fetch8(const int8_t* __restrict__ in, int k, int n, int nof_full, bool aligned, uint2 q,
                                        int& last, int& ragged, uint32_t& w0, uint32_t& w1)
 {
-  if (aligned && k >= 0 && k + 8 <= nof_full) {
-    const uint2 q = __ldg(reinterpret_cast<const uint2*>(in + k));
+  if (fetch_whole(k, nof_full, aligned)) {
     if ((q.x | q.y) != 0) {
       last = max(last, k + (q.y != 0 ? 8 - (__clz(q.y) >> 3) : 4 - (__clz(q.x) >> 3)));
     }
@@ -991,7 +1079,6 @@ __device__ __forceinline__ void decode_codeblock_pair(const pg_ldpc_cb& d, pair_
   const int          g        = bg - 1;
   const int          Kb       = bg == 1 ? 22 : 10;
   const int          nrows    = bg == 1 ? pg::kBg1Rows : pg::kBg2Rows;
-  const int          nedges   = bg == 1 ? pg::kBg1Edges : pg::kBg2Edges;
   const int          nfull    = bg == 1 ? 68 : 52;
   const int          msg_len  = Kb * Z;
   const int          n        = (int)d.nof_llrs;
@@ -1016,68 +1103,84 @@ __device__ __forceinline__ void decode_codeblock_pair(const pg_ldpc_cb& d, pair_
   const bool         active   = tid < T * H;
   const uint32_t     jp       = (uint32_t)(active ? tid / T : H - 1);
 
-  // Edge table of this lifting size, row list, constant column.
-  for (int e = tid; e < nedges; e += NT) {
-    const int      r    = tb.edge_row[g][e];
-    const uint32_t s    = (uint32_t)tb.edge_v[g][e][set] % (uint32_t)Z;
-    const bool     up   = s >= (uint32_t)H;
-    const uint32_t sp   = up ? s - (uint32_t)H : s;
+  // Edge table of this lifting size, row list, constant column. Meets the soft bits' loads below at one
+  // barrier.
+  for (int p = tid; p < tb.pad_e0[LG][g][nrows]; p += NT) {
+    const uint32_t c  = tb.pad_col[LG][g][p];
+    const uint32_t s  = (uint32_t)tb.pad_v[LG][g][p][set] % (uint32_t)Z;
+    const bool     up = s >= (uint32_t)H;
+    const uint32_t sp = up ? s - (uint32_t)H : s;
     // {shared address of (col, s'), 1 - (H - s') as a float, selector 0x3210 or (swapped) 0x1032, its change when
-    // the edge wraps (sign and magnitude)}
-    tab[tb.pad_e0[LG][g][r] + e - tb.row_e0[g][r]] =
-        make_uint4(E_s + h4 * (1u + tb.edge_col[g][e]) + 4u * sp, __float_as_uint(1.f - (float)(H - (int)sp)),
-                   up ? 0x1032u : 0x3210u, up ? 0x21deu : 0x800021deu);
+    // the edge wraps (sign and magnitude)}; the constant column's edges never wrap.
+    tab[p] = c == 0u ? make_uint4(E_s, __float_as_uint(-1024.f), 0x3210u, 0u)
+                     : make_uint4(E_s + h4 * c + 4u * sp, __float_as_uint(1.f - (float)(H - (int)sp)),
+                                  up ? 0x1032u : 0x3210u, up ? 0x21deu : 0x800021deu);
   }
   for (int r = tid; r < nrows; r += NT) {
-    const int deg = tb.row_deg[g][r];
     const int p0 = tb.pad_e0[LG][g][r], p1 = tb.pad_e0[LG][g][r + 1];
-    for (int k = deg; k < p1 - p0; ++k) {
-      tab[p0 + k] = make_uint4(E_s, __float_as_uint(-1024.f), 0x3210u, 0u); // the constant column
-    }
-    sh.row[r] = make_uint4(tab_s + 16u * (uint32_t)p0, (uint32_t)(nta * tb.msg0[LG][g][r]), (uint32_t)((p1 - p0) / T),
-                           (uint32_t)tb.row_sync[g][r]);
+    sh.row[r] = make_uint4(tab_s + 16u * (uint32_t)p0, 4u * (uint32_t)(nta * tb.msg0[LG][g][r]), (uint32_t)((p1 - p0) / T),
+                           tb.row_sync[g][r] != 0 ? (uint32_t)nta : 0u);
   }
   for (int k = tid; k < H; k += NT) {
     reinterpret_cast<uint32_t*>(E)[k] = kH8192;
   }
   if (tid == 0) {
-    sh.last   = 0;
-    sh.ragged = 0;
     sh.tb_crc = 0;
     sh.crc[0] = sh.crc[1] = 0;
     sh.zero[0] = sh.zero[1] = 0;
   }
-  __syncthreads();
 
   // Soft bits as f16 pairs (2Z punctured zeros, then the input): eight pairs per thread step when
   // the node halves are multiples of eight lanes, else one.
   {
     const int nof_full = (n / Z) * Z;
+    const int ncols    = min(nfull, max((n + Z - 1) / Z + 2, Kb + 4)); // the columns that the rows can use
     int       last = 0, ragged = 0;
     uint32_t* E0 = reinterpret_cast<uint32_t*>(E) + H;
     if ((H & 7) == 0) {
       const int      per_col = H >> 3;
-      const int      nchunks = nfull * per_col;
+      const int      nchunks = ncols * per_col;
       const uint32_t inv     = 0xffffffffu / (uint32_t)per_col + 1u;
       const bool     aligned = (reinterpret_cast<uintptr_t>(in) & 7u) == 0;
-#pragma unroll 2
-      for (int q = tid; q < nchunks; q += NT) {
-        const int col = per_col == 1 ? q : (int)__umulhi((uint32_t)q, inv);
-        const int w0  = (q - col * per_col) * 8;
-        const int k   = (col - 2) * Z + w0;
-        uint32_t  l0, l1, u0, u1;
-        fetch8(in, k, n, nof_full, aligned, last, ragged, l0, l1);
-        fetch8(in, k + H, n, nof_full, aligned, last, ragged, u0, u1);
-        const uint32_t p0 = __byte_perm(l0, u0, 0x5140), p1 = __byte_perm(l0, u0, 0x7362);
-        const uint32_t p2 = __byte_perm(l1, u1, 0x5140), p3 = __byte_perm(l1, u1, 0x7362);
-        uint32_t*      o = E0 + col * H + w0;
-        *reinterpret_cast<uint4*>(o) =
-            make_uint4(bytes_to_h2(p0), bytes_to_h2(p0 >> 16), bytes_to_h2(p1), bytes_to_h2(p1 >> 16));
-        *reinterpret_cast<uint4*>(o + 4) =
-            make_uint4(bytes_to_h2(p2), bytes_to_h2(p2 >> 16), bytes_to_h2(p3), bytes_to_h2(p3 >> 16));
+      for (int q0 = tid; q0 < nchunks; q0 += kFetchBatch * NT) {
+        // The batch's aligned whole-node loads are issued together; other pieces are read when they are used.
+        uint2 raw[kFetchBatch][2];
+        int   pos[kFetchBatch];
+#pragma unroll
+        for (int u = 0; u < kFetchBatch; ++u) {
+          const int q   = q0 + u * NT;
+          const int col = per_col == 1 ? q : (int)__umulhi((uint32_t)q, inv);
+          const int k   = (col - 2) * Z + (q - col * per_col) * 8;
+          pos[u]        = q < nchunks ? k : INT_MIN;
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            raw[u][i] = make_uint2(0u, 0u);
+            if (fetch_whole(k + i * H, nof_full, aligned) && q < nchunks) {
+              raw[u][i] = __ldg(reinterpret_cast<const uint2*>(in + k + i * H));
+            }
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < kFetchBatch; ++u) {
+          if (pos[u] == INT_MIN) {
+            break;
+          }
+          const int q   = q0 + u * NT;
+          const int col = per_col == 1 ? q : (int)__umulhi((uint32_t)q, inv);
+          uint32_t  l0, l1, u0, u1;
+          fetch8(in, pos[u], n, nof_full, aligned, raw[u][0], last, ragged, l0, l1);
+          fetch8(in, pos[u] + H, n, nof_full, aligned, raw[u][1], last, ragged, u0, u1);
+          const uint32_t p0 = __byte_perm(l0, u0, 0x5140), p1 = __byte_perm(l0, u0, 0x7362);
+          const uint32_t p2 = __byte_perm(l1, u1, 0x5140), p3 = __byte_perm(l1, u1, 0x7362);
+          uint32_t*      o = E0 + col * H + (q - col * per_col) * 8;
+          *reinterpret_cast<uint4*>(o) =
+              make_uint4(bytes_to_h2(p0), bytes_to_h2(p0 >> 16), bytes_to_h2(p1), bytes_to_h2(p1 >> 16));
+          *reinterpret_cast<uint4*>(o + 4) =
+              make_uint4(bytes_to_h2(p2), bytes_to_h2(p2 >> 16), bytes_to_h2(p3), bytes_to_h2(p3 >> 16));
+        }
       }
     } else {
-      const int      nwords = nfull * H;
+      const int      nwords = ncols * H;
       const uint32_t inv    = 0xffffffffu / (uint32_t)H + 1u;
 #pragma unroll 4
       for (int q = tid; q < nwords; q += NT) {
@@ -1099,16 +1202,19 @@ __device__ __forceinline__ void decode_codeblock_pair(const pg_ldpc_cb& d, pair_
       }
     }
     last = __reduce_max_sync(0xffffffffu, last);
-    if ((tid & 31) == 0 && last > 0) {
-      atomicMax(&sh.last, last);
-    }
-    if (ragged) {
-      sh.ragged = 1;
+    ragged = __any_sync(0xffffffffu, ragged);
+    if ((tid & 31) == 0) {
+      sh.seen[tid >> 5] = 2 * last + (ragged != 0 ? 1 : 0);
     }
   }
   __syncthreads();
 
-  const int input_size = sh.last;
+  int input_size = 0, ragged_any = 0;
+#pragma unroll
+  for (int w = 0; w < NT / 32; ++w) {
+    input_size = max(input_size, sh.seen[w] >> 1);
+    ragged_any |= sh.seen[w] & 1;
+  }
   if (input_size < msg_len) {
     for (int b = tid; b < nbytes; b += NT) {
       out[b] = 0xff;
@@ -1124,15 +1230,16 @@ __device__ __forceinline__ void decode_codeblock_pair(const pg_ldpc_cb& d, pair_
   int cb_len = max(input_size + 2 * Z, (Kb + 4) * Z);
   cb_len     = ((cb_len + Z - 1) / Z) * Z;
   const int      nof_layers = min(cb_len / Z - Kb, nrows);
-  const bool     ragged     = sh.ragged != 0;
+  const bool     ragged     = ragged_any != 0;
   const int      order      = crc_poly == PG_CRC16 ? 16 : 24;
   const uint32_t* pow_tab   = crc_pow + (size_t)(crc_poly <= PG_CRC24B ? crc_poly : 0) * pg::kCrcPowLen;
   const int      crc_len    = msg_len - (int)d.nof_filler_bits;
 
   // Messages: behind the columns of the rows that run (the columns past them hold only zeros).
-  const uint32_t o_msg   = kPairTabBytes + ((h4 * (uint32_t)(1 + Kb + nof_layers) + 15u) & ~15u);
-  const uint32_t msg_len_bytes = 4u * (uint32_t)nta * tb.msg0[LG][g][nof_layers];
-  uint32_t* msg = (o_msg + msg_len_bytes <= smem_bytes ? reinterpret_cast<uint32_t*>(smem + o_msg) : slab);
+  const uint32_t o_msg    = kPairTabBytes + ((h4 * (uint32_t)(1 + Kb + nof_layers) + 15u) & ~15u);
+  const bool     in_smem  = o_msg + 4u * (uint32_t)nta * tb.msg0[LG][g][nof_layers] <= smem_bytes;
+  const msg_shared msg_s{tab_s + o_msg};
+  const msg_global msg_g{reinterpret_cast<unsigned char*>(slab)};
 
   int       result = 0;
   const int max_it = d.max_iterations;
@@ -1146,19 +1253,26 @@ __device__ __forceinline__ void decode_codeblock_pair(const pg_ldpc_cb& d, pair_
   const float nh4d = __uint_as_float(0x80000000u | h4);
   for (int it = 0; it < max_it; ++it) {
     if (tid < nta) {
-      for (int r = 0; r < nof_layers; ++r) {
-        const uint4  rd = sh.row[r];
-        const int    ne = (int)rd.z;
-        uint32_t*    mr = msg + rd.y;
-        if (it > 0) {
-          pair_row_dispatch<false, T>(ne, tpart16, rd.x, jf, j4d, nh4d, mr, active);
-        } else if (!ragged) {
-          pair_row_dispatch<true, T>(ne, tpart16, rd.x, jf, j4d, nh4d, mr, active);
+      if (it > 0) {
+        if (in_smem) {
+          pair_rows<false, T>(sh, nof_layers, tpart16, jf, j4d, nh4d, msg_s, active);
         } else {
-          pair_row_ragged<T>(ne, rd.x + tpart16 * ne, jf, j4d, nh4d, mr + tid * ((ne + 1) / 2), active);
+          pair_rows<false, T>(sh, nof_layers, tpart16, jf, j4d, nh4d, msg_g, active);
         }
-        if (rd.w != 0 && r + 1 < nof_layers) {
-          asm volatile("bar.sync 1, %0;" ::"r"(nta) : "memory");
+      } else if (!ragged) {
+        if (in_smem) {
+          pair_rows<true, T>(sh, nof_layers, tpart16, jf, j4d, nh4d, msg_s, active);
+        } else {
+          pair_rows<true, T>(sh, nof_layers, tpart16, jf, j4d, nh4d, msg_g, active);
+        }
+      } else {
+        uint32_t* const msg = in_smem ? reinterpret_cast<uint32_t*>(smem + o_msg) : slab;
+        uint32_t        sync = 0;
+        for (int r = 0; r < nof_layers; ++r) {
+          const uint4 rd = sh.row[r];
+          const int   ne = (int)rd.z;
+          pair_row_ragged<T>(ne, rd.x + tpart16 * ne, jf, j4d, nh4d, msg + rd.y / 4 + tid * ((ne + 1) / 2), active, sync);
+          sync = rd.w;
         }
       }
     }
@@ -1171,19 +1285,16 @@ __device__ __forceinline__ void decode_codeblock_pair(const pg_ldpc_cb& d, pair_
     if (cgrp < ngrp) {
       const int       k  = tid - cgrp * H;
       const uint32_t* Ec = reinterpret_cast<const uint32_t*>(E) + H + k;
-#pragma unroll 4
+#pragma unroll 6
       for (int c = cgrp; c < Kb; c += ngrp) {
         const uint32_t x  = Ec[c * H];
         const int      i0 = c * Z + k, i1 = i0 + H;
+        // The powers are loaded whatever the soft bits are, so that the loads of several columns overlap.
+        const uint32_t q0 = crc_poly != PG_CRC_NONE && i0 < crc_len ? __ldg(pow_tab + (crc_len - 1 - i0 + order)) : 0u;
+        const uint32_t q1 = crc_poly != PG_CRC_NONE && i1 < crc_len ? __ldg(pow_tab + (crc_len - 1 - i1 + order)) : 0u;
         zero |= (x & 0x7fffu) == 0 || (x & 0x7fff0000u) == 0;
-        if (crc_poly != PG_CRC_NONE) {
-          if (pair_hard(x & 0xffffu) && i0 < crc_len) {
-            crc ^= __ldg(pow_tab + (crc_len - 1 - i0 + order));
-          }
-          if (pair_hard(x >> 16) && i1 < crc_len) {
-            crc ^= __ldg(pow_tab + (crc_len - 1 - i1 + order));
-          }
-        }
+        crc ^= pair_hard(x & 0xffffu) ? q0 : 0u;
+        crc ^= pair_hard(x >> 16) ? q1 : 0u;
       }
     }
     crc  = __reduce_xor_sync(0xffffffffu, crc);
@@ -1290,7 +1401,6 @@ __device__ __forceinline__ void decode_codeblock_pair(const pg_ldpc_cb& d, pair_
   }
 }
 
-constexpr int kPairThreads = 384;
 constexpr int kPairPerSm   = 2;
 constexpr int kPairMaxSmem = 227 * 1024 - (((int)sizeof(pair_shared) + 15) & ~15); // dynamic, one CTA per SM
 
@@ -1307,11 +1417,14 @@ static_assert(kPairMinSmem + 2048 <= 228 * 1024 / kPairPerSm, "every column fits
 // threads per lane pair above Z = 192, four below; odd lifting sizes (Z <= 15) with the one-lane
 // arithmetic.
 //
-// Bound: at 512 codeblocks the ALU pipe and latency (24 warps per SM), with few codeblocks latency
-// alone (12 warps). B200, against the kernel this one replaced (two lanes per thread, one thread per
-// lane pair, Z = 384 only, messages in L2): 512 codeblocks BG1/BG2 Z = 384, 0.528 -> 0.364 ms; 6
-// codeblocks BG1 Z = 384, 257 -> 155 us; 200 codeblocks of many sizes, 302 -> 190 us. One thread per
-// lane pair (192 threads, three CTAs per SM) took 0.415 ms, 200 us and 268 us.
+// Bound: at 512 codeblocks instruction issue (69 % of the slots with 24 warps per SM), with few codeblocks
+// latency (12 warps, 46 %). B200, against the kernel this one replaced (two lanes per thread, one thread per
+// lane pair, Z = 384 only, messages in L2): 512 codeblocks BG1/BG2 Z = 384, 528 -> 327 us; 6 codeblocks BG1
+// Z = 384, 257 -> 123 us; 200 codeblocks of many sizes, 302 -> 134 us. One thread per lane pair (192 threads,
+// three CTAs per SM) took 415, 200 and 268 us where this split took 364, 155 and 190. From there: the step's
+// barrier moved behind the next row's tables and messages 336, 138 and 156 us; message addresses of their
+// space (shared or global) in place of generic ones 330, 128 and 137; the table and the soft bits loaded in one
+// latency, the CRC powers by address alone 327, 123 and 134.
 __global__ void __launch_bounds__(kPairThreads, kPairPerSm)
     ldpc_decode_pair_kernel(const pg_ldpc_cb* __restrict__ descs, const int8_t* __restrict__ llrs,
                             uint8_t* __restrict__ bits, int32_t* __restrict__ iterations, int8_t* __restrict__ c2v_all,
@@ -1589,18 +1702,16 @@ int ldpc_upload_tables(pg_context* ctx)
   for (int gi = 0; gi < 2; ++gi) {
     const int rows = gi == 0 ? PG_BG1_ROWS : PG_BG2_ROWS;
     for (int r = 0; r < rows; ++r) {
-      pt.row_deg[gi][r]    = deg[gi][r];
-      pt.row_e0[gi][r + 1] = row_e0[gi][r + 1];
-      for (int e = row_e0[gi][r]; e < row_e0[gi][r + 1]; ++e) {
-        pt.edge_row[gi][e] = (uint8_t)r;
-        pt.edge_col[gi][e] = col[gi][e];
-        std::copy(v[gi][e], v[gi][e] + 8, pt.edge_v[gi][e]);
-      }
       for (int lg = 0; lg < 2; ++lg) {
         const int t                = 2 << lg;
         const int ne               = (deg[gi][r] + t - 1) / t;
         pt.pad_e0[lg][gi][r + 1]   = (uint16_t)(pt.pad_e0[lg][gi][r] + ne * t);
         pt.msg0[lg][gi][r + 1]     = (uint16_t)(pt.msg0[lg][gi][r] + (ne + 1) / 2);
+        for (int k = 0; k < deg[gi][r]; ++k) {
+          const int e = row_e0[gi][r] + k, p = pt.pad_e0[lg][gi][r] + k;
+          pt.pad_col[lg][gi][p] = (uint8_t)(col[gi][e] + 1);
+          std::copy(v[gi][e], v[gi][e] + 8, pt.pad_v[lg][gi][p]);
+        }
       }
     }
     for (int st = 0; st < nsteps[gi]; ++st) {
@@ -1631,12 +1742,14 @@ int ldpc_launch(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_
   return ldpc_launch_scratch(ctx, descs_dev, n, llrs, bits, iterations, ctx->dev.c2v, stream);
 }
 
-// CTAs of the decoder the context's batch decodes launch for n codeblocks: one per SM up to one and a half
-// codeblocks per SM (their messages then stay in shared memory: 200 codeblocks of many sizes 234 us
-// against 245 with two per SM), two per SM above (512 codeblocks 378 us against 462 with one).
+// CTAs of the decoder the context's batch decodes launch for n codeblocks: one per SM up to one and three
+// quarter codeblocks per SM (their messages then stay in shared memory), two per SM above. One against two
+// per SM, whole calls: 200 codeblocks of many sizes 196 and 231 us; BG1/BG2 mixed, Z = 384, 222 codeblocks
+// 228 and 299, 260 238 and 308, 350 300 and 291, 512 399 and 353; Z = 96, 200 codeblocks 153 and 160, 296
+// 182 and 166.
 static int batch_ctas(const pg_context* ctx, int n)
 {
-  const int per_sm = ctx->ldpc_ctas_per_sm > 0 ? ctx->ldpc_ctas_per_sm : (2 * n <= 3 * ctx->sm_count ? 1 : kPairPerSm);
+  const int per_sm = ctx->ldpc_ctas_per_sm > 0 ? ctx->ldpc_ctas_per_sm : (4 * n <= 7 * ctx->sm_count ? 1 : kPairPerSm);
   return std::min(n, ldpc_max_ctas(ctx, per_sm, ctx->ldpc_kernel));
 }
 
