@@ -163,12 +163,19 @@ int rate_dematch_launch(pg_context* ctx, const pg_rm_cb* descs_dev, int n, const
 // descs_dev when list is not NULL (a plan's codeblocks that the demodulator does not store in place).
 int rate_dematch_launch(pg_context* ctx, const pg_rm_cb* descs_dev, int n, const int8_t* in, int8_t* out,
                         cudaStream_t stream, int ctas_per_cb, const uint32_t* list = nullptr);
-// Writes what rate dematching leaves at the positions no LLR reaches (+127 at the fillers, 0
-// elsewhere) over the whole circular buffer of every codeblock with placed[c] = 1, to be done
-// before the demodulator stores those codeblocks' LLRs in place.
-// The same launch zeroes tb_out (tb_bytes) and *counter.
-int rm_prefill_launch(pg_context* ctx, const pg_rm_cb* descs_dev, int n, const uint8_t* placed, int8_t* out,
-                      uint8_t* tb_out, size_t tb_bytes, int* counter, cudaStream_t stream);
+// Before a slot plan's demodulator stores LLRs in place: the circular buffers of the codeblocks with
+// placed[c] = 1 get what rate dematching leaves at the positions no LLR reaches (+127 at the fillers, 0
+// elsewhere), and tb_out and *counter are zeroed (rm_prefill, kRmFillCtas CTAs per codeblock).
+struct rm_fill {
+  const pg_rm_cb* cbs;
+  const uint8_t*  placed;
+  int8_t*         out;
+  uint8_t*        tb_out;
+  size_t          tb_bytes;
+  int*            counter;
+  int             n;
+};
+constexpr int kRmFillCtas = 4;
 void crc_tables_host(uint32_t* tab);
 int crc_launch(pg_context* ctx, const pg_crc_item* items_dev, int n, const uint8_t* data, uint32_t* out,
                cudaStream_t stream);
@@ -245,11 +252,12 @@ int validate_ues(pg_context* ctx, const pg_pusch_ue* ues, int n);
 // *pilot_words words in total), and returns the item count. work_dev holds that blob on the device,
 // partials nwork float4, arrivals 4 n ints that are zero before the launch (and again after it).
 // pilot_bits (may be NULL: the kernel then forms the pilots from the Gold basis) holds the rows
-// written by dmrs_bits_launch for the same UEs and blob.
+// written by dmrs_bits_launch for the same UEs and blob. fill (may be NULL): the launch's last CTAs run it.
 int est_work_build(const pg_pusch_ue* ues, int n, std::vector<uint32_t>& blob, uint32_t* pilot_words = nullptr);
 int estimate_launch(pg_context* ctx, const pg_pusch_ue* ues_dev, int n, const uint32_t* work_dev, int nwork,
                     void* partials, int* arrivals, const uint32_t* grids, float* est, float* ls,
-                    pg_port_result* results, cudaStream_t s, const uint32_t* pilot_bits = nullptr);
+                    pg_port_result* results, cudaStream_t s, const uint32_t* pilot_bits = nullptr,
+                    const rm_fill* fill = nullptr);
 // The DM-RS sequence bits of every UE (their slot, N_ID, n_SCID and symbols), once per plan.
 int dmrs_bits_launch(pg_context* ctx, const pg_pusch_ue* ues_dev, int n, const uint32_t* work_dev, int nwork,
                      uint32_t* bits_dev, cudaStream_t s);

@@ -20,6 +20,7 @@
 // c is linear in c_init, so 32 precomputed basis sequences give any sequence word by word.
 #include "pg_internal.h"
 #include "pg_device.cuh"
+#include "rm_prefill.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -458,8 +459,15 @@ __global__ void __launch_bounds__(kChunkThreads) pusch_estimate_chunk_kernel(con
                                                                              int* __restrict__ arrivals,
                                                                              pg_port_result* __restrict__ results,
                                                                              const uint32_t* __restrict__ pilot_bits,
-                                                                             int nof_ues)
+                                                                             int nof_ues, int nwork,
+                                                                             const __grid_constant__ pg::rm_fill fill)
 {
+  // A slot plan's buffers are filled by CTAs behind the estimator's. On a branch of its own beside this kernel
+  // the fill's fork and join cost 1.7 us of a 45 us slot.
+  if ((int)blockIdx.x >= nwork) {
+    pg::rm_prefill<kChunkThreads>(fill, (int)blockIdx.x - nwork);
+    return;
+  }
   __shared__ uint32_t s_bits[kMaxDmrs][(2 * kChunkTile) / 32 + 2];
   __shared__ float2   s_y[kMaxDmrs][kChunk]; // the received pilots of the chunk (LS, then noise)
   __shared__ float2   s_ls[kMaxDmrs][2][kChunkTile];
@@ -507,7 +515,7 @@ __global__ void __launch_bounds__(kChunkThreads) pusch_estimate_chunk_kernel(con
   // bits (dmrs_bits_launch; bit b of symbol d's row = c(12 rb_start + b)) or from the Gold basis.
   const int nwords = (2 * (pe - pb) + 31) / 32;
   if (pilot_bits != nullptr) {
-    const uint32_t* pbits = pilot_bits + work[gridDim.x + 4 * nof_ues + 1 + u];
+    const uint32_t* pbits = pilot_bits + work[nwork + 4 * nof_ues + 1 + u];
     const int       W     = dmrs_bit_words(nrb);
     const int       w0    = (2 * pb) >> 5;
     const int       sh    = (2 * pb) & 31;
@@ -651,7 +659,7 @@ __global__ void __launch_bounds__(kChunkThreads) pusch_estimate_chunk_kernel(con
   __syncthreads();
   __shared__ int s_last;
   const int       pi    = 4 * u + port;
-  const uint32_t* first = work + gridDim.x; // the work list (one item per CTA), then each port's first item
+  const uint32_t* first = work + nwork; // the work list (one item per CTA), then each port's first item
   if (tid == 0) {
     float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int w = 0; w < kChunkThreads / 32; ++w) {
@@ -980,14 +988,16 @@ int dmrs_bits_launch(pg_context* ctx, const pg_pusch_ue* ues_dev, int n, const u
 
 int estimate_launch(pg_context* ctx, const pg_pusch_ue* ues_dev, int n, const uint32_t* work_dev, int nwork,
                     void* partials, int* arrivals, const uint32_t* grids, float* est, float* ls,
-                    pg_port_result* results, cudaStream_t s, const uint32_t* pilot_bits)
+                    pg_port_result* results, cudaStream_t s, const uint32_t* pilot_bits, const rm_fill* fill)
 {
-  if (n == 0 || nwork == 0) {
+  const int nfill = fill != nullptr ? kRmFillCtas * fill->n : 0;
+  if (nwork + nfill == 0) {
     return PG_OK;
   }
-  pusch_estimate_chunk_kernel<<<nwork, kChunkThreads, 0, s>>>(
+  pusch_estimate_chunk_kernel<<<nwork + nfill, kChunkThreads, 0, s>>>(
       ues_dev, work_dev, grids, reinterpret_cast<float2*>(est), reinterpret_cast<float2*>(ls),
-      static_cast<float4*>(partials), ctx->dev.gold, kGoldWords, arrivals, results, pilot_bits, n);
+      static_cast<float4*>(partials), ctx->dev.gold, kGoldWords, arrivals, results, pilot_bits, n, nwork,
+      fill != nullptr ? *fill : rm_fill{});
   return check_cuda(ctx, cudaGetLastError(), "pusch_estimate_chunk_kernel launch");
 }
 

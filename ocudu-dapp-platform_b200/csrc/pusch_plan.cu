@@ -73,12 +73,8 @@ struct pg_pusch_plan {
   uint8_t*        d_placed   = nullptr; // per codeblock: 1 when the demodulator places its LLRs
   uint32_t*       d_unplaced = nullptr; // capacity nof_cbs
   uint32_t*       d_pilot_bits = nullptr; // DM-RS sequence bits of every UE (dmrs_bits_launch)
-  // Side branch of every execution: the in-place codeblocks' circular buffers are prefilled on
-  // `aux` (forked from and joined back into the execution's stream) beside the channel estimation.
-  cudaStream_t    aux        = nullptr;
-  cudaEvent_t     ev_fork    = nullptr;
-  cudaEvent_t     ev_join    = nullptr;
-  cudaEvent_t     ev_ufork   = nullptr; // UCI decoding on the aux stream, beside the UL-SCH stages
+  cudaStream_t    aux        = nullptr; // plans with UCI: its decoding, beside the UL-SCH stages
+  cudaEvent_t     ev_ufork   = nullptr; // from and back into the execution's stream
   cudaEvent_t     ev_ujoin   = nullptr;
   cudaEvent_t     ev_uread   = nullptr; // orders the host's reads of the UCI results
   uint32_t*       d_est_work = nullptr; // channel-estimation work list and per-(UE, port) first items
@@ -190,7 +186,7 @@ size_t al(size_t x)
 // buffers when every codeblock holds new data without repetition (E <= N_cb - F), as a
 // consecutive run of E values with the smaller ones first and buffers a constant stride apart;
 // other UEs keep the codeword buffer and the rate-dematch kernel. placed[c] = 1 for the codeblocks
-// of the enabled UEs (prefilled with rm_prefill_launch, left alone by the rate-dematch kernel).
+// of the enabled UEs (prefilled by the estimation launch, left alone by the rate-dematch kernel).
 void build_direct(const std::vector<pg_pusch_ue>& ues, const std::vector<pg_rm_cb>& rm, const std::vector<int>& first,
                   const std::vector<int>& ncb, std::vector<rm_direct>& direct, std::vector<uint8_t>& placed)
 {
@@ -287,22 +283,12 @@ int enqueue(pg_pusch_plan* p, const uint32_t* grids, uint8_t* tb_out, pg_sch_res
             pg_port_result* port_results, cudaStream_t s)
 {
   pg_context* ctx = p->ctx;
-  // Fork: the in-place codeblocks' prefill depends on nothing of this execution (the previous
-  // execution on this stream, whose decoder read the buffers, precedes the fork).
-  int rc = check_cuda(ctx, cudaEventRecord(p->ev_fork, s), "cudaEventRecord(fork)");
-  if (rc == PG_OK) {
-    rc = estimate_launch(ctx, p->d_ues, p->nof_ues, p->d_est_work, p->est_nwork, p->d_est_part, p->d_est_arr, grids,
-                         p->d_est, p->le_net != nullptr ? p->d_ls : nullptr, port_results, s, p->d_pilot_bits);
-  }
-  if (rc == PG_OK) {
-    rc = check_cuda(ctx, cudaStreamWaitEvent(p->aux, p->ev_fork, 0), "cudaStreamWaitEvent(fork)");
-  }
-  if (rc == PG_OK) {
-    rc = rm_prefill_launch(ctx, p->d_rm, p->nof_cbs, p->d_placed, p->d_rm_out, tb_out, p->tb_bytes, p->d_counter, p->aux);
-  }
-  if (rc == PG_OK) {
-    rc = check_cuda(ctx, cudaEventRecord(p->ev_join, p->aux), "cudaEventRecord(join)");
-  }
+  // The estimator's launch also fills the in-place codeblocks' buffers (the previous execution on this stream,
+  // whose decoder read them, precedes it).
+  const rm_fill fill{p->d_rm, p->d_placed, p->d_rm_out, tb_out, p->tb_bytes, p->d_counter, p->nof_cbs};
+  int           rc = estimate_launch(ctx, p->d_ues, p->nof_ues, p->d_est_work, p->est_nwork, p->d_est_part, p->d_est_arr,
+                                     grids, p->d_est, p->le_net != nullptr ? p->d_ls : nullptr, port_results, s,
+                                     p->d_pilot_bits, &fill);
   if (rc == PG_OK && p->le_net != nullptr) {
     const unsigned int flags = timing_record_flags(ctx, s);
     if (ctx->timed) {
@@ -314,9 +300,6 @@ int enqueue(pg_pusch_plan* p, const uint32_t* grids, uint8_t* tb_out, pg_sch_res
       cudaEventRecordWithFlags(ctx->ev_le_stop, s, flags);
       ctx->le_recorded = true;
     }
-  }
-  if (rc == PG_OK) {
-    rc = check_cuda(ctx, cudaStreamWaitEvent(s, p->ev_join, 0), "cudaStreamWaitEvent(join)");
   }
   if (rc == PG_OK) {
     rc = demod_only_launch(ctx, p->d_ues, p->nof_ues, p->total_tiles, p->d_tile_map, grids, p->d_est, port_results,
@@ -397,7 +380,7 @@ void release(pg_pusch_plan* p)
     cudaStreamDestroy(p->aux);
   }
   for (cudaEvent_t e : {p->ev_h2d, p->ev_stage_free[0], p->ev_stage_free[1], p->ev_done[0], p->ev_done[1],
-                        p->ev_done[2], p->ev_fork, p->ev_join, p->ev_ufork, p->ev_ujoin, p->ev_uread}) {
+                        p->ev_done[2], p->ev_ufork, p->ev_ujoin, p->ev_uread}) {
     if (e) {
       cudaEventDestroy(e);
     }
@@ -786,7 +769,7 @@ int pg_pusch_plan_create_uci(pg_context* ctx, const pg_pusch_ue* ues, const pg_p
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaStreamCreateWithFlags(&p->aux, cudaStreamNonBlocking), "cudaStreamCreate(aux)");
   }
-  for (cudaEvent_t* e : {&p->ev_fork, &p->ev_join, &p->ev_ufork, &p->ev_ujoin, &p->ev_uread}) {
+  for (cudaEvent_t* e : {&p->ev_ufork, &p->ev_ujoin, &p->ev_uread}) {
     if (rc == PG_OK) {
       rc = check_cuda(ctx, cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate(fork/join)");
     }

@@ -237,73 +237,6 @@ __global__ void __launch_bounds__(kRmThreads) rate_dematch_kernel(const pg_rm_cb
   }
 }
 
-// The circular buffers of the codeblocks whose LLRs the demodulator stores in place (placed[c]
-// = 1: new data, E <= V), before it does: +127 at the filler positions [inf, (Kb - 2) Z) and 0
-// everywhere else, which is what rate dematching leaves at every position that no LLR reaches.
-// 16-byte stores; the first and last bytes of a buffer that does not start or end on a 16-byte
-// boundary are stored one by one.
-__global__ void __launch_bounds__(kRmThreads) rm_prefill_kernel(const pg_rm_cb* __restrict__ cbs,
-                                                                const uint8_t* __restrict__ placed,
-                                                                int8_t* __restrict__ out_all, uint8_t* __restrict__ tb_out,
-                                                                size_t tb_bytes, int* __restrict__ counter)
-{
-  // The TB buffer (bytes between the TBs stay zero) and the decoders' work counter.
-  {
-    const size_t nthr = (size_t)gridDim.x * gridDim.y * kRmThreads;
-    const size_t t0   = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kRmThreads + threadIdx.x;
-    const size_t head = min(tb_bytes, (size_t)((16u - (unsigned)(reinterpret_cast<uintptr_t>(tb_out) & 15u)) & 15u));
-    const size_t nvec = (tb_bytes - head) / 16;
-    uint4*       v    = reinterpret_cast<uint4*>(tb_out + head);
-    for (size_t q = t0; q < nvec; q += nthr) {
-      v[q] = make_uint4(0u, 0u, 0u, 0u);
-    }
-    if (t0 < head) {
-      tb_out[t0] = 0;
-    }
-    if (head + 16 * nvec + t0 < tb_bytes) {
-      tb_out[head + 16 * nvec + t0] = 0;
-    }
-    if (t0 == 0) {
-      *counter = 0;
-    }
-  }
-  if (placed[blockIdx.x] == 0) {
-    return;
-  }
-  const pg_rm_cb d    = cbs[blockIdx.x];
-  const int      Z    = d.lifting_size;
-  const int      N    = (d.base_graph == 1 ? 66 : 50) * Z;
-  const int      sys  = ((d.base_graph == 1 ? 22 : 10) - 2) * Z;
-  const int      inf  = sys - (int)d.nof_filler_bits;
-  int8_t*        out  = out_all + d.out_offset;
-  const int      head = min(N, (int)((16u - (unsigned)(reinterpret_cast<uintptr_t>(out) & 15u)) & 15u));
-  const int      nch  = (N - head) / 16;
-  const int      tail = head + 16 * nch;
-  const int      tid  = blockIdx.y * kRmThreads + threadIdx.x;
-  const int      nthr = gridDim.y * kRmThreads;
-  auto value = [&](int p) { return (int8_t)((p >= inf && p < sys) ? 127 : 0); };
-  if (tid < head) {
-    out[tid] = value(tid);
-  }
-  if (tail + tid < N) {
-    out[tail + tid] = value(tail + tid);
-  }
-  for (int q = tid; q < nch; q += nthr) {
-    const int c   = head + 16 * q;
-    const int fil = max(0, min(c + 16, sys) - max(c, inf));
-    uint4     w   = make_uint4(0u, 0u, 0u, 0u);
-    if (fil == 16) {
-      w = make_uint4(0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu);
-    } else if (fil > 0) {
-      int8_t* b = reinterpret_cast<int8_t*>(&w);
-      for (int i = 0; i < 16; ++i) {
-        b[i] = value(c + i);
-      }
-    }
-    *reinterpret_cast<uint4*>(out + c) = w;
-  }
-}
-
 } // namespace
 
 namespace pg {
@@ -367,17 +300,6 @@ int rate_dematch_launch(pg_context* ctx, const pg_rm_cb* descs_dev, int n, const
   ctas_per_cb = std::max(1, std::min(32, ctas_per_cb));
   rate_dematch_kernel<<<dim3(n, ctas_per_cb), kRmThreads, 0, stream>>>(descs_dev, in, out, list);
   return check_cuda(ctx, cudaGetLastError(), "rate_dematch_kernel launch");
-}
-
-int rm_prefill_launch(pg_context* ctx, const pg_rm_cb* descs_dev, int n, const uint8_t* placed, int8_t* out,
-                      uint8_t* tb_out, size_t tb_bytes, int* counter, cudaStream_t stream)
-{
-  if (n == 0) {
-    return PG_OK;
-  }
-  // N <= 25,344 bytes = 1,584 chunks: two CTAs of 256 threads per codeblock, about three stores each.
-  rm_prefill_kernel<<<dim3(n, 2), kRmThreads, 0, stream>>>(descs_dev, placed, out, tb_out, tb_bytes, counter);
-  return check_cuda(ctx, cudaGetLastError(), "rm_prefill_kernel launch");
 }
 
 } // namespace pg
