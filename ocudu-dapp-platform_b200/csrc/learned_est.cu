@@ -381,15 +381,19 @@ size_t al(size_t x)
 // completed, which precedes every write of B).
 //
 // Dataflow: the window is two M tiles of 128 pairs; the taps of either tile reach one pair into the
-// other. A producer warp waits for tile 0's epilogue barrier of layer l - 1 and issues the shifts
-// of tile 0 that read tile 0 only, loads the next layer's weights once layer l - 1's MMAs are
-// complete, waits for tile 1's epilogue barrier, issues tile 0's two remaining shifts (they read
-// tile 1's first pair) and commits tile 0, then issues and commits tile 1. Sixteen epilogue warps
-// (four per TMEM lane quarter, 32 accumulator columns each) take tile 0 as soon as its MMAs
-// complete - while tile 1's run - then tile 1: they add bias and residual, apply the ReLU and the
-// row mask, store bf16 to shared memory, make the stores visible to the tensor cores and arrive on
-// the tile's barrier. MMAs complete in issue order, so the epilogue of layer l writes its
-// destination only after every MMA of layer l - 1 that read it.
+// other. One warp issues tile 0's MMAs, another tile 1's. The first waits for tile 0's epilogue barrier of
+// layer l - 1 and issues the shifts of tile 0 that read tile 0 only, waits for tile 1's, issues tile 0's two
+// remaining shifts (they read tile 1's first pair), commits, and loads the next layer's weights. The second
+// waits for tile 1's barrier, issues tile 1 and commits. Sixteen epilogue warps (four per TMEM lane quarter,
+// 32 accumulator columns each) take tile 0 as soon as its MMAs complete - while tile 1's run - then tile 1:
+// they add bias and residual, apply the ReLU and the row mask, store bf16 to shared memory, make the stores
+// visible to the tensor cores and arrive on the tile's barrier. A tile's MMAs of layer l complete after the
+// epilogues of layer l - 1, hence after every MMA of layer l - 1, so the epilogue of layer l overwrites
+// nothing that is still read.
+//
+// Bound: the chain MMA - epilogue - MMA of tile 0. The tensor cores' operand reads take nearly all of the
+// shared-memory cycles, and a barrier probe under them 200 cycles or more: with one issuing warp, its five
+// waits stood between the MMAs and a layer took 5,600 cycles (tensor pipe busy for 3,000 of them).
 constexpr int      kFTiles    = 2;
 constexpr int      kFPairs    = 128 * kFTiles;
 constexpr int      kFWin      = 2 * kFPairs;
@@ -398,7 +402,7 @@ constexpr int      kFMargin   = 2 * kLayers;
 constexpr int      kFOut      = kFWin - 2 * kFMargin;
 constexpr int      kFOutHalf  = kFWin / 2 - 2 * kFMargin; // exact rows of a one-tile window
 constexpr int      kFEpiWarps = 16;
-constexpr int      kFThreads  = 32 * (kFEpiWarps + 1); // + producer warp
+constexpr int      kFThreads  = 32 * (kFEpiWarps + 2); // + one issuing warp per tile
 constexpr uint32_t kFChunkB   = kFPRows * 16;         // one 8-channel chunk of one plane
 constexpr uint32_t kFActB     = 2 * 8 * kFChunkB;     // [plane][chunk][pair]
 constexpr uint32_t kFWB       = kTaps * 8 * kCh * 16;
@@ -442,6 +446,23 @@ __device__ __forceinline__ uint32_t mask_positive(uint32_t w, uint32_t m)
 {
   const __nv_bfloat162 z = __floats2bfloat162_rn(0.f, 0.f);
   return w & __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&m), z);
+}
+
+// ReLU of packed bf16 values: the sign survives the rounding, and a NaN gives 0, as with fmaxf(x, 0).
+__device__ __forceinline__ uint32_t relu_bf16x2(uint32_t w)
+{
+  const __nv_bfloat162 r = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&w), __floats2bfloat162_rn(0.f, 0.f));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+
+__device__ __forceinline__ float2 add2(float2 a, float2 b) // one packed FP32 addition
+{
+  float2 r;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 z, x, y;\n\t"
+      "mov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
 }
 
 __device__ __forceinline__ uint32_t layer_weight_bytes(int l)
@@ -519,15 +540,18 @@ __device__ __forceinline__ void fused_issue_tile(int c, int part, uint32_t src, 
   }
 }
 
-// Bounded wait that gives up at once when another thread has recorded a failure.
+// Bounded wait that gives up when another thread has recorded a failure. The flag is read only between
+// probes: under the tensor cores' operand reads a shared-memory round trip takes 200 cycles or more.
 __device__ __forceinline__ bool fused_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_sm,
                                            int* __restrict__ err)
 {
-  if (*abort_sm != 0) {
-    return false;
-  }
-  if (mbar_wait_bounded(bar, parity)) {
-    return true;
+  for (uint32_t i = 0; i < kWaitLimit; ++i) {
+    if (mbar_try_wait(bar, parity)) {
+      return true;
+    }
+    if (*abort_sm != 0) {
+      return false;
+    }
   }
   *abort_sm = 1;
   atomicExch(err, 1);
@@ -578,7 +602,8 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
     *reinterpret_cast<uint4*>(smem + kFOffZero + 16 * i) = make_uint4(0, 0, 0, 0);
   }
   const uint32_t zero_s   = smem_u32(smem + kFOffZero);
-  const bool     producer = warp == kFEpiWarps;
+  const bool     issuer0  = warp == kFEpiWarps;
+  const bool     issuer1  = warp == kFEpiWarps + 1;
   const uint32_t bar_mma  = smem_u32(&bars[0]);           // + 8c
   const uint32_t bar_epi  = smem_u32(&bars[kFTiles]);     // + 8c
   const uint32_t bar_w    = smem_u32(&bars[2 * kFTiles]); // + 8b
@@ -588,7 +613,7 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
   if (warp == 0) {
     tmem_alloc(smem_u32(tmem_sm), kFCols);
   }
-  if (producer && lane == 0) {
+  if (issuer0 && lane == 0) {
     for (int c = 0; c < kFTiles; ++c) {
       mbar_init(bar_mma + 8u * c, 1);
       mbar_init(bar_epi + 8u * c, kFEpiWarps);
@@ -608,8 +633,8 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
   const int      q          = warp & 3;
   const int      cs         = (warp >> 2) & 3;
   uint32_t       step       = 0; // layer steps of this CTA (all roles count alike)
-  uint32_t       w_issued   = 1; // producer: weight loads issued (load k went to buffer k & 1)
-  uint32_t       mma_issued = 0; // producer: layer steps whose MMAs were issued
+  uint32_t       w_issued   = 1; // issuer of tile 0: weight loads issued (load k went to buffer k & 1)
+  uint32_t       mma_issued = 0; // issuers: layer steps whose MMAs were issued
 
   for (int win = blockIdx.x; win < n_win; win += gridDim.x) {
     // Windows 0 .. n_full - 1 have two M tiles, the rest one (kFOutHalf exact rows): the host picks
@@ -636,16 +661,14 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
     if (*abort_sm != 0) {
       break;
     }
-    if (producer) {
+    if (issuer0 || issuer1) {
       if (lane == 0) {
+        const int c = issuer0 ? 0 : 1;
         for (int l = 0; l < NL; ++l) {
           const uint32_t s   = step + (uint32_t)l;
           const uint32_t src = (l & 1) ? act_a : act_b;
-          if (!fused_wait(bar_w + 8u * (s & 1), (s >> 1) & 1u, abort_sm, err)) {
-            break;
-          }
-          const uint32_t wb    = wbuf0 + (s & 1) * kFWB;
-          auto           issue = [&](int c, int part) {
+          const uint32_t wb  = wbuf0 + (s & 1) * kFWB;
+          auto issue = [&](int part) {
             if (l == 0) {
               fused_issue_tile<kInCh, kCh, MODE != kFInfer>(c, part, src, wb, tmem, zero_s);
             } else if (MODE != kFBackward && l == kLayers - 1) {
@@ -654,49 +677,48 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
               fused_issue_tile<kCh, kCh, MODE != kFInfer>(c, part, src, wb, tmem, zero_s);
             }
           };
-          // Layer 0 follows the window barrier. Later layers: tile 0's first part reads tile 0 of
-          // layer l - 1 only, its second part and tile 1 also read tile 1 (and tile 1 overwrites
-          // tile 1's accumulator), so the epilogue barriers are waited in between.
+          if (!fused_wait(bar_w + 8u * (s & 1), (s >> 1) & 1u, abort_sm, err)) {
+            break;
+          }
+          // Layer 0 follows the window barrier. Later layers: tile 0's first part reads tile 0 of layer l - 1
+          // only; its second part and tile 1 also read the other tile. Tile 1's epilogue comes after tile 0's
+          // in every epilogue warp, so its barrier tells that both are done.
+          if (issuer0) {
+            if (l > 0) {
+              if (!fused_wait(bar_epi, (s - 1) & 1u, abort_sm, err)) {
+                break;
+              }
+              tc_fence_after();
+            }
+            issue(0);
+          }
           if (l > 0) {
-            if (!fused_wait(bar_epi, (s - 1) & 1u, abort_sm, err)) {
+            if (!fused_wait(bar_epi + 8u, (s - 1) & 1u, abort_sm, err)) {
+              if (issuer0) {
+                // Tile 0's first part is in flight: its barrier takes the completion, so that the wait
+                // after a failure below covers it.
+                mma_commit(bar_mma);
+                mma_issued = s + 1;
+              }
               break;
             }
             tc_fence_after();
           }
-          issue(0, 0);
-          // The MMAs of layer l - 1 are complete once its last commit (tile 1's barrier) has
-          // arrived, which precedes the epilogue waited next; before layer 0, the window barrier.
-          // Then its weight buffer takes the next layer (layer 0 of the next window after the
-          // last layer), in flight while this layer's MMAs run.
-          if (l > 0 && !fused_wait(bar_mma + 8u, (s - 1) & 1u, abort_sm, err)) {
-            mma_commit(bar_mma);
-            mma_commit(bar_mma + 8u);
-            mma_issued = s + 1;
-            break;
+          if (issuer0) {
+            issue(1);
+          } else if (two) {
+            issue(2);
           }
-          if (l + 1 < NL || win + (int)gridDim.x < n_win) {
+          mma_commit(bar_mma + 8u * c);
+          mma_issued = s + 1;
+          // Every MMA of layer l - 1 is complete (its epilogues are; before layer 0, the window barrier): its
+          // weight buffer takes the next layer (layer 0 of the next window after the last layer), in flight
+          // while this layer's MMAs and epilogues run.
+          if (issuer0 && (l + 1 < NL || win + (int)gridDim.x < n_win)) {
             const int nx = (l + 1) % NL;
             fused_load_weights(wp, MODE == kFBackward ? kLayers - 1 - nx : nx, wbuf0 + ((s + 1) & 1) * kFWB, bar_w + 8u * ((s + 1) & 1));
             ++w_issued;
           }
-          if (l > 0) {
-            if (!fused_wait(bar_epi + 8u, (s - 1) & 1u, abort_sm, err)) {
-              // Tile 0's first part is in flight: both barriers take its completion, so that the
-              // wait after a failure below covers it.
-              mma_commit(bar_mma);
-              mma_commit(bar_mma + 8u);
-              mma_issued = s + 1;
-              break;
-            }
-            tc_fence_after();
-          }
-          issue(0, 1);
-          mma_commit(bar_mma);
-          if (two) {
-            issue(1, 2);
-          }
-          mma_commit(bar_mma + 8u);
-          mma_issued = s + 1;
         }
       }
       __syncwarp();
@@ -714,6 +736,38 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
               mk[k] = (g >= 0 && g < R) ? __ldg(mp + (size_t)k * R) : make_uint4(0, 0, 0, 0);
             }
           }
+          // What the step needs beside its accumulators is read before the wait: the row mask, the bias and,
+          // in the second layer of a block, the residual (packed bf16 in TMEM, stored by this thread).
+          const bool     hidden = MODE == kFBackward || l < kLayers - 1;
+          const int      pr     = c * 128 + q * 32 + lane; // window row pair
+          const int      plane  = cs >> 1, hh = cs & 1;
+          const bool     second = l >= 2 && (l & 1) == 0;
+          const uint32_t tres   = tmem + ((uint32_t)(q * 32) << 16) + kFColRes + (uint32_t)(c * 64 + cs * 16);
+          bool           valid = false, all_valid = false;
+          float2         bb[16];
+          uint32_t       res[16];
+          if (hidden && (two || c == 0)) {
+            valid     = valid_s[2 * pr + plane] != 0;
+            all_valid = __all_sync(0xffffffffu, valid);
+            if (MODE != kFBackward) {
+              const float4* bl = reinterpret_cast<const float4*>(bias_s + l * kCh + hh * 32);
+#pragma unroll
+              for (int k = 0; k < 8; ++k) {
+                const float4 b4 = bl[k];
+                bb[2 * k]       = make_float2(b4.x, b4.y);
+                bb[2 * k + 1]   = make_float2(b4.z, b4.w);
+              }
+            }
+            if (second) {
+              tmem_wait_st();
+              float rf[16];
+              tmem_ld16(tres, rf);
+#pragma unroll
+              for (int k = 0; k < 16; ++k) {
+                res[k] = __float_as_uint(rf[k]);
+              }
+            }
+          }
           // One lane polls the barrier and tells the others: probes from all 32 lanes take
           // shared-memory cycles from the tensor cores' operand reads (measured 13 % slower).
           bool ok = false;
@@ -723,16 +777,12 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
           ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
           if (ok && (two || c == 0)) {
             tc_fence_after();
-            const int      pr  = c * 128 + q * 32 + lane;                 // window row pair
             const uint32_t tad = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 128);
-            if (MODE == kFBackward || l < kLayers - 1) {
+            if (hidden) {
               // 32 output channels (chunks 4 hh .. 4 hh + 3) of one row: one TMEM load of the
-              // accumulators, then straight-line arithmetic. Layers 0, 2, .. 12 write the block
+              // accumulators, then straight-line arithmetic on pairs. Layers 0, 2, .. 12 write the block
               // input, kept as packed bf16 in TMEM as well, where the second layer of the next block
               // reads its residual (no shared-memory reads beside the tensor cores').
-              const int      plane  = cs >> 1, hh = cs & 1;
-              const bool     valid  = valid_s[2 * pr + plane] != 0;
-              const bool     second = l >= 2 && (l & 1) == 0;
               const bool     keep   = (l & 1) == 0;
               unsigned char* dst    = (l & 1) ? buf_b : buf_a;
               const int      wr     = 2 * pr + plane; // window row
@@ -740,70 +790,48 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
               uint4*         op     = MODE != kFInfer ? io.out[l] + (size_t)(hh * 4) * R + (base + wr) : nullptr;
               uint4*         p      = reinterpret_cast<uint4*>(dst + fused_line(plane, hh * 4, pr + 1));
               constexpr int  kStep  = kFChunkB / 16; // uint4 per chunk
-              const float*   bl     = bias_s + l * kCh + hh * 32;
-              const uint32_t tres   = tmem + ((uint32_t)(q * 32) << 16) + kFColRes + (uint32_t)(c * 64 + cs * 16);
-              uint32_t       res[16];
-              if (second) {
-                float rf[16];
-                tmem_ld16(tres, rf);
-#pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                  res[k] = __float_as_uint(rf[k]);
-                }
-              }
-              float v[32];
+              float          v[32];
               tmem_ld32(tad + (uint32_t)(32 * cs), v);
               uint32_t kept[16];
 #pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const float4 b0 = reinterpret_cast<const float4*>(bl)[2 * k];
-                const float4 b1 = reinterpret_cast<const float4*>(bl)[2 * k + 1];
-                const float  bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-                float        o[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                  o[j] = v[8 * k + j] + (MODE == kFBackward ? 0.f : bb[j]);
-                }
+              for (int k = 0; k < 16; ++k) {
+                float2 o = add2(make_float2(v[2 * k], v[2 * k + 1]), MODE == kFBackward ? make_float2(0.f, 0.f) : bb[k]);
                 if (second) {
-#pragma unroll
-                  for (int j = 0; j < 4; ++j) {
-                    const __nv_bfloat162 rb = *reinterpret_cast<const __nv_bfloat162*>(&res[4 * k + j]);
-                    o[2 * j] += __low2float(rb);
-                    o[2 * j + 1] += __high2float(rb);
-                  }
+                  const __nv_bfloat162 rb = *reinterpret_cast<const __nv_bfloat162*>(&res[k]);
+                  o = add2(o, make_float2(__low2float(rb), __high2float(rb)));
                 }
-                uint4 pk = make_uint4(0, 0, 0, 0);
+                kept[k] = pack_bf16x2(o.x, o.y);
                 if (MODE == kFBackward) {
-                  if (valid) {
-                    pk = make_uint4(mask_positive(pack_bf16x2(o[0], o[1]), mk[k].x),
-                                    mask_positive(pack_bf16x2(o[2], o[3]), mk[k].y),
-                                    mask_positive(pack_bf16x2(o[4], o[5]), mk[k].z),
-                                    mask_positive(pack_bf16x2(o[6], o[7]), mk[k].w));
-                  }
-                } else if (valid) {
-                  pk = make_uint4(pack_bf16x2(fmaxf(o[0], 0.f), fmaxf(o[1], 0.f)),
-                                  pack_bf16x2(fmaxf(o[2], 0.f), fmaxf(o[3], 0.f)),
-                                  pack_bf16x2(fmaxf(o[4], 0.f), fmaxf(o[5], 0.f)),
-                                  pack_bf16x2(fmaxf(o[6], 0.f), fmaxf(o[7], 0.f)));
+                  const uint4 m4 = mk[k >> 2];
+                  kept[k] = mask_positive(kept[k], (k & 3) == 0 ? m4.x : (k & 3) == 1 ? m4.y : (k & 3) == 2 ? m4.z : m4.w);
+                } else {
+                  kept[k] = relu_bf16x2(kept[k]);
                 }
-                p[k * kStep] = pk;
+              }
+              if (!all_valid) {
+#pragma unroll
+                for (int k = 0; k < 16; ++k) {
+                  kept[k] = valid ? kept[k] : 0u;
+                }
+              }
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const uint4 pk = make_uint4(kept[4 * k], kept[4 * k + 1], kept[4 * k + 2], kept[4 * k + 3]);
+                p[k * kStep]   = pk;
                 if (MODE != kFInfer && store) {
                   op[(size_t)k * R] = pk;
                 }
-                kept[4 * k] = pk.x, kept[4 * k + 1] = pk.y, kept[4 * k + 2] = pk.z, kept[4 * k + 3] = pk.w;
-              }
-              if (keep) {
-                tmem_st16(tres, kept);
-                tmem_wait_st();
               }
               fence_async_shared();
+              if (keep) {
+                tmem_st16(tres, kept); // waited for before it is read
+              }
             } else if (cs < 2) {
-              const int    plane = cs;
-              const int    wr    = 2 * pr + plane; // window row
+              const int    wr    = 2 * pr + cs; // plane cs
               const bool   valid = valid_s[wr] != 0;
               const float* bl    = bias_s + l * kCh;
               float        v[16];
-              tmem_ld16(tad + (uint32_t)(kOutCh * plane), v);
+              tmem_ld16(tad + (uint32_t)(kOutCh * cs), v);
               const int g = base + wr;
               if (wr >= kFMargin && wr < kFMargin + nout && g < R) {
 #pragma unroll
@@ -836,18 +864,17 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
       break;
     }
   }
-  // After a failure: the producer waits (bounded) for the MMAs and weight loads it issued, so that
+  // After a failure: the issuers wait (bounded) for the MMAs and weight loads they issued, so that
   // nothing asynchronous is in flight when the tensor memory and shared memory go away.
-  if (producer && lane == 0 && *abort_sm != 0) {
+  if ((issuer0 || issuer1) && lane == 0 && *abort_sm != 0) {
     if (mma_issued > 0) {
-      for (int c = 0; c < kFTiles; ++c) {
-        (void)mbar_wait_bounded(bar_mma + 8u * c, (mma_issued - 1) & 1u);
-      }
+      (void)mbar_wait_bounded(bar_mma + (issuer0 ? 0u : 8u), (mma_issued - 1) & 1u);
     }
-    for (uint32_t k = mma_issued; k < w_issued; ++k) {
+    for (uint32_t k = mma_issued; issuer0 && k < w_issued; ++k) {
       (void)mbar_wait_bounded(bar_w + 8u * (k & 1), (k >> 1) & 1u);
     }
   }
+  tmem_wait_st();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
