@@ -490,7 +490,7 @@ __device__ __forceinline__ void fused_load_weights(const uint16_t* __restrict__ 
 // order, as one convolution per layer (conv1d_fwd_kernel) does, and the activations and gradients equal
 // those of such a chain bit for bit.
 template <int CIN, int COUT, int S, bool ZEROED>
-__device__ __forceinline__ void fused_issue_shift(uint64_t a0, uint64_t b0, uint32_t d)
+__device__ __forceinline__ void fused_issue_shift(uint32_t go, uint64_t a0, uint64_t b0, uint32_t d)
 {
   constexpr uint32_t idesc_pair = make_idesc(128, 2 * COUT, false, false);
   constexpr uint32_t idesc_one  = make_idesc(128, COUT, false, false);
@@ -505,11 +505,11 @@ __device__ __forceinline__ void fused_issue_shift(uint64_t a0, uint64_t b0, uint
     const uint64_t ad    = a0 + (uint64_t)(a_off >> 4);
     const uint64_t bd    = b0 + (uint64_t)(b_off >> 4);
     if (S == 3) {
-      mma_bf16(d + COUT, ad, bd, idesc_one, 1u);
+      mma_bf16_warp(go, d + COUT, ad, bd, idesc_one, 1u);
     } else if (S == -2) {
-      mma_bf16(d, ad, bd, idesc_one, 1u);
+      mma_bf16_warp(go, d, ad, bd, idesc_one, 1u);
     } else {
-      mma_bf16(d, ad, bd, idesc_pair, (!ZEROED && S == -1 && kc == 0) ? 0u : 1u);
+      mma_bf16_warp(go, d, ad, bd, idesc_pair, (!ZEROED && S == -1 && kc == 0) ? 0u : 1u);
     }
   }
 }
@@ -517,26 +517,26 @@ __device__ __forceinline__ void fused_issue_shift(uint64_t a0, uint64_t b0, uint
 // The MMAs of M tile c of one layer: part 0 the shifts that read no pair beyond the tile's end
 // (-1, -2, 0, 1), part 1 the two that read the next tile's first pair (2, 3), part 2 all six.
 template <int CIN, int COUT, bool ZEROED>
-__device__ __forceinline__ void fused_issue_tile(int c, int part, uint32_t src, uint32_t wb, uint32_t tmem, uint32_t zero)
+__device__ __forceinline__ void fused_issue_tile(uint32_t go, int c, int part, uint32_t src, uint32_t wb, uint32_t tmem, uint32_t zero)
 {
   const uint64_t a0 = make_desc(src + (uint32_t)(c * 128) * 16u, kFChunkB, 128);
   const uint64_t b0 = make_desc(wb, (uint32_t)kTaps * COUT * 16, 128);
   const uint32_t d  = tmem + (uint32_t)(c * 128);
   if (part != 1) {
     if (ZEROED) {
-      mma_bf16(d, make_desc(zero, kFZeroB / 2, 128), b0, make_idesc(128, 2 * COUT, false, false), 0u);
-      fused_issue_shift<CIN, COUT, -2, ZEROED>(a0, b0, d);
-      fused_issue_shift<CIN, COUT, -1, ZEROED>(a0, b0, d);
+      mma_bf16_warp(go, d, make_desc(zero, kFZeroB / 2, 128), b0, make_idesc(128, 2 * COUT, false, false), 0u);
+      fused_issue_shift<CIN, COUT, -2, ZEROED>(go, a0, b0, d);
+      fused_issue_shift<CIN, COUT, -1, ZEROED>(go, a0, b0, d);
     } else {
-      fused_issue_shift<CIN, COUT, -1, ZEROED>(a0, b0, d);
-      fused_issue_shift<CIN, COUT, -2, ZEROED>(a0, b0, d);
+      fused_issue_shift<CIN, COUT, -1, ZEROED>(go, a0, b0, d);
+      fused_issue_shift<CIN, COUT, -2, ZEROED>(go, a0, b0, d);
     }
-    fused_issue_shift<CIN, COUT, 0, ZEROED>(a0, b0, d);
-    fused_issue_shift<CIN, COUT, 1, ZEROED>(a0, b0, d);
+    fused_issue_shift<CIN, COUT, 0, ZEROED>(go, a0, b0, d);
+    fused_issue_shift<CIN, COUT, 1, ZEROED>(go, a0, b0, d);
   }
   if (part != 0) {
-    fused_issue_shift<CIN, COUT, 2, ZEROED>(a0, b0, d);
-    fused_issue_shift<CIN, COUT, 3, ZEROED>(a0, b0, d);
+    fused_issue_shift<CIN, COUT, 2, ZEROED>(go, a0, b0, d);
+    fused_issue_shift<CIN, COUT, 3, ZEROED>(go, a0, b0, d);
   }
 }
 
@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
   uint32_t*          tmem_sm  = reinterpret_cast<uint32_t*>(bars + kFBars);
   volatile uint32_t* abort_sm = tmem_sm + 1;
   const int          tid      = threadIdx.x;
-  const int          warp     = tid >> 5;
+  const int          warp     = __shfl_sync(0xffffffffu, tid >> 5, 0); // uniform
   const int          lane     = tid & 31;
   if ((int)blockIdx.x >= n_win) {
     return;
@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_sm;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_sm, 0);
   // Epilogue role: TMEM lane quarter q, accumulator columns 32 cs .. 32 cs + 31 of each tile (plane
   // cs >> 1, channel half cs & 1; in the last layer warps cs < 2 take plane cs, 16 columns).
   const int      q          = warp & 3;
@@ -662,22 +662,32 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
       break;
     }
     if (issuer0 || issuer1) {
-      if (lane == 0) {
-        const int c = issuer0 ? 0 : 1;
+      {
+        // The whole warp takes the same path (lane 0 polls, issues and commits).
+        const int      c    = issuer0 ? 0 : 1;
+        const uint32_t go   = lane == 0 ? 1u : 0u;
+        auto           wait = [&](uint32_t bar, uint32_t parity) {
+          return __all_sync(0xffffffffu, lane != 0 || fused_wait(bar, parity, abort_sm, err)) != 0;
+        };
+        auto commit = [&](uint32_t bar) {
+          if (lane == 0) {
+            mma_commit(bar);
+          }
+        };
         for (int l = 0; l < NL; ++l) {
           const uint32_t s   = step + (uint32_t)l;
           const uint32_t src = (l & 1) ? act_a : act_b;
           const uint32_t wb  = wbuf0 + (s & 1) * kFWB;
           auto issue = [&](int part) {
             if (l == 0) {
-              fused_issue_tile<kInCh, kCh, MODE != kFInfer>(c, part, src, wb, tmem, zero_s);
+              fused_issue_tile<kInCh, kCh, MODE != kFInfer>(go, c, part, src, wb, tmem, zero_s);
             } else if (MODE != kFBackward && l == kLayers - 1) {
-              fused_issue_tile<kCh, kOutCh, MODE != kFInfer>(c, part, src, wb, tmem, zero_s);
+              fused_issue_tile<kCh, kOutCh, MODE != kFInfer>(go, c, part, src, wb, tmem, zero_s);
             } else {
-              fused_issue_tile<kCh, kCh, MODE != kFInfer>(c, part, src, wb, tmem, zero_s);
+              fused_issue_tile<kCh, kCh, MODE != kFInfer>(go, c, part, src, wb, tmem, zero_s);
             }
           };
-          if (!fused_wait(bar_w + 8u * (s & 1), (s >> 1) & 1u, abort_sm, err)) {
+          if (!wait(bar_w + 8u * (s & 1), (s >> 1) & 1u)) {
             break;
           }
           // Layer 0 follows the window barrier. Later layers: tile 0's first part reads tile 0 of layer l - 1
@@ -685,7 +695,7 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
           // in every epilogue warp, so its barrier tells that both are done.
           if (issuer0) {
             if (l > 0) {
-              if (!fused_wait(bar_epi, (s - 1) & 1u, abort_sm, err)) {
+              if (!wait(bar_epi, (s - 1) & 1u)) {
                 break;
               }
               tc_fence_after();
@@ -693,11 +703,11 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
             issue(0);
           }
           if (l > 0) {
-            if (!fused_wait(bar_epi + 8u, (s - 1) & 1u, abort_sm, err)) {
+            if (!wait(bar_epi + 8u, (s - 1) & 1u)) {
               if (issuer0) {
                 // Tile 0's first part is in flight: its barrier takes the completion, so that the wait
                 // after a failure below covers it.
-                mma_commit(bar_mma);
+                commit(bar_mma);
                 mma_issued = s + 1;
               }
               break;
@@ -709,22 +719,41 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
           } else if (two) {
             issue(2);
           }
-          mma_commit(bar_mma + 8u * c);
+          commit(bar_mma + 8u * c);
           mma_issued = s + 1;
           // Every MMA of layer l - 1 is complete (its epilogues are; before layer 0, the window barrier): its
           // weight buffer takes the next layer (layer 0 of the next window after the last layer), in flight
           // while this layer's MMAs and epilogues run.
           if (issuer0 && (l + 1 < NL || win + (int)gridDim.x < n_win)) {
             const int nx = (l + 1) % NL;
-            fused_load_weights(wp, MODE == kFBackward ? kLayers - 1 - nx : nx, wbuf0 + ((s + 1) & 1) * kFWB, bar_w + 8u * ((s + 1) & 1));
+            if (lane == 0) {
+              fused_load_weights(wp, MODE == kFBackward ? kLayers - 1 - nx : nx, wbuf0 + ((s + 1) & 1) * kFWB, bar_w + 8u * ((s + 1) & 1));
+            }
             ++w_issued;
           }
         }
       }
       __syncwarp();
     } else {
+      const int  plane     = cs >> 1, hh = cs & 1; // of the hidden layers
+      const bool valid0    = valid_s[2 * (q * 32 + lane) + plane] != 0;
+      const bool valid1    = valid_s[2 * (128 + q * 32 + lane) + plane] != 0;
+      const bool all_valid = __all_sync(0xffffffffu, valid0 && valid1) != 0;
       for (int l = 0; l < NL; ++l) {
-        const uint32_t s = step + (uint32_t)l;
+        const uint32_t s      = step + (uint32_t)l;
+        const bool     hidden = MODE == kFBackward || l < kLayers - 1;
+        // The bias, for both tiles: before tile 0's wait the epilogue warps have time, before tile 1's not.
+        float2 bb[16];
+        if (MODE != kFBackward && hidden) {
+          const float4* bl = reinterpret_cast<const float4*>(bias_s + l * kCh + hh * 32);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const float4 b4 = bl[k];
+            bb[2 * k]       = make_float2(b4.x, b4.y);
+            bb[2 * k + 1]   = make_float2(b4.z, b4.w);
+          }
+        }
+#pragma unroll 1
         for (int c = 0; c < kFTiles; ++c) {
           // Backward: the forward activations of this step's outputs, loaded while its MMAs run.
           uint4 mk[4];
@@ -736,36 +765,20 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
               mk[k] = (g >= 0 && g < R) ? __ldg(mp + (size_t)k * R) : make_uint4(0, 0, 0, 0);
             }
           }
-          // What the step needs beside its accumulators is read before the wait: the row mask, the bias and,
-          // in the second layer of a block, the residual (packed bf16 in TMEM, stored by this thread).
-          const bool     hidden = MODE == kFBackward || l < kLayers - 1;
+          // The residual of a block's second layer (packed bf16 in TMEM, stored by this thread) is read before
+          // the wait.
           const int      pr     = c * 128 + q * 32 + lane; // window row pair
-          const int      plane  = cs >> 1, hh = cs & 1;
           const bool     second = l >= 2 && (l & 1) == 0;
           const uint32_t tres   = tmem + ((uint32_t)(q * 32) << 16) + kFColRes + (uint32_t)(c * 64 + cs * 16);
-          bool           valid = false, all_valid = false;
-          float2         bb[16];
+          const bool     valid  = c == 0 ? valid0 : valid1;
           uint32_t       res[16];
-          if (hidden && (two || c == 0)) {
-            valid     = valid_s[2 * pr + plane] != 0;
-            all_valid = __all_sync(0xffffffffu, valid);
-            if (MODE != kFBackward) {
-              const float4* bl = reinterpret_cast<const float4*>(bias_s + l * kCh + hh * 32);
+          if (hidden && second && (two || c == 0)) {
+            tmem_wait_st();
+            float rf[16];
+            tmem_ld16(tres, rf);
 #pragma unroll
-              for (int k = 0; k < 8; ++k) {
-                const float4 b4 = bl[k];
-                bb[2 * k]       = make_float2(b4.x, b4.y);
-                bb[2 * k + 1]   = make_float2(b4.z, b4.w);
-              }
-            }
-            if (second) {
-              tmem_wait_st();
-              float rf[16];
-              tmem_ld16(tres, rf);
-#pragma unroll
-              for (int k = 0; k < 16; ++k) {
-                res[k] = __float_as_uint(rf[k]);
-              }
+            for (int k = 0; k < 16; ++k) {
+              res[k] = __float_as_uint(rf[k]);
             }
           }
           // One lane polls the barrier and tells the others: probes from all 32 lanes take
@@ -828,7 +841,7 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
               }
             } else if (cs < 2) {
               const int    wr    = 2 * pr + cs; // plane cs
-              const bool   valid = valid_s[wr] != 0;
+              const bool   on    = valid_s[wr] != 0;
               const float* bl    = bias_s + l * kCh;
               float        v[16];
               tmem_ld16(tad + (uint32_t)(kOutCh * cs), v);
@@ -837,7 +850,7 @@ __global__ void __launch_bounds__(kFThreads, 1) le_fused_forward_kernel(const ui
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                   uint4 pk = make_uint4(0, 0, 0, 0);
-                  if (valid) {
+                  if (on) {
                     const float* b8 = bl + 8 * h;
                     const float* v8 = v + 8 * h;
                     pk = make_uint4(pack_bf16x2(v8[0] + b8[0], v8[1] + b8[1]), pack_bf16x2(v8[2] + b8[2], v8[3] + b8[3]),

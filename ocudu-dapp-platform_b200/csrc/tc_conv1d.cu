@@ -240,7 +240,7 @@ struct wg_args {
 // start-address fields (16-byte units, below 2^14, so no carry reaches the next field). Formed per MMA by
 // the one issuing thread they set the time of a tile (154 us for the 14 layers at 96,000 rows).
 template <int CIN, int COUT>
-__device__ __forceinline__ void wgrad_issue_tile(uint32_t ab, uint32_t d, uint32_t acc)
+__device__ __forceinline__ void wgrad_issue_tile(uint32_t go, uint32_t ab, uint32_t d, uint32_t acc)
 {
   constexpr int      kCopies = 16 / (CIN / 8);
   constexpr int      kMTiles = (kTapCount + kCopies - 1) / kCopies;
@@ -251,7 +251,7 @@ __device__ __forceinline__ void wgrad_issue_tile(uint32_t ab, uint32_t d, uint32
   for (int ks = 0; ks < kWgTile / 16; ++ks) {
 #pragma unroll
     for (int j = 0; j < kMTiles; ++j) {
-      mma_bf16(d + (uint32_t)(j * COUT), a0 + (uint64_t)(j * kCopies + ks * 16), b0 + (uint64_t)(ks * 16), idesc,
+      mma_bf16_warp(go, d + (uint32_t)(j * COUT), a0 + (uint64_t)(j * kCopies + ks * 16), b0 + (uint64_t)(ks * 16), idesc,
                ks > 0 ? 1u : acc);
     }
   }
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv1d_wgrad_kernel(const __gri
   const uint32_t     bar_read = smem_u32(&bars[2 * kWgStages + 2]); // + 8 set: they have been read
   const uint32_t     base     = smem_u32(smem);
   const int          tid      = threadIdx.x;
-  const int          warp     = tid >> 5;
+  const int          warp     = __shfl_sync(0xffffffffu, tid >> 5, 0); // uniform
   const int          lane     = tid & 31;
   if (warp == 0) {
     tmem_alloc(smem_u32(tmem_sm), kWgCols);
@@ -290,16 +290,18 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv1d_wgrad_kernel(const __gri
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem   = *tmem_sm;
+  const uint32_t tmem   = __shfl_sync(0xffffffffu, *tmem_sm, 0);
   const int      ntiles = (R + kWgTile - 1) / kWgTile;
   const long     total  = (long)args.n * ntiles;
   const long     t_end  = total * (blockIdx.x + 1) / gridDim.x;
   auto wait = [&](uint32_t bar, uint32_t parity) {
-    if (*abort_sm != 0) {
-      return false;
-    }
-    if (mbar_wait_bounded(bar, parity)) {
-      return true;
+    for (uint32_t i = 0; i < kWaitLimit; ++i) {
+      if (mbar_try_wait(bar, parity)) {
+        return true;
+      }
+      if (*abort_sm != 0) {
+        return false;
+      }
     }
     *abort_sm = 1;
     atomicExch(err, 1);
@@ -318,32 +320,36 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv1d_wgrad_kernel(const __gri
     const int              bch    = L.cout / 8;
     const int              ngrp   = (nt + kWgGroup - 1) / kWgGroup;
     if (warp == 0) {
-      if (lane == 0) {
-        for (int i = 0; i < nt; ++i) {
-          const uint32_t k = k0 + (uint32_t)i, st = k % kWgStages;
-          const uint32_t grp = g0 + (uint32_t)(i / kWgGroup), set = grp & 1u;
-          if (i % kWgGroup == 0 && grp >= 2 && !wait(bar_read + 8u * set, (grp / 2 - 1u) & 1u)) {
-            break;
-          }
-          if (!wait(bar_full + 8u * st, (k / kWgStages) & 1u)) {
-            break;
-          }
-          tc_fence_after();
-          const uint32_t ab = base + st * kWgStageB, acc = i % kWgGroup > 0 ? 1u : 0u, d = tmem + 256u * set;
-          if (L.cin == 16) {
-            wgrad_issue_tile<16, 64>(ab, d, acc);
-          } else if (L.cout == 16) {
-            wgrad_issue_tile<64, 16>(ab, d, acc);
-          } else {
-            wgrad_issue_tile<64, 64>(ab, d, acc);
-          }
+      // The whole warp takes the same path (lane 0 polls, issues and commits).
+      const uint32_t go = lane == 0 ? 1u : 0u;
+      for (int i = 0; i < nt; ++i) {
+        const uint32_t k = k0 + (uint32_t)i, st = k % kWgStages;
+        const uint32_t grp = g0 + (uint32_t)(i / kWgGroup), set = grp & 1u;
+        bool           ok = true;
+        if (lane == 0) {
+          ok = (i % kWgGroup != 0 || grp < 2 || wait(bar_read + 8u * set, (grp / 2 - 1u) & 1u)) &&
+               wait(bar_full + 8u * st, (k / kWgStages) & 1u);
+        }
+        if (__all_sync(0xffffffffu, ok) == 0) {
+          break;
+        }
+        tc_fence_after();
+        const uint32_t ab = base + st * kWgStageB, acc = i % kWgGroup > 0 ? 1u : 0u, d = tmem + 256u * set;
+        if (L.cin == 16) {
+          wgrad_issue_tile<16, 64>(go, ab, d, acc);
+        } else if (L.cout == 16) {
+          wgrad_issue_tile<64, 16>(go, ab, d, acc);
+        } else {
+          wgrad_issue_tile<64, 64>(go, ab, d, acc);
+        }
+        if (lane == 0) {
           mma_commit(bar_free + 8u * st);
           if (i % kWgGroup == kWgGroup - 1 || i + 1 == nt) {
             mma_commit(bar_acc + 8u * set);
           }
         }
+        __syncwarp();
       }
-      __syncwarp();
     } else if (warp == 1) {
       // Lane g: column g of A (copy g / inch, chunk g % inch), lane 16 + c: column c of B.
       const int    ak  = lane / inch;
