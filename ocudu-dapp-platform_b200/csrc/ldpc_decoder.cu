@@ -26,6 +26,7 @@
 
 #include <algorithm>
 #include <cstdio>
+#include <cstring>
 #include <mutex>
 
 namespace pg {
@@ -692,6 +693,15 @@ constexpr uint32_t kPairMinSmem  = kPairTabBytes + (pg::kMaxNodes + 1) * (pg::kM
 constexpr int      kOddMaxZ      = 16;   // odd lifting sizes are at most 15
 
 constexpr int kPairThreads = 384;
+
+// Descriptors of a batch passed in a launch's arguments.
+template <int N>
+struct desc_args {
+  pg_ldpc_cb cb[N];
+};
+constexpr int kDecodeArgs = 260;  // of the decoder: batches of one CTA per codeblock
+constexpr int kScoreArgs  = 1600; // of the ordering launch: 32,000 bytes of the 32,764 a launch takes
+static_assert(sizeof(desc_args<kScoreArgs>) <= 32000, "arguments of a launch");
 
 struct pair_shared {
   uint4    row[pg::kBg1Rows + 1]; // first padded edge, first message byte, edges per thread, threads to meet after it or 0
@@ -1429,7 +1439,8 @@ __global__ void __launch_bounds__(kPairThreads, kPairPerSm)
     ldpc_decode_pair_kernel(const pg_ldpc_cb* __restrict__ descs, const int8_t* __restrict__ llrs,
                             uint8_t* __restrict__ bits, int32_t* __restrict__ iterations, int8_t* __restrict__ c2v_all,
                             const uint32_t* __restrict__ crc_pow, const uint32_t* __restrict__ order, int n,
-                            int* __restrict__ counter, uint32_t smem_bytes, const __grid_constant__ pg::ldpc_tb_sink sink)
+                            int* __restrict__ counter, uint32_t smem_bytes, const __grid_constant__ pg::ldpc_tb_sink sink,
+                            const __grid_constant__ desc_args<kDecodeArgs> args)
 {
   extern __shared__ __align__(16) unsigned char smem_pair[];
   __shared__ pair_shared sh;
@@ -1437,7 +1448,7 @@ __global__ void __launch_bounds__(kPairThreads, kPairPerSm)
   uint32_t*     slab = reinterpret_cast<uint32_t*>(c2v_all + (size_t)blockIdx.x * pg::kPairSlab);
   for (int w = blockIdx.x; w < n;) {
     const int        cb = order != nullptr ? (int)order[w] : w;
-    const pg_ldpc_cb d  = descs[cb];
+    const pg_ldpc_cb d  = descs != nullptr ? descs[cb] : args.cb[cb];
     const int        Z  = d.lifting_size;
     if ((Z & 1) != 0 || Z < 2 || Z > pg::kMaxZ) {
       if (Z < kOddMaxZ) {
@@ -1500,13 +1511,26 @@ __device__ __forceinline__ void score_word(uint32_t w, int idx, uint32_t& sum, u
   }
 }
 
+//
+// The descriptors come from device memory (N = 1) or with the launch's arguments, and are then stored to
+// `store` for the decoder. The last CTA to finish sorts the keys (a counting sort) into order[0 .. n) and
+// leaves both counters (work counter, arrivals) at zero for the decoder and the next launch. Staging the
+// descriptors by a copy, a sort launch and a memset of the work counter put the decoder 20 us behind the call
+// instead of 10 (200 codeblocks).
+template <int N>
 __global__ void __launch_bounds__(kScoreThreads) ldpc_score_kernel(const pg_ldpc_cb* __restrict__ descs, int n,
-                                                                  const int8_t* __restrict__ llrs,
-                                                                  uint8_t* __restrict__ keys)
+                                                                  const int8_t* __restrict__ llrs, uint8_t* keys,
+                                                                  uint32_t* __restrict__ order, int* counters,
+                                                                  pg_ldpc_cb* __restrict__ store,
+                                                                  const __grid_constant__ desc_args<N> args)
 {
   __shared__ uint32_t s_red[3][kScoreThreads / 32];
-  const pg_ldpc_cb d    = descs[blockIdx.x];
+  __shared__ int      s_last;
+  const pg_ldpc_cb d    = N > 1 ? args.cb[blockIdx.x] : descs[blockIdx.x];
   const int8_t*    in   = llrs + d.llr_offset;
+  if (N > 1 && threadIdx.x == 0) {
+    store[blockIdx.x] = d;
+  }
   const int        len  = (int)d.nof_llrs;
   const int        head = min(len, (int)((16u - (unsigned)(reinterpret_cast<uintptr_t>(in) & 15u)) & 15u));
   const int        nvec = (len - head) / 16;
@@ -1558,21 +1582,25 @@ __global__ void __launch_bounds__(kScoreThreads) ldpc_score_kernel(const pg_ldpc
       key               = 255u - (uint32_t)min(255.f, 16.f * log2f(1.f + cost));
     }
     keys[blockIdx.x] = (uint8_t)key;
+    __threadfence();
+    s_last = atomicAdd(&counters[1], 1) == n - 1;
   }
-  (void)n;
-}
-
-// Counting sort of the keys in one CTA: order[0..n) = codeblocks by ascending key.
-__global__ void __launch_bounds__(1024) ldpc_sort_kernel(const uint8_t* __restrict__ keys, int n,
-                                                         uint32_t* __restrict__ order)
-{
+  __syncthreads();
+  if (!s_last) {
+    return;
+  }
+  __threadfence();
+  if (threadIdx.x == 0) {
+    counters[0] = 0;
+    counters[1] = 0;
+  }
   __shared__ uint32_t bin[256];
   for (int i = threadIdx.x; i < 256; i += blockDim.x) {
     bin[i] = 0;
   }
   __syncthreads();
   for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    atomicAdd(&bin[keys[k]], 1u);
+    atomicAdd(&bin[__ldcg(keys + k)], 1u);
   }
   __syncthreads();
   if (threadIdx.x < 32) {
@@ -1598,7 +1626,7 @@ __global__ void __launch_bounds__(1024) ldpc_sort_kernel(const uint8_t* __restri
   }
   __syncthreads();
   for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    order[atomicAdd(&bin[keys[k]], 1u)] = (uint32_t)k;
+    order[atomicAdd(&bin[__ldcg(keys + k)], 1u)] = (uint32_t)k;
   }
 }
 
@@ -1737,9 +1765,9 @@ int ldpc_upload_tables(pg_context* ctx)
 }
 
 int ldpc_launch(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* bits,
-                int32_t* iterations, cudaStream_t stream)
+                int32_t* iterations, cudaStream_t stream, const pg_ldpc_cb* descs_host)
 {
-  return ldpc_launch_scratch(ctx, descs_dev, n, llrs, bits, iterations, ctx->dev.c2v, stream);
+  return ldpc_launch_scratch(ctx, descs_dev, n, llrs, bits, iterations, ctx->dev.c2v, stream, descs_host);
 }
 
 // CTAs of the decoder the context's batch decodes launch for n codeblocks: one per SM up to one and three
@@ -1759,34 +1787,63 @@ int ldpc_max_ctas(const pg_context* ctx, int per_sm, int kernel)
                                            : std::min(per_sm, kPairPerSm) * ctx->sm_count;
 }
 
-int ldpc_launch_scratch(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* bits,
-                        int32_t* iterations, int8_t* c2v, cudaStream_t stream)
+// Whether the batch decodes run n codeblocks in longest-first order. With a CTA for every codeblock all start
+// at once, and their order decides nothing.
+static bool batch_ordered(const pg_context* ctx, int n)
 {
-  const int       ctas  = batch_ctas(ctx, n);
+  return ctx->ldpc_order_mode == PG_LDPC_ORDER_LONGEST_FIRST && n > batch_ctas(ctx, n) && n <= ctx->max_codeblocks;
+}
+
+bool ldpc_descs_by_value(const pg_context* ctx, int n)
+{
+  return batch_ordered(ctx, n) ? n <= kScoreArgs : n <= kDecodeArgs && ctx->ldpc_kernel != PG_LDPC_KERNEL_ONE_LANE;
+}
+
+int ldpc_launch_scratch(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* bits,
+                        int32_t* iterations, int8_t* c2v, cudaStream_t stream, const pg_ldpc_cb* descs_host)
+{
   const uint32_t* order = nullptr;
-  // With a CTA for every codeblock all start at once, and their order decides nothing.
-  if (ctx->ldpc_order_mode == PG_LDPC_ORDER_LONGEST_FIRST && n > ctas && n <= ctx->max_codeblocks) {
-    if (int rc = ldpc_order_launch(ctx, descs_dev, n, llrs, ctx->dev.ldpc_keys, ctx->dev.ldpc_order, stream)) {
+  if (batch_ordered(ctx, n)) {
+    if (int rc = ldpc_order_launch(ctx, descs_dev, n, llrs, ctx->dev.ldpc_keys, ctx->dev.ldpc_order,
+                                   ctx->dev.ldpc_counter, stream, descs_host)) {
       return rc;
     }
-    order = ctx->dev.ldpc_order;
+    order      = ctx->dev.ldpc_order;
+    descs_host = nullptr; // the ordering launch has stored them
   }
   return ldpc_launch_persistent(ctx, descs_dev, n, llrs, bits, iterations, c2v, order, ctx->dev.ldpc_counter, stream,
-                                ctas, ctx->ldpc_kernel);
+                                batch_ctas(ctx, n), ctx->ldpc_kernel, nullptr, order != nullptr, descs_host);
+}
+
+template <int N>
+static void score_launch(pg_context* ctx, pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* keys, uint32_t* order,
+                         int* counters, cudaStream_t stream, const pg_ldpc_cb* descs_host)
+{
+  desc_args<N> args;
+  if (descs_host != nullptr) {
+    std::memcpy(args.cb, descs_host, (size_t)n * sizeof(pg_ldpc_cb));
+  }
+  ldpc_score_kernel<N><<<n, kScoreThreads, 0, stream>>>(N > 1 ? nullptr : descs_dev, n, llrs, keys, order, counters,
+                                                       N > 1 ? descs_dev : nullptr, args);
 }
 
 int ldpc_order_launch(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* keys,
-                      uint32_t* order, cudaStream_t stream)
+                      uint32_t* order, int* counters, cudaStream_t stream, const pg_ldpc_cb* descs_host)
 {
   if (n <= 0) {
     return PG_OK;
   }
-  ldpc_score_kernel<<<n, kScoreThreads, 0, stream>>>(descs_dev, n, llrs, keys);
-  if (int rc = check_cuda(ctx, cudaGetLastError(), "ldpc_score_kernel launch")) {
-    return rc;
+  pg_ldpc_cb* dev = const_cast<pg_ldpc_cb*>(descs_dev); // written only when the descriptors come from the host
+  if (descs_host == nullptr) {
+    score_launch<1>(ctx, dev, n, llrs, keys, order, counters, stream, nullptr);
+  } else if (n <= kScoreArgs / 4) {
+    score_launch<kScoreArgs / 4>(ctx, dev, n, llrs, keys, order, counters, stream, descs_host);
+  } else if (n <= kScoreArgs / 2) {
+    score_launch<kScoreArgs / 2>(ctx, dev, n, llrs, keys, order, counters, stream, descs_host);
+  } else {
+    score_launch<kScoreArgs>(ctx, dev, n, llrs, keys, order, counters, stream, descs_host);
   }
-  ldpc_sort_kernel<<<1, 1024, 0, stream>>>(keys, n, order);
-  return check_cuda(ctx, cudaGetLastError(), "ldpc_sort_kernel launch");
+  return check_cuda(ctx, cudaGetLastError(), "ldpc_score_kernel launch");
 }
 
 unsigned int timing_record_flags(pg_context* ctx, cudaStream_t s)
@@ -1814,7 +1871,8 @@ int ldpc_resident_ctas(pg_context* ctx)
 
 int ldpc_launch_persistent(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* bits,
                            int32_t* iterations, int8_t* c2v, const uint32_t* order, int* counter,
-                           cudaStream_t stream, int max_ctas, int kernel, const ldpc_tb_sink* sink, bool counter_zero)
+                           cudaStream_t stream, int max_ctas, int kernel, const ldpc_tb_sink* sink, bool counter_zero,
+                           const pg_ldpc_cb* descs_host)
 {
   if (n == 0) {
     return PG_OK;
@@ -1832,9 +1890,13 @@ int ldpc_launch_persistent(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, 
   int rc = PG_OK;
   if (kernel != PG_LDPC_KERNEL_ONE_LANE) {
     const int smem = pair_smem((grid + ctx->sm_count - 1) / ctx->sm_count);
-    ldpc_decode_pair_kernel<<<grid, kPairThreads, smem, stream>>>(descs_dev, llrs, bits, iterations, c2v,
-                                                                  ctx->dev.crc_pow, order, n, counter, (uint32_t)smem,
-                                                                  sink != nullptr ? *sink : ldpc_tb_sink{});
+    desc_args<kDecodeArgs> args;
+    if (descs_host != nullptr) {
+      std::memcpy(args.cb, descs_host, (size_t)n * sizeof(pg_ldpc_cb));
+    }
+    ldpc_decode_pair_kernel<<<grid, kPairThreads, smem, stream>>>(
+        descs_host != nullptr ? nullptr : descs_dev, llrs, bits, iterations, c2v, ctx->dev.crc_pow, order, n, counter,
+        (uint32_t)smem, sink != nullptr ? *sink : ldpc_tb_sink{}, args);
     rc = check_cuda(ctx, cudaGetLastError(), "ldpc_decode_pair_kernel launch");
   } else {
     ldpc_decode_kernel<<<grid, kThreads, 0, stream>>>(descs_dev, llrs, bits, iterations, c2v, ctx->dev.crc_pow, order,

@@ -123,6 +123,17 @@ static int stage_descs(pg_context* ctx, const pg_ldpc_cb* cbs, int n, cudaStream
   return PG_OK;
 }
 
+// Whether s is being captured (or cannot tell).
+static bool capturing(cudaStream_t s)
+{
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return true;
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
+
 // Marks the staged descriptors busy until the work enqueued on s so far (the kernel reading
 // them included) has completed.
 static int release_descs_after(pg_context* ctx, cudaStream_t s)
@@ -297,6 +308,9 @@ int pg_create(const pg_config* cfg, pg_context** out)
     rc = check_cuda(ctx, cudaMalloc(&ctx->dev.ldpc_counter, 2 * sizeof(int)), "cudaMalloc(ldpc counter)");
   }
   if (rc == PG_OK) {
+    rc = check_cuda(ctx, cudaMemset(ctx->dev.ldpc_counter, 0, 2 * sizeof(int)), "cudaMemset(ldpc counter)");
+  }
+  if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaMalloc(&ctx->dev.ldpc_keys, (size_t)cfg->max_codeblocks), "cudaMalloc(ldpc keys)");
   }
   if (rc == PG_OK) {
@@ -433,11 +447,21 @@ int pg_ldpc_decode_batch_device(pg_context* ctx, const pg_ldpc_cb* cbs, int nof_
   if (llrs == nullptr || bits == nullptr || iterations == nullptr) {
     return set_error(ctx, PG_ERR_INVALID, "null device buffer");
   }
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (int rc = stage_descs(ctx, cbs, nof_cbs, s)) {
-    return rc;
+  // The descriptors travel with the launches where they fit. The context's decoder scratch is shared, so a call
+  // on another stream follows the one before it on the device. A captured call stages them as before: its graph
+  // must not wait for work outside it.
+  cudaStream_t s        = static_cast<cudaStream_t>(stream);
+  const bool   by_value = !capturing(s) && ldpc_descs_by_value(ctx, nof_cbs);
+  if (!by_value) {
+    if (int rc = stage_descs(ctx, cbs, nof_cbs, s)) {
+      return rc;
+    }
+  } else if (ctx->desc_pending) {
+    if (int rc = check_cuda(ctx, cudaStreamWaitEvent(s, ctx->ev_desc, 0), "cudaStreamWaitEvent(descriptors)")) {
+      return rc;
+    }
   }
-  if (int rc = ldpc_launch(ctx, ctx->dev.descs, nof_cbs, llrs, bits, iterations, s)) {
+  if (int rc = ldpc_launch(ctx, ctx->dev.descs, nof_cbs, llrs, bits, iterations, s, by_value ? cbs : nullptr)) {
     return rc;
   }
   return release_descs_after(ctx, s);

@@ -67,7 +67,7 @@ struct device_buffers {
   int8_t*      llrs        = nullptr; // staging for _host calls
   uint8_t*     bits        = nullptr;
   int32_t*     iterations  = nullptr;
-  int*         ldpc_counter = nullptr; // work counters of the persistent decoders (two ints)
+  int*         ldpc_counter = nullptr; // work counter of the persistent decoders, arrivals of ldpc_score_kernel
   uint8_t*     ldpc_keys    = nullptr; // max_codeblocks work-order keys of the batch decodes
   uint32_t*    ldpc_order   = nullptr; // max_codeblocks work-order entries
   size_t       llr_cap     = 0;
@@ -159,6 +159,10 @@ int ensure_scratch(pg_context* ctx, void** buf, size_t* cap, size_t bytes, const
 int validate_rm_descs(pg_context* ctx, const pg_rm_cb* cbs, int n, size_t in_total, size_t out_total);
 int rate_dematch_launch(pg_context* ctx, const pg_rm_cb* descs_dev, int n, const int8_t* in, int8_t* out,
                         cudaStream_t stream);
+// Same with host descriptors that travel with the launch, n <= kRmArgs.
+constexpr int kRmArgs = 1340;
+int rate_dematch_launch_args(pg_context* ctx, const pg_rm_cb* descs_host, int n, const int8_t* in, int8_t* out,
+                             cudaStream_t stream);
 // Same with ctas_per_cb CTAs per codeblock (1..32), over the n codeblocks list[0 .. n - 1] of
 // descs_dev when list is not NULL (a plan's codeblocks that the demodulator does not store in place).
 int rate_dematch_launch(pg_context* ctx, const pg_rm_cb* descs_dev, int n, const int8_t* in, int8_t* out,
@@ -270,15 +274,18 @@ int equalize_launch(pg_context* ctx, int nof_re, int nof_ports, int nof_layers, 
                     const float* nvar_port_host, float tx, float2* out, float* out_var, cudaStream_t s);
 int demap_launch(pg_context* ctx, int qm, int n, const float2* sym, const float* nvar, int8_t* llr, cudaStream_t s);
 
-// Enqueues the batched decoder; descs_dev holds n descriptors in device memory.
+// Enqueues the batched decoder; descs_dev holds n descriptors in device memory. With descs_host (where
+// ldpc_descs_by_value holds) they travel with the launches instead, and descs_dev is written when needed.
 int ldpc_launch(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* bits,
-                int32_t* iterations, cudaStream_t stream);
+                int32_t* iterations, cudaStream_t stream, const pg_ldpc_cb* descs_host = nullptr);
+bool ldpc_descs_by_value(const pg_context* ctx, int n);
 // Same with a caller-provided check-to-variable scratch of kLdpcSlabsPerSm * sm_count * kPairSlab bytes.
 int ldpc_launch_scratch(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* bits,
-                        int32_t* iterations, int8_t* c2v, cudaStream_t stream);
-// Hardest-first work order (ldpc_score_kernel + ldpc_sort_kernel): keys n bytes, order n entries.
+                        int32_t* iterations, int8_t* c2v, cudaStream_t stream, const pg_ldpc_cb* descs_host = nullptr);
+// Hardest-first work order (ldpc_score_kernel): keys n bytes, order n entries. counters: the decoder's work
+// counter, zeroed, and the launch's arrivals, zero before and after.
 int ldpc_order_launch(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* keys,
-                      uint32_t* order, cudaStream_t stream);
+                      uint32_t* order, int* counters, cudaStream_t stream, const pg_ldpc_cb* descs_host = nullptr);
 // Transport-block join of the lane-pair decoder: with tbs set, codeblock cb's payload goes to its place in
 // tb_out instead of the decoder's bit output, and the last codeblock of each TB writes results[tb]. Every
 // TB has one codeblock, or codeblocks of an even lifting size with payloads of whole bytes
@@ -308,7 +315,7 @@ int ldpc_max_ctas(const pg_context* ctx, int per_sm, int kernel);
 int ldpc_launch_persistent(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* bits,
                            int32_t* iterations, int8_t* c2v, const uint32_t* order, int* counter,
                            cudaStream_t stream, int max_ctas, int kernel, const ldpc_tb_sink* sink = nullptr,
-                           bool counter_zero = false);
+                           bool counter_zero = false, const pg_ldpc_cb* descs_host = nullptr);
 // CTAs of ldpc_decode_kernel resident on the whole device.
 int ldpc_resident_ctas(pg_context* ctx);
 

@@ -112,6 +112,9 @@ int pg_rate_dematch_batch_device(pg_context* ctx, const pg_rm_cb* cbs, int nof_c
   }
   cudaStream_t s   = static_cast<cudaStream_t>(stream);
   void*        dev = nullptr;
+  if (nof_cbs <= kRmArgs) {
+    return rate_dematch_launch_args(ctx, cbs, nof_cbs, in, out, s);
+  }
   if (int rc = stage_slot(ctx, SLOT_RM, cbs, (size_t)nof_cbs * sizeof(pg_rm_cb), s, &dev)) {
     return rc;
   }

@@ -103,7 +103,7 @@ struct pg_pusch_plan {
   uint32_t*       d_tb_chunks    = nullptr; // TB-assembly work items (TB | chunk << 16)
   int             tb_nchunks     = 0;
   uint8_t*        d_keys   = nullptr; // work-order keys of the codeblocks // LDPC work order: largest codeblocks first
-  int*            d_counter = nullptr; // work counter of the persistent decoder
+  int*            d_counter = nullptr; // work counter of the persistent decoder, arrivals of its ordering
   uint32_t*       d_grid   = nullptr; // grids of execute_host
   uint8_t*        d_tb_out = nullptr; // TBs of execute_host
   pg_sch_result*  d_res    = nullptr; // results of execute_host
@@ -337,7 +337,7 @@ int enqueue(pg_pusch_plan* p, const uint32_t* grids, uint8_t* tb_out, pg_sch_res
   const uint32_t* order = p->d_order_static;
   if (rc == PG_OK && ldpc_ordered(p)) {
     // Longest first: the decoders take the codeblocks by the predicted decoding time of their input.
-    rc    = ldpc_order_launch(ctx, p->d_ldpc, p->nof_cbs, p->d_rm_out, p->d_keys, p->d_order, s);
+    rc    = ldpc_order_launch(ctx, p->d_ldpc, p->nof_cbs, p->d_rm_out, p->d_keys, p->d_order, p->d_counter, s);
     order = p->d_order;
   }
   ldpc_tb_sink sink;
@@ -662,7 +662,7 @@ int pg_pusch_plan_create_uci(pg_context* ctx, const pg_pusch_ue* ues, const pg_p
   const size_t o_it     = o_crc + al((size_t)nof_ues * 4);
   const size_t o_keys   = o_it + al((size_t)p->nof_cbs * 4);
   const size_t o_cnt    = o_keys + al((size_t)p->nof_cbs);
-  const size_t o_c2v    = o_cnt + al(sizeof(int));
+  const size_t o_c2v    = o_cnt + al(2 * sizeof(int));
   const size_t o_grid   = o_c2v + al((size_t)ldpc_slabs * kPairSlab);
   const size_t o_tbout  = o_grid + al(grid_words * 4);
   const size_t o_res    = o_tbout + al(p->tb_bytes);
@@ -779,6 +779,9 @@ int pg_pusch_plan_create_uci(pg_context* ctx, const pg_pusch_ue* ues, const pg_p
   }
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaMemsetAsync(b + o_earr, 0, (size_t)nof_ues * 16, s), "cudaMemsetAsync(arrivals)");
+  }
+  if (rc == PG_OK) {
+    rc = check_cuda(ctx, cudaMemsetAsync(p->d_counter, 0, 2 * sizeof(int), s), "cudaMemsetAsync(work counter)");
   }
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaMemsetAsync(p->d_join, 0, (size_t)nof_ues * 8, s), "cudaMemsetAsync(TB join)");

@@ -13,6 +13,7 @@
 #include "pg_internal.h"
 
 #include <algorithm>
+#include <cstring>
 
 namespace {
 
@@ -198,12 +199,8 @@ struct rm_buffer {
 // positions: 7.0 us on new data, 8.7 us combining (12 us each as tiles of the input transposed through shared
 // memory with a second pass over the positions no LLR reaches; 10 us with every word taken the general way;
 // 12 us with the words ordered so that one CTA reads each input sector).
-__global__ void __launch_bounds__(kRmThreads) rate_dematch_kernel(const pg_rm_cb* __restrict__ cbs,
-                                                                  const int8_t* __restrict__ in_all,
-                                                                  int8_t* __restrict__ out_all,
-                                                                  const uint32_t* __restrict__ list)
+__device__ __forceinline__ void rate_dematch(const pg_rm_cb& d, const int8_t* __restrict__ in_all, int8_t* __restrict__ out_all)
 {
-  const pg_rm_cb d  = cbs[list != nullptr ? list[blockIdx.x] : blockIdx.x];
   const int      bg = d.base_graph;
   const int      Z  = d.lifting_size;
   const int      Kb = bg == 1 ? 22 : 10;
@@ -235,6 +232,32 @@ __global__ void __launch_bounds__(kRmThreads) rate_dematch_kernel(const pg_rm_cb
       c.word<false>(g);
     }
   }
+}
+
+__global__ void __launch_bounds__(kRmThreads) rate_dematch_kernel(const pg_rm_cb* __restrict__ cbs,
+                                                                  const int8_t* __restrict__ in_all,
+                                                                  int8_t* __restrict__ out_all,
+                                                                  const uint32_t* __restrict__ list)
+{
+  const pg_rm_cb d = cbs[list != nullptr ? list[blockIdx.x] : blockIdx.x];
+  rate_dematch(d, in_all, out_all);
+}
+
+// The descriptors in the launch's arguments: a copy staged in pinned memory started the kernel 6 us later, and
+// a second call waited on the host for the first one's kernel.
+template <int N>
+struct rm_args {
+  pg_rm_cb cb[N];
+};
+static_assert(sizeof(rm_args<pg::kRmArgs>) <= 32700, "arguments of a launch");
+
+template <int N>
+__global__ void __launch_bounds__(kRmThreads) rate_dematch_args_kernel(const __grid_constant__ rm_args<N> args,
+                                                                       const int8_t* __restrict__ in_all,
+                                                                       int8_t* __restrict__ out_all)
+{
+  const pg_rm_cb d = args.cb[blockIdx.x];
+  rate_dematch(d, in_all, out_all);
 }
 
 } // namespace
@@ -282,12 +305,40 @@ int validate_rm_descs(pg_context* ctx, const pg_rm_cb* cbs, int n, size_t in_tot
   return PG_OK;
 }
 
+// CTAs per codeblock of a batch. A CTA's set-up is worth several words of its threads: five CTAs per SM shared
+// among the codeblocks, at least four each. 200 codeblocks: 7.0 us at 4 CTAs each, 7.5 at 8, 8.3 at 13, 10.9 at
+// 25 (one word a thread).
+static int batch_ctas_per_cb(const pg_context* ctx, int n)
+{
+  return std::max(4, std::min(16, 5 * ctx->sm_count / std::max(1, n)));
+}
+
 int rate_dematch_launch(pg_context* ctx, const pg_rm_cb* descs_dev, int n, const int8_t* in, int8_t* out,
                         cudaStream_t stream)
 {
-  // A CTA's set-up is worth several words of its threads: five CTAs per SM shared among the codeblocks, at
-  // least four each. 200 codeblocks: 7.0 us at 4 CTAs each, 7.5 at 8, 8.3 at 13, 10.9 at 25 (one word a thread).
-  return rate_dematch_launch(ctx, descs_dev, n, in, out, stream, std::max(4, std::min(16, 5 * ctx->sm_count / std::max(1, n))));
+  return rate_dematch_launch(ctx, descs_dev, n, in, out, stream, batch_ctas_per_cb(ctx, n));
+}
+
+template <int N>
+static void launch_args(pg_context* ctx, const pg_rm_cb* descs, int n, const int8_t* in, int8_t* out, cudaStream_t stream)
+{
+  rm_args<N> args;
+  std::memcpy(args.cb, descs, (size_t)n * sizeof(pg_rm_cb));
+  rate_dematch_args_kernel<N><<<dim3(n, batch_ctas_per_cb(ctx, n)), kRmThreads, 0, stream>>>(args, in, out);
+}
+
+int rate_dematch_launch_args(pg_context* ctx, const pg_rm_cb* descs, int n, const int8_t* in, int8_t* out,
+                             cudaStream_t stream)
+{
+  // A launch copies its arguments whole: three sizes.
+  if (n <= kRmArgs / 4) {
+    launch_args<kRmArgs / 4>(ctx, descs, n, in, out, stream);
+  } else if (n <= kRmArgs / 2) {
+    launch_args<kRmArgs / 2>(ctx, descs, n, in, out, stream);
+  } else {
+    launch_args<kRmArgs>(ctx, descs, n, in, out, stream);
+  }
+  return check_cuda(ctx, cudaGetLastError(), "rate_dematch_args_kernel launch");
 }
 
 int rate_dematch_launch(pg_context* ctx, const pg_rm_cb* descs_dev, int n, const int8_t* in, int8_t* out,
