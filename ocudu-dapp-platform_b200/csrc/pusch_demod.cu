@@ -68,39 +68,43 @@ __device__ __forceinline__ float rcp_est(float x)
   return r;
 }
 
-__device__ __forceinline__ int8_t quantize(float v, float scale)
+// LLR v, descrambled by bit k of c, to an integer: rounding to nearest, the limits and NaN (0) are taken after
+// the conversion, which saturates, and the sign is flipped before it (rounding is symmetric).
+__device__ __forceinline__ int quantize(float v, float scale, uint32_t c, int k)
 {
-  v = __fmul_rn(v, scale);
-  v = v > 120.f ? 120.f : (v < -120.f ? -120.f : v);
-  if (!(v == v)) {
-    return 0;
-  }
-  return (int8_t)__float2int_rn(v);
+  const float f = __uint_as_float(__float_as_uint(__fmul_rn(v, scale)) ^ ((c << (31 - k)) & 0x80000000u));
+  return max(-120, min(120, __float2int_rn(f)));
 }
 
+struct demap_tables {
+  const float2* line;  // (slope, intercept) of [modulation][bit pair][interval]
+  const float*  width; // interval widths, then their reciprocals
+};
+
+// The QM LLRs of one symbol, descrambled by the bits of c. Symbol parts of magnitude up to 1e-9 give zeros (a
+// zero in place of the reciprocal).
 template <int QM>
-__device__ __forceinline__ void demap(float xr, float xi, float nvar, int8_t* llr, const float* s_slope,
-                                      const float* s_icpt, const float* s_width)
+__device__ __forceinline__ void demap(float xr, float xi, float nvar, uint32_t c, int* llr, const demap_tables& tb)
 {
   const float rcp = (nvar > 0.f) ? rcp_est(nvar) : 0.f;
   if (QM == 2) {
     const float g = 2.0f * 1.41421353816986083984375f;
-    llr[0]        = quantize(__fmul_rn(__fmul_rn(g, xr), rcp), 5.0f);
-    llr[1]        = quantize(__fmul_rn(__fmul_rn(g, xi), rcp), 5.0f);
+    llr[0]        = quantize(__fmul_rn(__fmul_rn(g, xr), rcp), 5.0f, c, 0);
+    llr[1]        = quantize(__fmul_rn(__fmul_rn(g, xi), rcp), 5.0f, c, 1);
     return;
   }
+  const float x[2]  = {xr, xi};
+  const float rz[2] = {fabsf(xr) <= 1e-9f ? 0.f : rcp, fabsf(xi) <= 1e-9f ? 0.f : rcp};
   if (QM == 4) {
-    const float s10  = 0.3162277638912200927734375f;
-    const float x[2] = {xr, xi};
+    const float s10 = 0.3162277638912200927734375f;
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const float first  = __fmul_rn(4.0f * s10, x[c]);
-      const float second = __fsub_rn(__fmul_rn(2.0f, first), copysignf(0.8f, x[c]));
-      const float v01    = fabsf(x[c]) > 2.0f * s10 ? second : first;
+    for (int i = 0; i < 2; ++i) {
+      const float first  = __fmul_rn(4.0f * s10, x[i]);
+      const float second = __fsub_rn(__fmul_rn(2.0f, first), copysignf(0.8f, x[i]));
+      const float v01    = fabsf(x[i]) > 2.0f * s10 ? second : first;
       const float v23    = __fsub_rn(0.8f, fabsf(first));
-      const bool  z      = fabsf(x[c]) <= 1e-9f;
-      llr[c]             = quantize(z ? 0.f : __fmul_rn(v01, rcp), 6.0f);
-      llr[2 + c]         = quantize(z ? 0.f : __fmul_rn(v23, rcp), 6.0f);
+      llr[i]             = quantize(__fmul_rn(v01, rz[i]), 6.0f, c, i);
+      llr[2 + i]         = quantize(__fmul_rn(v23, rz[i]), 6.0f, c, 2 + i);
     }
     return;
   }
@@ -109,19 +113,15 @@ __device__ __forceinline__ void demap(float xr, float xi, float nvar, int8_t* ll
   // Interval index floor(x / width) as x times the stored reciprocal width: where the two differ
   // (x / width within an ulp of an integer) the neighbouring interval's line meets this one at
   // the boundary (the interval functions are continuous), so the LLR is the same within rounding.
-  const float   iwidth = s_width[3 + t];
-  const float   x[2]   = {xr, xi};
+  const float iwidth = tb.width[3 + t];
 #pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    int idx      = (int)floorf(__fmul_rn(x[c], iwidth)) + nint / 2;
-    idx          = idx < 0 ? 0 : (idx > nint - 1 ? nint - 1 : idx);
-    const bool z = fabsf(x[c]) <= 1e-9f;
+  for (int i = 0; i < 2; ++i) {
+    int idx = (int)floorf(__fmul_rn(x[i], iwidth)) + nint / 2;
+    idx     = idx < 0 ? 0 : (idx > nint - 1 ? nint - 1 : idx);
 #pragma unroll
     for (int b = 0; b < QM / 2; ++b) {
-      const float v  = __fmul_rn(__fadd_rn(__fmul_rn(s_slope[(t * 4 + b) * 16 + idx], x[c]),
-                                           s_icpt[(t * 4 + b) * 16 + idx]),
-                                 rcp);
-      llr[2 * b + c] = quantize(z ? 0.f : v, 6.0f);
+      const float2 ln = tb.line[(t * 4 + b) * 16 + idx];
+      llr[2 * b + i]  = quantize(__fmul_rn(__fadd_rn(__fmul_rn(ln.x, x[i]), ln.y), rz[i]), 6.0f, c, 2 * b + i);
     }
   }
 }
@@ -157,12 +157,6 @@ __global__ void descramble_kernel(uint32_t c_init, const int8_t* __restrict__ in
     out[32 * w + b]    = (int8_t)(((c >> b) & 1u) ? -x : x);
   }
 }
-
-struct demap_tables {
-  const float* slope;
-  const float* icpt;
-  const float* width;
-};
 
 template <int L, int P, int QM>
 __device__ __forceinline__ void demod_re(const pg_pusch_ue& ue, const uint32_t* __restrict__ grid,
@@ -301,16 +295,16 @@ __device__ __forceinline__ void demod_re(const pg_pusch_ue& ue, const uint32_t* 
     }
   }
   // Demap, descramble, store: LLR index (re * L + l) * QM + b.
-  int8_t        llr[L * QM];
-#pragma unroll
-  for (int l = 0; l < L; ++l) {
-    demap<QM>(s[l].r, s[l].i, nv[l], llr + l * QM, tb.slope, tb.icpt, tb.width);
-  }
   const uint32_t bit0 = (uint32_t)re_idx * L * QM;
   const uint32_t wa   = __ldg(seq + (bit0 >> 5));
   const uint32_t wb   = __ldg(seq + (bit0 >> 5) + 1);
   const uint32_t sh   = bit0 & 31u;
   const uint32_t cbits = sh ? ((wa >> sh) | (wb << (32 - sh))) : wa;
+  int            llr[L * QM];
+#pragma unroll
+  for (int l = 0; l < L; ++l) {
+    demap<QM>(s[l].r, s[l].i, nv[l], cbits >> (l * QM), llr + l * QM, tb);
+  }
   if (dr != nullptr) {
     // Fused rate dematching: the RE's L*QM bits lie in one codeblock (E is a multiple of L*QM);
     // bit l*QM + b is de-interleaver row b, column i0 + l, placed in the circular buffer.
@@ -329,17 +323,19 @@ __device__ __forceinline__ void demod_re(const pg_pusch_ue& ue, const uint32_t* 
     const uint32_t kq  = E / QM;
     const uint32_t i0  = (bit0 - off) / QM;
     int8_t*        cbo = rm_out + dr->out0 + (size_t)r * dr->cb_len;
+    const uint32_t V = dr->V, inf = dr->inf, F = dr->F;
+    uint32_t       v = dr->v0 + i0; // valid position of (row 0, layer 0), less than 2 V
 #pragma unroll
     for (int b = 0; b < QM; ++b) {
-#pragma unroll
-      for (int l = 0; l < L; ++l) {
-        uint32_t v = dr->v0 + (uint32_t)b * kq + i0 + (uint32_t)l;
-        v          = v >= dr->V ? v - dr->V : v;
-        const uint32_t pos = v < dr->inf ? v : v + dr->F;
-        const int      k   = l * QM + b;
-        const int      x   = llr[k];
-        cbo[pos]           = (int8_t)(((cbits >> k) & 1u) ? -x : x);
+      v                   = v >= V ? v - V : v;
+      const uint32_t pos  = v < inf ? v : v + F;
+      cbo[pos]            = (int8_t)llr[b];
+      if (L == 2) {
+        // The next position, but at the fillers and at the buffer's end.
+        const uint32_t v1 = v + 1u >= V ? 0u : v + 1u;
+        cbo[v1 < inf ? v1 : v1 + F] = (int8_t)llr[QM + b];
       }
+      v += kq;
     }
     return;
   }
@@ -355,8 +351,7 @@ __device__ __forceinline__ void demod_re(const pg_pusch_ue& ue, const uint32_t* 
   }
 #pragma unroll
   for (int b = 0; b < NB; ++b) {
-    const int v = llr[b];
-    wd[b / 4] |= (uint32_t)(uint8_t)(int8_t)(((cbits >> b) & 1u) ? -v : v) << (8 * (b % 4));
+    wd[b / 4] |= (uint32_t)(uint8_t)llr[b] << (8 * (b % 4));
   }
   const uintptr_t a = reinterpret_cast<uintptr_t>(out);
   if (NB == 16 && (a & 15u) == 0) {
@@ -439,8 +434,7 @@ __global__ void __launch_bounds__(256) pusch_demod_kernel(const pg_pusch_ue* __r
                                                           int tiles_per_cta, const pg::rm_direct* __restrict__ direct,
                                                           int8_t* __restrict__ rm_out)
 {
-  __shared__ float  s_slope[3 * 4 * 16];
-  __shared__ float  s_icpt[3 * 4 * 16];
+  __shared__ float2 s_line[3 * 4 * 16];
   __shared__ float  s_width[6]; // interval widths, then their reciprocals
   __shared__ float2 s_est[4 * 2 * 2 * kDemodTile];
   __shared__ float2 s_bas[4 * 2 * 2 * kDemodTile];
@@ -449,14 +443,13 @@ __global__ void __launch_bounds__(256) pusch_demod_kernel(const pg_pusch_ue* __r
   __shared__ pg_port_result s_pres[4];
   __shared__ pg::rm_direct  s_dr;
   for (int i = threadIdx.x; i < 3 * 4 * 16; i += blockDim.x) {
-    s_slope[i] = (&c_slope_d[0][0][0])[i];
-    s_icpt[i]  = (&c_intercept_d[0][0][0])[i];
+    s_line[i] = make_float2((&c_slope_d[0][0][0])[i], (&c_intercept_d[0][0][0])[i]);
   }
   if (threadIdx.x < 3) {
     s_width[threadIdx.x]     = c_width_d[threadIdx.x];
     s_width[3 + threadIdx.x] = 1.0f / c_width_d[threadIdx.x];
   }
-  const demap_tables tb = {s_slope, s_icpt, s_width};
+  const demap_tables tb = {s_line, s_width};
   for (int k = 0; k < tiles_per_cta; ++k) {
     const uint32_t t = blockIdx.x * (uint32_t)tiles_per_cta + (uint32_t)k;
     if (t >= ntiles) {
