@@ -1,6 +1,9 @@
 // Device helpers shared by the pusch_b200 kernels.
 #pragma once
 
+#include <cuda_runtime.h>
+
+#include <cstddef>
 #include <cstdint>
 
 namespace pg {
@@ -31,6 +34,36 @@ __device__ __forceinline__ uint32_t gold_word(const uint32_t* __restrict__ tab, 
     }
   }
   return sh ? ((lo >> sh) | (hi << (32 - sh))) : lo;
+}
+
+// Programmatic dependent launch. launch_dependents: the next kernel of the stream, if launched to allow it
+// (launch_overlapped), may start once every CTA of this grid has called it or exited. wait_prerequisites: until
+// the kernels before this one have completed and their memory is visible; without such a launch it returns at
+// once. Everything before it may touch only memory that no earlier kernel of the stream writes.
+__device__ __forceinline__ void launch_dependents()
+{
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_prerequisites()
+{
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Launches a kernel that calls wait_prerequisites and may start before the kernel ahead of it has completed.
+template <class... P, class... A>
+inline cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args)
+{
+  cudaLaunchAttribute attr = {};
+  attr.id                  = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim            = grid;
+  cfg.blockDim           = block;
+  cfg.dynamicSmemBytes   = smem;
+  cfg.stream             = s;
+  cfg.attrs              = &attr;
+  cfg.numAttrs           = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
 } // namespace pg

@@ -166,7 +166,7 @@ int rate_dematch_launch_args(pg_context* ctx, const pg_rm_cb* descs_host, int n,
 // Same with ctas_per_cb CTAs per codeblock (1..32), over the n codeblocks list[0 .. n - 1] of
 // descs_dev when list is not NULL (a plan's codeblocks that the demodulator does not store in place).
 int rate_dematch_launch(pg_context* ctx, const pg_rm_cb* descs_dev, int n, const int8_t* in, int8_t* out,
-                        cudaStream_t stream, int ctas_per_cb, const uint32_t* list = nullptr);
+                        cudaStream_t stream, int ctas_per_cb, const uint32_t* list = nullptr, bool overlap = false);
 // Before a slot plan's demodulator stores LLRs in place: the circular buffers of the codeblocks with
 // placed[c] = 1 get what rate dematching leaves at the positions no LLR reaches (+127 at the fillers, 0
 // elsewhere), and tb_out and *counter are zeroed (rm_prefill, kRmFillCtas CTAs per codeblock).
@@ -244,7 +244,8 @@ int demod_only_launch(pg_context* ctx, const pg_pusch_ue* ues_dev, int n, uint32
                       const uint32_t* tile_map_dev, const uint32_t* grids, const float* est,
                       const pg_port_result* port_results, const uint32_t* seq_offsets_dev, const uint32_t* seq_dev,
                       int8_t* llrs, cudaStream_t s, int block, int res_per_thread, const float* basis = nullptr,
-                      const uint8_t* basis_use = nullptr, const rm_direct* direct = nullptr, int8_t* rm_out = nullptr);
+                      const uint8_t* basis_use = nullptr, const rm_direct* direct = nullptr, int8_t* rm_out = nullptr,
+                      bool overlap = false); // overlap: the launch may start before the kernel ahead of it ends
 // Decodes transport blocks whose codeword LLRs are already in device memory (d_llrs, nof_llrs);
 // uses scratch_b; results and TB payloads land in host memory.
 int sch_decode_device_llrs(pg_context* ctx, const pg_sch_tb* tbs, int nof_tbs, const int8_t* d_llrs,
@@ -311,11 +312,13 @@ std::vector<ldpc_tb_cb> tb_join_in_decoder(const std::vector<pg_tb_desc>& tbs, c
 int ldpc_max_ctas(const pg_context* ctx, int per_sm, int kernel);
 // Persistent launch: min(n, max_ctas) CTAs (max_ctas from ldpc_max_ctas) take codeblocks order[0..n)
 // (identity when order is null) from *counter (device int, zeroed here on the stream unless counter_zero);
-// c2v holds one slab (kPairSlab bytes) per CTA.
+// overlap: the launch may start before the kernel ahead of it ends (that kernel writes neither the order nor
+// the descriptors); c2v holds one slab (kPairSlab bytes) per CTA.
 int ldpc_launch_persistent(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* bits,
                            int32_t* iterations, int8_t* c2v, const uint32_t* order, int* counter,
                            cudaStream_t stream, int max_ctas, int kernel, const ldpc_tb_sink* sink = nullptr,
-                           bool counter_zero = false, const pg_ldpc_cb* descs_host = nullptr);
+                           bool counter_zero = false, const pg_ldpc_cb* descs_host = nullptr,
+                           bool overlap = false);
 // CTAs of ldpc_decode_kernel resident on the whole device.
 int ldpc_resident_ctas(pg_context* ctx);
 

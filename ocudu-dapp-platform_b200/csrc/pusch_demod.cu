@@ -329,11 +329,14 @@ __device__ __forceinline__ void demod_re(const pg_pusch_ue& ue, const uint32_t* 
     for (int b = 0; b < QM; ++b) {
       v                   = v >= V ? v - V : v;
       const uint32_t pos  = v < inf ? v : v + F;
-      cbo[pos]            = (int8_t)llr[b];
-      if (L == 2) {
-        // The next position, but at the fillers and at the buffer's end.
-        const uint32_t v1 = v + 1u >= V ? 0u : v + 1u;
-        cbo[v1 < inf ? v1 : v1 + F] = (int8_t)llr[QM + b];
+      if (L == 1) {
+        cbo[pos] = (int8_t)llr[b];
+      } else if (v + 1u < V && v + 1u != inf && (reinterpret_cast<uintptr_t>(cbo + pos) & 1u) == 0) {
+        *reinterpret_cast<uint16_t*>(cbo + pos) = (uint16_t)__byte_perm((uint32_t)llr[b], (uint32_t)llr[L == 2 ? QM + b : b], 0x0040);
+      } else { // an odd address, the fillers or the buffer's end between the two layers
+        const uint32_t v1           = v + 1u >= V ? 0u : v + 1u;
+        cbo[pos]                    = (int8_t)llr[b];
+        cbo[v1 < inf ? v1 : v1 + F] = (int8_t)llr[L == 2 ? QM + b : b];
       }
       v += kq;
     }
@@ -450,6 +453,7 @@ __global__ void __launch_bounds__(256) pusch_demod_kernel(const pg_pusch_ue* __r
     s_width[3 + threadIdx.x] = 1.0f / c_width_d[threadIdx.x];
   }
   const demap_tables tb = {s_line, s_width};
+  pg::launch_dependents();
   for (int k = 0; k < tiles_per_cta; ++k) {
     const uint32_t t = blockIdx.x * (uint32_t)tiles_per_cta + (uint32_t)k;
     if (t >= ntiles) {
@@ -480,6 +484,9 @@ __global__ void __launch_bounds__(256) pusch_demod_kernel(const pg_pusch_ue* __r
       s_sym[r]         = s;
       s_w[r]           = nd == 2 ? (float)(s - d0) / (float)(d1 - d0) : 0.f;
     }
+    // Up to here constants of the plan or the batch; the estimates and the buffers that the estimation fills
+    // come after.
+    pg::wait_prerequisites();
     if (threadIdx.x >= 32 && threadIdx.x < 32 + ue.nof_rx_ports) {
       s_pres[threadIdx.x - 32] = port_results[(size_t)u * 4 + threadIdx.x - 32];
     }
@@ -586,7 +593,7 @@ int demod_only_launch(pg_context* ctx, const pg_pusch_ue* ues_dev, int n, uint32
                       const uint32_t* tile_map_dev, const uint32_t* grids, const float* est,
                       const pg_port_result* port_results, const uint32_t* seq_offsets_dev, const uint32_t* seq_dev,
                       int8_t* llrs, cudaStream_t s, int block, int res_per_thread, const float* basis,
-                      const uint8_t* basis_use, const rm_direct* direct, int8_t* rm_out)
+                      const uint8_t* basis_use, const rm_direct* direct, int8_t* rm_out, bool overlap)
 {
   if (n == 0 || total_tiles == 0) {
     return PG_OK;
@@ -599,6 +606,14 @@ int demod_only_launch(pg_context* ctx, const pg_pusch_ue* ues_dev, int n, uint32
   }
   res_per_thread       = std::max(1, std::min(8, res_per_thread));
   const uint32_t per   = (uint32_t)res_per_thread; // tiles per CTA
+  if (overlap) {
+    return check_cuda(ctx,
+                      launch_overlapped(pusch_demod_kernel, (total_tiles + per - 1) / per, block, 0, s, ues_dev,
+                                        total_tiles, tile_map_dev, grids, reinterpret_cast<const float2*>(est),
+                                        reinterpret_cast<const float2*>(basis), basis_use, port_results,
+                                        seq_offsets_dev, seq_dev, llrs, res_per_thread, direct, rm_out),
+                      "pusch_demod_kernel launch");
+  }
   pusch_demod_kernel<<<(total_tiles + per - 1) / per, block, 0, s>>>(
       ues_dev, total_tiles, tile_map_dev, grids, reinterpret_cast<const float2*>(est), reinterpret_cast<const float2*>(basis),
       basis_use, port_results, seq_offsets_dev, seq_dev, llrs, res_per_thread, direct, rm_out);

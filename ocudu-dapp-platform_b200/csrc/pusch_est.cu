@@ -462,6 +462,7 @@ __global__ void __launch_bounds__(kChunkThreads) pusch_estimate_chunk_kernel(con
                                                                              int nof_ues, int nwork,
                                                                              const __grid_constant__ pg::rm_fill fill)
 {
+  pg::launch_dependents();
   // A slot plan's buffers are filled by CTAs behind the estimator's. On a branch of its own beside this kernel
   // the fill's fork and join cost 1.7 us of a 45 us slot.
   if ((int)blockIdx.x >= nwork) {

@@ -11,6 +11,7 @@
 // previous buffer content (soft combining). Filler positions hold +127; positions at or beyond N_cb
 // are zeroed on new data and untouched otherwise.
 #include "pg_internal.h"
+#include "pg_device.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -239,7 +240,9 @@ __global__ void __launch_bounds__(kRmThreads) rate_dematch_kernel(const pg_rm_cb
                                                                   int8_t* __restrict__ out_all,
                                                                   const uint32_t* __restrict__ list)
 {
+  pg::launch_dependents();
   const pg_rm_cb d = cbs[list != nullptr ? list[blockIdx.x] : blockIdx.x];
+  pg::wait_prerequisites();
   rate_dematch(d, in_all, out_all);
 }
 
@@ -342,13 +345,19 @@ int rate_dematch_launch_args(pg_context* ctx, const pg_rm_cb* descs, int n, cons
 }
 
 int rate_dematch_launch(pg_context* ctx, const pg_rm_cb* descs_dev, int n, const int8_t* in, int8_t* out,
-                        cudaStream_t stream, int ctas_per_cb, const uint32_t* list)
+                        cudaStream_t stream, int ctas_per_cb, const uint32_t* list, bool overlap)
 {
   if (n == 0) {
     return PG_OK;
   }
   // Each codeblock's N <= 25,344 output positions spread over ctas_per_cb CTAs.
   ctas_per_cb = std::max(1, std::min(32, ctas_per_cb));
+  if (overlap) {
+    return check_cuda(ctx,
+                      launch_overlapped(rate_dematch_kernel, dim3(n, ctas_per_cb), kRmThreads, 0, stream, descs_dev, in, out,
+                                        list),
+                      "rate_dematch_kernel launch");
+  }
   rate_dematch_kernel<<<dim3(n, ctas_per_cb), kRmThreads, 0, stream>>>(descs_dev, in, out, list);
   return check_cuda(ctx, cudaGetLastError(), "rate_dematch_kernel launch");
 }
