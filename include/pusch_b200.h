@@ -548,7 +548,9 @@ int pg_pusch_plan_set_graph(pg_pusch_plan* plan, int enabled);
 int pg_pusch_plan_set_harq(pg_pusch_plan* plan, const uint8_t* new_data, const uint8_t* rv);
 
 /* Launch shapes of a plan's stages (the autotuner's search space). No counterpart in the
- * reference, whose stages are sized per UE and per codeblock by its thread pools. */
+ * reference, whose stages are sized per UE and per codeblock by its thread pools. Until a tuning is set or
+ * searched, a plan takes ldpc_ctas_per_sm and ldpc_order from its number of codeblocks: one CTA per SM up to
+ * 1.75 codeblocks per SM, else two, in the fixed order. */
 typedef struct pg_pusch_plan_tuning {
   int rm_ctas_per_cb;       /* rate dematching: CTAs per codeblock, 1..32 (default 8) */
   int demod_res_per_thread; /* demodulation: resource elements per thread, 1..8 (default 1) */
