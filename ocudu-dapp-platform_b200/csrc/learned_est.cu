@@ -393,7 +393,8 @@ size_t al(size_t x)
 //
 // Bound: the chain MMA - epilogue - MMA of tile 0. The tensor cores' operand reads take nearly all of the
 // shared-memory cycles, and a barrier probe under them 200 cycles or more: with one issuing warp, its five
-// waits stood between the MMAs and a layer took 5,600 cycles (tensor pipe busy for 3,000 of them).
+// waits stood between the MMAs and a layer took 5,600 cycles (tensor pipe busy for 3,000 of them); with two
+// 4,900. The network of a 16-cell slot (172,000 rows) takes 114 us, 128 us before.
 constexpr int      kFTiles    = 2;
 constexpr int      kFPairs    = 128 * kFTiles;
 constexpr int      kFWin      = 2 * kFPairs;
@@ -432,8 +433,8 @@ static_assert(kFChunkB % 16 == 0 && kFSmem < (1u << 18), "descriptor start addre
 // the block), and the ReLU replaced by the mask of the forward activation (its values are positive where
 // the ReLU passed), read from memory while the layer's MMAs run. Both passes are one launch instead of
 // one per layer, whose tile loads, MMAs and epilogues ran one after the other: at 96,000 rows the forward
-// pass takes 92 us (446 us in 14 launches before), the input gradients 122 us (545 us in 13). Bound: the
-// epilogues and the activation traffic (tensor pipe 31 % and 24 % of active cycles).
+// pass takes 90 us (446 us in 14 launches before), the input gradients 112 us (545 us in 13). Bound: the
+// chain of MMAs and epilogues and the activation traffic.
 enum fused_mode { kFInfer, kFTrain, kFBackward };
 
 struct fused_io {

@@ -216,9 +216,9 @@ __global__ void __launch_bounds__(kConvThreads) conv1d_fwd_kernel(const uint4* _
 // the same stage, and warps 4 to 7 add each group of four tiles' FP32 accumulators (two sets in tensor
 // memory, one filled while the other is read) to FP32 sums in registers, so that no sum of more than 512
 // rows is formed in the tensor cores. When a CTA's run of tiles of one layer ends, its sums are added to
-// dw[t][ci][co] with vector atomics. At 96,000 rows the 14 layers take 105 us (722 us with one launch per
-// layer, two synchronous stages and a second launch for the bias); bound by the rate at which one thread
-// issues the MMAs and by the loads.
+// dw[t][ci][co] with vector atomics. At 96,000 rows the 14 layers take 100 us (722 us with one launch per
+// layer, two synchronous stages and a second launch for the bias); bound by the MMAs' shared-memory operand
+// reads and by the loads.
 constexpr int      kWgTile     = 128;
 constexpr int      kWgCopyRows = kWgTile + 8;
 constexpr int      kWgStages   = 4;
