@@ -15,7 +15,7 @@ The line also carries: the same plan with the plain estimator (batched_plain); t
 GPU path on the same slot (one plan per UE, executed one after another with the host waiting for
 each UE's result); the end-to-end value through the host entry (pg_pusch_plan_execute_host: pinned
 host grids in, TBs and results out, every step); the rooflines of the learned estimator's network
-(tensor cores) and of ldpc_decode_kernel (integer pipe), both timed with CUDA events inside the
+(tensor cores) and of the LDPC decoder (integer pipe), both timed with CUDA events inside the
 step; the LDPC decoder batch (512 codeblocks, BG1/BG2 Z=384) in Gbit/s; clocks sampled during the
 timed region; and the reference's CPU receive path (oracle/_ref, the reference's own stage objects)
 on this host's cores as cpu_baseline.
@@ -57,7 +57,7 @@ LDPC_KERNEL_NAMES = (["ldpc_decode_kernel (one lifted lane per thread)"]
                      + 4 * ["ldpc_decode_pair_kernel (two lifted lanes per lane pair, 2 or 4 threads per pair)"])
 # ncu figures of one launch of the LDPC batch with the lane-pair kernel: pipe utilisation in % of active
 # cycles.
-LDPC_NCU = {k: {"pipes": {"alu": 56.0, "fma": 46.0, "issue_active": 64.0, "sm_active_pct_of_elapsed": 89.0}}
+LDPC_NCU = {k: {"pipes": {"alu": 57.3, "fma": 26.1, "fma_fp16": 21.8, "lsu": 26.6, "issue_active": 68.5}}
             for k in range(1, 5)}
 # Integer-instruction throughput probe (the LDPC roofline denominator), built by
 # ocudu-dapp-platform_b200/measure/Makefile.
@@ -1133,6 +1133,8 @@ def ldpc_measure(args, dev, rank, world):
 
 def main():
     args = parse_args()
+    if not os.path.exists(os.path.join(ROOT, "oracle", "_ref", "libocudu_ref.so")):
+        args.no_cpu_baseline = True  # the reference is not built here: no CPU baseline beside the measurement
     if args.impl == "reference":
         return run_reference_pusch(args) if args.workload == "uneven" else run_reference(args)
     return run_ours_pusch(args) if args.workload == "uneven" else run_ours_ldpc(args)
