@@ -1135,6 +1135,10 @@ def main():
     args = parse_args()
     if not os.path.exists(os.path.join(ROOT, "oracle", "_ref", "libocudu_ref.so")):
         args.no_cpu_baseline = True  # the reference is not built here: no CPU baseline beside the measurement
+        if args.impl == "reference":
+            if int(os.environ.get("RANK", "0")) == 0:
+                print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/libocudu_ref.so is not built"}))
+            return 0
     if args.impl == "reference":
         return run_reference_pusch(args) if args.workload == "uneven" else run_reference(args)
     return run_ours_pusch(args) if args.workload == "uneven" else run_ours_ldpc(args)
