@@ -309,7 +309,7 @@ __device__ __forceinline__ void decode_codeblock(const pg_ldpc_cb& d, smem_scala
   for (int k0 = 4 * tid; k0 < n; k0 += 4 * NT) {
     int v[4];
     if (aligned && k0 + 3 < n) {
-      const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(in + k0));
+      const uint32_t w = pg::load_written(reinterpret_cast<const uint32_t*>(in + k0));
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         v[j] = (int)(int8_t)(w >> (8 * j));
@@ -317,7 +317,7 @@ __device__ __forceinline__ void decode_codeblock(const pg_ldpc_cb& d, smem_scala
     } else {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        v[j] = k0 + j < n ? (int)in[k0 + j] : 0;
+        v[j] = k0 + j < n ? pg::load_written(in + k0 + j) : 0;
       }
     }
 #pragma unroll
@@ -985,7 +985,7 @@ __device__ __forceinline__ void fetch8(const int8_t* __restrict__ in, int k, int
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int kk = k + i;
-    int       x  = (kk >= 0 && kk < n) ? (int)__ldg(in + kk) : 0;
+    int       x  = (kk >= 0 && kk < n) ? pg::load_written(in + kk) : 0;
     last         = x != 0 ? max(last, kk + 1) : last;
     if (kk < nof_full) {
       x = max(-64, min(64, x));
@@ -1169,7 +1169,7 @@ __device__ __forceinline__ void decode_codeblock_pair(const pg_ldpc_cb& d, pair_
           for (int i = 0; i < 2; ++i) {
             raw[u][i] = make_uint2(0u, 0u);
             if (fetch_whole(k + i * H, nof_full, aligned) && q < nchunks) {
-              raw[u][i] = __ldg(reinterpret_cast<const uint2*>(in + k + i * H));
+              raw[u][i] = pg::load_written(reinterpret_cast<const uint2*>(in + k + i * H));
             }
           }
         }
@@ -1203,7 +1203,7 @@ __device__ __forceinline__ void decode_codeblock_pair(const pg_ldpc_cb& d, pair_
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           const int kk = k + i * H;
-          x[i]         = (kk >= 0 && kk < n) ? (int)__ldg(in + kk) : 0;
+          x[i]         = (kk >= 0 && kk < n) ? pg::load_written(in + kk) : 0;
           last         = x[i] != 0 ? max(last, kk + 1) : last;
           if (kk < nof_full) {
             x[i] = max(-64, min(64, x[i]));

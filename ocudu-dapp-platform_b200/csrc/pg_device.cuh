@@ -39,7 +39,10 @@ __device__ __forceinline__ uint32_t gold_word(const uint32_t* __restrict__ tab, 
 // Programmatic dependent launch. launch_dependents: the next kernel of the stream, if launched to allow it
 // (launch_overlapped), may start once every CTA of this grid has called it or exited. wait_prerequisites: until
 // the kernels before this one have completed and their memory is visible; without such a launch it returns at
-// once. Everything before it may touch only memory that no earlier kernel of the stream writes.
+// once. Everything before it may touch only memory that no earlier kernel of the stream writes. What an earlier
+// kernel does write is written while this one runs, so it is never read-only here: it is read after the wait and
+// with load_written, not with __ldg, which may be served from a line cached before the write, nor with a plain load
+// through const __restrict__, which the compiler may turn into the same and move ahead of the wait.
 __device__ __forceinline__ void launch_dependents()
 {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -47,6 +50,32 @@ __device__ __forceinline__ void launch_dependents()
 __device__ __forceinline__ void wait_prerequisites()
 {
   asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Coherent loads, in order with the wait (both are volatile).
+__device__ __forceinline__ int load_written(const int8_t* p)
+{
+  int v;
+  asm volatile("ld.global.s8 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint32_t load_written(const uint32_t* p)
+{
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint2 load_written(const uint2* p)
+{
+  uint2 v;
+  asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float2 load_written(const float2* p)
+{
+  float2 v;
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
 }
 
 // Launches a kernel that calls wait_prerequisites and may start before the kernel ahead of it has completed.

@@ -488,7 +488,13 @@ __global__ void __launch_bounds__(256) pusch_demod_kernel(const pg_pusch_ue* __r
     // come after.
     pg::wait_prerequisites();
     if (threadIdx.x >= 32 && threadIdx.x < 32 + ue.nof_rx_ports) {
-      s_pres[threadIdx.x - 32] = port_results[(size_t)u * 4 + threadIdx.x - 32];
+      const int       p   = (int)threadIdx.x - 32;
+      const uint32_t* src = reinterpret_cast<const uint32_t*>(port_results + (size_t)u * 4 + p);
+      static_assert(sizeof(pg_port_result) % 4 == 0, "copied by words");
+#pragma unroll
+      for (int i = 0; i < (int)sizeof(pg_port_result) / 4; ++i) {
+        reinterpret_cast<uint32_t*>(s_pres + p)[i] = pg::load_written(src + i);
+      }
     }
     const int ne = nd == 2 ? 2 : 1;
     const bool use_basis = basis_all != nullptr && basis_use != nullptr && nd == 2 && basis_use[u] != 0;
@@ -504,9 +510,9 @@ __global__ void __launch_bounds__(256) pusch_demod_kernel(const pg_pusch_ue* __r
         const int    d   = pd % ne;
         const int    p   = pd / ne;
         const size_t src = ((size_t)(p * nd + d) * ue.nof_layers + l) * nsc + j0 + jj;
-        s_est[row * kDemodTile + jj] = est[src];
+        s_est[row * kDemodTile + jj] = pg::load_written(est + src);
         if (bas != nullptr) {
-          s_bas[row * kDemodTile + jj] = bas[src];
+          s_bas[row * kDemodTile + jj] = pg::load_written(bas + src);
         }
       }
     }

@@ -37,13 +37,20 @@ __device__ __forceinline__ int llr_sum(int a, int b)
 
 constexpr int kRmRepBatch = 4;   // repetitions whose loads a thread issues together
 
-// One codeblock's buffer, and the store of one aligned word of it (positions 4 g - mis ..).
+// One codeblock's buffer, and the store of one aligned word of it (positions 4 g - mis ..). EARLY: the kernel
+// may have started before the one that writes the LLRs ended.
+template <bool EARLY>
 struct rm_buffer {
   int8_t*       out;
   const int8_t* in;
   int           mis, N, Ncb, inf, sys, F, V, v0, E, Qm, Kq;
   float         inv_kq;
   bool          nd;
+
+  __device__ __forceinline__ static int llr(const int8_t* p)
+  {
+    return EARLY ? pg::load_written(p) : (int)__ldg(p);
+  }
 
   // LLR t of the de-interleaved order is at row t mod Kq, column t div Kq; the quotient comes from a float
   // reciprocal, corrected to the exact value (t < 2^24).
@@ -63,7 +70,7 @@ struct rm_buffer {
   {
     int r, q;
     split(t, r, q);
-    return (int)__ldg(in + (r * Qm + q));
+    return llr(in + (r * Qm + q));
   }
   __device__ __forceinline__ static uint32_t pack(const int* x)
   {
@@ -97,7 +104,7 @@ struct rm_buffer {
     int                 x[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      x[j] = (int)__ldg(f + j * Qm);
+      x[j] = llr(f + j * Qm);
     }
     if (nd) {
 #pragma unroll
@@ -200,6 +207,7 @@ struct rm_buffer {
 // positions: 7.0 us on new data, 8.7 us combining (12 us each as tiles of the input transposed through shared
 // memory with a second pass over the positions no LLR reaches; 10 us with every word taken the general way;
 // 12 us with the words ordered so that one CTA reads each input sector).
+template <bool EARLY>
 __device__ __forceinline__ void rate_dematch(const pg_rm_cb& d, const int8_t* __restrict__ in_all, int8_t* __restrict__ out_all)
 {
   const int      bg = d.base_graph;
@@ -207,7 +215,7 @@ __device__ __forceinline__ void rate_dematch(const pg_rm_cb& d, const int8_t* __
   const int      Kb = bg == 1 ? 22 : 10;
   const int      sh = bg == 1 ? (d.rv == 0 ? 0 : d.rv == 1 ? 17 : d.rv == 2 ? 33 : 56)
                               : (d.rv == 0 ? 0 : d.rv == 1 ? 13 : d.rv == 2 ? 25 : 43);
-  rm_buffer      c;
+  rm_buffer<EARLY> c;
   c.N            = (bg == 1 ? 66 : 50) * Z;
   c.Ncb          = (d.nref > 0 && d.nref < (uint32_t)c.N) ? (int)d.nref : c.N;
   c.F            = d.nof_filler_bits;
@@ -228,9 +236,9 @@ __device__ __forceinline__ void rate_dematch(const pg_rm_cb& d, const int8_t* __
   const int tid  = threadIdx.x;
   for (int g = blockIdx.y * kRmThreads + tid; g < nw; g += gridDim.y * kRmThreads) {
     if (c.E > c.V) {
-      c.word<true>(g);
+      c.template word<true>(g);
     } else if (!c.plain_word(g)) {
-      c.word<false>(g);
+      c.template word<false>(g);
     }
   }
 }
@@ -243,7 +251,7 @@ __global__ void __launch_bounds__(kRmThreads) rate_dematch_kernel(const pg_rm_cb
   pg::launch_dependents();
   const pg_rm_cb d = cbs[list != nullptr ? list[blockIdx.x] : blockIdx.x];
   pg::wait_prerequisites();
-  rate_dematch(d, in_all, out_all);
+  rate_dematch<true>(d, in_all, out_all);
 }
 
 // The descriptors in the launch's arguments: a copy staged in pinned memory started the kernel 6 us later, and
@@ -260,7 +268,7 @@ __global__ void __launch_bounds__(kRmThreads) rate_dematch_args_kernel(const __g
                                                                        int8_t* __restrict__ out_all)
 {
   const pg_rm_cb d = args.cb[blockIdx.x];
-  rate_dematch(d, in_all, out_all);
+  rate_dematch<false>(d, in_all, out_all);
 }
 
 } // namespace
