@@ -93,7 +93,10 @@ int pg_ldpc_decode_batch_device(pg_context* ctx, const pg_ldpc_cb* cbs, int nof_
                                 uint8_t* bits, int32_t* iterations, void* stream);
 
 /* Same, with the descriptors already in device memory (nothing is staged: suitable for CUDA
- * graph capture and device-built work lists). */
+ * graph capture and device-built work lists).
+ * The batch decodes and transport-block decodes of a context share its decoder scratch: each call, on any
+ * stream, follows the one before it on the device. Captured calls are not ordered like this: the caller keeps
+ * the replays of a captured decode apart from each other and from the context's other decodes. */
 int pg_ldpc_decode_batch_resident(pg_context* ctx, const pg_ldpc_cb* cbs_dev, int nof_cbs, const int8_t* llrs,
                                   uint8_t* bits, int32_t* iterations, void* stream);
 

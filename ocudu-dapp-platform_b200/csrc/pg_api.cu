@@ -102,6 +102,36 @@ static int ensure_host_capacity(pg_context* ctx, size_t llrs, size_t bits)
   return PG_OK;
 }
 
+bool capturing(cudaStream_t s)
+{
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return true;
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
+
+int decoder_acquire(pg_context* ctx, cudaStream_t s)
+{
+  if (ctx->desc_pending && !ctx->desc_captured) {
+    if (int rc = check_cuda(ctx, cudaStreamWaitEvent(s, ctx->ev_desc, 0), "cudaStreamWaitEvent(descriptors)")) {
+      return rc;
+    }
+  }
+  return ctx->decoder_pending ? check_cuda(ctx, cudaStreamWaitEvent(s, ctx->ev_decoder, 0), "cudaStreamWaitEvent(decoder)")
+                              : PG_OK;
+}
+
+int decoder_release(pg_context* ctx, cudaStream_t s)
+{
+  if (int rc = check_cuda(ctx, cudaEventRecord(ctx->ev_decoder, s), "cudaEventRecord(decoder)")) {
+    return rc;
+  }
+  ctx->decoder_pending = true;
+  return PG_OK;
+}
+
 // Copies descriptors into the pinned staging buffer and uploads them on stream s. The staging
 // and device descriptor buffers are reused only after the previous kernel that read them has
 // completed (see release_descs_after).
@@ -123,25 +153,15 @@ static int stage_descs(pg_context* ctx, const pg_ldpc_cb* cbs, int n, cudaStream
   return PG_OK;
 }
 
-// Whether s is being captured (or cannot tell).
-static bool capturing(cudaStream_t s)
-{
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return true;
-  }
-  return st != cudaStreamCaptureStatusNone;
-}
-
-// Marks the staged descriptors busy until the work enqueued on s so far (the kernel reading
-// them included) has completed.
-static int release_descs_after(pg_context* ctx, cudaStream_t s)
+// Marks the staged descriptors and the decoder scratch busy until the work enqueued on s so far (the kernels
+// using them included) has completed.
+static int release_descs_after(pg_context* ctx, cudaStream_t s, bool captured)
 {
   if (int rc = check_cuda(ctx, cudaEventRecord(ctx->ev_desc, s), "cudaEventRecord(descriptors)")) {
     return rc;
   }
-  ctx->desc_pending = true;
+  ctx->desc_pending  = true;
+  ctx->desc_captured = captured;
   return PG_OK;
 }
 
@@ -288,6 +308,9 @@ int pg_create(const pg_config* cfg, pg_context** out)
     rc = check_cuda(ctx, cudaEventCreateWithFlags(&ctx->ev_desc, cudaEventDisableTiming), "cudaEventCreate");
   }
   if (rc == PG_OK) {
+    rc = check_cuda(ctx, cudaEventCreateWithFlags(&ctx->ev_decoder, cudaEventDisableTiming), "cudaEventCreate");
+  }
+  if (rc == PG_OK) {
     // One slab per resident decoder CTA.
     rc = check_cuda(ctx, cudaMalloc(&ctx->dev.c2v, (size_t)kLdpcSlabsPerSm * ctx->sm_count * kPairSlab),
                     "cudaMalloc(check-to-variable scratch)");
@@ -426,6 +449,9 @@ void pg_destroy(pg_context* ctx)
   if (ctx->ev_desc) {
     cudaEventDestroy(ctx->ev_desc);
   }
+  if (ctx->ev_decoder) {
+    cudaEventDestroy(ctx->ev_decoder);
+  }
   if (ctx->stream) {
     cudaStreamDestroy(ctx->stream);
   }
@@ -447,24 +473,19 @@ int pg_ldpc_decode_batch_device(pg_context* ctx, const pg_ldpc_cb* cbs, int nof_
   if (llrs == nullptr || bits == nullptr || iterations == nullptr) {
     return set_error(ctx, PG_ERR_INVALID, "null device buffer");
   }
-  // The descriptors travel with the launches where they fit. The context's decoder scratch is shared, so a call
-  // on another stream follows the one before it on the device. A captured call stages them as before: its graph
-  // must not wait for work outside it.
+  // The descriptors travel with the launches where they fit. A captured call stages them, and so does a call
+  // after it, which that capture's event refuses.
   cudaStream_t s        = static_cast<cudaStream_t>(stream);
-  const bool   by_value = !capturing(s) && ldpc_descs_by_value(ctx, nof_cbs);
-  if (!by_value) {
-    if (int rc = stage_descs(ctx, cbs, nof_cbs, s)) {
-      return rc;
-    }
-  } else if (ctx->desc_pending) {
-    if (int rc = check_cuda(ctx, cudaStreamWaitEvent(s, ctx->ev_desc, 0), "cudaStreamWaitEvent(descriptors)")) {
-      return rc;
-    }
+  const bool   captured = capturing(s);
+  const bool   by_value = !captured && !ctx->desc_captured && ldpc_descs_by_value(ctx, nof_cbs);
+  int          rc       = captured ? PG_OK : decoder_acquire(ctx, s);
+  if (rc == PG_OK && !by_value) {
+    rc = stage_descs(ctx, cbs, nof_cbs, s);
   }
-  if (int rc = ldpc_launch(ctx, ctx->dev.descs, nof_cbs, llrs, bits, iterations, s, by_value ? cbs : nullptr)) {
-    return rc;
+  if (rc == PG_OK) {
+    rc = ldpc_launch(ctx, ctx->dev.descs, nof_cbs, llrs, bits, iterations, s, by_value ? cbs : nullptr);
   }
-  return release_descs_after(ctx, s);
+  return rc == PG_OK ? release_descs_after(ctx, s, captured) : rc;
 }
 
 int pg_ldpc_decode_batch_resident(pg_context* ctx, const pg_ldpc_cb* cbs_dev, int nof_cbs, const int8_t* llrs,
@@ -479,7 +500,13 @@ int pg_ldpc_decode_batch_resident(pg_context* ctx, const pg_ldpc_cb* cbs_dev, in
   if (cbs_dev == nullptr || llrs == nullptr || bits == nullptr || iterations == nullptr) {
     return set_error(ctx, PG_ERR_INVALID, "null device buffer");
   }
-  return ldpc_launch(ctx, cbs_dev, nof_cbs, llrs, bits, iterations, static_cast<cudaStream_t>(stream));
+  cudaStream_t s        = static_cast<cudaStream_t>(stream);
+  const bool   captured = capturing(s);
+  int          rc       = captured ? PG_OK : decoder_acquire(ctx, s);
+  if (rc == PG_OK) {
+    rc = ldpc_launch(ctx, cbs_dev, nof_cbs, llrs, bits, iterations, s);
+  }
+  return rc == PG_OK && !captured ? decoder_release(ctx, s) : rc;
 }
 
 int pg_ldpc_decode_batch_host(pg_context* ctx, const pg_ldpc_cb* cbs, int nof_cbs, const int8_t* llrs,
@@ -504,7 +531,10 @@ int pg_ldpc_decode_batch_host(pg_context* ctx, const pg_ldpc_cb* cbs, int nof_cb
     return rc;
   }
   cudaStream_t s  = ctx->stream;
-  int          rc = stage_descs(ctx, cbs, nof_cbs, s);
+  int          rc = decoder_acquire(ctx, s);
+  if (rc == PG_OK) {
+    rc = stage_descs(ctx, cbs, nof_cbs, s);
+  }
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaMemcpyAsync(ctx->dev.llrs, llrs, nof_llrs_total, cudaMemcpyHostToDevice, s),
                     "cudaMemcpyAsync(llrs)");
@@ -513,7 +543,7 @@ int pg_ldpc_decode_batch_host(pg_context* ctx, const pg_ldpc_cb* cbs, int nof_cb
     rc = ldpc_launch(ctx, ctx->dev.descs, nof_cbs, ctx->dev.llrs, ctx->dev.bits, ctx->dev.iterations, s);
   }
   if (rc == PG_OK) {
-    rc = release_descs_after(ctx, s);
+    rc = release_descs_after(ctx, s, false);
   }
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaMemcpyAsync(bits, ctx->dev.bits, bits_bytes, cudaMemcpyDeviceToHost, s),

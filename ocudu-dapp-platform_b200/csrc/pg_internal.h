@@ -91,8 +91,11 @@ struct pg_context {
   cudaEvent_t         ev_le_start    = nullptr; // learned-estimator stage of slot plans (timed contexts)
   cudaEvent_t         ev_le_stop     = nullptr;
   bool                le_recorded    = false;
-  cudaEvent_t         ev_desc        = nullptr; // completion of the last descriptor upload
+  cudaEvent_t         ev_desc        = nullptr; // last batch decode with descriptors from the host
   bool                desc_pending   = false;
+  bool                desc_captured  = false;   // ev_desc was last recorded in a capture
+  cudaEvent_t         ev_decoder     = nullptr; // last other use of the decoder scratch
+  bool                decoder_pending = false;
   pg::staging_slot    slots[8];                  // rate-dematch, CRC, TB, PUSCH, UE and UCI work lists
   void*               est_partials     = nullptr;  // partial sums of the batched channel estimation
   size_t              est_partials_cap = 0;
@@ -112,6 +115,16 @@ namespace pg {
 
 int set_error(pg_context* ctx, int code, const std::string& msg);
 int check_cuda(pg_context* ctx, cudaError_t err, const char* what);
+
+// Whether s is being captured (or cannot tell).
+bool capturing(cudaStream_t s);
+// The batch decodes of a context share its decoder scratch (dev.c2v, ldpc_counter, ldpc_keys, ldpc_order and, for
+// descriptors that the ordering launch stores, dev.descs). Every call on a stream s that is not being captured
+// starts with decoder_acquire, which puts it behind the calls before it on the device, and ends by recording its
+// event: ev_desc where the descriptors come from the host, else ev_decoder (decoder_release). A captured call
+// waits for neither (its graph must not depend on work outside it): its replays are ordered by the caller.
+int decoder_acquire(pg_context* ctx, cudaStream_t s);
+int decoder_release(pg_context* ctx, cudaStream_t s);
 
 // Validates descriptors on the host; returns PG_OK or PG_ERR_INVALID with a message.
 int validate_ldpc_descs(pg_context* ctx, const pg_ldpc_cb* cbs, int n, size_t nof_llrs_total, size_t bits_bytes);

@@ -495,8 +495,14 @@ int sch_decode_device_llrs(pg_context* ctx, const pg_sch_tb* tbs, int nof_tbs, c
     rc = stage_slot(ctx, SLOT_PUSCH, ldpc.data(), ldpc.size() * sizeof(pg_ldpc_cb), s, &d_ldpc);
   }
   if (rc == PG_OK) {
+    rc = decoder_acquire(ctx, s);
+  }
+  if (rc == PG_OK) {
     rc = ldpc_launch(ctx, static_cast<const pg_ldpc_cb*>(d_ldpc), ncb, reinterpret_cast<const int8_t*>(base + o_rm),
                      base + o_bits, reinterpret_cast<int32_t*>(base + o_it), s);
+  }
+  if (rc == PG_OK) {
+    rc = decoder_release(ctx, s);
   }
   if (rc == PG_OK) {
     rc = release_slot_after(ctx, SLOT_PUSCH, s);
