@@ -489,7 +489,8 @@ __device__ __forceinline__ void decode_codeblock(const pg_ldpc_cb& d, smem_scala
 // counter == nullptr: one CTA per codeblock (blockIdx.x), slab blockIdx.x. Otherwise a persistent
 // grid: each CTA takes the next work index from *counter (zeroed before the launch), decodes
 // codeblock order[w] (or w) with its own slab blockIdx.x, and stops when the n codeblocks are
-// taken. Codeblocks are independent, so the order of work changes no result.
+// taken. Codeblocks are independent, so the order of work changes no result. With an order, counter[1] (the
+// arrivals of the ordering launch) is left at zero.
 __global__ void __launch_bounds__(kThreads, 2) ldpc_decode_kernel(const pg_ldpc_cb* __restrict__ descs,
                                                               const int8_t* __restrict__ llrs,
                                                               uint8_t* __restrict__ bits,
@@ -518,6 +519,9 @@ __global__ void __launch_bounds__(kThreads, 2) ldpc_decode_kernel(const pg_ldpc_
     const int w = s_work;
     __syncthreads();
     if (w >= n) {
+      if (order != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
+        counter[1] = 0;
+      }
       break;
     }
     const int        cb = order != nullptr ? (int)order[w] : w;
@@ -1054,9 +1058,8 @@ __device__ __forceinline__ void tb_arrive(const pg::ldpc_tb_sink& sink, const pg
   sum = __reduce_add_sync(0xffffffffu, sum);
   mx  = __reduce_max_sync(0xffffffffu, mx);
   if (lane == 0) {
-    const uint32_t crc   = atomicExch(&sink.crc[tb], 0u); // zero again for the next execution
-    sink.arrivals[tb]    = 0;
-    pg_sch_result r;
+    const uint32_t crc   = __ldcg(&sink.crc[tb]);
+    pg_sch_result  r;
     r.tb_crc_ok          = (ok == t.nof_cbs && (t.nof_cbs == 1 || crc == 0)) ? 1u : 0u;
     r.nof_cbs            = t.nof_cbs;
     r.nof_cbs_crc_ok     = ok;
@@ -1489,6 +1492,12 @@ __global__ void __launch_bounds__(kPairThreads, kPairPerSm)
     }
     __syncthreads();
     w = sh.work;
+  }
+  // The arrivals of the ordering launch ahead of this one. Its last CTA clears them too, but knows that it is the
+  // last from the count: cleared here, a count that was off (ordering launches that ran at the same time, from
+  // replays of captured decodes) spoils no later batch.
+  if (order != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
+    counter[1] = 0;
   }
 }
 

@@ -182,14 +182,16 @@ int rate_dematch_launch(pg_context* ctx, const pg_rm_cb* descs_dev, int n, const
                         cudaStream_t stream, int ctas_per_cb, const uint32_t* list = nullptr, bool overlap = false);
 // Before a slot plan's demodulator stores LLRs in place: the circular buffers of the codeblocks with
 // placed[c] = 1 get what rate dematching leaves at the positions no LLR reaches (+127 at the fillers, 0
-// elsewhere), and tb_out and *counter are zeroed (rm_prefill, kRmFillCtas CTAs per codeblock).
+// elsewhere), and tb_out, counters (two) and join are zeroed (rm_prefill, kRmFillCtas CTAs per codeblock).
 struct rm_fill {
   const pg_rm_cb* cbs;
   const uint8_t*  placed;
   int8_t*         out;
   uint8_t*        tb_out;
   size_t          tb_bytes;
-  int*            counter;
+  int*            counters;
+  uint32_t*       join;
+  int             njoin;
   int             n;
 };
 constexpr int kRmFillCtas = 4;
@@ -304,7 +306,7 @@ int ldpc_order_launch(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const
 // tb_out instead of the decoder's bit output, and the last codeblock of each TB writes results[tb]. Every
 // TB has one codeblock, or codeblocks of an even lifting size with payloads of whole bytes
 // (tb_join_in_decoder). cbs[cb]: TB and x^((C - 1 - c) P) mod the TB's CRC polynomial for codeblock c of C
-// with P payload bits. crc and arrivals (one entry per TB) are zero before a launch and after it.
+// with P payload bits. crc and arrivals (one entry per TB) are zero before a launch.
 struct ldpc_tb_cb {
   uint32_t tb;
   uint32_t factor;
@@ -324,7 +326,8 @@ std::vector<ldpc_tb_cb> tb_join_in_decoder(const std::vector<pg_tb_desc>& tbs, c
 // kernel's own limit.
 int ldpc_max_ctas(const pg_context* ctx, int per_sm, int kernel);
 // Persistent launch: min(n, max_ctas) CTAs (max_ctas from ldpc_max_ctas) take codeblocks order[0..n)
-// (identity when order is null) from *counter (device int, zeroed here on the stream unless counter_zero);
+// (identity when order is null) from *counter (device int, zeroed here on the stream unless counter_zero; with an
+// order, the ordering launch's arrivals follow it);
 // overlap: the launch may start before the kernel ahead of it ends (that kernel writes neither the order nor
 // the descriptors); c2v holds one slab (kPairSlab bytes) per CTA.
 int ldpc_launch_persistent(pg_context* ctx, const pg_ldpc_cb* descs_dev, int n, const int8_t* llrs, uint8_t* bits,

@@ -99,7 +99,7 @@ struct pg_pusch_plan {
   uint32_t*       d_order  = nullptr; // per-execution work order (device ordering)
   uint32_t*       d_order_static = nullptr; // largest codeblocks first, fixed at creation
   ldpc_tb_cb*     d_tb_cbs       = nullptr; // TB join in the decoder (null: separate kernels)
-  uint32_t*       d_join         = nullptr; // its per-TB CRC and arrival words, zero between executions
+  uint32_t*       d_join         = nullptr; // its per-TB CRC and arrival words, zeroed by every execution
   uint32_t*       d_tb_chunks    = nullptr; // TB-assembly work items (TB | chunk << 16)
   int             tb_nchunks     = 0;
   uint8_t*        d_keys   = nullptr; // work-order keys of the codeblocks // LDPC work order: largest codeblocks first
@@ -295,7 +295,8 @@ int enqueue(pg_pusch_plan* p, const uint32_t* grids, uint8_t* tb_out, pg_sch_res
   // each kernel started behind the last), a 100 MHz cell 52.0 (55.3), 3 cells 70.6 (72.9).
   // The estimator's launch also fills the in-place codeblocks' buffers (the previous execution on this stream,
   // whose decoder read them, precedes it).
-  const rm_fill fill{p->d_rm, p->d_placed, p->d_rm_out, tb_out, p->tb_bytes, p->d_counter, p->nof_cbs};
+  const rm_fill fill{p->d_rm,      p->d_placed, p->d_rm_out,    tb_out,    p->tb_bytes,
+                     p->d_counter, p->d_join,   2 * p->nof_ues, p->nof_cbs};
   int           rc = estimate_launch(ctx, p->d_ues, p->nof_ues, p->d_est_work, p->est_nwork, p->d_est_part, p->d_est_arr,
                                      grids, p->d_est, p->le_net != nullptr ? p->d_ls : nullptr, port_results, s,
                                      p->d_pilot_bits, &fill);
@@ -790,12 +791,6 @@ int pg_pusch_plan_create_uci(pg_context* ctx, const pg_pusch_ue* ues, const pg_p
   }
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaMemsetAsync(b + o_earr, 0, (size_t)nof_ues * 16, s), "cudaMemsetAsync(arrivals)");
-  }
-  if (rc == PG_OK) {
-    rc = check_cuda(ctx, cudaMemsetAsync(p->d_counter, 0, 2 * sizeof(int), s), "cudaMemsetAsync(work counter)");
-  }
-  if (rc == PG_OK) {
-    rc = check_cuda(ctx, cudaMemsetAsync(p->d_join, 0, (size_t)nof_ues * 8, s), "cudaMemsetAsync(TB join)");
   }
   if (rc == PG_OK) {
     rc = scrambling_launch(ctx, p->d_ues, nof_ues, max_words, p->d_seq_off, p->d_seq, s);

@@ -9,8 +9,8 @@ namespace pg {
 // = 1: new data, E <= V), before it does: +127 at the filler positions [inf, (Kb - 2) Z) and 0
 // everywhere else, which is what rate dematching leaves at every position that no LLR reaches.
 // 16-byte stores; the first and last bytes of a buffer that does not start or end on a 16-byte
-// boundary are stored one by one. Also zeroes the TB buffer (bytes between the TBs stay zero) and the
-// decoders' work counter. CTA `cta` of kRmFillCtas * n, NT threads each.
+// boundary are stored one by one. Also zeroes the TB buffer (bytes between the TBs stay zero), the decoders'
+// work counter, the arrivals of their ordering launch, and the CRC and arrival words of the TB join. CTA `cta` of kRmFillCtas * n, NT threads each.
 template <int NT>
 __device__ __forceinline__ void rm_prefill(const rm_fill& f, const int cta)
 {
@@ -29,8 +29,11 @@ __device__ __forceinline__ void rm_prefill(const rm_fill& f, const int cta)
     if (head + 16 * nvec + t0 < f.tb_bytes) {
       f.tb_out[head + 16 * nvec + t0] = 0;
     }
-    if (t0 == 0) {
-      *f.counter = 0;
+    if (t0 < 2) {
+      f.counters[t0] = 0;
+    }
+    for (size_t q = t0; q < (size_t)f.njoin; q += nthr) {
+      f.join[q] = 0u;
     }
   }
   const int c = cta / kRmFillCtas;
