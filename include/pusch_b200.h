@@ -524,12 +524,12 @@ typedef struct pg_pusch_uci_result {
  * message without a polar code for its encoded size makes the creation PG_ERR_INVALID). */
 int  pg_pusch_plan_create_uci(pg_context* ctx, const pg_pusch_ue* ues, const pg_pusch_uci* uci, int nof_ues,
                               size_t grid_words, pg_pusch_plan** out);
-/* UCI results of the plan's last execution (nof_ues entries, host memory). Reads device memory
- * synchronously: call after that execution's stream has completed. */
+/* UCI results of the plan's last execution (nof_ues entries, host memory), which the decoders store to pinned
+ * host memory: call after that execution's stream has completed. Any device may be current. */
 int  pg_pusch_plan_uci_results(pg_pusch_plan* plan, pg_pusch_uci_result* out);
 /* One UCI message of the plan's last execution, any size: UE ue, field 0 HARQ-ACK / 1 CSI Part 1;
  * bits receives the message's bits (one per byte; len at least its size) and *valid its validity.
- * PG_ERR_INVALID when the UE carries no such message. Synchronous, as pg_pusch_plan_uci_results. */
+ * PG_ERR_INVALID when the UE carries no such message. To be called as pg_pusch_plan_uci_results. */
 int  pg_pusch_plan_uci_message(pg_pusch_plan* plan, int ue, int field, uint8_t* bits, size_t len, uint8_t* valid);
 void pg_pusch_plan_destroy(pg_pusch_plan* plan);
 int  pg_pusch_plan_info(const pg_pusch_plan* plan, pg_pusch_plan_info_t* info);

@@ -924,11 +924,26 @@ int pg_pusch_plan_set_learned(pg_pusch_plan* plan, pg_le_net* net, const uint8_t
 
 // Waits for the executions whose UCI results the caller reads. The decoders store them to pinned host
 // memory, so a read needs no copy; recording an event on the default stream keeps the order a copy on that
-// stream would have. (Two copies to pageable memory took 37 us a message.)
+// stream would have: the default stream of the plan's device, whichever is current. (Two copies to pageable
+// memory took 37 us a message.)
 static int wait_uci(pg_pusch_plan* plan)
 {
-  int rc = check_cuda(plan->ctx, cudaEventRecord(plan->ev_uread, nullptr), "cudaEventRecord(UCI read)");
-  return rc != PG_OK ? rc : check_cuda(plan->ctx, cudaEventSynchronize(plan->ev_uread), "cudaEventSynchronize(UCI read)");
+  pg_context* ctx  = plan->ctx;
+  int         prev = -1;
+  int         rc   = check_cuda(ctx, cudaGetDevice(&prev), "cudaGetDevice");
+  if (rc == PG_OK && prev != ctx->device) {
+    rc = check_cuda(ctx, cudaSetDevice(ctx->device), "cudaSetDevice");
+  }
+  if (rc == PG_OK) {
+    rc = check_cuda(ctx, cudaEventRecord(plan->ev_uread, nullptr), "cudaEventRecord(UCI read)");
+  }
+  if (rc == PG_OK) {
+    rc = check_cuda(ctx, cudaEventSynchronize(plan->ev_uread), "cudaEventSynchronize(UCI read)");
+  }
+  if (prev >= 0 && prev != ctx->device) {
+    cudaSetDevice(prev);
+  }
+  return rc;
 }
 
 int pg_pusch_plan_uci_results(pg_pusch_plan* plan, pg_pusch_uci_result* out)
