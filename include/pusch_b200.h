@@ -551,20 +551,18 @@ int pg_pusch_plan_set_graph(pg_pusch_plan* plan, int enabled);
 int pg_pusch_plan_set_harq(pg_pusch_plan* plan, const uint8_t* new_data, const uint8_t* rv);
 
 /* Launch shapes of a plan's stages (the autotuner's search space). No counterpart in the
- * reference, whose stages are sized per UE and per codeblock by its thread pools. Until a tuning is set or
- * searched, a plan takes ldpc_ctas_per_sm and ldpc_order from its number of codeblocks: one CTA per SM up to
- * 1.75 codeblocks per SM, else two, in the fixed order. */
+ * reference, whose stages are sized per UE and per codeblock by its thread pools. */
 typedef struct pg_pusch_plan_tuning {
   int rm_ctas_per_cb;       /* rate dematching: CTAs per codeblock, 1..32 (default 8) */
   int demod_res_per_thread; /* demodulation: resource elements per thread, 1..8 (default 1) */
   int demod_block;          /* demodulation: threads per CTA, 64, 128 or 256 (default 256) */
-  int ldpc_ctas_per_sm;     /* persistent LDPC decoders: CTAs per SM, 1..4 (default 2, which is also the most
-                               a kernel holds) */
+  int ldpc_ctas_per_sm;     /* persistent LDPC decoders: CTAs per SM, 1..4 (a kernel holds 2 at most; a new
+                               plan has 1 up to 1.75 codeblocks per SM, else 2) */
   int ldpc_kernel;          /* LDPC decoder (pg_ldpc_kernel), PG_LDPC_KERNEL_ONE_LANE .. _Z384_SPLIT
                                (default PG_LDPC_KERNEL_Z384, the lane-pair decoder) */
   int ldpc_order;           /* work order of the persistent decoders: 0 = largest codeblocks first, fixed
                                when the plan is created; 1 = longest predicted decode first, from every
-                               execution's LLRs (pg_set_ldpc_order's estimate; default 1) */
+                               execution's LLRs (pg_set_ldpc_order's estimate; default 0) */
 } pg_pusch_plan_tuning;
 
 int pg_pusch_plan_get_tuning(const pg_pusch_plan* plan, pg_pusch_plan_tuning* out);

@@ -137,8 +137,7 @@ struct pg_pusch_plan {
   int             le_nseq   = 0;
   int             le_rows   = 0;
   // Launch shapes (defaults, or the autotuner's choice).
-  pg_pusch_plan_tuning tuning = {8, 1, 256, 2, PG_LDPC_KERNEL_Z384, 1};
-  bool                 tuned  = false; // the tuning was set or searched
+  pg_pusch_plan_tuning tuning = {8, 1, 256, 2, PG_LDPC_KERNEL_Z384, 0};
   // CUDA graph of execute_device.
   bool            use_graph = false;
   cudaGraphExec_t exec      = nullptr;
@@ -264,20 +263,14 @@ std::vector<uint32_t> unplaced_list(const std::vector<uint8_t>& placed)
 
 // Decoder CTAs of the plan's launch, and whether an execution orders the codeblocks on the device: only
 // when they outnumber the CTAs (otherwise all start at once).
-// A plan whose tuning was never set or searched: one CTA per SM up to 1.75 codeblocks per SM, whose messages then
-// stay in shared memory, two above; the work order fixed at creation. One CTA and the fixed order against two
-// (with the predicted order, which runs above two codeblocks per SM): slots of 171 codeblocks 89 and 95 us, 163
-// 80 and 88, 228 95 and 103, 156 91 and 93, 210 94.5 and 96, 166 77.0 and 76.5; 263 101 and 98. Two CTAs at 300
-// codeblocks: fixed order 107 us, predicted 119 (its launch reads every LLR again).
 int ldpc_ctas(const pg_pusch_plan* p)
 {
-  const int per_sm = p->tuned ? p->tuning.ldpc_ctas_per_sm : (4 * p->nof_cbs <= 7 * p->ctx->sm_count ? 1 : 2);
-  return std::min(p->nof_cbs, ldpc_max_ctas(p->ctx, per_sm, p->tuning.ldpc_kernel));
+  return std::min(p->nof_cbs, ldpc_max_ctas(p->ctx, p->tuning.ldpc_ctas_per_sm, p->tuning.ldpc_kernel));
 }
 
 bool ldpc_ordered(const pg_pusch_plan* p)
 {
-  return p->tuned && p->tuning.ldpc_order != 0 && p->nof_cbs > ldpc_ctas(p);
+  return p->tuning.ldpc_order != 0 && p->nof_cbs > ldpc_ctas(p);
 }
 
 // Whether the decoder joins the TBs and writes the results (the lane-pair kernel, TBs it can join).
@@ -628,6 +621,12 @@ int pg_pusch_plan_create_uci(pg_context* ctx, const pg_pusch_ue* ues, const pg_p
     cost[c]             = (uint64_t)l.lifting_size * std::min<uint64_t>(w.rm[c].rm_length + l.nof_filler_bits, l.nof_llrs);
   }
   std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return cost[a] > cost[b]; });
+  // A new plan's decoder: one CTA per SM up to 1.75 codeblocks per SM, whose messages then stay in shared memory,
+  // two above; the work order fixed here. One CTA and the fixed order against two (with the predicted order, which
+  // runs above two codeblocks per SM): slots of 171 codeblocks 89 and 95 us, 163 80 and 88, 228 95 and 103, 156 91
+  // and 93, 210 94.5 and 96, 166 77.0 and 76.5; 263 101 and 98. Two CTAs at 300 codeblocks: fixed order 107 us,
+  // predicted 119 (its launch reads every LLR again).
+  p->tuning.ldpc_ctas_per_sm = 4 * p->nof_cbs <= 7 * ctx->sm_count ? 1 : 2;
   // One check-to-variable slab per decoder CTA, at most one per codeblock.
   const int ldpc_slabs = std::max(1, std::min(p->nof_cbs, kLdpcSlabsPerSm * ctx->sm_count));
 
@@ -1096,7 +1095,6 @@ int pg_pusch_plan_set_tuning(pg_pusch_plan* plan, const pg_pusch_plan_tuning* t)
     return rc;
   }
   plan->tuning = *t;
-  plan->tuned  = true;
   if (plan->exec != nullptr) {
     cudaGraphExecDestroy(plan->exec);
     plan->exec = nullptr;
@@ -1182,8 +1180,7 @@ int pg_pusch_plan_autotune(pg_pusch_plan* plan, const uint32_t* grids, int reps,
       return rc;
     }
   }
-  plan->tuned = true;
-  rc          = time_plan(plan, grids, plan->d_tb_out, plan->d_res, reps, &cur_ms);
+  rc = time_plan(plan, grids, plan->d_tb_out, plan->d_res, reps, &cur_ms);
   auto try_set = [&](pg_pusch_plan_tuning cand) -> int {
     if (!tuning_valid(cand, ctx)) {
       return PG_OK;
