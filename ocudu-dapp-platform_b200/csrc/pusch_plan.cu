@@ -1217,6 +1217,11 @@ int pg_pusch_plan_autotune(pg_pusch_plan* plan, const uint32_t* grids, int reps,
       c.ldpc_ctas_per_sm     = v;
       if (rc == PG_OK) rc = try_set(c);
     }
+    for (int v : {PG_LDPC_KERNEL_ONE_LANE, PG_LDPC_KERNEL_Z384}) { // the others name the second
+      pg_pusch_plan_tuning c = cur;
+      c.ldpc_kernel          = v;
+      if (rc == PG_OK) rc = try_set(c);
+    }
     for (int v : {0, 1}) {
       pg_pusch_plan_tuning c = cur;
       c.ldpc_order           = v;
