@@ -98,7 +98,8 @@ struct pg_le_net {
   uint16_t*   mid[kBlocks] = {};  // [8][R][8]
   uint16_t*   y        = nullptr; // [2][R][8]
   uint16_t*   dy       = nullptr; // [2][R][8]
-  uint16_t*   g[kLayers - 1] = {}; // g[l]: [8][R][8] gradient of layer l's output (before it: dy)
+  uint16_t*   g[kLayers - 1] = {}; // g[l]: [8][R][8] gradient of layer l's output (before it: dy); see grad_buffers
+  void*       dev_g     = nullptr;
   uint8_t*    row_valid = nullptr;
   pg::le_seq* seqs      = nullptr;
   float*      gseq      = nullptr;
@@ -963,6 +964,38 @@ int forward(pg_le_net* net, int R, cudaStream_t s)
   return fused_launch<kFTrain>(net, net->x, net->wp, R, io, s);
 }
 
+// The layers' gradient buffers, half of a training net's memory: allocated by the first call that trains, so that
+// a net which only infers does not hold them. That call may be captured, hence the relaxed mode. They are written
+// before they are read.
+int grad_buffers(pg_le_net* net, int rows)
+{
+  if (net->dev_g != nullptr || rows <= 0) {
+    return PG_OK;
+  }
+  pg_context*           ctx  = net->ctx;
+  const size_t          one  = al((size_t)net->max_rows * 128);
+  int                   prev = -1;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  int rc = pg::check_cuda(ctx, cudaGetDevice(&prev), "cudaGetDevice");
+  if (rc == PG_OK && prev != ctx->device) {
+    rc = pg::check_cuda(ctx, cudaSetDevice(ctx->device), "cudaSetDevice");
+  }
+  if (rc == PG_OK) {
+    rc = pg::check_cuda(ctx, cudaThreadExchangeStreamCaptureMode(&mode), "cudaThreadExchangeStreamCaptureMode");
+    if (rc == PG_OK) {
+      rc = pg::check_cuda(ctx, cudaMalloc(&net->dev_g, (kLayers - 1) * one), "cudaMalloc(learned estimator gradients)");
+      (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+  }
+  if (prev >= 0 && prev != ctx->device) {
+    cudaSetDevice(prev);
+  }
+  for (int i = 0; rc == PG_OK && i < kLayers - 1; ++i) {
+    net->g[i] = reinterpret_cast<uint16_t*>(static_cast<uint8_t*>(net->dev_g) + i * one);
+  }
+  return rc;
+}
+
 // Gradients of every parameter (added to net->grads) from net->dy and the activations of the last
 // forward pass: the input gradients of every layer in one launch, then the weight and bias gradients of
 // every layer in another.
@@ -1141,17 +1174,12 @@ int pg_le_create(pg_context* ctx, int max_rows, pg_le_net** out)
   }
   const size_t o_rv = take(R), o_seq = take((size_t)n->max_seqs * sizeof(le_seq)),
                o_gs = take((size_t)n->max_seqs * 4), o_err = take(4), o_loss = take(8);
-  const size_t cleared = off; // the gradients are written before they are read
-  size_t o_grad[kLayers - 1] = {};
-  for (int i = 0; i < kLayers - 1; ++i) {
-    o_grad[i] = take(R * 128);
-  }
   int rc = check_cuda(ctx, cudaSetDevice(ctx->device), "cudaSetDevice");
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaMalloc(&n->dev, off), "cudaMalloc(learned estimator)");
   }
   if (rc == PG_OK) {
-    rc = check_cuda(ctx, cudaMemset(n->dev, 0, cleared), "cudaMemset(learned estimator)");
+    rc = check_cuda(ctx, cudaMemset(n->dev, 0, off), "cudaMemset(learned estimator)");
   }
   if (rc == PG_OK) {
     rc = check_cuda(ctx,
@@ -1198,9 +1226,6 @@ int pg_le_create(pg_context* ctx, int max_rows, pg_le_net** out)
   for (int i = 0; i < kBlocks; ++i) {
     n->mid[i] = reinterpret_cast<uint16_t*>(b + o_mid[i]);
   }
-  for (int i = 0; i < kLayers - 1; ++i) {
-    n->g[i] = reinterpret_cast<uint16_t*>(b + o_grad[i]);
-  }
   n->row_valid = b + o_rv;
   n->seqs      = reinterpret_cast<le_seq*>(b + o_seq);
   n->gseq      = reinterpret_cast<float*>(b + o_gs);
@@ -1216,6 +1241,7 @@ void pg_le_destroy(pg_le_net* net)
     return;
   }
   cudaDeviceSynchronize();
+  cudaFree(net->dev_g);
   cudaFree(net->dev);
   delete net;
 }
@@ -1324,8 +1350,10 @@ int pg_le_backward_device(pg_le_net* net, const void* dy, int rows, void* stream
     return set_error(net->ctx, PG_ERR_INVALID, "learned estimator: null gradient or bad row count");
   }
   cudaStream_t s  = static_cast<cudaStream_t>(stream);
-  int          rc = check_cuda(net->ctx, cudaMemsetAsync(net->grads, 0, (size_t)layers().nparams * 4, s),
-                               "cudaMemsetAsync(grads)");
+  int          rc = grad_buffers(net, rows);
+  if (rc == PG_OK) {
+    rc = check_cuda(net->ctx, cudaMemsetAsync(net->grads, 0, (size_t)layers().nparams * 4, s), "cudaMemsetAsync(grads)");
+  }
   if (rc == PG_OK) {
     rc = check_cuda(net->ctx, cudaMemcpyAsync(net->dy, dy, (size_t)rows * 32, cudaMemcpyDeviceToDevice, s),
                     "D2D output gradient");
@@ -1395,6 +1423,9 @@ int pg_le_train_step_device(pg_le_net* net, const pg_pusch_ue* ues, int nof_ues,
   }
   if (nseq == 0) {
     return PG_OK;
+  }
+  if (int rc = grad_buffers(net, R)) {
+    return rc;
   }
   le_features_kernel<<<(R + 255) / 256, 256, 0, s>>>(net->seqs, nseq, R, reinterpret_cast<const float2*>(est),
                                                      reinterpret_cast<const float2*>(ls), port_results,
