@@ -291,15 +291,22 @@ __device__ __forceinline__ void polar_rate_dematch(const polar_cb& d, polar_cb_s
   const int     K   = d.K;
   const int8_t* f   = llrs + d.llr_offset;
 
-  // By aligned words; an unaligned stream is shifted into place.
+  // By aligned words that hold soft bits only; an unaligned stream is shifted into place. The few soft bits
+  // before and behind come by bytes: nothing outside the stream is read.
   {
-    const uint32_t  sh = (uint32_t)(reinterpret_cast<uintptr_t>(f) & 3u);
+    const int       sh = (int)(reinterpret_cast<uintptr_t>(f) & 3u);
     const uint32_t* w  = reinterpret_cast<const uint32_t*>(f - sh);
-    const int       nw = (E + 3) / 4, last = (int)(sh + (uint32_t)E - 1u) / 4; // last word that holds a soft bit
+    const int       i0 = sh != 0 ? 1 : 0;                         // words i0 .. i1 - 1 of the shared copy
+    const int       i1 = max(i0, (E + sh) / 4 - (sh != 0 ? 1 : 0));
 #pragma unroll 8
-    for (int i = tid; i < nw; i += kPolarThreads) {
-      const uint32_t lo = __ldg(w + i), hi = sh != 0 && i < last ? __ldg(w + i + 1) : 0u;
+    for (int i = i0 + tid; i < i1; i += kPolarThreads) {
+      const uint32_t lo = __ldg(w + i), hi = sh != 0 ? __ldg(w + i + 1) : 0u;
       sm.in[i]          = __funnelshift_r(lo, hi, 8 * sh);
+    }
+    int8_t* const in8 = reinterpret_cast<int8_t*>(sm.in);
+    for (int b = tid; b < 4 * i0 + E - 4 * i1; b += kPolarThreads) {
+      const int p = b < 4 * i0 ? b : b - 4 * i0 + 4 * i1;
+      in8[p]      = __ldg(f + p);
     }
   }
   __syncthreads();
