@@ -1740,28 +1740,32 @@ int ldpc_upload_tables(pg_context* ctx)
   if (rc == PG_OK) {
     rc = check_cuda(ctx, cudaMemcpyToSymbol(c_row_e0, row_e0, sizeof(row_e0)), "cudaMemcpyToSymbol(row_e0)");
   }
-  static pair_tables pt; // the same values in every call
-  for (int gi = 0; gi < 2; ++gi) {
-    const int rows = gi == 0 ? PG_BG1_ROWS : PG_BG2_ROWS;
-    for (int r = 0; r < rows; ++r) {
-      for (int lg = 0; lg < 2; ++lg) {
-        const int t                = 2 << lg;
-        const int ne               = (deg[gi][r] + t - 1) / t;
-        pt.pad_e0[lg][gi][r + 1]   = (uint16_t)(pt.pad_e0[lg][gi][r] + ne * t);
-        pt.msg0[lg][gi][r + 1]     = (uint16_t)(pt.msg0[lg][gi][r] + (ne + 1) / 2);
-        for (int k = 0; k < deg[gi][r]; ++k) {
-          const int e = row_e0[gi][r] + k, p = pt.pad_e0[lg][gi][r] + k;
-          pt.pad_col[lg][gi][p] = (uint8_t)(col[gi][e] + 1);
-          std::copy(v[gi][e], v[gi][e] + 8, pt.pad_v[lg][gi][p]);
+  // Formed by the first call (the values are the same in every one), while calls of other threads wait.
+  static const pair_tables tables = [&] {
+    pair_tables pt = {};
+    for (int gi = 0; gi < 2; ++gi) {
+      const int rows = gi == 0 ? PG_BG1_ROWS : PG_BG2_ROWS;
+      for (int r = 0; r < rows; ++r) {
+        for (int lg = 0; lg < 2; ++lg) {
+          const int t                = 2 << lg;
+          const int ne               = (deg[gi][r] + t - 1) / t;
+          pt.pad_e0[lg][gi][r + 1]   = (uint16_t)(pt.pad_e0[lg][gi][r] + ne * t);
+          pt.msg0[lg][gi][r + 1]     = (uint16_t)(pt.msg0[lg][gi][r] + (ne + 1) / 2);
+          for (int k = 0; k < deg[gi][r]; ++k) {
+            const int e = row_e0[gi][r] + k, p = pt.pad_e0[lg][gi][r] + k;
+            pt.pad_col[lg][gi][p] = (uint8_t)(col[gi][e] + 1);
+            std::copy(v[gi][e], v[gi][e] + 8, pt.pad_v[lg][gi][p]);
+          }
         }
       }
+      for (int st = 0; st < nsteps[gi]; ++st) {
+        pt.row_sync[gi][step_row0[gi][st] + step_nrows[gi][st] - 1] = 1;
+      }
     }
-    for (int st = 0; st < nsteps[gi]; ++st) {
-      pt.row_sync[gi][step_row0[gi][st] + step_nrows[gi][st] - 1] = 1;
-    }
-  }
+    return pt;
+  }();
   if (rc == PG_OK) {
-    rc = check_cuda(ctx, cudaMemcpyToSymbol(g_pair_tables, &pt, sizeof(pt)), "cudaMemcpyToSymbol(pair tables)");
+    rc = check_cuda(ctx, cudaMemcpyToSymbol(g_pair_tables, &tables, sizeof(tables)), "cudaMemcpyToSymbol(pair tables)");
   }
   if (rc == PG_OK) {
     rc = check_cuda(ctx,
