@@ -419,7 +419,7 @@ constexpr uint32_t kFCopy     = kFWB;  // bytes per bulk copy: one per layer (16
 constexpr uint32_t kFCols     = 512;   // TMEM columns: 128 accumulators per M tile, then 64 per tile
                                        // of packed bf16 block input (the residual two layers on)
 constexpr uint32_t kFColRes   = 256;
-constexpr uint32_t kFZeroB    = 2 * 128 * 16;          // training: a zero A tile (two chunks of 128 pairs)
+constexpr uint32_t kFZeroB    = 2 * 128 * 16;          // training: a zero tile (two chunks of 128 rows)
 constexpr uint32_t kFOffZero  = ((uint32_t)kFSmem + 127u) & ~127u;
 constexpr size_t   kFSmemTrain = kFOffZero + kFZeroB;
 static_assert(kFSmemTrain <= 227 * 1024, "shared memory of the fused kernel's training modes");
@@ -487,8 +487,8 @@ __device__ __forceinline__ void fused_load_weights(const uint16_t* __restrict__ 
 // formed once; each MMA adds its constant offset (16-byte units) to the start-address field, which
 // stays below 2^14 (shared memory < 256 KB), so no carry reaches the LBO field. Inference: shift -1 comes
 // first in each tile and initialises both halves of the accumulator (N = 2 cout, no accumulation on the
-// first chunk); every other MMA accumulates. Training (ZEROED): an MMA of a zero A tile initialises both
-// halves and the shifts follow in ascending order, so that every output row sums its taps 0 to 4 in
+// first chunk); every other MMA accumulates. Training (ZEROED): an MMA of zeros (in both operands: zero times
+// an infinite weight is NaN) initialises both halves and the shifts follow in ascending order, so that every output row sums its taps 0 to 4 in
 // order, as one convolution per layer (conv1d_fwd_kernel) does, and the activations and gradients equal
 // those of such a chain bit for bit.
 template <int CIN, int COUT, int S, bool ZEROED>
@@ -526,7 +526,9 @@ __device__ __forceinline__ void fused_issue_tile(uint32_t go, int c, int part, u
   const uint32_t d  = tmem + (uint32_t)(c * 128);
   if (part != 1) {
     if (ZEROED) {
-      mma_bf16_warp(go, d, make_desc(zero, kFZeroB / 2, 128), b0, make_idesc(128, 2 * COUT, false, false), 0u);
+      static_assert(2 * COUT <= 128, "the zero tile serves as both operands");
+      const uint64_t z = make_desc(zero, kFZeroB / 2, 128);
+      mma_bf16_warp(go, d, z, z, make_idesc(128, 2 * COUT, false, false), 0u);
       fused_issue_shift<CIN, COUT, -2, ZEROED>(go, a0, b0, d);
       fused_issue_shift<CIN, COUT, -1, ZEROED>(go, a0, b0, d);
     } else {
