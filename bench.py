@@ -55,9 +55,9 @@ WORKLOAD = ("LDPC decoder batch: 512 codeblocks, BG1 Z=384 (K=8448, rate 1/3) an
 INT_OPS_PER_EDGE = 10
 LDPC_KERNEL_NAMES = (["ldpc_decode_kernel (one lifted lane per thread)"]
                      + 4 * ["ldpc_decode_pair_kernel (two lifted lanes per lane pair, 2 or 4 threads per pair)"])
-# ncu figures of one launch of the LDPC batch with the lane-pair kernel: pipe utilisation in % of active
-# cycles.
-LDPC_NCU = {k: {"pipes": {"alu": 57.3, "fma": 26.1, "fma_fp16": 21.8, "lsu": 26.6, "issue_active": 68.5}}
+# ncu figures of one launch of the LDPC batch with the lane-pair kernel: DRAM bytes read and written, and pipe
+# utilisation in % of active cycles.
+LDPC_NCU = {k: {"traffic": 12874752, "pipes": {"alu": 57.0, "fma": 27.2, "fma_fp16": 21.8, "lsu": 26.7, "issue_active": 70.9}}
             for k in range(1, 5)}
 # Integer-instruction throughput probe (the LDPC roofline denominator), built by
 # ocudu-dapp-platform_b200/measure/Makefile.
@@ -87,7 +87,7 @@ def parse_args():
     p.add_argument("--ldpc-kernel", type=int, default=None,
                    help="LDPC batch kernel of the --workload ldpc line (pg_ldpc_kernel; default: the library's)")
     p.add_argument("--ldpc-ctas-per-sm", type=int, default=2,
-                   help="resident LDPC CTAs per SM of the --workload ldpc line (0: the kernel limit)")
+                   help="resident LDPC CTAs per SM of the --workload ldpc line (0: by the batch size)")
     p.add_argument("--ldpc-order", default="longest", choices=["given", "longest"],
                    help="work order of the --workload ldpc line's persistent decoders (pg_set_ldpc_order)")
     return p.parse_args()
@@ -586,9 +586,24 @@ def run_ours_pusch(args):
                                                          ctypes.addressof(h_res), None))
             return time.perf_counter() - t0
 
+        # The host link beside it: the rate of plain pinned copies of the same size, before and after, since
+        # machines differ (and share their links) by more than anything in the pipeline does.
+        d_copy = torch.empty_like(h_grid, device=dev)
+
+        def link_gbs(copies=20):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            for _ in range(copies):
+                d_copy.copy_(h_grid, non_blocking=True)
+            e1.record()
+            torch.cuda.synchronize()
+            return copies * h_grid.numel() * h_grid.element_size() / (e0.elapsed_time(e1) * 1e6)
+
         pipelined(max(args.warmup, 2), args.e2e_depth)
+        link = [link_gbs(5) and link_gbs()]
         np_steps = min(args.steps, 200)
         p_ms = 1e3 * pipelined(np_steps, args.e2e_depth) / np_steps
+        link.append(link_gbs())
         assert [bool(h_res[i].tb_crc_ok) for i in range(n)] == [r.tb_crc_ok for r in results]
         p_ms = max_over_ranks(p_ms, world)
         # The headline end-to-end figure is the pipelined one (consecutive slots, as a PHY runs them);
@@ -598,6 +613,7 @@ def run_ours_pusch(args):
                "d2h_bytes_per_step": int(plan.tb_bytes + n * ctypes.sizeof(PgSchResult)),
                "ms_per_step": round(p_ms, 3),
                "slots_in_flight": args.e2e_depth,
+               "pinned_copy_gbs": [round(x, 1) for x in link],
                "entry": "pg_pusch_plan_submit_host / pg_pusch_plan_collect_host (slots in flight as above; every step "
                         "copies its grids in and its results out)",
                "synchronous": e2e}
@@ -895,7 +911,7 @@ def ldpc_core(args, dev, rank, world, with_cpu=True, with_e2e=True, steps=None):
     roofline = {
         "bound": "int",
         "kernel": LDPC_KERNEL_NAMES[kernel_id] + " (every codeblock of the batch has Z=384)",
-        "ctas_per_sm": args.ldpc_ctas_per_sm or "kernel limit",
+        "ctas_per_sm": args.ldpc_ctas_per_sm or "by batch size",
         "achieved": round(achieved, 3), "peak": round(peak, 3),
         "unit": "Tops/s", "frac": round(achieved / peak, 4),
         "peak_source": ("measured: full-rate int32 instruction throughput (add.s32/min.s32 probe, libpg_probe.so)"

@@ -51,7 +51,7 @@ typedef struct pg_context pg_context;
 
 typedef struct pg_config {
   int device;         /* CUDA device ordinal */
-  int max_codeblocks; /* largest LDPC batch one call may carry (sizes the message scratch) */
+  int max_codeblocks; /* largest LDPC batch one call may carry */
   int max_llrs;       /* largest total LLR count one _host call may carry */
 } pg_config;
 

@@ -3,13 +3,18 @@
 // (lib/phy/upper/channel_coding/ldpc/ldpc_decoder_impl.cpp:41-306,
 //  lib/phy/upper/channel_coding/ldpc/ldpc_decoder_avx512.cpp:69-253).
 //
-// Mapping: one CTA per codeblock, one thread per lifted check lane j (0 <= j < Z). For base-graph
-// row r, edge e (variable node v_e, lifted shift s_e), lane j reads soft bit (v_e, (j+s_e) mod Z):
-// the rows of a layer touch every lifted variable lane exactly once, so the Z lanes of a row are
-// independent and one __syncthreads separates consecutive rows (the layer schedule). Soft bits
-// live in shared memory; check-to-variable messages live in a per-codeblock global scratch slab
-// (edge-major, lane-minor: coalesced, L2 resident), indexed by (edge, check lane) rather than
-// the reference's rotated-back (variable slot, variable lane): the stored values are identical.
+// Mapping: one CTA per codeblock at a time. For base-graph row r, edge e (variable node v_e, lifted shift
+// s_e), check lane j (0 <= j < Z) reads soft bit (v_e, (j+s_e) mod Z): the rows of a layer touch every
+// lifted variable lane exactly once, so the Z lanes of a row are independent and a barrier separates rows
+// that share columns (the layer schedule). Soft bits live in shared memory; check-to-variable messages are
+// indexed by (edge, check lane) rather than the reference's rotated-back (variable slot, variable lane):
+// the stored values are identical. Two kernels:
+// - ldpc_decode_pair_kernel ("Lane-pair decoder" below) runs the batch decodes and the slot plans: even
+//   lifting sizes as pairs of lanes in f16x2, messages in shared memory or a global slab per CTA; the
+//   odd ones (Z <= 15) with the one-lane code.
+// - ldpc_decode_kernel, one thread per lane, messages in global memory (one byte per edge and lane, L2
+//   resident): PG_LDPC_KERNEL_ONE_LANE and the static-scratch entry, whose fixed array has room for this
+//   layout and not for the padded rows of the other.
 //
 // Arithmetic, per lane and edge (all exactly as the reference's AVX-512 kernels):
 //   v2c = soft == +-127 ? soft : clamp(soft - c2v, -120, 120)
@@ -1433,8 +1438,8 @@ static_assert(kPairMinSmem + 2048 <= 228 * 1024 / kPairPerSm, "every column fits
 // threads per lane pair above Z = 192, four below; odd lifting sizes (Z <= 15) with the one-lane
 // arithmetic.
 //
-// Bound: at 512 codeblocks instruction issue (69 % of the slots with 24 warps per SM), with few codeblocks
-// latency (12 warps, 46 %). B200, against the kernel this one replaced (two lanes per thread, one thread per
+// Bound: at 512 codeblocks instruction issue (71 % of the slots with 24 warps per SM), with few codeblocks
+// latency (12 warps, 47 %). B200, against the kernel this one replaced (two lanes per thread, one thread per
 // lane pair, Z = 384 only, messages in L2): 512 codeblocks BG1/BG2 Z = 384, 528 -> 327 us; 6 codeblocks BG1
 // Z = 384, 257 -> 123 us; 200 codeblocks of many sizes, 302 -> 134 us. One thread per lane pair (192 threads,
 // three CTAs per SM) took 415, 200 and 268 us where this split took 364, 155 and 190. From there: the step's

@@ -59,7 +59,7 @@ struct staging_slot {
 };
 
 struct device_buffers {
-  int8_t*      c2v         = nullptr; // max_codeblocks * kC2vStride check-to-variable messages
+  int8_t*      c2v         = nullptr; // check-to-variable messages, a slab (kPairSlab) per decoder CTA
   pg_ldpc_cb*  descs       = nullptr; // staged descriptors
   uint32_t*    crc_pow     = nullptr; // [3][kCrcPowLen]
   uint32_t*    crc_tabs    = nullptr; // [3][1024 + 2048]: x^k and x^(1024k) mod g
@@ -106,7 +106,7 @@ struct pg_context {
   bool                timed          = false;
   int8_t*             static_c2v     = nullptr;  // device address of the module-static LDPC scratch
   int                 ldpc_kernel    = PG_LDPC_KERNEL_Z384; // kernel of the batch decodes (pg_ldpc_kernel)
-  int                 ldpc_ctas_per_sm = 0;   // resident CTAs per SM of the batch decodes (0: kernel limit)
+  int                 ldpc_ctas_per_sm = 0;   // resident CTAs per SM of the batch decodes (0: by the batch size)
   int                 ldpc_order_mode  = PG_LDPC_ORDER_LONGEST_FIRST; // work order of the batch decodes
   std::string         last_error;
 };

@@ -143,7 +143,7 @@ class LdpcBatchDecoder:
         self.ctx.check(self.lib.pg_set_ldpc_order(self.ctx.handle, int(mode)))
 
     def set_ctas_per_sm(self, ctas_per_sm: int):
-        """Resident CTAs per SM of the batch decodes (0: the kernel's limit); results do not depend on it."""
+        """Resident CTAs per SM of the batch decodes (0: by the batch size); results do not depend on it."""
         self.ctx.check(self.lib.pg_set_ldpc_ctas_per_sm(self.ctx.handle, int(ctas_per_sm)))
 
     def set_kernel_timing(self, enabled: bool):
