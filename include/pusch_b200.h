@@ -650,9 +650,10 @@ typedef struct pg_le_adam {
 size_t pg_le_nof_params(void);
 /* Rows of the network's layout for a list of UEs (12 nof_rb per port and layer, plus gaps). */
 size_t pg_le_rows(const pg_pusch_ue* ues, int nof_ues);
-/* Creates a network with buffers for max_rows rows (about 1.8 KB of device memory per row; the first
- * pg_le_backward_device or pg_le_train_step_device allocates another 1.7 KB per row). The parameters start at
- * zero: set them with pg_le_set_params. */
+/* Creates a network with buffers for max_rows rows: about 1.8 KB of device memory per row, and 1.7 KB per row for
+ * training where they fit. A network that has not trained gives the latter back when a plan uses it
+ * (pg_pusch_plan_set_learned); the next pg_le_backward_device or pg_le_train_step_device allocates them again. The
+ * parameters start at zero: set them with pg_le_set_params. */
 int  pg_le_create(pg_context* ctx, int max_rows, pg_le_net** out);
 void pg_le_destroy(pg_le_net* net);
 /* Host FP32 parameters in and out (count = pg_le_nof_params()); setting them resets Adam. */

@@ -100,6 +100,7 @@ struct pg_le_net {
   uint16_t*   dy       = nullptr; // [2][R][8]
   uint16_t*   g[kLayers - 1] = {}; // g[l]: [8][R][8] gradient of layer l's output (before it: dy); see grad_buffers
   void*       dev_g     = nullptr;
+  bool        trained   = false;   // a training call has used the gradient buffers: they stay
   uint8_t*    row_valid = nullptr;
   pg::le_seq* seqs      = nullptr;
   float*      gseq      = nullptr;
@@ -966,12 +967,13 @@ int forward(pg_le_net* net, int R, cudaStream_t s)
   return fused_launch<kFTrain>(net, net->x, net->wp, R, io, s);
 }
 
-// The layers' gradient buffers, half of a training net's memory: allocated by the first call that trains, so that
-// a net which only infers does not hold them. That call may be captured, hence the relaxed mode. They are written
-// before they are read.
-int grad_buffers(pg_le_net* net, int rows)
+// The layers' gradient buffers, half of a training net's memory, written before they are read. A net has them from
+// its creation where they fit (allocated by the first training call they made it 0.75 to 4 ms longer); a net that
+// has not trained gives them back when a plan uses it (le_infer_only), and the next training call, which may be
+// captured (hence the relaxed mode), allocates them again.
+int grad_buffers(pg_le_net* net)
 {
-  if (net->dev_g != nullptr || rows <= 0) {
+  if (net->dev_g != nullptr) {
     return PG_OK;
   }
   pg_context*           ctx  = net->ctx;
@@ -996,6 +998,15 @@ int grad_buffers(pg_le_net* net, int rows)
     net->g[i] = reinterpret_cast<uint16_t*>(static_cast<uint8_t*>(net->dev_g) + i * one);
   }
   return rc;
+}
+
+int train_buffers(pg_le_net* net, int rows)
+{
+  if (rows <= 0) {
+    return PG_OK;
+  }
+  net->trained = true;
+  return grad_buffers(net);
 }
 
 // Gradients of every parameter (added to net->grads) from net->dy and the activations of the last
@@ -1112,6 +1123,14 @@ int le_refine_launch(pg_le_net* net, const le_seq* seqs_dev, int nseq, int R, co
 int le_capacity(const pg_le_net* net, size_t rows, int nseq)
 {
   return rows <= (size_t)net->max_rows && nseq <= net->max_seqs ? PG_OK : PG_ERR_CAPACITY;
+}
+
+void le_infer_only(pg_le_net* net)
+{
+  if (!net->trained && net->dev_g != nullptr) {
+    cudaFree(net->dev_g);
+    net->dev_g = nullptr;
+  }
 }
 
 pg_context* le_context(const pg_le_net* net)
@@ -1233,7 +1252,10 @@ int pg_le_create(pg_context* ctx, int max_rows, pg_le_net** out)
   n->gseq      = reinterpret_cast<float*>(b + o_gs);
   n->err       = reinterpret_cast<int*>(b + o_err);
   n->loss      = reinterpret_cast<float*>(b + o_loss);
-  *out         = n;
+  if (grad_buffers(n) != PG_OK) { // no room for them now: the net can infer, and a training call tries again
+    (void)cudaGetLastError();
+  }
+  *out = n;
   return PG_OK;
 }
 
@@ -1352,7 +1374,7 @@ int pg_le_backward_device(pg_le_net* net, const void* dy, int rows, void* stream
     return set_error(net->ctx, PG_ERR_INVALID, "learned estimator: null gradient or bad row count");
   }
   cudaStream_t s  = static_cast<cudaStream_t>(stream);
-  int          rc = grad_buffers(net, rows);
+  int          rc = train_buffers(net, rows);
   if (rc == PG_OK) {
     rc = check_cuda(net->ctx, cudaMemsetAsync(net->grads, 0, (size_t)layers().nparams * 4, s), "cudaMemsetAsync(grads)");
   }
@@ -1426,7 +1448,7 @@ int pg_le_train_step_device(pg_le_net* net, const pg_pusch_ue* ues, int nof_ues,
   if (nseq == 0) {
     return PG_OK;
   }
-  if (int rc = grad_buffers(net, R)) {
+  if (int rc = train_buffers(net, R)) {
     return rc;
   }
   le_features_kernel<<<(R + 255) / 256, 256, 0, s>>>(net->seqs, nseq, R, reinterpret_cast<const float2*>(est),

@@ -379,6 +379,8 @@ size_t le_build_seqs(const pg_pusch_ue* ues, int n, const uint8_t* use, std::vec
 // PG_OK when the net's buffers hold `rows` rows and `nseq` sequences, else PG_ERR_CAPACITY.
 int le_capacity(const pg_le_net* net, size_t rows, int nseq);
 pg_context* le_context(const pg_le_net* net);
+// A plan uses the net: its gradient buffers are given back unless it has trained.
+void le_infer_only(pg_le_net* net);
 // Features -> network -> est += correction, for sequences already in device memory.
 int le_refine_launch(pg_le_net* net, const le_seq* seqs_dev, int nseq, int R, const float* ls, float* est, float* basis,
                      const pg_port_result* pr, cudaStream_t s);

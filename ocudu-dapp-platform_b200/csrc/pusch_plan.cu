@@ -918,6 +918,7 @@ int pg_pusch_plan_set_learned(pg_pusch_plan* plan, pg_le_net* net, const uint8_t
   plan->le_nseq   = (int)seqs.size();
   plan->le_rows   = (int)rows;
   plan->le_net    = net;
+  le_infer_only(net);
   return PG_OK;
 }
 

@@ -1,14 +1,17 @@
-"""A net that only infers holds no gradient buffers: they come with the first backward pass, also where that pass is
-captured into a graph."""
+"""A net that a plan uses and that has not trained holds no gradient buffers; a training call allocates them again,
+also where it is captured into a graph, and a net that has trained keeps them."""
 import numpy as np
 import pytest
 
-from pusch_b200 import learned
+from pusch_b200 import learned, sim
 from pusch_b200 import tclayout as tl
+from pusch_b200.pusch import PuschSlotPlan
 
 pytestmark = pytest.mark.gpu
 
 ROWS = 100_000
+GRADIENTS = 13 * 128 * ROWS
+SLACK = 8 << 20  # granularity of the allocations
 
 
 def inputs(rows):
@@ -19,59 +22,66 @@ def inputs(rows):
     return bf(), bf(), torch.ones(rows, dtype=torch.uint8, device="cuda")
 
 
-def test_gradient_buffers_come_with_training(ctx):
+def free():
     import torch
-    rows = 300
-    x, dy, valid = inputs(rows)
-    y = torch.zeros((2, rows, 8), dtype=torch.int16, device="cuda")
-    st = torch.cuda.current_stream().cuda_stream
     torch.cuda.synchronize()
-    free = lambda: torch.cuda.mem_get_info()[0]
-    f0 = free()
-    net = learned.LearnedEstimator(ctx, ROWS, params=learned.init_params(3))
-    f1 = free()
-    net.forward(x.data_ptr(), valid.data_ptr(), rows, y.data_ptr(), st)
-    net.status()
-    f2 = free()
-    net.backward(dy.data_ptr(), rows, st)
-    net.status()
-    f3 = free()
-    net.backward(dy.data_ptr(), rows, st)
-    net.status()
-    slack = 8 << 20  # granularity of the allocations
-    assert f0 - f1 < 1900 * ROWS + slack
-    assert f2 > f1 - slack
-    assert 13 * 128 * ROWS <= f2 - f3 + slack and f2 - f3 < 13 * 128 * ROWS + slack
-    assert free() > f3 - slack
-    net.close()
-    torch.cuda.synchronize()
-    assert free() > f0 - slack
+    return torch.cuda.mem_get_info()[0]
 
 
-def test_first_backward_captured(ctx):
+@pytest.fixture(scope="module")
+def plan(ctx):
+    p = PuschSlotPlan(ctx, sim.uneven_cells(seed=3, nof_cells=1, max_ues=4))
+    yield p
+    p.close()
+
+
+def train(net, rows, x, dy, valid, y, stream, graph):
+    """Gradients of one forward and backward pass; the backward pass captured and replayed when graph is set."""
+    import torch
+    net.forward(x.data_ptr(), valid.data_ptr(), rows, y.data_ptr(), stream.cuda_stream)
+    stream.synchronize()
+    if graph:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            net.backward(dy.data_ptr(), rows, stream.cuda_stream)
+        g.replay()
+        torch.cuda.synchronize()
+        del g
+    else:
+        net.backward(dy.data_ptr(), rows, stream.cuda_stream)
+    grads = net.grads()
+    net.status()
+    return grads
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_gradient_buffers_of_a_plan_s_net(ctx, plan, graph):
     import torch
     rows = 1025
     x, dy, valid = inputs(rows)
     y = torch.zeros((2, rows, 8), dtype=torch.int16, device="cuda")
-    grads = []
-    for captured in (False, True):
-        net = learned.LearnedEstimator(ctx, rows, params=learned.init_params(3))
-        s = torch.cuda.Stream()
-        torch.cuda.synchronize()
-        net.forward(x.data_ptr(), valid.data_ptr(), rows, y.data_ptr(), s.cuda_stream)
-        s.synchronize()
-        if captured:
-            g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g, stream=s):
-                net.backward(dy.data_ptr(), rows, s.cuda_stream)
-            g.replay()
-        else:
-            net.backward(dy.data_ptr(), rows, s.cuda_stream)
-        torch.cuda.synchronize()
-        grads.append(net.grads())
-        net.status()
-        if captured:
-            del g
-        net.close()
+    s = torch.cuda.Stream()
+    fresh = learned.LearnedEstimator(ctx, rows, params=learned.init_params(3))
+    want = train(fresh, rows, x, dy, valid, y, s, False)
+    fresh.close()
+    f0 = free()
+    net = learned.LearnedEstimator(ctx, ROWS, params=learned.init_params(3))
+    f1 = free()
+    assert f0 - f1 < 1900 * ROWS + GRADIENTS + SLACK
+    plan.set_learned(net)
+    f2 = free()
+    assert f2 - f1 > GRADIENTS - SLACK
+    a = [r.tb_crc_ok for r in plan.execute_host()]
+    got = train(net, rows, x, dy, valid, y, s, graph)
+    f3 = free()
+    assert abs(f2 - f3 - GRADIENTS) < SLACK + (64 << 20 if graph else 0)  # a capture may hold memory of its own
+    plan.set_learned(None)
+    plan.set_learned(net)  # trained: kept
+    assert free() < f3 + GRADIENTS // 2
+    assert [r.tb_crc_ok for r in plan.execute_host()] == a
+    again = train(net, rows, x, dy, valid, y, s, False)
+    plan.set_learned(None)
+    net.close()
     # The same kernels on the same inputs; the order of the FP32 atomics differs.
-    assert np.linalg.norm(grads[1] - grads[0]) <= 2e-6 * np.linalg.norm(grads[0])
+    for g in (got, again):
+        assert np.linalg.norm(g - want) <= 2e-6 * np.linalg.norm(want)
